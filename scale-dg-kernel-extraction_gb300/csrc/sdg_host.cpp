@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "sdg_fix.cuh"
 #include "sdg_internal.h"
 
 namespace sdg {
@@ -263,6 +264,43 @@ int eo_tables(int Nq, const double* D1D, const double* Lift_mat, std::vector<dou
   return SDG_OK;
 }
 
+void fix_tables(int Nq, const Box& box, const std::vector<double>& eo, FixTables& t) {
+  const int N = Nq, H = N / 2, HR = (N + 1) / 2, ODD = N & 1;
+  const int TE = H * H + HR * H + ODD * H + HR + H;
+  const int oO = H * H, oM = oO + HR * H, oA = oM + ODD * H, oB = oA + HR;
+  t.ok = 0;
+  t.coef.assign(2 * 3 * (size_t)TE, 0);
+  t.row.assign(3 * (size_t)HR, 0);
+  for (int d = 0; d < 3; d++) {
+    const double* T = eo.data() + (size_t)d * TE;
+    auto value = [&](int w) { return -(long double)T[w] * (w < oA ? box.Es[d] : box.Fs[d]); };
+    for (int i = 0; i < HR; i++) {
+      std::vector<int> even, odd{oA + i};
+      for (int l = 0; l < H; l++) odd.push_back(oO + i * H + l);
+      if (i < H) {
+        even.push_back(oB + i);
+        if (ODD) even.push_back(oM + i);
+        for (int l = 0; l < H; l++) even.push_back(i * H + l);
+      }
+      long double se = 0.0L, so = 0.0L;
+      for (int w : even) se += std::fabs(value(w));
+      for (int w : odd) so += std::fabs(value(w));
+      const long double most = std::fmax(se, so);
+      if (!std::isfinite((double)most)) return;
+      int k = 0;
+      if (most > 0.0L) std::frexp(most, &k);
+      if (k < -200 || k > 200) return;
+      t.row[(size_t)d * HR + i] = k - 59;
+      even.insert(even.end(), odd.begin(), odd.end());
+      for (int w : even) {
+        const fixlimb x = fix_coef((int64_t)std::llround(std::ldexp(value(w), 60 - k)));
+        t.coef[2 * ((size_t)d * TE + w)] = x.hi;
+        t.coef[2 * ((size_t)d * TE + w) + 1] = x.lo;
+      }
+    }
+  }
+  t.ok = 1;
+}
 
 }  // namespace sdg
 

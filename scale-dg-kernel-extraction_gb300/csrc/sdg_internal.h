@@ -57,6 +57,20 @@ struct Box {
 };
 Box make_box(int NeX, int NeY, int NeZ, double Lx, double Ly, double Lz);
 
+// Coefficients of the fixed-point stage (sdg_stage_fix.cuh) on the host: per
+// direction the even-odd table of EoShape as limb pairs (hi, lo) of
+// c 2^(60 - k), c = -(derivative entry) Es_d or -(lift entry) Fs_d, k the
+// row's exponent: the smallest that keeps the sums of magnitudes of the row's
+// two halves (E, D(mid), B and O, A) at or below 2^k.  row: k - 59.  ok = 0
+// when an exponent lies outside +-200: every line is then formed in FP64.
+struct FixTables {
+  std::vector<int32_t> coef;
+  std::vector<int> row;
+  int ok = 0;
+};
+// Fills t from the unscaled tables of eo_tables.
+void fix_tables(int Nq, const Box& box, const std::vector<double>& eo, FixTables& t);
+
 // Arguments of one fused stage launch.
 struct StageArgs {
   const double* q_in;   // state read by the stage (Np*Ne)
@@ -88,6 +102,9 @@ struct StageArgs {
   // advect3d_eq_cal_tend call), form them once.  Both null: formed inline.
   double* fc_out;
   const double* fc_in;
+  // even-odd FP64 stage: its fixed-point coefficients (host memory, copied
+  // into the launch)
+  const FixTables* fix;
 };
 
 // Even-odd tables (3 directions, unscaled) from D1D and Lift_mat after the

@@ -41,6 +41,8 @@ struct sdg_solver {
   // Measured on GB300 against forming them in every stage: 1.04-1.13x for the
   // FP64 stage (p = 7: 19.3 against 18.5 GDOF-updates/s), 1.01-1.14x emulated.
   double* fc = nullptr;
+  // coefficients of the fixed-point stage (even-odd FP64)
+  FixTables fix;
   // elements a stage advances: [elem_begin, elem_begin + elem_count) of the
   // box (the whole box by default; a z-slab partition advances its owned
   // layers and keeps a ghost layer on each side)
@@ -129,6 +131,7 @@ int one_stage_on(sdg_solver* s, int stage, double dt, const double* qin, const d
   a.tend_only = tend_only ? 1 : 0;
   a.fc_out = (s->fc && fc == 1) ? s->fc : nullptr;
   a.fc_in = (s->fc && fc == 2) ? s->fc : nullptr;
+  a.fix = &s->fix;
   const double c = tend_only ? 1.0 : a.b * dt;
   for (int d = 0; d < 3; d++) {
     a.eo_sD[d] = -c * s->box.Es[d];
@@ -276,6 +279,7 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
     } else {
       dtab.resize(8 * tab.size());
       std::memcpy(dtab.data(), tab.data(), dtab.size());
+      fix_tables(s->Nq, s->box, tab, s->fix);
     }
   }
   cudaError_t e = cudaSuccess;

@@ -1,12 +1,11 @@
 // Fused RK-stage kernel with the even-odd factorisation of the 1D operators
-// (opt type SDG_OPT_EVENODD), for the FP64 form and the FP32-compute form.
+// (opt type SDG_OPT_EVENODD) in the FP32-compute form, and the even-odd line
+// pieces that the FP64 kernels of the reference-shaped entry points share (the
+// FP64 stage itself forms its lines in fixed point, sdg_stage_fix.cuh).
 //
-// On GB300 the FP64 pipe runs at 1/64 of the FP32 rate, so the plain FP64
-// stage is bound by its count of FP64 instructions, not by HBM.  This body
-// computes the same tendency and stage update as stage_block<P, double> with
-// about 30 % fewer FP64 instructions per node; in FP32 it also replaces the
-// node body's per-node shared-memory reads of a whole line by one read per
-// line value:
+// The pair sums cost about half the operations of the plain line sums, and
+// one thread a line replaces the node body's per-node shared-memory reads of a
+// whole line by one read per line value:
 //
 //  * Centro-antisymmetry of the GLL differentiation matrix,
 //    D(N-1-i, N-1-l) = -D(i, l), splits a line's N-term sums into pairs:
@@ -27,10 +26,6 @@
 //  * The face flux 0.5 Fs (qP VelP - qM VelM - α (qP - qM)) is formed as
 //    qP (2VelP - 2α) - qM (2VelM - 2α) with 2α = |uP + uM| (the normal sign
 //    applied through the constant ±2): five FP64 operations per face node.
-//    Three of them form the velocity factors tP = ±2VelP - 2α and tM, which
-//    every stage of one solver call shares (the velocity cannot change
-//    within a call): the call's first stage stores them (fc_out) and every
-//    later stage reads them (fc_in), two operations a face node there.
 //
 // Thread layout: phase 0 and the face flux run one thread per node / face
 // node as in stage_block; the three contraction phases run one thread per
@@ -68,8 +63,8 @@ struct EoShape {
 // halves the registers a thread needs and doubles the warps that hide memory
 // latency; at low orders a line has one or two output pairs, and one thread
 // a line measured faster on GB300 up to p = 3 in the single-box kernel (p = 3:
-// 91.8 against 72.5 GDOF-updates/s).  The FP64 body is bound by the FP64 pipe
-// and keeps one.  The batched kernels pick their own count (batch_eo_parts).
+// 91.8 against 72.5 GDOF-updates/s).
+// The batched kernels pick their own count (batch_eo_parts).
 // At p = 4 and 6 one thread a line measured faster (77.5 against 70.0
 // GDOF-updates/s at p = 4 with 256 threads and six blocks an SM; 77.3 against
 // 69.1 at p = 6 with four); likewise at p = 5 with five blocks of 256 threads
@@ -79,28 +74,23 @@ struct EoShape {
 // level or slower at p = 8..10 and 15.
 template <int P, typename CT>
 __host__ __device__ constexpr int eo_parts() {
-  return (sizeof(CT) == 4 && P >= 7 && (P < 11 || P > 14)) ? 2 : 1;
+  return (P >= 7 && (P < 11 || P > 14)) ? 2 : 1;
 }
 
 // Lines of a block: 256, or 128 for the FP32 body at p = 7, 9 and 10, where
 // twice as many half-size blocks (the same 64 warps an SM) measured 1.04-1.05x
-// on GB300 (108 against 103 GDOF-updates/s at p = 7; 0.95x at p = 8), and for
-// the FP64 body at p = 7 (eight blocks of 128 threads for four of 256, the
-// same 61 registers: 19.81 against 19.68 GDOF-updates/s; at p = 1..5 the
-// same change measured 0.97-1.008x).
+// on GB300 (108 against 103 GDOF-updates/s at p = 7; 0.95x at p = 8).
 template <int P, typename CT>
 __host__ __device__ constexpr int eo_lines() {
-  return ((sizeof(CT) == 4 && (P == 7 || P == 9 || P == 10)) || (sizeof(CT) == 8 && P == 7))
-             ? 128
-             : 256;
+  return (P == 7 || P == 9 || P == 10) ? 128 : 256;
 }
 
 template <int P, typename CT>
 __host__ __device__ constexpr bool eo_exact() {
-  return sizeof(CT) == 4 && (P == 11 || P == 12);
+  return P == 11 || P == 12;
 }
 
-template <int P, typename CT = double>
+template <int P, typename CT>
 struct EoCfg {
   // FP32 at p = 11 and 12: one element a block, the block sized to its
   // lines instead of 256 lines of which 144 / 169 had work; measured on
@@ -108,7 +98,7 @@ struct EoCfg {
   // GDOF-updates/s (now one thread a line, eo_parts: 160 and 192 threads).
   // At p = 13 and 14 the 256-line shape stays faster (78.2 against 77.3,
   // 72.1 against 71.6 with two threads a line), at p = 9 level (87.0 against
-  // 86.5), and the FP64 form at p = 11..13, bound by its FP64 pipe, level.
+  // 86.5).
   static constexpr bool EXACT = eo_exact<P, CT>();
   static constexpr int LINES = eo_lines<P, CT>();
   static constexpr int THREADS = EXACT ? ((Ord<P>::NQ2 * eo_parts<P, CT>() + 31) / 32) * 32
@@ -118,30 +108,17 @@ struct EoCfg {
 
 // Dynamic shared memory of one block with nloc elements: the three scaled
 // direction tables, then per element the arrays below and the 6 Nfp face
-// fluxes, then the neighbour indices.
-// The FP64 body does not stage q: the face flux and the RK update read it
-// from global memory (L1 / L2 hits after phase 0), which saves shared memory
-// for a fourth resident block.
-template <typename CT>
-__host__ __device__ constexpr bool eo_stages_q() {
-  return sizeof(CT) == 4;
-}
-
-// The FP64 body keeps one array: the x lines' pair values, then the sums; the
-// y and z line threads form their lines' pair values from q and v / w in
-// cache.  That leaves room for four resident blocks.  The FP32 body keeps q
-// (FP32), F_x and the line-result sums (in their own array, since two threads
-// share a line and one may write before the other has read), and either
-// stages F_y and F_z as well or (FLY) has the y and z line threads form
-// F = q v / q w from the staged q and the velocity in cache: two arrays less,
-// which keeps more blocks resident at high orders, for two extra velocity
-// reads per line node.
+// fluxes, then the neighbour indices.  q (FP32), F_x and
+// the line-result sums (in their own array where two threads share a line and
+// one may write before the other has read), and either F_y and F_z as well or
+// (FLY) the y and z line threads form F = q v / q w from the staged q and the
+// velocity in cache: two arrays less, which keeps more blocks resident at high
+// orders, for two extra velocity reads per line node.
 template <int P, typename CT, bool FLY = false, int PARTS_SET = 0>
 __host__ __device__ constexpr size_t eo_block_smem(int nloc) {
   using O = Ord<P>;
   constexpr int parts = PARTS_SET > 0 ? PARTS_SET : eo_parts<P, CT>();
-  constexpr int arrays =
-      sizeof(CT) == 8 ? 1 : (eo_stages_q<CT>() ? 2 : 1) + (FLY ? 0 : 2) + (parts > 1 ? 1 : 0);
+  constexpr int arrays = 2 + (FLY ? 0 : 2) + (parts > 1 ? 1 : 0);
   return sizeof(CT) * (size_t)(3 * EoShape<P>::TE + nloc * (arrays * O::NP + O::NFT)) +
          sizeof(int) * 6 * (size_t)nloc;
 }
@@ -243,10 +220,9 @@ __device__ __forceinline__ void eo_pairs_f64(const double* __restrict__ q,
 }
 
 // One block advances elements [eb, eb + nloc) through one stage with the
-// even-odd body.  CT = double: FP64 throughout (tables scaled by eo_sD /
-// eo_sL).  CT = float: the FP32-compute form (FP32 tables, velocity and
-// sums, scaled by eo_sDf / eo_sLf), with the increment widened by bits and
-// the RK combination in FP64.  Block size and nloc are runtime values, so the
+// even-odd body of the FP32-compute form (CT = float: FP32 tables, velocity
+// and sums, scaled by eo_sDf / eo_sLf), with the increment widened by bits
+// and the RK combination in FP64.  Block size and nloc are runtime values, so the
 // batched persistent kernel can use the same body.
 // PREF (FP32 body): start q0 towards L2 in phase 0 and unroll the staging
 // loop by 4, so more loads are in flight per warp.  (Four nodes a thread as
@@ -262,13 +238,11 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
   using Sh = EoShape<P>;
   constexpr int NQ = O::NQ, NQ2 = O::NQ2, NP = O::NP, NFP = O::NFP, NFT = O::NFT;
   constexpr int TE = Sh::TE;
-  constexpr bool kF64 = sizeof(CT) == 8;
   const int T = blockDim.x;
   CT* sT = reinterpret_cast<CT*>(smem);  // 3 directions x TE
-  constexpr bool kSQ = eo_stages_q<CT>();
-  CT* sq = sT + 3 * TE;      // q (FP32 body only)
-  CT* sFx = sq + (kSQ ? nloc * NP : 0);  // F_x (FP64: x pair values), then the sums
-  constexpr bool kSYZ = !kF64 && !FLY;    // F_y, F_z staged (FP32 only)
+  CT* sq = sT + 3 * TE;      // q
+  CT* sFx = sq + nloc * NP;  // F_x, then the sums
+  constexpr bool kSYZ = !FLY;             // F_y, F_z staged
   CT* sFy = sFx + (kSYZ ? nloc * NP : 0);
   CT* sFz = sFy + (kSYZ ? nloc * NP : 0);
   constexpr int PARTS = PARTS_SET > 0 ? PARTS_SET : eo_parts<P, CT>();
@@ -289,13 +263,8 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
   CT fD[3], fL[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    if constexpr (kF64) {
-      fD[d] = a.eo_sD[d];
-      fL[d] = a.eo_sL[d];
-    } else {
-      fD[d] = a.eo_sDf[d];
-      fL[d] = a.eo_sLf[d];
-    }
+    fD[d] = a.eo_sDf[d];
+    fL[d] = a.eo_sLf[d];
   }
   for (int t = threadIdx.x; t < 3 * TE; t += T) {
     const int dir = t / TE, w = t - dir * TE;
@@ -305,50 +274,27 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
   }
   for (int t = threadIdx.x; t < 6 * nloc; t += T)
     snb[t] = (int)neighbor(a.box, eb + t / 6, t % 6);
-  if constexpr (kF64) {
-    // x pair values: one task per (element, x line, c < ceil(N/2)), c fastest
-    constexpr int HR = Sh::HR, H = Sh::H;
-    for (int t = threadIdx.x; t < nloc * NQ2 * HR; t += T) {
-      const int le = t / (NQ2 * HR), w = t - le * NQ2 * HR;
-      const int r = w / HR, c = w - r * HR;
-      const long long g = g0 + (long long)le * NP + (long long)r * NQ;
-      CT* row = sFx + le * NP + r * NQ;
-      if (c < H) {
-        const double q1 = qin[g + c], u1 = gu[g + c];
-        const double p2 = qin[g + NQ - 1 - c] * gu[g + NQ - 1 - c];
-        row[c] = fma(q1, u1, p2);
-        row[NQ - 1 - c] = fma(q1, u1, -p2);
-      } else {
-        row[c] = qin[g + c] * gu[g + c];
-      }
+  auto stage_node = [&](int t) {
+    const CT qq = to_ct<CT>(qin[g0 + t]);
+    sq[t] = qq;
+    sFx[t] = qq * gu[g0 + t];
+    if constexpr (kSYZ) {
+      sFy[t] = qq * gv[g0 + t];
+      sFz[t] = qq * gw[g0 + t];
     }
-  } else {
-    auto stage_node = [&](int t) {
-      const CT qq = to_ct<CT>(qin[g0 + t]);
-      if constexpr (kSQ) sq[t] = qq;
-      sFx[t] = qq * gu[g0 + t];
-      if constexpr (kSYZ) {
-        sFy[t] = qq * gv[g0 + t];
-        sFz[t] = qq * gw[g0 + t];
-      }
-    };
-    if constexpr (PREF) {
-      // q0, read only by the last phase's RK update, starts towards L2 now
-      if (rk_kind(a) == kRkGeneral)
-        for (int t = 16 * threadIdx.x; t < nloc * NP; t += 16 * T) prefetch_l2(a.q0 + g0 + t);
+  };
+  if constexpr (PREF) {
+    // q0, read only by the last phase's RK update, starts towards L2 now
+    if (rk_kind(a) == kRkGeneral)
+      for (int t = 16 * threadIdx.x; t < nloc * NP; t += 16 * T) prefetch_l2(a.q0 + g0 + t);
 #pragma unroll 4
-      for (int t = threadIdx.x; t < nloc * NP; t += T) stage_node(t);
-    } else {
-      for (int t = threadIdx.x; t < nloc * NP; t += T) stage_node(t);
-    }
+    for (int t = threadIdx.x; t < nloc * NP; t += T) stage_node(t);
+  } else {
+    for (int t = threadIdx.x; t < nloc * NP; t += T) stage_node(t);
   }
   __syncthreads();
 
-  // phase 1: face fluxes qP (2VelP - 2α) - qM (2VelM - 2α), unscaled.  The
-  // velocity factors tP = ±2VelP - 2α and tM come from fc_in when a stage
-  // before this one in the step stored them (FP64 body).
-  const double2* __restrict__ fcin = reinterpret_cast<const double2*>(a.fc_in);
-  double2* __restrict__ fcout = reinterpret_cast<double2*>(a.fc_out);
+  // phase 1: face fluxes qP (2VelP - 2α) - qM (2VelM - 2α), unscaled;
   // tasks face-major below p = 5 (FaceTasks)
   const FaceTasks<NQ> ftask(nloc);
   for (int t = threadIdx.x; t < nloc * NFT; t += T) {
@@ -360,26 +306,14 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
     face_nodes<NQ>(f, fp % NQ, fp / NQ, nM, nP, axis, sg);
     const long long gM = g0 + (long long)le * NP + nM;
     const long long gP = (long long)snb[6 * le + f] * NP + nP;
-    CT qM;
-    if constexpr (kSQ)
-      qM = sq[le * NP + nM];
-    else
-      qM = to_ct<CT>(qin[gM]);
+    const CT qM = sq[le * NP + nM];
     const CT qP = to_ct<CT>(qin[gP]);
-    CT tP, tM;
-    if (kF64 && fcin != nullptr) {
-      const double2 c = fcin[eb * NFT + ti];
-      tP = CT(c.x);
-      tM = CT(c.y);
-    } else {
-      const CT* gvel = (axis == 0) ? gu : (axis == 1) ? gv : gw;
-      const CT uM = gvel[gM], uP = gvel[gP];
-      const CT a2 = abs_ct(uP + uM);
-      const CT tw = (sg > 0) ? CT(2) : CT(-2);
-      tP = fma(tw, uP, -a2);
-      tM = fma(tw, uM, -a2);
-      if (kF64 && fcout != nullptr) fcout[eb * NFT + ti] = make_double2(tP, tM);
-    }
+    const CT* gvel = (axis == 0) ? gu : (axis == 1) ? gv : gw;
+    const CT uM = gvel[gM], uP = gvel[gP];
+    const CT a2 = fabsf(uP + uM);
+    const CT tw = (sg > 0) ? CT(2) : CT(-2);
+    const CT tP = fma(tw, uP, -a2);
+    const CT tM = fma(tw, uM, -a2);
     sf[ti] = fma(qP, tP, -(qM * tM));
   }
   __syncthreads();
@@ -392,7 +326,7 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
     const CT* F = sFx + le * NP + r * NQ;
     CT* acc = sAcc + le * NP + r * NQ;
     const CT* fl = sf + le * NFT + r;
-    eo_line<P, 1, PARTS, kF64>(F, sT, fl[3 * NFP], fl[1 * NFP], part,
+    eo_line<P, 1, PARTS, false>(F, sT, fl[3 * NFP], fl[1 * NFP], part,
                          [&](int m, CT v) { acc[m] = v; });
   }
   __syncthreads();
@@ -404,12 +338,7 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
     const int off = le * NP + (r % NQ) + (r / NQ) * NQ2;
     CT* acc = sAcc + off;
     const CT* fl = sf + le * NFT + r;
-    if constexpr (kF64) {
-      double row[NQ];
-      eo_pairs_f64<P>(qin, gv, g0 + off, NQ, row);
-      eo_line<P, 1, PARTS, true>(row, sT + TE, fl[0], fl[2 * NFP], part,
-                                 [&](int m, CT v) { acc[m * NQ] += v; });
-    } else if constexpr (kSYZ) {
+    if constexpr (kSYZ) {
       eo_line<P, NQ, PARTS, false>(sFy + off, sT + TE, fl[0], fl[2 * NFP], part,
                                    [&](int m, CT v) { acc[m * NQ] += v; });
     } else {
@@ -443,21 +372,13 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
       auto emitz = [&](int m, CT v) {
         const int n = off + m * NQ2;
         const long long g = g0 + n;
-        double inc;
-        if constexpr (kF64)
-          inc = sAcc[n] + v;
-        else
-          inc = f32_to_f64_bits(sAcc[n] + v);
+        const double inc = f32_to_f64_bits(sAcc[n] + v);
         if constexpr (RK == kRkTend)
           qout[g] = inc;
         else
           qout[g] = rk_combine<RK>(inc, qin[g], RK == kRkGeneral ? q0[g] : 0.0, rk_a, rk_b);
       };
-      if constexpr (kF64) {
-        double row[NQ];
-        eo_pairs_f64<P>(qin, gw, g0 + off, NQ2, row);
-        eo_line<P, 1, PARTS, true>(row, sT + 2 * TE, fl[4 * NFP], fl[5 * NFP], part, emitz);
-      } else if constexpr (kSYZ) {
+      if constexpr (kSYZ) {
         eo_line<P, NQ2, PARTS, false>(sFz + off, sT + 2 * TE, fl[4 * NFP], fl[5 * NFP], part,
                                       emitz);
       } else {
@@ -477,18 +398,8 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
 // GDOF-updates/s at p = 7); at p = 15 shared memory admits three blocks and
 // the cap would only spill.  One thread a line (p <= 6 and 11..14): the
 // counts below, each measured on GB300 against its neighbours.
-// FP64: four or five blocks of 256 threads (registers capped at 64 or 48): a
-// block in its load or flux phase leaves the others feeding the FP64 pipe.
-// Five measured faster on GB300 at most orders once stages 2-3 read the face
-// factors (1.02-1.06x up to p = 4, 1.005-1.013x at p = 6 and 8..13, 48
-// registers with small spills) and four at p = 5, 7, 14 and 15 (by 0.2-1.1 %).
-// At p = 1 eight blocks (32 registers, 68 bytes of spills) measured 20.5
-// against 19.8 GDOF-updates/s for five (20.4 for six); at p = 2 six were level.
-// At p = 7 the blocks have 128 threads (eo_lines), so four blocks' worth of
-// warps is eight blocks (ten, at 48 registers with spills: 19.75).
 template <int P, typename CT>
 __host__ __device__ constexpr int eo_min_blocks() {
-  if (sizeof(CT) == 8) return P == 7 ? 8 : (P == 5 || P >= 14) ? 4 : P == 1 ? 8 : 5;
   if (P == 4) return 6;  // 40 registers, one thread a line (above)
   if (P == 5) return 5;  // 48 registers, one thread a line
   // one thread a line from p = 11 to 14 (eo_parts); p = 11, 12 in blocks

@@ -1,0 +1,374 @@
+// Fused RK-stage kernel of the FP64 form with the line sums in 60-bit fixed
+// point (sdg_fix.cuh).
+//
+// An FP64 even-odd stage spends 28.8 FP64 instructions a DOF at p = 7 and kept
+// the FP64 pipe 90 % busy at 19.8 GDOF-updates/s.  Here the even-odd pair
+// sums, the derivative and the lift are integer multiply-adds, and FP64 keeps
+// the products q u_d, the face flux and the RK update (6.8 instructions a
+// DOF): 62 GDOF-updates/s at p = 7 on 32^3 elements (270 us a stage, from
+// 848), 39-62 across p = 1..15 (from 13-22), the FP64 pipe 60-67 % and the
+// issue slots 41-47 % busy, with 32 warps an SM waiting on the loads of its
+// two ends.  Error of a tendency against a long-double one: 0.5-1.1 times the
+// FP64 body's at every order, on smooth, narrow and random fields (the
+// coefficients' symmetrisation, common to both, dominates from p = 5).
+//
+// The pairs: S(l) = F(l) + F(N-1-l), d(l) = F(l) -
+// F(N-1-l), e_i = sum E(i,l) S(l) [+ D(i,mid) F(mid)] + B(i) (g- - g+),
+// o_i = sum O(i,l) d(l) + A(i) (g- + g+), out(i) = o_i + e_i, out(N-1-i) =
+// o_i - e_i.  The coefficients (Escale, Fscale and the minus sign of dqdt
+// folded in) are kernel parameters, so a multiply-add takes them from the
+// constant bank.  The x, y and z results of a node add up as integers; the
+// increment is their sum times one factor of the element and the stage.
+//
+// Scale: a line's values share the power of two that bounds its fluxes q u_d
+// and its two face fluxes, and a row of coefficients has a power of two of its
+// own, so every line result keeps about 2^-59 of its own bound.  The three
+// results of a node are added as integers on the largest of their scales and
+// become one double.  A line with infinities, NaN, or magnitudes near the ends
+// of the exponent range is formed in FP64 by its thread, and its nodes add up
+// in FP64.
+//
+// Thread layout: thread r of an element's N^2 owns line r of each direction
+// and node r of each face, so a line's face fluxes never leave their thread.
+//   0  the z line's x and y fluxes to shared memory, the six face fluxes
+//   1  x line and y line r, results over the fluxes
+//   2  z line r, and the RK update of its nodes
+#pragma once
+
+#include "sdg_fix.cuh"
+#include "sdg_stage_eo.cuh"
+
+namespace sdg {
+
+template <int P>
+struct FixShape {
+  static constexpr int N = P + 1, N2 = N * N;
+  static constexpr int NS = (N & 1) ? N : N + 1;  // padded x row: odd, so that
+                                                  // rows start on distinct banks
+  static constexpr int EW = NS * N2;              // words of an element's array
+  // threads: whole elements of N^2 lines in 128 or 256 threads, whichever
+  // leaves fewer idle; one element in whole warps from p = 10
+  static constexpr int THREADS = (N2 > 100) ? ((N2 + 31) / 32) * 32
+                                 : (N2 == 49 || N2 == 81) ? 256 : 128;
+  static constexpr int EPB = THREADS / N2;
+};
+
+template <int P>
+struct FixStageArgs {
+  StageArgs s;
+  double c;                       // b dt (1: tendency)
+  fixlimb tab[3 * EoShape<P>::TE];
+  int row[3 * EoShape<P>::HR];    // exponent of a row's scale, less 59
+  int ok;                         // 0: the box's coefficients are out of range,
+                                  // every line is formed in FP64
+};
+
+template <int P>
+__host__ __device__ constexpr size_t fix_smem() {
+  return sizeof(double) * 2 * FixShape<P>::EPB * FixShape<P>::EW +
+         sizeof(int) * 2 * FixShape<P>::EPB * FixShape<P>::N2;
+}
+
+// A line in FP64, for values the fixed-point path does not take (E: their
+// largest exponent, 0 when there is nothing but zeros and subnormals): F
+// holds the line's fluxes with stride fs, results to out[0..N).  A call of
+// its own, so that its registers do not count against the kernel's.
+template <int P>
+__device__ __noinline__ void fix_line_fp64(const double* F, int fs, const double* __restrict__ T,
+                                           double sD, double sL, double gm, double gp,
+                                           double* out) {
+  using Sh = EoShape<P>;
+  constexpr int N = Sh::N, H = Sh::H;
+  const double gs = gm + gp, gd = gm - gp;
+  bool some = gm != 0.0 || gp != 0.0;
+  for (int l = 0; l < N; l++) {
+    out[l] = 0.0;
+    some = some || F[l * fs] != 0.0;
+  }
+  if (!some) return;
+#pragma unroll 1
+  for (int i = 0; i < Sh::HR; i++) {
+    double e = 0.0, o = 0.0;
+#pragma unroll 1
+    for (int l = 0; l < H; l++) {
+      const double f1 = F[l * fs], f2 = F[(N - 1 - l) * fs];
+      if (i < H) e = fma(T[Sh::OFF_E + i * H + l], f1 + f2, e);
+      o = fma(T[Sh::OFF_O + i * H + l], f1 - f2, o);
+    }
+    if (Sh::ODD != 0 && i < H) e = fma(T[Sh::OFF_DM + i], F[H * fs], e);
+    o = fma(sD, o, sL * (T[Sh::OFF_A + i] * gs));
+    if (i < H) {
+      e = fma(sD, e, sL * (T[Sh::OFF_B + i] * gd));
+      out[i] = o + e;
+      out[N - 1 - i] = o - e;
+    } else {
+      out[i] = o;
+    }
+  }
+}
+
+// One line of direction AX: F its fluxes q u_d, gm / gp the face fluxes of its
+// - and + faces, all in range of the scale E; emit(m, I): the result is I times
+// two to the line's exponent (fix_line_exp) plus its row's.
+template <int P, int AX, typename Emit>
+__device__ __forceinline__ void fix_line(const FixStageArgs<P>& a, const double* F, int32_t E,
+                                         double gm, double gp, Emit&& emit) {
+  using Sh = EoShape<P>;
+  constexpr int N = Sh::N, H = Sh::H;
+  const fixlimb* T = a.tab + AX * Sh::TE;
+  fixlimb s[H], d[H], fm{0, 0};
+#pragma unroll
+  for (int l = 0; l < H; l++) {
+    const int64_t f1 = fix_align(F[l], E), f2 = fix_align(F[N - 1 - l], E);
+    s[l] = fix_split(f1 + f2);
+    d[l] = fix_split(f1 - f2);
+  }
+  if constexpr (Sh::ODD != 0) fm = fix_split(fix_align(F[H], E));
+  const int64_t im = fix_align_face(gm, E), ip = fix_align_face(gp, E);
+  const fixlimb gs = fix_split(im + ip), gd = fix_split(im - ip);
+#pragma unroll
+  for (int i = 0; i < H; i++) {
+    fixacc e, o;
+    fix_mul(e, T[Sh::OFF_B + i], gd);
+    fix_mul(o, T[Sh::OFF_A + i], gs);
+#pragma unroll
+    for (int l = 0; l < H; l++) {
+      fix_fma(e, T[Sh::OFF_E + i * H + l], s[l]);
+      fix_fma(o, T[Sh::OFF_O + i * H + l], d[l]);
+    }
+    if constexpr (Sh::ODD != 0) fix_fma(e, T[Sh::OFF_DM + i], fm);
+    const int64_t es = fix_sum(e), os = fix_sum(o);
+    emit(i, os + es);
+    emit(N - 1 - i, os - es);
+  }
+  if constexpr (Sh::ODD != 0) {
+    fixacc o;
+    fix_mul(o, T[Sh::OFF_A + H], gs);
+#pragma unroll
+    for (int l = 0; l < H; l++) fix_fma(o, T[Sh::OFF_O + H * H + l], d[l]);
+    emit(H, fix_sum(o));
+  }
+}
+
+// Exponent of a line formed in FP64: its results are doubles.
+constexpr int kFixDouble = 1 << 20;
+
+// The line of direction AX held in shared memory with stride S, its results
+// over it as integers (or doubles); returns the line's exponent.
+template <int P, int AX, int S>
+__device__ __forceinline__ int fix_line_shared(const FixStageArgs<P>& a, double* line, double gm,
+                                               double gp) {
+  constexpr int N = P + 1;
+  double F[N];
+  int32_t E = max(0, max(fix_face_exp(gm), fix_face_exp(gp)));
+#pragma unroll
+  for (int l = 0; l < N; l++) {
+    F[l] = line[l * S];
+    E = max(E, fix_value_exp(F[l]));
+  }
+  if (a.ok && fix_in_range(E)) {
+    int64_t* out = reinterpret_cast<int64_t*>(line);
+    fix_line<P, AX>(a, F, E, gm, gp, [&](int m, int64_t v) { out[m * S] = v; });
+    return fix_line_exp(E);
+  }
+  double out[N];
+  fix_line_fp64<P>(line, S, static_cast<const double*>(a.s.D) + AX * EoShape<P>::TE, a.s.eo_sD[AX],
+                   a.s.eo_sL[AX], gm, gp, out);
+  for (int m = 0; m < N; m++) line[m * S] = out[m];
+  return kFixDouble;
+}
+
+// A node's tendency from its three line results v with exponents e (at least
+// one a double): the sum in FP64.
+static __device__ __noinline__ double fix_node_fp64(int64_t x, int ex, int64_t y, int ey, int64_t z,
+                                             int ez) {
+  auto value = [](int64_t v, int e) {
+    return e >= kFixDouble / 2 ? __longlong_as_double(v) : v == 0 ? 0.0 : fix_to_double(v, e);
+  };
+  return (value(x, ex) + value(y, ey)) + value(z, ez);
+}
+
+// Neighbour elements of e across the faces -y, +x, +y, -x, -z, +z with
+// periodic wrap.
+__device__ __forceinline__ void fix_neighbors(const Box& b, unsigned e, unsigned nb[6]) {
+  const unsigned NX = b.NeX, NY = b.NeY, NZ = b.NeZ, sy = NX, sz = NX * NY;
+  const unsigned rxy = e / NX, ex = e - rxy * NX, ez = rxy / NY, ey = rxy - ez * NY;
+  nb[0] = (ey == 0) ? e + (NY - 1) * sy : e - sy;
+  nb[2] = (ey == NY - 1) ? e - (NY - 1) * sy : e + sy;
+  nb[3] = (ex == 0) ? e + (NX - 1) : e - 1;
+  nb[1] = (ex == NX - 1) ? e - (NX - 1) : e + 1;
+  nb[4] = (ez == 0) ? e + (NZ - 1) * sz : e - sz;
+  nb[5] = (ez == NZ - 1) ? e - (NZ - 1) * sz : e + sz;
+}
+
+template <int P>
+__host__ __device__ constexpr int fix_min_blocks() {
+  return P >= 14 ? 3 : 1024 / FixShape<P>::THREADS;
+}
+
+// RK: the stage's update kind; FCIN: the velocity factors of the face flux
+// come from an earlier stage of the call.
+template <int P, int RK, bool FCIN>
+__global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
+    stage_fix_kernel(const __grid_constant__ FixStageArgs<P> a) {
+  using Sh = FixShape<P>;
+  constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NFT = 6 * N2, NS = Sh::NS, EW = Sh::EW,
+                EPB = Sh::EPB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const long long eb = a.s.elem_begin + (long long)blockIdx.x * EPB;
+  const long long left = a.s.elem_begin + a.s.elem_count - eb;
+  const int nloc = (int)(left < EPB ? left : EPB);
+  const int le = threadIdx.x / N2, r = threadIdx.x - le * N2;
+  const bool on = le < nloc;
+  const int i = r % N, j = r / N;
+  double* sX = reinterpret_cast<double*>(smem_raw) + le * EW;
+  double* sY = sX + EPB * EW;
+  // exponents of the element's x and y lines
+  int* sEx = reinterpret_cast<int*>(reinterpret_cast<double*>(smem_raw) + 2 * EPB * EW) + le * N2;
+  int* sEy = sEx + EPB * N2;
+  const long long ge = (eb + le) * NP;  // the element's first node
+  const double* __restrict__ q = a.s.q_in;
+  const int zat = i + NS * j;  // the z line's first node in the padded arrays
+
+  // 0: the z line's x and y fluxes, the six face fluxes; what phase 2 reads
+  // starts towards L2
+  double g[6];
+  if (on) {
+    for (int t = 16 * r; t < NP; t += 16 * N2) {
+      prefetch_l2(static_cast<const double*>(a.s.w) + ge + t);
+      if constexpr (RK == kRkGeneral) prefetch_l2(a.s.q0 + ge + t);
+    }
+    const double* __restrict__ u = static_cast<const double*>(a.s.u);
+    const double* __restrict__ v = static_cast<const double*>(a.s.v);
+#pragma unroll
+    for (int m = 0; m < N; m++) {
+      const double qv = q[ge + r + m * N2];
+      sX[zat + m * NS * N] = qv * u[ge + r + m * N2];
+      sY[zat + m * NS * N] = qv * v[ge + r + m * N2];
+    }
+    unsigned nb[6];
+    fix_neighbors(a.s.box, (unsigned)(eb + le), nb);
+    // node of face f on this side and on the neighbour's
+    const int x0 = i * N + j * N2, y0 = i + j * N2;
+    const int nM[6] = {y0, x0 + (N - 1), y0 + (N - 1) * N, x0, r, r + (N - 1) * N2};
+    const int nP[6] = {y0 + (N - 1) * N, x0, y0, x0 + (N - 1), r + (N - 1) * N2, r};
+#pragma unroll
+    for (int f = 0; f < 6; f++) {
+      const long long gP = (long long)nb[f] * NP + nP[f];
+      const double qP = q[gP], qM = q[ge + nM[f]];
+      const long long fi = (eb + le) * NFT + f * N2 + r;
+      double2 fc;
+      if constexpr (FCIN) {
+        fc = reinterpret_cast<const double2*>(a.s.fc_in)[fi];
+      } else {
+        const double* vel = static_cast<const double*>((f == 1 || f == 3)   ? a.s.u
+                                                       : (f == 0 || f == 2) ? a.s.v
+                                                                            : a.s.w);
+        const double uM = vel[ge + nM[f]], uP = vel[gP];
+        const double a2 = abs_ct(uP + uM);
+        const double tw = (f == 1 || f == 2 || f == 5) ? 2.0 : -2.0;
+        fc = make_double2(fma(tw, uP, -a2), fma(tw, uM, -a2));
+        if (a.s.fc_out) reinterpret_cast<double2*>(a.s.fc_out)[fi] = fc;
+      }
+      g[f] = fma(qP, fc.x, -(qM * fc.y));
+    }
+  }
+  __syncthreads();
+  if (on) {
+    // lines along i (r = j + N k), faces -x (3) and +x (1)
+    sEx[r] = fix_line_shared<P, 0, 1>(a, sX + NS * r, g[3], g[1]);
+    // lines along j (r = i + N k), faces -y (0) and +y (2)
+    sEy[r] = fix_line_shared<P, 1, NS>(a, sY + i + NS * N * j, g[0], g[2]);
+  }
+  // lines along k (r = i + N j), faces -z (4) and +z (5); the RK update
+  double F[N];
+  int32_t E = 0;
+  if (on) {
+    const double* __restrict__ w = static_cast<const double*>(a.s.w);
+    E = max(0, max(fix_face_exp(g[4]), fix_face_exp(g[5])));
+#pragma unroll
+    for (int m = 0; m < N; m++) {
+      F[m] = q[ge + r + m * N2] * w[ge + r + m * N2];
+      E = max(E, fix_value_exp(F[m]));
+    }
+  }
+  __syncthreads();
+  if (on) {
+    const double* __restrict__ q0 = a.s.q0;
+    double* __restrict__ qout = a.s.q_out;
+    const double c = a.c, ra = a.s.a, rb = a.s.b;
+    // the node's three results on the largest of their scales, added as
+    // integers (each below 2^61)
+    const int Bz = a.ok && fix_in_range(E) ? fix_line_exp(E) : kFixDouble;
+    const int rx = a.row[min(i, N - 1 - i)], ry = a.row[EoShape<P>::HR + min(j, N - 1 - j)];
+    const int64_t* iX = reinterpret_cast<const int64_t*>(sX) + zat;
+    const int64_t* iY = reinterpret_cast<const int64_t*>(sY) + zat;
+    auto emit = [&](int m, int64_t z) {
+      const int64_t x = iX[m * NS * N], y = iY[m * NS * N];
+      const int ex = sEx[j + N * m] + rx, ey = sEy[i + N * m] + ry;
+      const int ez = Bz + a.row[2 * EoShape<P>::HR + (m < N - 1 - m ? m : N - 1 - m)];
+      const int e = max(ex, max(ey, ez));
+      double t;
+      if (e < kFixDouble / 2)
+        t = fix_to_double(fix_sar(x, e - ex) + fix_sar(y, e - ey) + fix_sar(z, e - ez), e);
+      else
+        t = fix_node_fp64(x, ex, y, ey, z, ez);
+      const long long n = ge + r + m * N2;
+      if constexpr (RK == kRkTend)
+        qout[n] = t;
+      else if constexpr (RK == kRkFirst)
+        qout[n] = fma(c, t, q[n]);
+      else
+        qout[n] = rk_combine<RK>(c * t, q[n], q0[n], ra, rb);  // c t rounds below q's last bit
+    };
+    if (Bz != kFixDouble) {
+      fix_line<P, 2>(a, F, E, g[4], g[5], emit);
+    } else {
+      double in[N], out[N];  // in: F itself stays in registers
+#pragma unroll
+      for (int m = 0; m < N; m++) in[m] = F[m];
+      fix_line_fp64<P>(in, 1, static_cast<const double*>(a.s.D) + 2 * EoShape<P>::TE,
+                       a.s.eo_sD[2], a.s.eo_sL[2], g[4], g[5], out);
+#pragma unroll 1
+      for (int m = 0; m < N; m++) emit(m, __double_as_longlong(out[m]));
+    }
+  }
+}
+
+template <int P, int RK, bool FCIN>
+int launch_stage_fix_kind(const FixStageArgs<P>& a, unsigned nblk, cudaStream_t st) {
+  constexpr size_t smem = fix_smem<P>();
+  SDG_TRY(set_kernel_smem((const void*)stage_fix_kernel<P, RK, FCIN>, (int)smem, true));
+  stage_fix_kernel<P, RK, FCIN><<<nblk, FixShape<P>::THREADS, smem, st>>>(a);
+  SDG_CUDA_TRY(cudaGetLastError());
+  return SDG_OK;
+}
+
+template <int P>
+int launch_stage_fix_impl(const StageArgs& s, cudaStream_t st) {
+  FixStageArgs<P> a;
+  a.s = s;
+  a.c = s.tend_only ? 1.0 : s.b * s.dt;
+  for (int d = 0; d < 3; d++) {
+    // the FP64 lines' factors, without the stage's (which a.c carries)
+    a.s.eo_sD[d] = -s.box.Es[d];
+    a.s.eo_sL[d] = -(0.25 * s.box.Fs[d]);
+  }
+  for (int t = 0; t < 3 * EoShape<P>::TE; t++)
+    a.tab[t] = fixlimb{s.fix->coef[2 * t], s.fix->coef[2 * t + 1]};
+  for (int t = 0; t < 3 * EoShape<P>::HR; t++) a.row[t] = s.fix->row[t];
+  a.ok = s.fix->ok;
+  const long long nblk = (s.elem_count + FixShape<P>::EPB - 1) / FixShape<P>::EPB;
+  if (nblk <= 0) return SDG_OK;
+  if (nblk > 0x7fffffffLL) return fail(SDG_ERR_INVALID_ARG, "too many elements");
+  const bool in = s.fc_in != nullptr;
+  switch (rk_kind(s)) {
+    case kRkTend: return launch_stage_fix_kind<P, kRkTend, false>(a, (unsigned)nblk, st);
+    case kRkFirst:
+      return in ? launch_stage_fix_kind<P, kRkFirst, true>(a, (unsigned)nblk, st)
+                : launch_stage_fix_kind<P, kRkFirst, false>(a, (unsigned)nblk, st);
+    default: return launch_stage_fix_kind<P, kRkGeneral, true>(a, (unsigned)nblk, st);
+  }
+}
+
+}  // namespace sdg
