@@ -52,14 +52,17 @@ extern "C" {
 #define SDG_OPT_GENERAL 1
 #define SDG_OPT_OPT1 2
 /* The even-odd factorisation of D1D and of the face lift (needs their
- * centro-symmetry, which GLL operators have to rounding): in the solver and
- * batched forms the fused stage with ~30 % fewer FP64 operations in the FP64
- * form and about half the instructions in the FP32 and emulated forms; in
- * cal_tend the even-odd tendency kernel.  Same result to rounding. */
+ * centro-symmetry, which GLL operators have to rounding): half the products of
+ * a line sum, in the solver and batched forms and in cal_tend's even-odd
+ * tendency kernel.  Same result to rounding. */
 #define SDG_OPT_EVENODD 3
 
 /* Arithmetic of a solver (the reference is FP64 throughout). */
-#define SDG_PREC_FP64 0   /* FP64 state and FP64 arithmetic on the DFMA pipe */
+#define SDG_PREC_FP64 0   /* FP64 state, fluxes and RK update; the line sums of
+                             the fused stage as exact integer sums of 60-bit
+                             fixed-point products, as near to the exact sum as
+                             FP64 arithmetic, which forms the lines that hold
+                             infinities, NaN or extreme magnitudes */
 #define SDG_PREC_FP32 1   /* FP32 flux/derivative/lift, FP64 RK state */
 #define SDG_PREC_FP64_EMU 2 /* FP64 state and RK combine; flux/derivative/lift in
                                double-float (two FP32 numbers, ~48 bits) on the
@@ -344,15 +347,17 @@ int sdg_advect3d_eq_step_dev(double* q, const double* u, const double* v,
 typedef struct sdg_solver sdg_solver;
 
 /* D1D(Nq,Nq) and Lift_mat(Nq,Nq,Nq,6) as read from operator_data (or from
- * sdg_operator_generate).  opt = SDG_OPT_GENERAL / SDG_OPT_OPT1 selects the
- * summation order of the divergence (they differ only for p > 7);
+ * sdg_operator_generate).  opt = SDG_OPT_GENERAL / SDG_OPT_OPT1 takes any
+ * operators and selects the summation order of the divergence (they differ
+ * only for p > 7, and not in SDG_PREC_FP64, whose integer sums have none);
  * SDG_OPT_EVENODD the even-odd stage (returns SDG_ERR_INVALID_ARG if
  * D1D or Lift_mat lacks the centro-symmetry beyond 1e-13 relative).
  * precision = SDG_PREC_*.  stream may be NULL.
- * With SDG_OPT_EVENODD and SDG_PREC_FP64 or SDG_PREC_FP64_EMU the solver also
- * holds the face-flux velocity factors of one step (16 bytes per face node,
- * 96/Nq bytes per DOF): the first stage of every step forms them from the
- * current velocity and the other two stages read them. */
+ * With SDG_PREC_FP64, or SDG_OPT_EVENODD and SDG_PREC_FP64_EMU, the solver also
+ * holds the face-flux velocity factors of one call (16 bytes per face node,
+ * 96/Nq bytes per DOF): the first stage of every sdg_solver_step forms them
+ * from the current velocity and the others read them.  (With GENERAL and OPT1
+ * a solver whose device memory does not hold them forms them in every stage.) */
 int sdg_solver_create(sdg_solver** out, int NeX, int NeY, int NeZ, int p,
                       double Lx, double Ly, double Lz, const double* D1D,
                       const double* Lift_mat, int opt, int precision,

@@ -264,6 +264,26 @@ int eo_tables(int Nq, const double* D1D, const double* Lift_mat, std::vector<dou
   return SDG_OK;
 }
 
+namespace {
+// The limbs of -x y 2^(60 - k), the product exact (its rounding error added
+// back as an integer); double arithmetic, since long double is software on
+// some hosts.
+void fix_put(int32_t* out, double x, double y, int k) {
+  const double scale = std::ldexp(1.0, 60 - k), hi = x * y, lo = std::fma(x, y, -hi);
+  const fixlimb c = fix_coef(-(int64_t)(std::llrint(hi * scale) + std::llrint(lo * scale)));
+  out[0] = c.hi;
+  out[1] = c.lo;
+}
+// The exponent of a row whose magnitudes add up to `sum` (with room for the
+// rounding of the sum); false outside +-200.
+bool fix_row_exp(double sum, int* k) {
+  *k = 0;
+  if (!std::isfinite(sum)) return false;
+  if (sum > 0.0) std::frexp(sum * (1.0 + 1e-13), k);
+  return *k >= -200 && *k <= 200;
+}
+}  // namespace
+
 void fix_tables(int Nq, const Box& box, const std::vector<double>& eo, FixTables& t) {
   const int N = Nq, H = N / 2, HR = (N + 1) / 2, ODD = N & 1;
   const int TE = H * H + HR * H + ODD * H + HR + H;
@@ -273,7 +293,7 @@ void fix_tables(int Nq, const Box& box, const std::vector<double>& eo, FixTables
   t.row.assign(3 * (size_t)HR, 0);
   for (int d = 0; d < 3; d++) {
     const double* T = eo.data() + (size_t)d * TE;
-    auto value = [&](int w) { return -(long double)T[w] * (w < oA ? box.Es[d] : box.Fs[d]); };
+    auto scale = [&](int w) { return w < oA ? box.Es[d] : box.Fs[d]; };
     for (int i = 0; i < HR; i++) {
       std::vector<int> even, odd{oA + i};
       for (int l = 0; l < H; l++) odd.push_back(oO + i * H + l);
@@ -282,20 +302,51 @@ void fix_tables(int Nq, const Box& box, const std::vector<double>& eo, FixTables
         if (ODD) even.push_back(oM + i);
         for (int l = 0; l < H; l++) even.push_back(i * H + l);
       }
-      long double se = 0.0L, so = 0.0L;
-      for (int w : even) se += std::fabs(value(w));
-      for (int w : odd) so += std::fabs(value(w));
-      const long double most = std::fmax(se, so);
-      if (!std::isfinite((double)most)) return;
+      double se = 0.0, so = 0.0;
+      for (int w : even) se += std::fabs(T[w] * scale(w));
+      for (int w : odd) so += std::fabs(T[w] * scale(w));
       int k = 0;
-      if (most > 0.0L) std::frexp(most, &k);
-      if (k < -200 || k > 200) return;
+      if (!fix_row_exp(se > so ? se : so, &k)) return;
       t.row[(size_t)d * HR + i] = k - 59;
       even.insert(even.end(), odd.begin(), odd.end());
-      for (int w : even) {
-        const fixlimb x = fix_coef((int64_t)std::llround(std::ldexp(value(w), 60 - k)));
-        t.coef[2 * ((size_t)d * TE + w)] = x.hi;
-        t.coef[2 * ((size_t)d * TE + w) + 1] = x.lo;
+      for (int w : even) fix_put(&t.coef[2 * ((size_t)d * TE + w)], T[w], scale(w), k);
+    }
+  }
+  t.ok = 1;
+}
+
+void fix_tables_general(int Nq, const Box& box, const double* D1D, const double* Lift_mat,
+                        FixTables& t, std::vector<int32_t>& lift) {
+  const int N = Nq, N2 = N * N, NP = N * N2;
+  const int fminus[3] = {3, 0, 4}, fplus[3] = {1, 2, 5};
+  t.ok = 0;
+  t.coef.assign(2 * 3 * (size_t)N2, 0);
+  t.row.assign(3 * (size_t)N, 0);
+  lift.assign(4 * 3 * (size_t)NP, 0);
+  for (int d = 0; d < 3; d++) {
+    const double Es = box.Es[d], Fs = box.Fs[d];
+    const double* Lm = Lift_mat + (long long)fminus[d] * NP;
+    const double* Lp = Lift_mat + (long long)fplus[d] * NP;
+    for (int i = 0; i < N; i++) {
+      auto node = [&](int r) {  // node i of line r along axis d
+        return d == 0 ? i + N * r : d == 1 ? r % N + N * i + N2 * (r / N) : r + N2 * i;
+      };
+      double most = 0.0, sum = 0.0;
+      for (int r = 0; r < N2; r++) {
+        const double s = std::fabs(Lm[node(r)]) + std::fabs(Lp[node(r)]);
+        if (!std::isfinite(s)) return;
+        most = s > most ? s : most;
+      }
+      for (int l = 0; l < N; l++) sum += std::fabs(D1D[i + l * N] * Es);
+      int k = 0;
+      if (!fix_row_exp(sum + most * Fs, &k)) return;
+      t.row[(size_t)d * N + i] = k - 59;
+      for (int l = 0; l < N; l++)
+        fix_put(&t.coef[2 * ((size_t)d * N2 + i * N + l)], D1D[i + l * N], Es, k);
+      for (int r = 0; r < N2; r++) {
+        int32_t* out = &lift[4 * ((size_t)d * NP + (size_t)i * N2 + r)];
+        fix_put(out, Lm[node(r)], Fs, k);
+        fix_put(out + 2, Lp[node(r)], Fs, k);
       }
     }
   }

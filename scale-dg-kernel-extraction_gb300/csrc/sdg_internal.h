@@ -70,6 +70,12 @@ struct FixTables {
 };
 // Fills t from the unscaled tables of eo_tables.
 void fix_tables(int Nq, const Box& box, const std::vector<double>& eo, FixTables& t);
+// The same for operators as given (coef: per direction D(i,l) at i Nq + l; one
+// scale a row, over all its nodes' lift entries).  lift receives, per direction
+// d, row i and line r of the direction, the limb pairs of the - and the + face's
+// lift entry at that node: 4 * 3 * Nq^3 values.
+void fix_tables_general(int Nq, const Box& box, const double* D1D, const double* Lift_mat,
+                        FixTables& t, std::vector<int32_t>& lift);
 
 // Arguments of one fused stage launch.
 struct StageArgs {
@@ -102,9 +108,11 @@ struct StageArgs {
   // advect3d_eq_cal_tend call), form them once.  Both null: formed inline.
   double* fc_out;
   const double* fc_in;
-  // even-odd FP64 stage: its fixed-point coefficients (host memory, copied
-  // into the launch)
+  // FP64 stage: its fixed-point coefficients (host memory, copied into the
+  // launch), and for operators as given the nodes' lift limbs (device memory,
+  // one int4 a node and direction)
   const FixTables* fix;
+  const void* fix_lift;
 };
 
 // Even-odd tables (3 directions, unscaled) from D1D and Lift_mat after the

@@ -41,8 +41,10 @@ struct sdg_solver {
   // Measured on GB300 against forming them in every stage: 1.04-1.13x for the
   // FP64 stage (p = 7: 19.3 against 18.5 GDOF-updates/s), 1.01-1.14x emulated.
   double* fc = nullptr;
-  // coefficients of the fixed-point stage (even-odd FP64)
+  // coefficients of the FP64 stage, and for operators as given (GENERAL, OPT1)
+  // its device table of lift limbs
   FixTables fix;
+  void* fix_lift = nullptr;
   // elements a stage advances: [elem_begin, elem_begin + elem_count) of the
   // box (the whole box by default; a z-slab partition advances its owned
   // layers and keeps a ghost layer on each side)
@@ -88,6 +90,7 @@ void release(sdg_solver* s) {
   cudaFree(s->Lift);
   cudaFree(s->dqdt);
   cudaFree(s->fc);
+  cudaFree(s->fix_lift);
 }
 
 // fc: 0 = the stage forms the face-flux velocity factors inline, 1 = it also
@@ -132,6 +135,7 @@ int one_stage_on(sdg_solver* s, int stage, double dt, const double* qin, const d
   a.fc_out = (s->fc && fc == 1) ? s->fc : nullptr;
   a.fc_in = (s->fc && fc == 2) ? s->fc : nullptr;
   a.fix = &s->fix;
+  a.fix_lift = s->fix_lift;
   const double c = tend_only ? 1.0 : a.b * dt;
   for (int d = 0; d < 3; d++) {
     a.eo_sD[d] = -c * s->box.Es[d];
@@ -282,6 +286,9 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
       fix_tables(s->Nq, s->box, tab, s->fix);
     }
   }
+  std::vector<int32_t> fix_lift;
+  if (precision == SDG_PREC_FP64 && opt != SDG_OPT_EVENODD)
+    fix_tables_general(s->Nq, s->box, D1D, Lift_mat, s->fix, fix_lift);
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < 3 && e == cudaSuccess; i++)
     e = cudaMalloc(&s->q[i], 8 * (size_t)s->ndof);
@@ -290,8 +297,18 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
   if (e == cudaSuccess) e = cudaMalloc(&s->w, es * (size_t)s->ndof);
   if (e == cudaSuccess) e = cudaMalloc(&s->D, dtab.size());
   if (e == cudaSuccess) e = cudaMalloc(&s->Lift, ltab.size());
+  const size_t fc_bytes = 16 * (size_t)(6 * s->Nq * s->Nq) * (size_t)s->box.Ne;
   if (e == cudaSuccess && precision != SDG_PREC_FP32 && opt == SDG_OPT_EVENODD)
-    e = cudaMalloc(&s->fc, 16 * (size_t)(6 * s->Nq * s->Nq) * (size_t)s->box.Ne);
+    e = cudaMalloc(&s->fc, fc_bytes);
+  if (e == cudaSuccess && !fix_lift.empty()) e = cudaMalloc(&s->fix_lift, 4 * fix_lift.size());
+  if (e == cudaSuccess && !fix_lift.empty())
+    e = cudaMemcpy(s->fix_lift, fix_lift.data(), 4 * fix_lift.size(), cudaMemcpyHostToDevice);
+  // GENERAL and OPT1 in FP64 share the velocity factors too, but a box whose
+  // other buffers fill the memory runs without them
+  if (e == cudaSuccess && !fix_lift.empty() && cudaMalloc(&s->fc, fc_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    s->fc = nullptr;
+  }
   if (e == cudaSuccess) e = cudaMemcpy(s->D, dtab.data(), dtab.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(s->Lift, ltab.data(), ltab.size(), cudaMemcpyHostToDevice);

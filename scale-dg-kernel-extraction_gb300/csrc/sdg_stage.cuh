@@ -1,4 +1,6 @@
-// Fused RK-stage kernel for the periodic structured box.
+// Fused RK-stage kernel for the periodic structured box: the node body of the
+// FP32-compute form, and what every stage kernel shares (RK kinds, face
+// geometry, neighbours).  The FP64 form is in sdg_stage_fix.cuh.
 //
 // One launch advances every element of the box through one SSP-RK3 stage,
 // replacing, per stage, the reference's update_halo (mod_mesh.f90:209-221),
@@ -257,19 +259,10 @@ __device__ __forceinline__ void stage_block(const StageArgs& a, long long eb, in
   __syncthreads();
 
   // phase 1: element-boundary flux (mod_advect3d_eq.f90:116-140); 0.5*Fscale
-  // is exact in either type and prepared on the host for FP32.  The velocity
+  // is prepared on the host.  The velocity
   // of both sides is read from global memory (the own element's values were
   // just loaded by phase 0 and sit in L1).
-  CT hfx, hfy, hfz;
-  if constexpr (sizeof(CT) == 4) {
-    hfx = a.box.hFsf[0];
-    hfy = a.box.hFsf[1];
-    hfz = a.box.hFsf[2];
-  } else {
-    hfx = 0.5 * a.box.Fs[0];
-    hfy = 0.5 * a.box.Fs[1];
-    hfz = 0.5 * a.box.Fs[2];
-  }
+  const CT hfx = a.box.hFsf[0], hfy = a.box.hFsf[1], hfz = a.box.hFsf[2];
   const FaceTasks<NQ> ftask(nloc);
   for (int t = threadIdx.x; t < nloc * NFT; t += T) {
     int le, f, fp;
@@ -295,20 +288,11 @@ __device__ __forceinline__ void stage_block(const StageArgs& a, long long eb, in
 
   // phase 3: divergence + lift + combine + RK (mod_advect3d_eq.f90:185-198,
   // main.f90:69-73)
-  CT Ex, Ey, Ez;
-  if constexpr (sizeof(CT) == 4) {
-    Ex = a.box.Esf[0];
-    Ey = a.box.Esf[1];
-    Ez = a.box.Esf[2];
-  } else {
-    Ex = a.box.Es[0];
-    Ey = a.box.Es[1];
-    Ez = a.box.Es[2];
-  }
+  const CT Ex = a.box.Esf[0], Ey = a.box.Esf[1], Ez = a.box.Esf[2];
   const CT* __restrict__ L = static_cast<const CT*>(a.Lift);
   double* __restrict__ qout = a.q_out;
   const double* __restrict__ q0 = a.q0;
-  const double ra = a.a, rb = a.b, rdt = a.dt;
+  const double ra = a.a, rb = a.b;
   const CT cdt = a.cdt_hi;
   with_rk_kind<RKFIX>(rk_kind(a), [&](auto rkc) {
     constexpr int RK = decltype(rkc)::value;
@@ -327,26 +311,13 @@ __device__ __forceinline__ void stage_block(const StageArgs& a, long long eb, in
       const CT lf = lift_node<P>(L + n, sf + le * NFT, i, j, k);
       const CT dq = -(((Ex * dx + Ey * dy) + Ez * dz) + lf);
       const long long g = g0 + t;
-      if constexpr (sizeof(CT) == 8) {
-        // the reference's order, a*q0 + b*(q + dt*dqdt) (main.f90:69-73);
-        // stage 1 (a = 0, b = 1) is q + dt*dqdt exactly
-        if constexpr (RK == kRkTend) {
-          qout[g] = (double)dq;
-        } else if constexpr (RK == kRkFirst) {
-          qout[g] = qin[g] + rdt * (double)dq;
-        } else {
-          const double r = rb * (qin[g] + rdt * (double)dq);
-          qout[g] = ra * q0[g] + r;
-        }
-      } else {
-        // FP32 form: the increment (b*dt)*dqdt is an FP32 product widened by
-        // bits; the state combination a*q0 + b*q + increment stays FP64
-        if constexpr (RK == kRkTend)
-          qout[g] = f32_to_f64_bits(dq);
-        else
-          qout[g] = rk_combine<RK>(f32_to_f64_bits(cdt * dq), qin[g],
-                                   RK == kRkGeneral ? q0[g] : 0.0, ra, rb);
-      }
+      // the increment (b*dt)*dqdt is an FP32 product widened by bits; the
+      // state combination a*q0 + b*q + increment stays FP64
+      if constexpr (RK == kRkTend)
+        qout[g] = f32_to_f64_bits(dq);
+      else
+        qout[g] = rk_combine<RK>(f32_to_f64_bits(cdt * dq), qin[g], RK == kRkGeneral ? q0[g] : 0.0,
+                                 ra, rb);
     }
   });
 }

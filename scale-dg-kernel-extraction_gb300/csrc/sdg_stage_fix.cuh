@@ -20,6 +20,14 @@
 // constant bank.  The x, y and z results of a node add up as integers; the
 // increment is their sum times one factor of the element and the stage.
 //
+// Face flux: qP tP - qM tM with tP = 2VelP - 2a, tM = 2VelM - 2a, 2a = |uP + uM|
+// (a quarter of Fscale is in the lift coefficients).  With operators as given
+// it is formed as qP (tP - tM) + (qP - qM) tM: a rounding of tM or of its product
+// then weighs with the jump, not with q, which keeps the tendency's error on
+// smooth fields at 0.6-0.95 of the FP64 node body's (p = 11: 7e-16 against
+// 8.8e-16; 1.7e-15 with the first form).  The factors, (tP, tM) or
+// (tP - tM, tM), come from the first stage of a call, which stores them.
+//
 // Scale: a line's values share the power of two that bounds its fluxes q u_d
 // and its two face fluxes, and a row of coefficients has a power of two of its
 // own, so every line result keeps about 2^-59 of its own bound.  The three
@@ -34,6 +42,8 @@
 //   1  x line and y line r, results over the fluxes
 //   2  z line r, and the RK update of its nodes
 #pragma once
+
+#include <algorithm>
 
 #include "sdg_fix.cuh"
 #include "sdg_stage_eo.cuh"
@@ -53,39 +63,61 @@ struct FixShape {
   static constexpr int EPB = THREADS / N2;
 };
 
-template <int P>
+// EO: coefficients of the even-odd pairs; else those of D1D as given, with the
+// lift entries of every node (operators without the symmetries, and the
+// GENERAL and OPT1 types, whose sums differ only in an order that integer sums
+// do not have).
+template <int P, bool EO>
 struct FixStageArgs {
+  static constexpr int TAB = EO ? EoShape<P>::TE : (P + 1) * (P + 1);
+  static constexpr int ROWS = EO ? EoShape<P>::HR : P + 1;
   StageArgs s;
-  double c;                       // b dt (1: tendency)
-  fixlimb tab[3 * EoShape<P>::TE];
-  int row[3 * EoShape<P>::HR];    // exponent of a row's scale, less 59
-  int ok;                         // 0: the box's coefficients are out of range,
-                                  // every line is formed in FP64
+  double c;              // EO: b dt, else dt
+  fixlimb tab[3 * TAB];  // per direction: EoShape's table, or D(i,l) at i N + l
+  int row[3 * ROWS];     // exponent of a row's scale, less 59
+  int ok;                // 0: coefficients out of range, every line in FP64
+  static __host__ __device__ constexpr int row_of(int m) {
+    return EO ? (m < P - m ? m : P - m) : m;
+  }
 };
 
 template <int P>
-__host__ __device__ constexpr size_t fix_smem() {
-  return sizeof(double) * 2 * FixShape<P>::EPB * FixShape<P>::EW +
-         sizeof(int) * 2 * FixShape<P>::EPB * FixShape<P>::N2;
+__host__ __device__ constexpr size_t fix_smem(int epb) {
+  return sizeof(double) * 2 * epb * FixShape<P>::EW + sizeof(int) * 2 * epb * FixShape<P>::N2;
 }
 
 // A line in FP64, for values the fixed-point path does not take (E: their
 // largest exponent, 0 when there is nothing but zeros and subnormals): F
 // holds the line's fluxes with stride fs, results to out[0..N).  A call of
 // its own, so that its registers do not count against the kernel's.
-template <int P>
-__device__ __noinline__ void fix_line_fp64(const double* F, int fs, const double* __restrict__ T,
-                                           double sD, double sL, double gm, double gp,
-                                           double* out) {
+template <int P, bool EO>
+__device__ __noinline__ void fix_line_fp64(const StageArgs* a, int ax, int r, const double* F,
+                                           int fs, double gm, double gp, double* out) {
   using Sh = EoShape<P>;
-  constexpr int N = Sh::N, H = Sh::H;
-  const double gs = gm + gp, gd = gm - gp;
+  constexpr int N = Sh::N, H = Sh::H, N2 = N * N, NP = N * N2;
+  const double sD = -a->box.Es[ax], sL = -(0.25 * a->box.Fs[ax]);
   bool some = gm != 0.0 || gp != 0.0;
   for (int l = 0; l < N; l++) {
     out[l] = 0.0;
     some = some || F[l * fs] != 0.0;
   }
   if (!some) return;
+  const double* __restrict__ T = static_cast<const double*>(a->D);
+  if constexpr (!EO) {
+    const int fm = ax == 0 ? 3 : ax == 1 ? 0 : 4, fp = ax == 0 ? 1 : ax == 1 ? 2 : 5;
+    const double* __restrict__ L = static_cast<const double*>(a->Lift);
+#pragma unroll 1
+    for (int i = 0; i < N; i++) {
+      double d = 0.0;
+#pragma unroll 1
+      for (int l = 0; l < N; l++) d = fma(T[i + l * N], F[l * fs], d);
+      const int n = ax == 0 ? i + N * r : ax == 1 ? r % N + N * i + N2 * (r / N) : r + N2 * i;
+      out[i] = fma(sD, d, sL * fma(L[n + fm * NP], gm, L[n + fp * NP] * gp));
+    }
+    return;
+  }
+  T += ax * Sh::TE;
+  const double gs = gm + gp, gd = gm - gp;
 #pragma unroll 1
   for (int i = 0; i < Sh::HR; i++) {
     double e = 0.0, o = 0.0;
@@ -107,15 +139,34 @@ __device__ __noinline__ void fix_line_fp64(const double* F, int fs, const double
   }
 }
 
-// One line of direction AX: F its fluxes q u_d, gm / gp the face fluxes of its
+// Line r of direction AX: F its fluxes q u_d, gm / gp the face fluxes of its
 // - and + faces, all in range of the scale E; emit(m, I): the result is I times
 // two to the line's exponent (fix_line_exp) plus its row's.
-template <int P, int AX, typename Emit>
-__device__ __forceinline__ void fix_line(const FixStageArgs<P>& a, const double* F, int32_t E,
-                                         double gm, double gp, Emit&& emit) {
+template <int P, bool EO, int AX, typename Emit>
+__device__ __forceinline__ void fix_line(const FixStageArgs<P, EO>& a, int r, const double* F,
+                                         int32_t E, double gm, double gp, Emit&& emit) {
   using Sh = EoShape<P>;
   constexpr int N = Sh::N, H = Sh::H;
-  const fixlimb* T = a.tab + AX * Sh::TE;
+  const fixlimb* T = a.tab + AX * a.TAB;
+  const int64_t im = fix_align_face(gm, E), ip = fix_align_face(gp, E);
+  if constexpr (!EO) {
+    const fixlimb lm = fix_split(im), lp = fix_split(ip);
+    fixlimb f[N];
+#pragma unroll
+    for (int l = 0; l < N; l++) f[l] = fix_split(fix_align(F[l], E));
+    const int4* __restrict__ lift = static_cast<const int4*>(a.s.fix_lift) + AX * N * N * N + r;
+#pragma unroll 2
+    for (int i = 0; i < N; i++) {
+      const int4 c = lift[i * N * N];
+      fixacc o;
+      fix_mul(o, fixlimb{c.x, c.y}, lm);
+      fix_fma(o, fixlimb{c.z, c.w}, lp);
+#pragma unroll
+      for (int l = 0; l < N; l++) fix_fma(o, T[i * N + l], f[l]);
+      emit(i, fix_sum(o));
+    }
+    return;
+  }
   fixlimb s[H], d[H], fm{0, 0};
 #pragma unroll
   for (int l = 0; l < H; l++) {
@@ -124,7 +175,6 @@ __device__ __forceinline__ void fix_line(const FixStageArgs<P>& a, const double*
     d[l] = fix_split(f1 - f2);
   }
   if constexpr (Sh::ODD != 0) fm = fix_split(fix_align(F[H], E));
-  const int64_t im = fix_align_face(gm, E), ip = fix_align_face(gp, E);
   const fixlimb gs = fix_split(im + ip), gd = fix_split(im - ip);
 #pragma unroll
   for (int i = 0; i < H; i++) {
@@ -155,9 +205,9 @@ constexpr int kFixDouble = 1 << 20;
 
 // The line of direction AX held in shared memory with stride S, its results
 // over it as integers (or doubles); returns the line's exponent.
-template <int P, int AX, int S>
-__device__ __forceinline__ int fix_line_shared(const FixStageArgs<P>& a, double* line, double gm,
-                                               double gp) {
+template <int P, bool EO, int AX, int S>
+__device__ __forceinline__ int fix_line_shared(const FixStageArgs<P, EO>& a, int r, double* line,
+                                               double gm, double gp) {
   constexpr int N = P + 1;
   double F[N];
   int32_t E = max(0, max(fix_face_exp(gm), fix_face_exp(gp)));
@@ -168,12 +218,11 @@ __device__ __forceinline__ int fix_line_shared(const FixStageArgs<P>& a, double*
   }
   if (a.ok && fix_in_range(E)) {
     int64_t* out = reinterpret_cast<int64_t*>(line);
-    fix_line<P, AX>(a, F, E, gm, gp, [&](int m, int64_t v) { out[m * S] = v; });
+    fix_line<P, EO, AX>(a, r, F, E, gm, gp, [&](int m, int64_t v) { out[m * S] = v; });
     return fix_line_exp(E);
   }
   double out[N];
-  fix_line_fp64<P>(line, S, static_cast<const double*>(a.s.D) + AX * EoShape<P>::TE, a.s.eo_sD[AX],
-                   a.s.eo_sL[AX], gm, gp, out);
+  fix_line_fp64<P, EO>(&a.s, AX, r, line, S, gm, gp, out);
   for (int m = 0; m < N; m++) line[m * S] = out[m];
   return kFixDouble;
 }
@@ -208,24 +257,25 @@ __host__ __device__ constexpr int fix_min_blocks() {
 
 // RK: the stage's update kind; FCIN: the velocity factors of the face flux
 // come from an earlier stage of the call.
-template <int P, int RK, bool FCIN>
+template <int P, bool EO, int RK, bool FCIN>
 __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
-    stage_fix_kernel(const __grid_constant__ FixStageArgs<P> a) {
+    stage_fix_kernel(const __grid_constant__ FixStageArgs<P, EO> a) {
+  using Args = FixStageArgs<P, EO>;
   using Sh = FixShape<P>;
-  constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NFT = 6 * N2, NS = Sh::NS, EW = Sh::EW,
-                EPB = Sh::EPB;
+  constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NFT = 6 * N2, NS = Sh::NS, EW = Sh::EW;
+  const int epb = blockDim.x / N2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long long eb = a.s.elem_begin + (long long)blockIdx.x * EPB;
+  const long long eb = a.s.elem_begin + (long long)blockIdx.x * epb;
   const long long left = a.s.elem_begin + a.s.elem_count - eb;
-  const int nloc = (int)(left < EPB ? left : EPB);
+  const int nloc = (int)(left < epb ? left : epb);
   const int le = threadIdx.x / N2, r = threadIdx.x - le * N2;
   const bool on = le < nloc;
   const int i = r % N, j = r / N;
   double* sX = reinterpret_cast<double*>(smem_raw) + le * EW;
-  double* sY = sX + EPB * EW;
+  double* sY = sX + epb * EW;
   // exponents of the element's x and y lines
-  int* sEx = reinterpret_cast<int*>(reinterpret_cast<double*>(smem_raw) + 2 * EPB * EW) + le * N2;
-  int* sEy = sEx + EPB * N2;
+  int* sEx = reinterpret_cast<int*>(reinterpret_cast<double*>(smem_raw) + 2 * epb * EW) + le * N2;
+  int* sEy = sEx + epb * N2;
   const long long ge = (eb + le) * NP;  // the element's first node
   const double* __restrict__ q = a.s.q_in;
   const int zat = i + NS * j;  // the z line's first node in the padded arrays
@@ -267,18 +317,18 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
         const double uM = vel[ge + nM[f]], uP = vel[gP];
         const double a2 = abs_ct(uP + uM);
         const double tw = (f == 1 || f == 2 || f == 5) ? 2.0 : -2.0;
-        fc = make_double2(fma(tw, uP, -a2), fma(tw, uM, -a2));
+        fc = make_double2(EO ? fma(tw, uP, -a2) : tw * (uP - uM), fma(tw, uM, -a2));
         if (a.s.fc_out) reinterpret_cast<double2*>(a.s.fc_out)[fi] = fc;
       }
-      g[f] = fma(qP, fc.x, -(qM * fc.y));
+      g[f] = EO ? fma(qP, fc.x, -(qM * fc.y)) : fma(qP, fc.x, (qP - qM) * fc.y);
     }
   }
   __syncthreads();
   if (on) {
     // lines along i (r = j + N k), faces -x (3) and +x (1)
-    sEx[r] = fix_line_shared<P, 0, 1>(a, sX + NS * r, g[3], g[1]);
+    sEx[r] = fix_line_shared<P, EO, 0, 1>(a, r, sX + NS * r, g[3], g[1]);
     // lines along j (r = i + N k), faces -y (0) and +y (2)
-    sEy[r] = fix_line_shared<P, 1, NS>(a, sY + i + NS * N * j, g[0], g[2]);
+    sEy[r] = fix_line_shared<P, EO, 1, NS>(a, r, sY + i + NS * N * j, g[0], g[2]);
   }
   // lines along k (r = i + N j), faces -z (4) and +z (5); the RK update
   double F[N];
@@ -300,13 +350,13 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
     // the node's three results on the largest of their scales, added as
     // integers (each below 2^61)
     const int Bz = a.ok && fix_in_range(E) ? fix_line_exp(E) : kFixDouble;
-    const int rx = a.row[min(i, N - 1 - i)], ry = a.row[EoShape<P>::HR + min(j, N - 1 - j)];
+    const int rx = a.row[Args::row_of(i)], ry = a.row[Args::ROWS + Args::row_of(j)];
     const int64_t* iX = reinterpret_cast<const int64_t*>(sX) + zat;
     const int64_t* iY = reinterpret_cast<const int64_t*>(sY) + zat;
     auto emit = [&](int m, int64_t z) {
       const int64_t x = iX[m * NS * N], y = iY[m * NS * N];
       const int ex = sEx[j + N * m] + rx, ey = sEy[i + N * m] + ry;
-      const int ez = Bz + a.row[2 * EoShape<P>::HR + (m < N - 1 - m ? m : N - 1 - m)];
+      const int ez = Bz + a.row[2 * Args::ROWS + Args::row_of(m)];
       const int e = max(ex, max(ey, ez));
       double t;
       if (e < kFixDouble / 2)
@@ -319,55 +369,60 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
       else if constexpr (RK == kRkFirst)
         qout[n] = fma(c, t, q[n]);
       else
-        qout[n] = rk_combine<RK>(c * t, q[n], q0[n], ra, rb);  // c t rounds below q's last bit
+        // the even-odd type adds b dt t to b q; the others keep the reference's
+        // a q0 + b (q + dt t) (main.f90:69-73)
+        qout[n] = EO ? rk_combine<RK>(c * t, q[n], q0[n], ra, rb)
+                     : fma(ra, q0[n], rb * fma(c, t, q[n]));
     };
     if (Bz != kFixDouble) {
-      fix_line<P, 2>(a, F, E, g[4], g[5], emit);
+      fix_line<P, EO, 2>(a, r, F, E, g[4], g[5], emit);
     } else {
       double in[N], out[N];  // in: F itself stays in registers
 #pragma unroll
       for (int m = 0; m < N; m++) in[m] = F[m];
-      fix_line_fp64<P>(in, 1, static_cast<const double*>(a.s.D) + 2 * EoShape<P>::TE,
-                       a.s.eo_sD[2], a.s.eo_sL[2], g[4], g[5], out);
+      fix_line_fp64<P, EO>(&a.s, 2, r, in, 1, g[4], g[5], out);
 #pragma unroll 1
       for (int m = 0; m < N; m++) emit(m, __double_as_longlong(out[m]));
     }
   }
 }
 
-template <int P, int RK, bool FCIN>
-int launch_stage_fix_kind(const FixStageArgs<P>& a, unsigned nblk, cudaStream_t st) {
-  constexpr size_t smem = fix_smem<P>();
-  SDG_TRY(set_kernel_smem((const void*)stage_fix_kernel<P, RK, FCIN>, (int)smem, true));
-  stage_fix_kernel<P, RK, FCIN><<<nblk, FixShape<P>::THREADS, smem, st>>>(a);
+template <int P, bool EO, int RK, bool FCIN>
+int launch_stage_fix_kind(const FixStageArgs<P, EO>& a, cudaStream_t st) {
+  // a small box takes blocks of a warp's elements, so that its blocks cover
+  // the chip: 8^3 elements at p = 3 as 256 blocks of 32 threads, not 64 of 128
+  constexpr int N2 = FixShape<P>::N2;
+  const long long want = std::max(a.s.elem_count / (2 * 152), 1LL);
+  const int threads = (int)std::min<long long>((want * N2 + 31) / 32 * 32, FixShape<P>::THREADS);
+  const int epb = threads / N2;
+  const long long nblk = (a.s.elem_count + epb - 1) / epb;
+  if (nblk <= 0) return SDG_OK;
+  if (nblk > 0x7fffffffLL) return fail(SDG_ERR_INVALID_ARG, "too many elements");
+  SDG_TRY(set_kernel_smem((const void*)stage_fix_kernel<P, EO, RK, FCIN>,
+                          (int)fix_smem<P>(FixShape<P>::EPB), true));
+  stage_fix_kernel<P, EO, RK, FCIN><<<(unsigned)nblk, threads, fix_smem<P>(epb), st>>>(a);
   SDG_CUDA_TRY(cudaGetLastError());
   return SDG_OK;
 }
 
-template <int P>
+template <int P, bool EO>
 int launch_stage_fix_impl(const StageArgs& s, cudaStream_t st) {
-  FixStageArgs<P> a;
+  FixStageArgs<P, EO> a;
   a.s = s;
-  a.c = s.tend_only ? 1.0 : s.b * s.dt;
-  for (int d = 0; d < 3; d++) {
-    // the FP64 lines' factors, without the stage's (which a.c carries)
-    a.s.eo_sD[d] = -s.box.Es[d];
-    a.s.eo_sL[d] = -(0.25 * s.box.Fs[d]);
-  }
-  for (int t = 0; t < 3 * EoShape<P>::TE; t++)
+  a.c = EO ? s.b * s.dt : s.dt;
+  for (int t = 0; t < 3 * a.TAB; t++)
     a.tab[t] = fixlimb{s.fix->coef[2 * t], s.fix->coef[2 * t + 1]};
-  for (int t = 0; t < 3 * EoShape<P>::HR; t++) a.row[t] = s.fix->row[t];
+  for (int t = 0; t < 3 * a.ROWS; t++) a.row[t] = s.fix->row[t];
   a.ok = s.fix->ok;
-  const long long nblk = (s.elem_count + FixShape<P>::EPB - 1) / FixShape<P>::EPB;
-  if (nblk <= 0) return SDG_OK;
-  if (nblk > 0x7fffffffLL) return fail(SDG_ERR_INVALID_ARG, "too many elements");
   const bool in = s.fc_in != nullptr;
   switch (rk_kind(s)) {
-    case kRkTend: return launch_stage_fix_kind<P, kRkTend, false>(a, (unsigned)nblk, st);
+    case kRkTend: return launch_stage_fix_kind<P, EO, kRkTend, false>(a, st);
     case kRkFirst:
-      return in ? launch_stage_fix_kind<P, kRkFirst, true>(a, (unsigned)nblk, st)
-                : launch_stage_fix_kind<P, kRkFirst, false>(a, (unsigned)nblk, st);
-    default: return launch_stage_fix_kind<P, kRkGeneral, true>(a, (unsigned)nblk, st);
+      return in ? launch_stage_fix_kind<P, EO, kRkFirst, true>(a, st)
+                : launch_stage_fix_kind<P, EO, kRkFirst, false>(a, st);
+    default:
+      return in ? launch_stage_fix_kind<P, EO, kRkGeneral, true>(a, st)
+                : launch_stage_fix_kind<P, EO, kRkGeneral, false>(a, st);
   }
 }
 
