@@ -308,17 +308,15 @@ int sdg_rk_stage_dev(double* q, const double* q0, const double* dqdt, int Np,
  * (main.f90:68-73).  Every array has its reference meaning and layout, as in
  * sdg_advect3d_eq_cal_tend_dev, plus halo_src_map (NhaloNode, 1-based) for
  * the halo slots that VMapP points into.
- *   opt SDG_OPT_EVENODD: one fused launch per stage on two scratch state
- *     buffers -- face flux from VMapM / VMapP, normal_fn and Fscale, the
- *     even-odd line sums with the caller's per-node Escale, the lift and the
- *     RK update.  Halo slots are resolved through halo_src_map once per call
- *     instead of being copied every stage; the velocity factors of the face
- *     flux are formed in a step's first stage and reused in its other two.
- *   opt SDG_OPT_OPT1 / SDG_OPT_GENERAL: the reference's sequence and
- *     summation order (q0 copy, halo update, flux, cal_dqdt, RK: 13 launches
- *     a step).
+ * One fused launch per stage on two scratch state buffers: face flux from
+ * VMapM / VMapP, normal_fn and Fscale, the line sums with the caller's Escale
+ * (SDG_OPT_EVENODD the even-odd pairs, SDG_OPT_OPT1 / SDG_OPT_GENERAL operators
+ * as given), the lift and the RK update.  Halo slots are resolved through
+ * halo_src_map and the velocity factors of the face flux formed once per call.
  * scratch: device memory of at least sdg_advect3d_eq_step_scratch_bytes(Nq,
- * Ne) bytes, 256-byte aligned.  Errors found on the device set *err_flag
+ * Ne) bytes, 256-byte aligned.  (Scratch short of that by no more than the
+ * operator tables, the last 48 Nq^3 bytes and some, is taken too: OPT1 / GENERAL
+ * then run the per-stage sequence, 10 launches a step and more.)  Errors found on the device set *err_flag
  * (not cleared here): 1 for a VMapM / VMapP / halo_src_map entry outside the
  * DOFs it may name, 2 for operators without the even-odd symmetries.  On
  * return the halo slots of q hold the final state's halo values.  Runs

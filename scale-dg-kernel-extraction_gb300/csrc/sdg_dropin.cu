@@ -18,8 +18,8 @@ SDG_DECL_DROPIN(9) SDG_DECL_DROPIN(10) SDG_DECL_DROPIN(11) SDG_DECL_DROPIN(12)
 SDG_DECL_DROPIN(13) SDG_DECL_DROPIN(14) SDG_DECL_DROPIN(15)
 #undef SDG_DECL_DROPIN
 
-// what: 0 = cal_dqdt, 1 = divlike, 2 = lift, 3 = gradlike (mod_dg_optr_kernel.f90:87-133
-// and :155-186 select the per-order kernel the same way).
+// what: as dropin_order (mod_dg_optr_kernel.f90:87-133 and :155-186 select the
+// per-order kernel the same way).
 static int dropin(int p, int what, int opt, const void* args, cudaStream_t st) {
   switch (p) {
     case 1: return dropin_p1(what, opt, args, st);
@@ -115,9 +115,44 @@ __global__ void flux_kernel(const TendArgs a, int NfpTot) {
   }
 }
 
+// One tendency: the tables of step_ref_kernel in the flux scratch (its fluxes
+// stay in registers), then the kernel.  GENERAL and OPT1 keep the flux kernel
+// and the FP64 cal_dqdt kernel where the scratch does not hold the tables, and
+// on small meshes, where the time is the latency of one block and a line kernel
+// waits longer than a node kernel.  Measured per call (fixed point / FP64): at
+// p = 7 22.7 / 16.5 us at 64k DOF, 22.9 / 26.8 at 175k, 105 / 186 at 2.1M; p = 3
+// 16.6 / 12.5 at 64k, 20.7 / 22.7 at 175k, 120 / 169 at 1.9M; p = 11 35 / 35 at
+// 110k; p = 15 44 / 82 at 110k.
 int tend_dev(const TendArgs& a, int p, int NfpTot, int opt, cudaStream_t st) {
   if (a.Ne == 0) return SDG_OK;
   const long long NT = (long long)NfpTot * a.Ne;
+  size_t need[2] = {0, 0};
+  SDG_TRY(dropin(p, 6, opt, need, st));
+  const uintptr_t at = (reinterpret_cast<uintptr_t>(a.flux) + 15) & ~uintptr_t(15);
+  const uintptr_t end = reinterpret_cast<uintptr_t>(a.flux + NT);
+  const long long dof = (long long)(p + 1) * (p + 1) * (p + 1) * a.Ne;
+  if (at + need[0] <= end && (opt == SDG_OPT_EVENODD || dof >= 160000 || p >= 12)) {
+    RefArgs r{};
+    r.q_in = a.q;
+    r.out = a.dqdt;
+    r.u = a.u;
+    r.v = a.v;
+    r.w = a.w;
+    r.D = a.D;
+    r.Dt = a.Dt;
+    r.Lift = a.Lift;
+    r.VMapM = a.VMapM;
+    r.VMapP = a.VMapP;
+    r.normal_fn = a.normal_fn;
+    r.Fscale = a.Fscale;
+    r.err = a.err;
+    r.NpNeA = a.NpNeA;
+    r.Escale = a.Escale;
+    r.Ne = a.Ne;
+    RefCall c{&r, kRkTend, reinterpret_cast<void*>(at), (size_t)(end - at)};
+    SDG_TRY(dropin(p, 5, opt, &c, st));
+    return dropin(p, 4, opt, &c, st);
+  }
   long long nb = (NT + 255) / 256;
   if (nb > 152LL * 64) nb = 152LL * 64;
   flux_kernel<<<(unsigned)nb, 256, 0, st>>>(a, NfpTot);
@@ -156,8 +191,9 @@ __global__ void rk_kernel(double* q, const double* q0, const double* dqdt,
 
 // Once per call, one thread per face node m: the owned nodes its qM and qP
 // come from (VMapM(m), VMapP(m), a halo slot b followed through
-// halo_src_map(b)) and the velocity factors (tP, tM) of its flux from the
-// caller's velocity at VMapM / VMapP, normal_fn and Fscale.  An entry out of
+// halo_src_map(b)) and the velocity factors of its flux qP tP - qM tM from the
+// caller's velocity at VMapM / VMapP, normal_fn and Fscale: (tP, tM), or with
+// `jump` (tP - tM, tM).  An entry out of
 // range sets *err = 1 and gives the face node a zero flux.
 __global__ void step_face_kernel(const int* __restrict__ VMapM, const int* __restrict__ VMapP,
                                  const int* __restrict__ halo_src_map,
@@ -166,7 +202,7 @@ __global__ void step_face_kernel(const int* __restrict__ VMapM, const int* __res
                                  const double* __restrict__ normal_fn,
                                  const double* __restrict__ Fscale, int2* res, double2* fc,
                                  long long NT, long long NpNe, long long NpNeA,
-                                 long long NhaloNode, int* err) {
+                                 long long NhaloNode, int jump, int* err) {
   for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < NT;
        m += (long long)gridDim.x * blockDim.x) {
     const long long vM = (long long)VMapM[m] - 1, vP = (long long)VMapP[m] - 1;
@@ -189,7 +225,7 @@ __global__ void step_face_kernel(const int* __restrict__ VMapM, const int* __res
     const double velP = u[vP] * n1 + v[vP] * n2 + w[vP] * n3;
     const double alpha = 0.5 * fabs(velP + velM);
     const double hf = 0.5 * Fscale[m];
-    fc[m] = make_double2(hf * (velP - alpha), hf * (velM - alpha));
+    fc[m] = make_double2(hf * (jump ? velP - velM : velP - alpha), hf * (velM - alpha));
   }
 }
 
@@ -535,18 +571,28 @@ int sdg_rk_stage_dev(double* q, const double* q0, const double* dqdt, int Np,
 // ---- the time loop on the reference's arrays ---------------------------------
 
 // Scratch of sdg_advect3d_eq_step_dev, 256-byte aligned pieces: two stage
-// states (Np*Ne), the face factors (tP, tM) per face node, the resolved
-// gather indices (M, P) per face node, the even-odd tables, and per element
-// its Escale when that is one value per direction.
-static size_t step_layout(int Nq, long long Ne, size_t off[6]) {
+// states (Np*Ne), the face factors per face node, the resolved gather indices
+// (M, P) per face node, per element its Escale when that is one value per
+// direction (in a piece that also holds the even-odd tables without the shared
+// coefficients), and the whole tables of either kind.  `least` receives the
+// size without the last piece, all that earlier versions asked for: with less
+// than the whole, EVENODD keeps its tables in the fifth piece and its stages
+// read Escale themselves, GENERAL and OPT1 run the per-stage sequence.
+static size_t step_layout(int Nq, long long Ne, size_t off[6], size_t* least) {
   const long long np = (long long)Nq * Nq * Nq, nft = 6LL * Nq * Nq * Ne;
   const int N = Nq, H = N / 2, HR = (N + 1) / 2;
   const long long te = (long long)H * H + (long long)HR * H + (N & 1) * H + HR + H;
+  size_t eo[2] = {0, 0}, general[2] = {0, 0};
+  dropin(Nq - 1, 6, SDG_OPT_EVENODD, eo, nullptr);
+  dropin(Nq - 1, 6, SDG_OPT_GENERAL, general, nullptr);
   const size_t sizes[6] = {(size_t)(8 * np * Ne), (size_t)(8 * np * Ne), (size_t)(16 * nft),
-                           (size_t)(8 * nft), (size_t)(8 * 3 * te), (size_t)(32 * Ne)};
+                           (size_t)(8 * nft),
+                           (((size_t)(8 * 3 * te) + 255) & ~size_t(255)) + (size_t)(32 * Ne),
+                           eo[1] > general[1] ? eo[1] : general[1]};
   size_t total = 0;
   for (int k = 0; k < 6; k++) {
     off[k] = total;
+    if (k == 5) *least = total;
     total += (sizes[k] + 255) & ~size_t(255);
   }
   return total;
@@ -554,8 +600,8 @@ static size_t step_layout(int Nq, long long Ne, size_t off[6]) {
 
 size_t sdg_advect3d_eq_step_scratch_bytes(int Nq, int Ne) {
   if (Nq - 1 < 1 || Nq - 1 > kMaxOrder || Ne < 0) return 0;
-  size_t off[6];
-  return step_layout(Nq, Ne, off);
+  size_t off[6], least;
+  return step_layout(Nq, Ne, off, &least);
 }
 
 int sdg_advect3d_eq_step_dev(double* q, const double* u, const double* v, const double* w,
@@ -576,9 +622,9 @@ int sdg_advect3d_eq_step_dev(double* q, const double* u, const double* v, const 
   if ((long long)Np * NeA > 0x7fffffffLL)
     return fail(SDG_ERR_INVALID_ARG, "Np*NeA beyond the 32-bit DOF ids of VMapM/VMapP");
   if (Ne == 0 || nstep == 0) return SDG_OK;
-  size_t off[6];
-  const size_t need = step_layout(Nq, Ne, off);
-  if (!scratch || scratch_bytes < need)
+  size_t off[6], least = 0;
+  const size_t need = step_layout(Nq, Ne, off, &least);
+  if (!scratch || scratch_bytes < least)
     return fail(SDG_ERR_INVALID_ARG, "scratch of %zu bytes, %zu needed "
                 "(sdg_advect3d_eq_step_scratch_bytes)", scratch_bytes, need);
   if (!q || !u || !v || !w || !D1D || !D1D_tr || !Lift_mat || !VMapM || !VMapP ||
@@ -593,9 +639,9 @@ int sdg_advect3d_eq_step_dev(double* q, const double* u, const double* v, const 
   const long long np = Np, nft = (long long)NfpTot * Ne, npne = np * Ne;
   const int p = Nq - 1;
 
-  if (opt != SDG_OPT_EVENODD) {
-    // the reference's own sequence and summation order: q0 = q, then per
-    // stage update_halo(q), cal_tend into dqdt, the RK update (main.f90:51-80)
+  if (opt != SDG_OPT_EVENODD && scratch_bytes < need) {
+    // the reference's own sequence: q0 = q, then per stage update_halo(q),
+    // cal_tend into dqdt, the RK update (main.f90:51-80)
     double* flux = reinterpret_cast<double*>(base + off[2]);
     TendArgs ta{qC, q, u, v, w, D1D, D1D_tr, Lift_mat, VMapM, VMapP, normal_fn,
                 Escale, Fscale, flux, err_flag, Ne, np * NeA};
@@ -622,30 +668,37 @@ int sdg_advect3d_eq_step_dev(double* q, const double* u, const double* v, const 
     return SDG_OK;
   }
 
-  // even-odd: the per-call face data, then one fused launch per stage on
+  // the per-call tables and face data, then one fused launch per stage on
   // ping-pong buffers
+  const bool eo = opt == SDG_OPT_EVENODD;
   double2* fc = reinterpret_cast<double2*>(base + off[2]);
   int2* res = reinterpret_cast<int2*>(base + off[3]);
-  double* tab = reinterpret_cast<double*>(base + off[4]);
-  double4* esu = reinterpret_cast<double4*>(base + off[5]);
-  StepTablesArgs tb{D1D, D1D_tr, Lift_mat, tab, err_flag};
-  SDG_TRY(dropin(p, 5, opt, &tb, st));
-  step_face_kernel<<<grid_for(nft), 256, 0, st>>>(VMapM, VMapP, halo_src_map, u, v, w,
-                                                  normal_fn, Fscale, res, fc, nft, npne,
-                                                  np * NeA, NhaloNode, err_flag);
-  SDG_CUDA_TRY(cudaGetLastError());
-  step_escale_kernel<<<grid_for(32LL * Ne), 256, 0, st>>>(Escale, esu, Ne, Np);
-  SDG_CUDA_TRY(cudaGetLastError());
-  StepRefArgs a{};
-  a.esu = esu;
+  RefArgs a{};
   a.u = u;
   a.v = v;
   a.w = w;
-  a.tab = tab;
+  a.D = D1D;
+  a.Dt = D1D_tr;
+  a.Lift = Lift_mat;
+  a.err = err_flag;
   a.res = res;
   a.fc = fc;
   a.Escale = Escale;
   a.Ne = Ne;
+  a.dt = dt;
+  const bool whole = scratch_bytes >= need;
+  RefCall call{&a, 0, base + off[whole ? 5 : 4], whole ? need - off[5] : off[5] - off[4]};
+  SDG_TRY(dropin(p, 5, opt, &call, st));
+  if (whole) {
+    double4* esu = reinterpret_cast<double4*>(base + off[4]);
+    step_escale_kernel<<<grid_for(32LL * Ne), 256, 0, st>>>(Escale, esu, Ne, Np);
+    SDG_CUDA_TRY(cudaGetLastError());
+    a.esu = esu;
+  }
+  step_face_kernel<<<grid_for(nft), 256, 0, st>>>(VMapM, VMapP, halo_src_map, u, v, w,
+                                                  normal_fn, Fscale, res, fc, nft, npne,
+                                                  np * NeA, NhaloNode, eo ? 0 : 1, err_flag);
+  SDG_CUDA_TRY(cudaGetLastError());
   for (int s = 0; s < nstep; s++) {
     // stage 1: q -> B; 2: B, q0 = q -> C; 3: C, q0 = q -> q
     const double* ins[3] = {q, qB, qC};
@@ -653,12 +706,11 @@ int sdg_advect3d_eq_step_dev(double* q, const double* u, const double* v, const 
     for (int stage = 0; stage < 3; stage++) {
       a.q_in = ins[stage];
       a.q0 = q;
-      a.q_out = outs[stage];
+      a.out = outs[stage];
       a.a = rk_a[stage];
       a.b = rk_b[stage];
-      a.c = -rk_b[stage] * dt;
-      a.rk = stage == 0 ? kRkFirst : kRkGeneral;
-      SDG_TRY(dropin(p, 4, opt, &a, st));
+      call.mode = stage == 0 ? kRkFirst : kRkGeneral;
+      SDG_TRY(dropin(p, 4, opt, &call, st));
     }
   }
   // leave the halo slots of q consistent with the final state

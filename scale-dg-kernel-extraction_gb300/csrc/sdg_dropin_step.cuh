@@ -1,89 +1,155 @@
-// Fused SSP-RK3 stage for meshes given as the reference's arrays: the time
-// loop of main.f90:51-80 (q0 = q; per stage update_halo(q),
-// advect3d_eq_cal_tend (mod_advect3d_eq.f90:41-85), RK update) in one launch
-// per stage, with the even-odd line sums of the fused structured stage.
+// The tendency and the SSP-RK3 stages for meshes given as the reference's
+// arrays, with the line sums in fixed point (sdg_fix.cuh, sdg_stage_fix.cuh).
 //
-// What the caller's arrays decide, and how they are honoured:
+// One kernel serves advect3d_eq_cal_tend (mod_advect3d_eq.f90:41-85; MODE
+// kRkTend) and the time loop of main.f90:51-80 (per stage update_halo,
+// cal_tend and the RK update in one launch; the other MODEs).  What the
+// caller's arrays decide, and how they are honoured:
 //   * VMapM / VMapP (1-based flat DOF ids, halo slots for periodic
-//     neighbours): resolved once per call through halo_src_map to the owned
-//     node each one reads (step_face_kernel), so the stages gather q from
-//     the owned part of the previous stage's state -- the value update_halo
-//     would have copied into the slot -- and need no halo copy of their own.
-//     The velocity gathers use VMapM / VMapP as given (the caller's u, v, w
-//     halos), as cal_elembnd_flux does;
-//   * normal_fn and Fscale: the face flux
-//       0.5 Fs ((qP VelP - qM VelM) - alpha (qP - qM)),  Vel = u.n,
-//       alpha = 0.5 |VelP + VelM|  (mod_advect3d_eq.f90:116-140)
-//     is formed as qP tP - qM tM with tP = 0.5 Fs (VelP - alpha) and
-//     tM = 0.5 Fs (VelM - alpha).  tP and tM depend only on the velocity and
-//     the geometry, which every stage of the loop shares (main.f90:58-67
-//     passes the same u, v, w each time and never changes them), so
-//     step_face_kernel forms them once per call and every stage reads them;
-//   * Escale (per node, per direction): applied to each direction's
-//     derivative sum before the lift is added, as cal_dqdt does
-//     (mod_advect3d_eq.f90:185-198).  Where an element's Escale is one value
-//     per direction (mesh_setup's affine elements, mod_mesh.f90:147-149;
-//     step_escale_kernel checks every node once per call) the value is
-//     folded into that element's copy of the derivative tables instead, and
-//     its lines run the structured stage's body (eo_line); elements with
-//     Escale varying node by node keep the per-node form (eo_line_esc).
-// The summation order is the even-odd one of dqdt_eo_kernel: neither
-// GENERAL's nor OPT1's, equal to both to rounding.
+//     neighbours), normal_fn and Fscale: a tendency gathers q, u, v, w through
+//     them, range-checked, and forms the flux as cal_elembnd_flux does
+//     (mod_advect3d_eq.f90:116-140).  In the time loop step_face_kernel
+//     resolves them once per call to the owned node each entry reads (the
+//     value update_halo would have copied into the slot) and to the velocity
+//     factors of the flux, which every stage of the loop shares (main.f90:58-67
+//     passes the same u, v, w each time);
+//   * Escale (per node, per direction): where an element's is one value per
+//     direction over all its nodes (mesh_setup's affine elements,
+//     mod_mesh.f90:147-149), its significand is folded into the element's copy
+//     of the derivative coefficients and its exponent into the line's (the
+//     faces aligned against it); the lines of other elements are formed in FP64, Escale applied per node
+//     before the lift is added (mod_advect3d_eq.f90:185-198).
+//
+// EO: coefficients of the even-odd pairs, for operators with the symmetries
+// (type EVENODD); else rows of D1D (x) and D1D_tr (y, z) as given and every
+// node's lift entries (GENERAL, OPT1).
+//
+// Measured on GB300 at about 7M DOF against the FP64 kernels this replaced
+// (GDOF-updates/s): the time loop at p = 7 42.0 from 18.2 (EVENODD) and 35.2
+// from 10.7 (OPT1), p = 3 38.9 / 34.6 from 19.1 / 10.7, p = 15 34.4 / 22.3 from
+// 13.1 / 6.8; the per-stage calls 19.9 from 10.6 at p = 7.  A stage is bound by
+// the latency of its gathers and loads (long-scoreboard stalls 6.5 of 17 cycles
+// an instruction, 32 warps an SM) with the FP64 pipe 44-60 % busy; a tendency,
+// which gathers 14 values a face node, by them alone (the FP64 pipe 44 %).
 #pragma once
 
-#include "sdg_stage.cuh"
 #include "sdg_stage_eo.cuh"
+#include "sdg_stage_fix.cuh"
 
 namespace sdg {
 
-struct StepRefArgs {
-  const double* q_in;   // stage input state, owned part (Np*Ne)
+struct RefArgs {
+  const double* q_in;   // state (the tendency's with halos)
   const double* q0;     // step-start state (stages 2 and 3)
-  double* q_out;        // stage result (Np*Ne); may be q0 in the third stage
-  const double* u;      // caller's velocity with halos (Np*NeA)
+  double* out;          // dqdt, or the stage result (may be q0 in the third)
+  const double* u;      // caller's velocity
   const double* v;
   const double* w;
-  const double* tab;    // 3 x TE unscaled even-odd tables (step_tables_kernel)
-  const int2* res;      // per face node: the 0-based owned nodes qM and qP come
-                        //   from (-1: a map entry was out of range)
-  const double2* fc;    // per face node: the velocity factors (tP, tM)
+  const double* D;      // operators as given
+  const double* Dt;
+  const double* Lift;
+  // tables (ref_tables_kernel): rows of coefficients times 2^-row, the rows'
+  // exponents (kRefBadRow: out of range), the nodes' lift limbs (not EO)
+  const double* tab;
+  const int* row;
+  const int4* lift;
+  // faces of a tendency
+  const int* VMapM;
+  const int* VMapP;
+  const double* normal_fn;
+  const double* Fscale;
+  int* err;             // set to 1 on an out-of-range VMap entry
+  long long NpNeA;      // valid 1-based indices are 1..NpNeA
+  // faces of the time loop: the 0-based owned nodes qM and qP come from (-1: a
+  // map entry was out of range), and the velocity factors
+  const int2* res;
+  const double2* fc;
   const double* Escale;
-  const double4* esu;   // per element: (Es_x, Es_y, Es_z, 1) when its Escale is
-                        //   one value per direction, (.., 0) otherwise
+  // coefficients for the Escale of the mesh's first node (null: not built), and
+  // in the time loop per element (Es_x, Es_y, Es_z, 1) when its Escale is one
+  // value per direction, (.., 0) otherwise (null: read Escale)
+  const fixlimb* shared;
+  const double4* esu;
   int Ne;
-  double a, b, c;       // q_out = a q0 + b q_in + c S, c = -b dt, S = -dqdt
-                        // (the tables are scaled by c)
-  int rk;               // kRkFirst or kRkGeneral
+  double a, b, dt;      // q_out = a q0 + b (q + dt dqdt)
 };
 
-template <int P>
-struct StepRefCfg {
-  static constexpr int THREADS = 256;
-  static constexpr int EPB = (256 / Ord<P>::NQ2) > 0 ? 256 / Ord<P>::NQ2 : 1;
+constexpr int kRefBadRow = 1 << 20;
+
+template <int P, bool EO>
+struct RefShape {
+  static constexpr int N = P + 1;
+  static constexpr int TAB = EO ? EoShape<P>::TE : N * N;
+  static constexpr int ROWS = EO ? EoShape<P>::HR : N;
+  // bytes of the tables: lift limbs, coefficients, rows (16-byte aligned base)
+  static constexpr size_t LIFT = EO ? 0 : sizeof(int4) * 3 * N * N * N;
+  static constexpr size_t LEAST = LIFT + sizeof(double) * 3 * TAB + sizeof(int) * 3 * ROWS;
+  // with the coefficients for the first node's Escale
+  static constexpr size_t SHARED = (LEAST + 7) / 8 * 8;
+  static constexpr size_t BYTES = SHARED + sizeof(fixlimb) * 3 * TAB;
+  // a table entry's row, and whether Escale applies to it
+  static __host__ __device__ constexpr int row_of_entry(int w) {
+    using Sh = EoShape<P>;
+    constexpr int H1 = Sh::H;
+    return !EO                 ? w / N
+           : w < Sh::OFF_O     ? w / H1
+           : w < Sh::OFF_DM    ? (w - Sh::OFF_O) / H1
+           : w < Sh::OFF_A     ? w - Sh::OFF_DM
+           : w < Sh::OFF_B     ? w - Sh::OFF_A
+                               : w - Sh::OFF_B;
+  }
+  static __host__ __device__ constexpr bool derivative(int w) { return !EO || w < EoShape<P>::OFF_A; }
+  static __host__ __device__ constexpr int row_of(int m) {
+    return EO ? (m < P - m ? m : P - m) : m;
+  }
 };
 
-template <int P>
-constexpr size_t step_ref_smem_bytes() {
-  using O = Ord<P>;
-  return sizeof(double) * (size_t)(3 * EoShape<P>::TE +
-                                   StepRefCfg<P>::EPB * (O::NP + O::NFT + 3 * EoShape<P>::TE));
+// The exponent of a row whose magnitudes add up to sum (with room for the
+// rounding of the sum and of a coefficient's high limb), kRefBadRow outside +-200.
+__device__ __forceinline__ int ref_row_exp(double sum) {
+  const int e = (int)((unsigned)__double2hiint(sum * (1.0 + 1e-8)) >> 20 & 0x7FFu);
+  if (sum == 0.0) return 0;
+  return e < 1022 - 200 || e > 1022 + 200 ? kRefBadRow : e - 1022;
+}
+__device__ __forceinline__ double ref_pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
+// Escale of a direction: its exponent x (Es = sig 2^x, sig in [0.5, 1)), and
+// sig 2^60.
+__device__ __forceinline__ int ref_escale_exp(double es) {
+  return (int)((unsigned)__double2hiint(es) >> 20 & 0x7FFu) - 1022;
+}
+__device__ __forceinline__ int64_t ref_escale_sig(double es) {
+  return fix_unit(
+      __hiloint2double(__double2hiint(es) - (ref_escale_exp(es) << 20), __double2loint(es)));
+}
+// The limbs of a table entry (its minus sign is dqdt's), a derivative entry
+// with the significand of Escale.
+__device__ __forceinline__ fixlimb ref_coef(double entry, bool derivative, int64_t sig) {
+  const int64_t c = fix_unit(entry);
+  return fix_coef(derivative ? -fix_times(c, sig) : -c);
 }
 
 // The three directions' unscaled even-odd tables from D1D and Lift_mat (the
-// lift column of a face from its tangential node (0, 0)), one block; it
-// checks the symmetries the factorisation needs -- D1D centro-antisymmetric,
-// D1D_tr its transpose, each face's lift constant over the tangential nodes,
-// the + face's column the mirror of the - face's, all to 1e-13 of the largest
-// entry -- and sets *err = 2 when one fails.
+// lift column of a face from its tangential node (0, 0)) with their row scales,
+// and (shared not null) the coefficients for the Escale of the mesh's first
+// node, one block; it checks the symmetries the factorisation needs -- D1D
+// centro-antisymmetric, D1D_tr its transpose, each face's lift constant over
+// the tangential nodes, the + face's column the mirror of the - face's, all to
+// 1e-13 of the largest entry -- and sets *err = 2 when one fails.
 template <int P>
-__global__ void __launch_bounds__(256) step_tables_kernel(const double* __restrict__ D,
-                                                          const double* __restrict__ Dt,
-                                                          const double* __restrict__ L,
-                                                          double* tab, int* err) {
+__global__ void __launch_bounds__(256) ref_tables_eo_kernel(const double* __restrict__ D,
+                                                            const double* __restrict__ Dt,
+                                                            const double* __restrict__ L,
+                                                            const double* __restrict__ Es,
+                                                            long long NpNe, double* tab, int* row,
+                                                            fixlimb* shared, int* err) {
   using O = Ord<P>;
   using Sh = EoShape<P>;
+  using Rs = RefShape<P, true>;
   constexpr int NQ = O::NQ, NQ2 = O::NQ2, NP = O::NP, TE = Sh::TE, N = Sh::N, H = Sh::H;
   __shared__ unsigned long long smax[2];
+  __shared__ double sT[3 * TE];
+  __shared__ int sRow[3 * Sh::HR];
   auto Dv = [&](int i, int l) { return D[i + l * N]; };  // D1D(i,l), column-major
   auto Ds = [&](int i, int l) { return 0.5 * (Dv(i, l) - Dv(N - 1 - i, N - 1 - l)); };
   auto node = [](int ax, int m, int t1, int t2) {
@@ -97,26 +163,38 @@ __global__ void __launch_bounds__(256) step_tables_kernel(const double* __restri
   auto lam = [&](int ax, int m) { return 0.5 * (col(ax, 0, m) + col(ax, 1, N - 1 - m)); };
   for (int t = threadIdx.x; t < 3 * TE; t += blockDim.x) {
     const int ax = t / TE, w = t - ax * TE;
+    const int i = Rs::row_of_entry(w);
     double v;
     if (w < Sh::OFF_O) {
-      const int i = w / H, l = w - i * H;
+      const int l = w - i * H;
       v = 0.5 * (Ds(i, l) + Ds(i, N - 1 - l));
     } else if (w < Sh::OFF_DM) {
-      const int i = (w - Sh::OFF_O) / H, l = (w - Sh::OFF_O) - i * H;
+      const int l = (w - Sh::OFF_O) - i * H;
       v = 0.5 * (Ds(i, l) - Ds(i, N - 1 - l));
     } else if (w < Sh::OFF_A) {
-      v = Ds(w - Sh::OFF_DM, H);
+      v = Ds(i, H);
     } else if (w < Sh::OFF_B) {
-      const int i = w - Sh::OFF_A;
       v = 0.5 * (lam(ax, i) + lam(ax, N - 1 - i));
     } else {
-      const int i = w - Sh::OFF_B;
       v = 0.5 * (lam(ax, i) - lam(ax, N - 1 - i));
     }
-    tab[t] = v;
+    sT[t] = v;
   }
   if (threadIdx.x == 0) smax[0] = smax[1] = 0ull;
   __syncthreads();
+  for (int t = threadIdx.x; t < 3 * Sh::HR; t += blockDim.x) {
+    const double* T = sT + (t / Sh::HR) * TE;
+    const int i = t % Sh::HR;
+    // what the row's two outputs can reach on values and faces below one
+    auto pair = [&](int e, int o) {
+      // (0 * x keeps a NaN that fmax would drop)
+      return 2.0 * fmax(i < H ? fabs(T[e]) : 0.0, fabs(T[o])) + 0.0 * (T[e] + T[o]);
+    };
+    double most = pair(i < H ? Sh::OFF_B + i : Sh::OFF_A + i, Sh::OFF_A + i);
+    for (int l = 0; l < H; l++) most += pair(Sh::OFF_E + i * H + l, Sh::OFF_O + i * H + l);
+    if (i < H && Sh::ODD) most += fabs(T[Sh::OFF_DM + i]);
+    row[t] = sRow[t] = ref_row_exp(most);
+  }
   unsigned long long mD = 0, mL = 0;
   for (int t = threadIdx.x; t < NQ2; t += blockDim.x)
     mD = max(mD, (unsigned long long)__double_as_longlong(fabs(D[t])));
@@ -125,6 +203,13 @@ __global__ void __launch_bounds__(256) step_tables_kernel(const double* __restri
   atomicMax(&smax[0], mD);
   atomicMax(&smax[1], mL);
   __syncthreads();
+  for (int t = threadIdx.x; t < 3 * TE; t += blockDim.x) {
+    const int w = t % TE, k = sRow[t / TE * Sh::HR + Rs::row_of_entry(w)];
+    const double c = k == kRefBadRow ? sT[t] : sT[t] * ref_pow2(-k);
+    tab[t] = c;
+    if (shared)
+      shared[t] = ref_coef(c, Rs::derivative(w), ref_escale_sig(Es[(t / TE) * NpNe]));
+  }
   const double tD = 1e-13 * __longlong_as_double((long long)smax[0]);
   const double tL = 1e-13 * __longlong_as_double((long long)smax[1]);
   bool bad = false;
@@ -145,172 +230,385 @@ __global__ void __launch_bounds__(256) step_tables_kernel(const double* __restri
   if (bad) atomicExch(err, 2);
 }
 
-// One line in pair form with the caller's per-node Escale: row holds S(l) at
-// l and Δ(l) at N-1-l (l < N/2) and F(mid) for an odd N; T the direction's
-// tables scaled by the stage factor c; gm / gp the line's face fluxes; Es(m)
-// the node's Escale.  emit(m, r) receives r = Es(m) (D F)(m) + lift(m), both
-// times c.  Per output pair: the even and odd sums, e + o and o - e, one
-// product B gd shared by the two lifts (A gs +- B gd) and two FMAs with
-// Escale -- seven FP64 operations beside the sums.
-template <int P, typename EsAt, typename Emit>
-__device__ __forceinline__ void eo_line_esc(const double* row, const double* __restrict__ T,
-                                            double gm, double gp, EsAt&& Es, Emit&& emit) {
+// Operators as given: block (d, i) forms row i of direction d -- its scale over
+// the derivative entries and all its nodes' lift entries, the scaled
+// derivative entries (D1D for x, D1D_tr for y and z), the nodes' lift limbs
+// (-, + face) and the coefficients for the Escale of the mesh's first node.
+template <int P>
+__global__ void __launch_bounds__(256) ref_tables_kernel(const double* __restrict__ D,
+                                                         const double* __restrict__ Dt,
+                                                         const double* __restrict__ L,
+                                                         const double* __restrict__ Es,
+                                                         long long NpNe, double* tab, int* row,
+                                                         int4* lift, fixlimb* shared) {
+  constexpr int N = P + 1, N2 = N * N, NP = N * N2;
+  const int d = blockIdx.x / N, i = blockIdx.x - d * N, r = threadIdx.x;
+  const int fm = d == 0 ? 3 : d == 1 ? 0 : 4, fp = d == 0 ? 1 : d == 1 ? 2 : 5;
+  __shared__ unsigned long long smax;
+  if (r == 0) smax = 0ull;
+  __syncthreads();
+  const int n = d == 0 ? i + N * r : d == 1 ? r % N + N * i + N2 * (r / N) : r + N2 * i;
+  double m = 0.0, p = 0.0;
+  if (r < N2) {
+    m = L[n + fm * NP];
+    p = L[n + fp * NP];
+    atomicMax(&smax, (unsigned long long)__double_as_longlong(fabs(m) + fabs(p)));
+  }
+  __syncthreads();
+  auto Dv = [&](int l) { return d == 0 ? D[i + l * N] : Dt[l + i * N]; };
+  double sum = __longlong_as_double((long long)smax);
+  for (int l = 0; l < N; l++) sum += fabs(Dv(l));
+  const int k = ref_row_exp(sum);
+  if (r == 0) row[blockIdx.x] = k;
+  const double scale = k == kRefBadRow ? 1.0 : ref_pow2(-k);
+  if (r < N) {
+    const double c = Dv(r) * scale;
+    tab[blockIdx.x * N + r] = c;
+    if (shared) shared[blockIdx.x * N + r] = ref_coef(c, true, ref_escale_sig(Es[d * NpNe]));
+  }
+  if (r < N2) {
+    const fixlimb a = fix_coef(-fix_unit(m * scale)), b = fix_coef(-fix_unit(p * scale));
+    lift[(long long)blockIdx.x * N2 + r] = make_int4(a.hi, a.lo, b.hi, b.lo);
+  }
+}
+
+// A line in FP64 with the caller's Escale per node (Es, stride es): F its
+// fluxes (stride fs), out[m] = -(Es(m) (D F)(m) + lift(m)).
+template <int P, bool EO>
+__device__ __noinline__ void ref_line_fp64(const RefArgs* a, int ax, int r, const double* F, int fs,
+                                           double gm, double gp, const double* __restrict__ Es,
+                                           int es, double* out) {
   using Sh = EoShape<P>;
-  constexpr int N = Sh::N, H = Sh::H;
-  double sv[H], dv[H];
+  constexpr int N = Sh::N, H = Sh::H, N2 = N * N, NP = N * N2;
+  if constexpr (!EO) {
+    const int fm = ax == 0 ? 3 : ax == 1 ? 0 : 4, fp = ax == 0 ? 1 : ax == 1 ? 2 : 5;
+    double f[N];
+#pragma unroll
+    for (int l = 0; l < N; l++) f[l] = F[l * fs];
+    const double* __restrict__ D = ax == 0 ? a->D : a->Dt;
+#pragma unroll 1
+    for (int i = 0; i < N; i++) {
+      double s = 0.0;
+#pragma unroll
+      for (int l = 0; l < N; l++) s = fma(ax == 0 ? D[i + l * N] : D[l + i * N], f[l], s);
+      const int n = ax == 0 ? i + N * r : ax == 1 ? r % N + N * i + N2 * (r / N) : r + N2 * i;
+      out[i] = -fma(Es[i * es], s, fma(a->Lift[n + fm * NP], gm, a->Lift[n + fp * NP] * gp));
+    }
+    return;
+  }
+  double s[H], d[H];
 #pragma unroll
   for (int l = 0; l < H; l++) {
-    sv[l] = row[l];
-    dv[l] = row[N - 1 - l];
+    const double f1 = F[l * fs], f2 = F[(N - 1 - l) * fs];
+    s[l] = f1 + f2;
+    d[l] = f1 - f2;
   }
-  double fm = 0.0;
-  if constexpr (Sh::ODD != 0) fm = row[H];
+  const double fmid = Sh::ODD ? F[H * fs] : 0.0;
   const double gs = gm + gp, gd = gm - gp;
-  constexpr int kRowUnroll = (N <= 5) ? H : 1;
-#pragma unroll kRowUnroll
-  for (int i = 0; i < H; i++) {
-    double e = T[Sh::OFF_E + i * H] * sv[0];
+  const double* __restrict__ T = a->tab + ax * Sh::TE;
+#pragma unroll 1
+  for (int i = 0; i < Sh::HR; i++) {
+    const int k = a->row[ax * Sh::HR + i];
+    const double c = k == kRefBadRow ? -1.0 : -ref_pow2(k);
+    double o = T[Sh::OFF_O + i * H] * d[0];
 #pragma unroll
-    for (int l = 1; l < H; l++) e = fma(T[Sh::OFF_E + i * H + l], sv[l], e);
-    if constexpr (Sh::ODD != 0) e = fma(T[Sh::OFF_DM + i], fm, e);
-    double o = T[Sh::OFF_O + i * H] * dv[0];
+    for (int l = 1; l < H; l++) o = fma(T[Sh::OFF_O + i * H + l], d[l], o);
+    const double ag = c * (T[Sh::OFF_A + i] * gs);
+    if (i == H) {
+      out[H] = fma(c * Es[H * es], o, ag);
+      continue;
+    }
+    double e = T[Sh::OFF_E + i * H] * s[0];
 #pragma unroll
-    for (int l = 1; l < H; l++) o = fma(T[Sh::OFF_O + i * H + l], dv[l], o);
-    const double bg = T[Sh::OFF_B + i] * gd, ag = T[Sh::OFF_A + i];
-    emit(i, fma(Es(i), e + o, fma(ag, gs, bg)));
-    emit(N - 1 - i, fma(Es(N - 1 - i), o - e, fma(ag, gs, -bg)));
-  }
-  if constexpr (Sh::ODD != 0) {
-    double o = T[Sh::OFF_O + H * H] * dv[0];
-#pragma unroll
-    for (int l = 1; l < H; l++) o = fma(T[Sh::OFF_O + H * H + l], dv[l], o);
-    emit(H, fma(Es(H), o, T[Sh::OFF_A + H] * gs));
+    for (int l = 1; l < H; l++) e = fma(T[Sh::OFF_E + i * H + l], s[l], e);
+    if (Sh::ODD != 0) e = fma(T[Sh::OFF_DM + i], fmid, e);
+    const double bg = c * (T[Sh::OFF_B + i] * gd);
+    out[i] = fma(c * Es[i * es], o + e, ag + bg);
+    out[N - 1 - i] = fma(c * Es[(N - 1 - i) * es], o - e, ag - bg);
   }
 }
 
-// One stage over elements [blockIdx.x*EPB, ...): the face fluxes from the
-// per-call face data, the even-odd line sums with per-node Escale, the lift
-// and the RK update.  One thread per line in the line phases.
-template <int P, int RK>
-__global__ void __launch_bounds__(StepRefCfg<P>::THREADS, 4) step_ref_kernel(const StepRefArgs a) {
-  using O = Ord<P>;
-  using Sh = EoShape<P>;
-  constexpr int NQ = O::NQ, NQ2 = O::NQ2, NP = O::NP, NFP = O::NFP, NFT = O::NFT,
-                EPB = StepRefCfg<P>::EPB, T = StepRefCfg<P>::THREADS, TE = Sh::TE,
-                H = Sh::H, HR = Sh::HR;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* sT = reinterpret_cast<double*>(smem_raw);  // [3][TE]
-  double* sA = sT + 3 * TE;                          // [EPB][NP]: x pairs, then sums
-  double* sf = sA + EPB * NP;                        // [EPB][NFT] face fluxes
-  double* sTe = sf + EPB * NFT;                      // [EPB][3][TE] per element
-  const long long eb = (long long)blockIdx.x * EPB;
-  const int nloc = (int)min((long long)EPB, (long long)a.Ne - eb);
-  if (nloc <= 0) return;
-  // the tables times the stage factor c = -b dt: the line results are then
-  // the stage's increments, and the RK update needs no multiply of its own;
-  // an element with one Escale per direction gets its own copy with the
-  // derivative parts also times Es_d
-  for (int t = threadIdx.x; t < 3 * TE; t += T) sT[t] = a.tab[t] * a.c;
-  for (int t = threadIdx.x; t < nloc * 3 * TE; t += T) {
-    const int le = t / (3 * TE), w3 = t - le * 3 * TE, dir = w3 / TE, w = w3 - dir * TE;
-    const double4 es = a.esu[eb + le];
-    const double sd = (dir == 0) ? es.x : (dir == 1) ? es.y : es.z;
-    sTe[t] = (w < Sh::OFF_A) ? a.tab[w3] * (a.c * sd) : a.tab[w3] * a.c;
+// u . n with the components whose normal entry is a zero left out: the same
+// value, as long as those components are finite, for two of three FP64
+// operations a side on the axis-aligned normals of mesh_setup.
+__device__ __forceinline__ double ref_normal_velocity(double u, double v, double w, double n1,
+                                                      double n2, double n3, int axis) {
+  if (axis == 0) return u * n1;
+  if (axis == 1) return v * n2;
+  if (axis == 2) return w * n3;
+  return u * n1 + v * n2 + w * n3;
+}
+
+// Face flux of a tendency at face node m with map entries at
+// (cal_elembnd_flux, mod_advect3d_eq.f90:116-140).
+__device__ __forceinline__ double ref_flux(const RefArgs& a, long long m, long long NT, int2 at) {
+  // 1..NpNeA, which a map entry's 31 bits bound as well
+  const unsigned iM = (unsigned)at.x - 1u, iP = (unsigned)at.y - 1u;
+  const unsigned lim = a.NpNeA < 0x7fffffffLL ? (unsigned)a.NpNeA : 0x7fffffffu;
+  if (iM >= lim || iP >= lim) {
+    atomicExch(a.err, 1);
+    return 0.0;
   }
-  const long long g0 = eb * NP;
+  const double n1 = a.normal_fn[m], n2 = a.normal_fn[m + NT], n3 = a.normal_fn[m + 2 * NT];
+  const double qM = a.q_in[iM], qP = a.q_in[iP];
+  const double uM = a.u[iM], vM = a.v[iM], wM = a.w[iM], uP = a.u[iP], vP = a.v[iP],
+               wP = a.w[iP];
+  auto zero = [](double x) { return (__double2hiint(x) << 1 | __double2loint(x)) == 0; };
+  auto exp = [](double x) { return (unsigned)__double2hiint(x) & 0x7FF00000u; };
+  const bool z1 = zero(n1), z2 = zero(n2), z3 = zero(n3);
+  const unsigned top = max(max(max(exp(uM), exp(vM)), max(exp(wM), exp(uP))),
+                           max(exp(vP), exp(wP)));
+  const int axis = top == 0x7FF00000u ? 3 : z2 && z3 ? 0 : z1 && z3 ? 1 : z1 && z2 ? 2 : 3;
+  const double VelM = ref_normal_velocity(uM, vM, wM, n1, n2, n3, axis);
+  const double VelP = ref_normal_velocity(uP, vP, wP, n1, n2, n3, axis);
+  const double alpha = 0.5 * fabs(VelP + VelM);
+  return (0.5 * a.Fscale[m]) * ((qP * VelP - qM * VelM) - alpha * (qP - qM));
+}
+
+template <int P, bool EO>
+__host__ __device__ constexpr size_t ref_smem(int epb) {
+  return sizeof(double) * 2 * epb * FixShape<P>::EW +
+         sizeof(fixlimb) * 3 * epb * RefShape<P, EO>::TAB +
+         sizeof(short) * 2 * epb * FixShape<P>::N2;
+}
+
+// The line of direction AX held in shared memory with stride S, its results
+// over it; returns its exponent.  T: the element's coefficients of the
+// direction, xe: the exponent of its Escale, ok: they are usable.
+template <int P, bool EO, int AX, int S, int ES>
+__device__ __forceinline__ int ref_line_shared(const RefArgs& a, const fixlimb* T, int xe, bool ok,
+                                               int r, double* line, double gm, double gp,
+                                               const double* Es) {
+  constexpr int N = P + 1;
+  double F[N];
+  int32_t E = max(0, max(fix_value_exp(gm), fix_value_exp(gp)) - (xe << 20));
+#pragma unroll
+  for (int l = 0; l < N; l++) {
+    F[l] = line[l * S];
+    E = max(E, fix_value_exp(F[l]));
+  }
+  if (ok && fix_in_range(E)) {
+    int64_t* out = reinterpret_cast<int64_t*>(line);
+    const int32_t Ef = E + (xe << 20);
+    fix_line<P, EO>(T, EO ? nullptr : a.lift + AX * N * N * N + r, F, E, fix_align(gm, Ef),
+                    fix_align(gp, Ef), [&](int m, int64_t v) { out[m * S] = v; });
+    return fix_line_exp(E) + xe;
+  }
+  double out[N];
+  ref_line_fp64<P, EO>(&a, AX, r, line, S, gm, gp, Es, ES, out);
+  for (int m = 0; m < N; m++) line[m * S] = out[m];
+  return kFixDouble;
+}
+
+template <int P, bool EO>
+__host__ __device__ constexpr int ref_min_blocks() {
+  return P >= 12 ? 3 : 1024 / FixShape<P>::THREADS;
+}
+
+// MODE kRkTend: dqdt of elements [blockIdx.x*epb, ...); kRkFirst, kRkGeneral:
+// one stage of the time loop.  Thread layout as stage_fix_kernel.
+template <int P, bool EO, int MODE>
+__global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
+    step_ref_kernel(const __grid_constant__ RefArgs a) {
+  using Sh = FixShape<P>;
+  using Rs = RefShape<P, EO>;
+  constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NFT = 6 * N2, NS = Sh::NS, EW = Sh::EW,
+                TAB = Rs::TAB, ROWS = Rs::ROWS;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int sMix[FixShape<P>::EPB];  // elements whose lines go in FP64
+  const int epb = blockDim.x / N2;
+  const long long eb = (long long)blockIdx.x * epb;
+  const long long left = (long long)a.Ne - eb;
+  const int nloc = (int)(left < epb ? left : epb);
+  const int le = threadIdx.x / N2, r = threadIdx.x - le * N2;
+  const bool on = le < nloc;
+  const int i = r % N, j = r / N;
+  double* sX = reinterpret_cast<double*>(smem_raw) + le * EW;
+  double* sY = sX + epb * EW;
+  fixlimb* sT0 = reinterpret_cast<fixlimb*>(reinterpret_cast<double*>(smem_raw) + 2 * epb * EW);
+  fixlimb* sT = sT0 + le * 3 * TAB;
+  short* sEx = reinterpret_cast<short*>(sT0 + 3 * epb * TAB) + le * N2;
+  short* sEy = sEx + epb * N2;
+  const long long e = eb + le, ge = e * NP, NpNe = (long long)NP * a.Ne;
   const double* __restrict__ q = a.q_in;
-  const double* __restrict__ gu = a.u;
-  // x pair values: one task per (element, x line, c < ceil(N/2))
-  for (int t = threadIdx.x; t < nloc * NQ2 * HR; t += T) {
-    const int le = t / (NQ2 * HR), w = t - le * NQ2 * HR;
-    const int r = w / HR, c = w - r * HR;
-    const long long g = g0 + (long long)le * NP + (long long)r * NQ;
-    double* row = sA + le * NP + r * NQ;
-    if (c < H) {
-      const double q1 = q[g + c], u1 = gu[g + c];
-      const double p2 = q[g + NQ - 1 - c] * gu[g + NQ - 1 - c];
-      row[c] = fma(q1, u1, p2);
-      row[NQ - 1 - c] = fma(q1, u1, -p2);
+  const double* __restrict__ Es = a.Escale;
+  const int zat = i + NS * j;
+
+  if (threadIdx.x < nloc) sMix[threadIdx.x] = 0;
+  __syncthreads();
+  // 0: the z line's x and y fluxes, the element's coefficients, the face fluxes
+  double g[6];
+  int xe[3] = {0, 0, 0};
+  if (on) {
+    // the gathers wait for these: first
+    int2 at[6];
+    const long long NT = (long long)NFT * a.Ne;
+#pragma unroll
+    for (int f = 0; f < 6; f++) {
+      const long long m = e * NFT + f * N2 + r;
+      at[f] = MODE == kRkTend ? make_int2(a.VMapM[m], a.VMapP[m]) : a.res[m];
+    }
+    for (int t = 16 * r; t < NP; t += 16 * N2) {
+      prefetch_l2(a.w + ge + t);
+      if constexpr (MODE == kRkGeneral) prefetch_l2(a.q0 + ge + t);
+    }
+    bool mix = false;
+    double es[3];
+    if (MODE == kRkTend || a.esu == nullptr) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        es[d] = Es[ge + d * NpNe];
+#pragma unroll
+        for (int m = 0; m < N; m++)
+          mix |= __double_as_longlong(Es[ge + r + m * N2 + d * NpNe]) != __double_as_longlong(es[d]);
+      }
     } else {
-      row[c] = q[g + c] * gu[g + c];
+      const double4 x = a.esu[e];
+      es[0] = x.x;
+      es[1] = x.y;
+      es[2] = x.z;
+      mix = __double2hiint(x.w) == 0;
+    }
+    bool same = a.shared != nullptr;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      xe[d] = ref_escale_exp(es[d]);
+      mix |= xe[d] < -150 || xe[d] > 150;
+      same = same && __double_as_longlong(es[d]) == __double_as_longlong(Es[d * NpNe]);
+    }
+    for (int t = r; t < 3 * ROWS; t += N2) mix |= a.row[t] == kRefBadRow;
+    if (mix) sMix[le] = 1;
+#pragma unroll
+    for (int m = 0; m < N; m++) {
+      const double qv = q[ge + r + m * N2];
+      sX[zat + m * NS * N] = qv * a.u[ge + r + m * N2];
+      sY[zat + m * NS * N] = qv * a.v[ge + r + m * N2];
+    }
+    if (same) {
+      for (int t = r; t < 3 * TAB; t += N2) sT[t] = a.shared[t];
+    } else {
+      for (int t = r; t < 3 * TAB; t += N2) {
+        const int d = t / TAB, w = t - d * TAB;
+        sT[t] = ref_coef(a.tab[t], Rs::derivative(w),
+                         ref_escale_sig(d == 0 ? es[0] : d == 1 ? es[1] : es[2]));
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < 6; f++) {
+      const long long m = e * NFT + f * N2 + r;
+      if constexpr (MODE == kRkTend) {
+        g[f] = ref_flux(a, m, NT, at[f]);
+      } else {
+        const double2 fc = a.fc[m];
+        g[f] = 0.0;
+        if (at[f].x >= 0) {
+          const double qP = q[at[f].y], qM = q[at[f].x];
+          g[f] = EO ? fma(qP, fc.x, -(qM * fc.y)) : fma(qP, fc.x, (qP - qM) * fc.y);
+        }
+      }
     }
   }
-  // face fluxes qP tP - qM tM
-  for (int t = threadIdx.x; t < nloc * NFT; t += T) {
-    const long long m = eb * NFT + t;
-    const int2 rr = a.res[m];
-    const double2 fc = a.fc[m];
-    sf[t] = (rr.x >= 0) ? fma(q[rr.y], fc.x, -(q[rr.x] * fc.y)) : 0.0;
+  __syncthreads();
+  const bool ok = on && sMix[le] == 0;
+  if (on) {
+    // lines along i (r = j + N k), faces -x (3) and +x (1); along j (r = i + N k),
+    // faces -y (0) and +y (2)
+    sEx[r] = ref_line_shared<P, EO, 0, 1, 1>(a, sT, xe[0], ok, r, sX + NS * r, g[3], g[1],
+                                             Es + ge + N * r);
+    sEy[r] = ref_line_shared<P, EO, 1, NS, N>(a, sT + TAB, xe[1], ok, r, sY + i + NS * N * j, g[0],
+                                              g[2], Es + NpNe + ge + i + j * N2);
+  }
+  // lines along k (r = i + N j), faces -z (4) and +z (5); the node's result
+  double F[N];
+  int32_t E = 0;
+  if (on) {
+    E = max(0, max(fix_value_exp(g[4]), fix_value_exp(g[5])) - (xe[2] << 20));
+#pragma unroll
+    for (int m = 0; m < N; m++) {
+      F[m] = q[ge + r + m * N2] * a.w[ge + r + m * N2];
+      E = max(E, fix_value_exp(F[m]));
+    }
   }
   __syncthreads();
-  const long long NpNe = (long long)NP * a.Ne;
-  const double* __restrict__ Es = a.Escale;
-  const int r = threadIdx.x % NQ2, le = threadIdx.x / NQ2;
-  const bool has_line = threadIdx.x < nloc * NQ2;
-  const double* fl = sf + le * NFT + r;
-  // one Escale per direction for this line's element: the folded tables
-  const bool uni = has_line && a.esu[eb + le].w != 0.0;
-  const double* Te = sTe + le * 3 * TE;
-  // x lines: faces -x (3) and +x (1); Escale_x D F + lift over the pair values
-  if (has_line) {
-    double* row = sA + le * NP + r * NQ;
-    const long long g = g0 + (long long)le * NP + (long long)r * NQ;
-    auto emit = [&](int m, double r) { row[m] = r; };
-    if (uni)
-      eo_line<P, 1, 1, true>(row, Te, fl[3 * NFP], fl[1 * NFP], 0, emit);
-    else
-      eo_line_esc<P>(row, sT, fl[3 * NFP], fl[1 * NFP], [&](int m) { return Es[g + m]; }, emit);
-  }
-  __syncthreads();
-  // y lines: faces -y (0) and +y (2); added into the sums
-  if (has_line) {
-    const int off = le * NP + (r % NQ) + (r / NQ) * NQ2;
-    double row[NQ];
-    eo_pairs_f64<P>(q, a.v, g0 + off, NQ, row);
-    auto emit = [&](int m, double r) { sA[off + m * NQ] += r; };
-    if (uni)
-      eo_line<P, 1, 1, true>(row, Te + TE, fl[0], fl[2 * NFP], 0, emit);
-    else
-      eo_line_esc<P>(row, sT + TE, fl[0], fl[2 * NFP],
-                     [&](int m) { return Es[g0 + off + m * NQ + NpNe]; }, emit);
-  }
-  __syncthreads();
-  // z lines: faces -z (4) and +z (5); finish the node and the RK update
-  if (has_line) {
-    const int off = le * NP + r;
-    double row[NQ];
-    eo_pairs_f64<P>(q, a.w, g0 + off, NQ2, row);
-    double* __restrict__ qout = a.q_out;
-    const double* q0 = a.q0;
-    const double ra = a.a, rb = a.b;
-    auto emit = [&](int m, double r) {
-      const int n = off + m * NQ2;
-      const long long g = g0 + n;
-      // q0 is read before q_out is written at the same node, by this thread
-      // only, so the third stage may write the result over q0
-      qout[g] = rk_combine<RK>(sA[n] + r, q[g], RK == kRkGeneral ? q0[g] : 0.0, ra, rb);
+  if (on) {
+    const double dt = a.dt, ra = a.a, rb = a.b;
+    const bool zok = ok && fix_in_range(E);
+    const int Bz = zok ? fix_line_exp(E) + xe[2] : kFixDouble;
+    const int rx = a.row[Rs::row_of(i)] - 61, ry = a.row[ROWS + Rs::row_of(j)] - 61;
+    const int64_t* iX = reinterpret_cast<const int64_t*>(sX) + zat;
+    const int64_t* iY = reinterpret_cast<const int64_t*>(sY) + zat;
+    // a line in FP64 has doubles whatever its row (a bad row's exponent is large)
+    auto add = [](int line, int row) { return line == kFixDouble ? kFixDouble : line + row; };
+    auto emit = [&](int m, int64_t z) {
+      const double t = fix_node(iX[m * NS * N], add(sEx[j + N * m], rx), iY[m * NS * N],
+                                add(sEy[i + N * m], ry), z,
+                                add(Bz, a.row[2 * ROWS + Rs::row_of(m)] - 61));
+      const long long n = ge + r + m * N2;
+      if constexpr (MODE == kRkTend)
+        a.out[n] = t;
+      else if constexpr (MODE == kRkFirst)
+        a.out[n] = fma(dt, t, q[n]);
+      else
+        // q0 is read before out is written at the same node, by this thread
+        // only, so the third stage may write the result over q0.  The even-odd
+        // type adds b dt t to b q, the others keep the reference's order
+        // (main.f90:69-73)
+        a.out[n] = EO ? fma(ra, a.q0[n], fma(rb, q[n], (rb * dt) * t))
+                      : fma(ra, a.q0[n], rb * fma(dt, t, q[n]));
     };
-    if (uni)
-      eo_line<P, 1, 1, true>(row, Te + 2 * TE, fl[4 * NFP], fl[5 * NFP], 0, emit);
-    else
-      eo_line_esc<P>(row, sT + 2 * TE, fl[4 * NFP], fl[5 * NFP],
-                     [&](int m) { return Es[g0 + off + m * NQ2 + 2 * NpNe]; }, emit);
+    if (zok) {
+      const int32_t Ef = E + (xe[2] << 20);
+      fix_line<P, EO>(sT + 2 * TAB, EO ? nullptr : a.lift + 2 * NP + r, F, E,
+                      fix_align(g[4], Ef), fix_align(g[5], Ef), emit);
+    } else {
+      double in[N], out[N];  // in: F itself stays in registers
+#pragma unroll
+      for (int m = 0; m < N; m++) in[m] = F[m];
+      ref_line_fp64<P, EO>(&a, 2, r, in, 1, g[4], g[5], Es + 2 * NpNe + ge + r, N2, out);
+#pragma unroll 1
+      for (int m = 0; m < N; m++) emit(m, __double_as_longlong(out[m]));
+    }
   }
 }
 
-template <int P>
-int launch_step_ref_impl(const StepRefArgs& a, cudaStream_t st) {
-  constexpr size_t smem = step_ref_smem_bytes<P>();
-  const long long nblk = ((long long)a.Ne + StepRefCfg<P>::EPB - 1) / StepRefCfg<P>::EPB;
+template <int P, bool EO, int MODE>
+int launch_ref_mode(const RefArgs& a, cudaStream_t st) {
+  // blocks of fewer elements on small meshes, as launch_stage_fix_kind
+  constexpr int N2 = FixShape<P>::N2;
+  const long long want = std::max(a.Ne / (2 * 152), 1);
+  const int threads = (int)std::min<long long>((want * N2 + 31) / 32 * 32, FixShape<P>::THREADS);
+  const int epb = threads / N2;
+  const long long nblk = ((long long)a.Ne + epb - 1) / epb;
   if (nblk == 0) return SDG_OK;
-  if (a.rk == kRkFirst) {
-    SDG_TRY(set_kernel_smem((const void*)step_ref_kernel<P, kRkFirst>, (int)smem, false));
-    step_ref_kernel<P, kRkFirst><<<(unsigned)nblk, StepRefCfg<P>::THREADS, smem, st>>>(a);
-  } else {
-    SDG_TRY(set_kernel_smem((const void*)step_ref_kernel<P, kRkGeneral>, (int)smem, false));
-    step_ref_kernel<P, kRkGeneral><<<(unsigned)nblk, StepRefCfg<P>::THREADS, smem, st>>>(a);
-  }
+  SDG_TRY(set_kernel_smem((const void*)step_ref_kernel<P, EO, MODE>,
+                          (int)ref_smem<P, EO>(FixShape<P>::EPB), true));
+  step_ref_kernel<P, EO, MODE><<<(unsigned)nblk, threads, ref_smem<P, EO>(epb), st>>>(a);
   SDG_CUDA_TRY(cudaGetLastError());
+  return SDG_OK;
+}
+
+// Points a's tables into `base` (16-byte aligned, `bytes` of at least
+// RefShape::LEAST) and builds them there.
+template <int P, bool EO>
+int launch_ref_tables(RefArgs& a, void* base, size_t bytes, cudaStream_t st) {
+  using Rs = RefShape<P, EO>;
+  char* p = static_cast<char*>(base);
+  int4* lift = reinterpret_cast<int4*>(p);
+  double* tab = reinterpret_cast<double*>(p + Rs::LIFT);
+  int* row = reinterpret_cast<int*>(tab + 3 * Rs::TAB);
+  a.tab = tab;
+  a.row = row;
+  a.lift = EO ? nullptr : lift;
+  fixlimb* shared = bytes >= Rs::BYTES ? reinterpret_cast<fixlimb*>(p + Rs::SHARED) : nullptr;
+  const long long npne = (long long)(P + 1) * (P + 1) * (P + 1) * a.Ne;
+  if constexpr (EO)
+    ref_tables_eo_kernel<P><<<1, 256, 0, st>>>(a.D, a.Dt, a.Lift, a.Escale, npne, tab, row, shared,
+                                               a.err);
+  else
+    ref_tables_kernel<P><<<3 * (P + 1), 256, 0, st>>>(a.D, a.Dt, a.Lift, a.Escale, npne, tab, row,
+                                                      lift, shared);
+  SDG_CUDA_TRY(cudaGetLastError());
+  a.shared = shared;
   return SDG_OK;
 }
 

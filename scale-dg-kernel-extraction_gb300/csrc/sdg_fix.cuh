@@ -2,19 +2,24 @@
 //
 // GB300 issues a 32 x 32 + 64 bit integer multiply-add (IMAD.WIDE) 36 times
 // as fast as an FP64 FMA (58-61 against 1.66 a clock and SM, measured), so a
-// product of two 60-bit numbers, formed from 30-bit limbs by three of them,
-// costs a twelfth of a DFMA.  The values of one line share a power-of-two
+// product of two 60-bit numbers, formed from a 31-bit and a 29-bit limb by
+// three of them, costs a twelfth of a DFMA.  The values of one line share a power-of-two
 // scale; sums of products are then exact integer sums, independent of their
 // order, and their error is the quantisation of the operands and the dropped
-// low x low limb product: a few units of 2^-59 of the line's largest value,
-// where a chain of FP64 operations rounds every partial sum to 2^-53.
+// low x low limb product: about one unit of 2^-61 of the largest sum a line
+// could have, where a chain of FP64 operations rounds every partial sum to
+// 2^-53.  (Those sums cancel: a smooth line's derivative is a hundredth of
+// them, so the last bits count.)
 //
-//   values        |F| < 2^59, pair sums |S| < 2^60: hi 2^30 + lo, 0 <= lo < 2^30
-//   coefficients  |C| <= 2^60: hi 2^30 + lo, -2^29 <= lo < 2^29; a row of
-//                 coefficients has sum |C| <= 2^60
+//   values        |F| <= 2^59, pair sums |S| <= 2^60: hi 2^29 + lo,
+//                 0 <= lo < 2^29
+//   coefficients  c 2^60, |c| < 1: hi 2^29 + lo, -2^28 <= lo < 2^28; a row's
+//                 magnitudes add up to less than 1 over the line's values
+//                 (less than 1/2 over its pair sums)
 //   accumulator   hh = sum Ch Xh, x = sum (Ch Xl + Cl Xh); result
-//                 hh + (x >> 30) = sum C X / 2^60.  |hh| <= 2^60 and
-//                 |x| <= 2^60 + n 2^59 < 2^63 for n <= 14 terms.
+//                 hh + (x >> 29) = sum C X / 2^58, at most 2^61, so that a
+//                 node's three results add up in 64 bits.  |x| <= 2^60 + n 2^58
+//                 for n <= 18 values, 2^59 + n 2^59 for n <= 10 pair sums.
 //
 // The same code compiles for the host, where tests check it.
 #pragma once
@@ -29,21 +34,32 @@ struct fixlimb {
   int32_t hi, lo;
 };
 
-constexpr int kFixMask = (1 << 30) - 1;
+constexpr int kFixLow = 29;  // bits of the low limb
+constexpr int kFixMask = (1 << kFixLow) - 1;
 
 SDG_HD fixlimb fix_split(int64_t x) {
   fixlimb r;
-  r.hi = (int32_t)(x >> 30);
+  r.hi = (int32_t)(x >> kFixLow);
   r.lo = (int32_t)((uint32_t)x & (uint32_t)kFixMask);
   return r;
 }
 
-// Limbs of a coefficient c 2^60 (|c| <= 1): balanced low limb.
+// Limbs of a coefficient c 2^60 (|c| < 1): balanced low limb.
 SDG_HD fixlimb fix_coef(int64_t c) {
   fixlimb r;
-  r.hi = (int32_t)((c + (int64_t(1) << 29)) >> 30);
-  r.lo = (int32_t)(c - ((int64_t)r.hi << 30));
+  r.hi = (int32_t)((c + (int64_t(1) << (kFixLow - 1))) >> kFixLow);
+  r.lo = (int32_t)(c - ((int64_t)r.hi << kFixLow));
   return r;
+}
+
+// c 2^60 of a double |c| <= 1, truncated.
+SDG_HD int64_t fix_unit(double c) {
+  uint32_t hi, lo;
+  d2words(c, hi, lo);
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  const uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32 | lo) << 8;
+  const int64_t r = e + 63 < 1023 || e > 1023 ? 0 : (int64_t)(m >> (1023 - e));
+  return (int32_t)hi < 0 ? -r : r;
 }
 
 struct fixacc {
@@ -80,7 +96,14 @@ SDG_HD void fix_fma(fixacc& a, fixlimb c, fixlimb v) {
   a.hh = fix_wide(c.hi, v.hi, a.hh);
   a.x = fix_wide(c.lo, v.hi, fix_wide(c.hi, v.lo, a.x));
 }
-SDG_HD int64_t fix_sum(const fixacc& a) { return a.hh + (a.x >> 30); }
+SDG_HD int64_t fix_sum(const fixacc& a) { return a.hh + (a.x >> kFixLow); }
+
+// a b / 2^60 of two numbers below 2^60, two units off at most.
+SDG_HD int64_t fix_times(int64_t a, int64_t b) {
+  fixacc p;
+  fix_mul(p, fix_split(a), fix_split(b));
+  return fix_sum(p) >> (60 - 2 * kFixLow);
+}
 
 // a >> s, zero for s > 63 (the hardware shift clamps; C++ leaves it undefined).
 SDG_HD uint64_t fix_shr(uint64_t a, uint32_t s) {

@@ -275,11 +275,11 @@ void fix_put(int32_t* out, double x, double y, int k) {
   out[1] = c.lo;
 }
 // The exponent of a row whose magnitudes add up to `sum` (with room for the
-// rounding of the sum); false outside +-200.
+// rounding of the sum and of a coefficient's high limb); false outside +-200.
 bool fix_row_exp(double sum, int* k) {
   *k = 0;
   if (!std::isfinite(sum)) return false;
-  if (sum > 0.0) std::frexp(sum * (1.0 + 1e-13), k);
+  if (sum > 0.0) std::frexp(sum * (1.0 + 1e-8), k);
   return *k >= -200 && *k <= 200;
 }
 }  // namespace
@@ -302,12 +302,20 @@ void fix_tables(int Nq, const Box& box, const std::vector<double>& eo, FixTables
         if (ODD) even.push_back(oM + i);
         for (int l = 0; l < H; l++) even.push_back(i * H + l);
       }
-      double se = 0.0, so = 0.0;
-      for (int w : even) se += std::fabs(T[w] * scale(w));
-      for (int w : odd) so += std::fabs(T[w] * scale(w));
+      // what the row's two outputs can reach on values and faces below one:
+      // D's row holds E + O and E - O, the faces' columns A + B and A - B
+      auto pair = [&](int e, int o) {
+        const double x = e < 0 ? 0.0 : std::fabs(T[e]), y = std::fabs(T[o]);
+        return 2.0 * (x > y ? x : y) * scale(o);
+      };
+      double most = pair(i < H ? oB + i : -1, oA + i);
+      for (int l = 0; l < H; l++) most += pair(i < H ? i * H + l : -1, oO + i * H + l);
+      if (ODD && i < H) most += std::fabs(T[oM + i] * scale(oM + i));
+      bool finite = true;
+      for (int w : even) finite = finite && std::isfinite(T[w]);
       int k = 0;
-      if (!fix_row_exp(se > so ? se : so, &k)) return;
-      t.row[(size_t)d * HR + i] = k - 59;
+      if (!finite || !fix_row_exp(most, &k)) return;
+      t.row[(size_t)d * HR + i] = k - 61;
       even.insert(even.end(), odd.begin(), odd.end());
       for (int w : even) fix_put(&t.coef[2 * ((size_t)d * TE + w)], T[w], scale(w), k);
     }
@@ -340,7 +348,7 @@ void fix_tables_general(int Nq, const Box& box, const double* D1D, const double*
       for (int l = 0; l < N; l++) sum += std::fabs(D1D[i + l * N] * Es);
       int k = 0;
       if (!fix_row_exp(sum + most * Fs, &k)) return;
-      t.row[(size_t)d * N + i] = k - 59;
+      t.row[(size_t)d * N + i] = k - 61;
       for (int l = 0; l < N; l++)
         fix_put(&t.coef[2 * ((size_t)d * N2 + i * N + l)], D1D[i + l * N], Es, k);
       for (int r = 0; r < N2; r++) {

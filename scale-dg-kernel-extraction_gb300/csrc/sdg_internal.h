@@ -60,8 +60,8 @@ Box make_box(int NeX, int NeY, int NeZ, double Lx, double Ly, double Lz);
 // Coefficients of the fixed-point stage (sdg_stage_fix.cuh) on the host: per
 // direction the even-odd table of EoShape as limb pairs (hi, lo) of
 // c 2^(60 - k), c = -(derivative entry) Es_d or -(lift entry) Fs_d, k the
-// row's exponent: the smallest that keeps the sums of magnitudes of the row's
-// two halves (E, D(mid), B and O, A) at or below 2^k.  row: k - 59.  ok = 0
+// row's exponent: what its outputs can reach on values below one is below 2^k.
+// row: k - 61.  ok = 0
 // when an exponent lies outside +-200: every line is then formed in FP64.
 struct FixTables {
   std::vector<int32_t> coef;

@@ -1,7 +1,6 @@
 // Fused RK-stage kernel with the even-odd factorisation of the 1D operators
-// (opt type SDG_OPT_EVENODD) in the FP32-compute form, and the even-odd line
-// pieces that the FP64 kernels of the reference-shaped entry points share (the
-// FP64 stage itself forms its lines in fixed point, sdg_stage_fix.cuh).
+// (opt type SDG_OPT_EVENODD) in the FP32-compute form.  (The FP64 form's lines
+// are in sdg_stage_fix.cuh, on the same tables.)
 //
 // The pair sums cost about half the operations of the plain line sums, and
 // one thread a line replaces the node body's per-node shared-memory reads of a
@@ -197,26 +196,6 @@ template <int P, int S, int PARTS, bool PAIRED, typename CT, typename Emit>
 __device__ __forceinline__ void eo_line(const CT* F, const CT* __restrict__ T, CT gm, CT gp,
                                         int part, Emit&& emit) {
   eo_line_f<P, PARTS, PAIRED, CT>([&](int l) { return F[l * S]; }, T, gm, gp, part, emit);
-}
-
-// Pair values of one line from q and the axis velocity in global memory (FP64
-// body): S(c) = F(c) + F(N-1-c) and Δ(c) = F(c) - F(N-1-c) with F = q u, as
-// P' = q' u' and fma(q, u, ±P') -- three operations a pair instead of four.
-template <int P>
-__device__ __forceinline__ void eo_pairs_f64(const double* __restrict__ q,
-                                             const double* __restrict__ vel, long long g,
-                                             int stride, double* row) {
-  using Sh = EoShape<P>;
-  constexpr int N = Sh::N, H = Sh::H;
-#pragma unroll
-  for (int c = 0; c < H; c++) {
-    const long long a = g + (long long)c * stride, b = g + (long long)(N - 1 - c) * stride;
-    const double q1 = q[a], u1 = vel[a];
-    const double p2 = q[b] * vel[b];
-    row[c] = fma(q1, u1, p2);
-    row[N - 1 - c] = fma(q1, u1, -p2);
-  }
-  if constexpr (Sh::ODD != 0) row[H] = q[g + (long long)H * stride] * vel[g + (long long)H * stride];
 }
 
 // One block advances elements [eb, eb + nloc) through one stage with the

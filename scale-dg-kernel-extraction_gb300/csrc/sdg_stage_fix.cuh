@@ -30,7 +30,7 @@
 //
 // Scale: a line's values share the power of two that bounds its fluxes q u_d
 // and its two face fluxes, and a row of coefficients has a power of two of its
-// own, so every line result keeps about 2^-59 of its own bound.  The three
+// own, so every line result keeps about 2^-61 of its own bound.  The three
 // results of a node are added as integers on the largest of their scales and
 // become one double.  A line with infinities, NaN, or magnitudes near the ends
 // of the exponent range is formed in FP64 by its thread, and its nodes add up
@@ -74,16 +74,19 @@ struct FixStageArgs {
   StageArgs s;
   double c;              // EO: b dt, else dt
   fixlimb tab[3 * TAB];  // per direction: EoShape's table, or D(i,l) at i N + l
-  int row[3 * ROWS];     // exponent of a row's scale, less 59
+  int row[3 * ROWS];     // exponent of a row's scale, less 61
   int ok;                // 0: coefficients out of range, every line in FP64
   static __host__ __device__ constexpr int row_of(int m) {
     return EO ? (m < P - m ? m : P - m) : m;
+  }
+  __device__ const int4* lift(int ax, int r) const {
+    return static_cast<const int4*>(s.fix_lift) + ax * (P + 1) * (P + 1) * (P + 1) + r;
   }
 };
 
 template <int P>
 __host__ __device__ constexpr size_t fix_smem(int epb) {
-  return sizeof(double) * 2 * epb * FixShape<P>::EW + sizeof(int) * 2 * epb * FixShape<P>::N2;
+  return sizeof(double) * 2 * epb * FixShape<P>::EW + sizeof(short) * 2 * epb * FixShape<P>::N2;
 }
 
 // A line in FP64, for values the fixed-point path does not take (E: their
@@ -139,22 +142,21 @@ __device__ __noinline__ void fix_line_fp64(const StageArgs* a, int ax, int r, co
   }
 }
 
-// Line r of direction AX: F its fluxes q u_d, gm / gp the face fluxes of its
-// - and + faces, all in range of the scale E; emit(m, I): the result is I times
-// two to the line's exponent (fix_line_exp) plus its row's.
-template <int P, bool EO, int AX, typename Emit>
-__device__ __forceinline__ void fix_line(const FixStageArgs<P, EO>& a, int r, const double* F,
-                                         int32_t E, double gm, double gp, Emit&& emit) {
+// One line: F its fluxes q u_d on the scale E, im / ip its - and + face's
+// fluxes as integers, T its direction's coefficients and (operators as given)
+// lift its nodes' lift limbs, N^2 apart; emit(m, I): the result is I times two
+// to the line's exponent (fix_line_exp) plus its row's.
+template <int P, bool EO, typename Emit>
+__device__ __forceinline__ void fix_line(const fixlimb* T, const int4* __restrict__ lift,
+                                         const double* F, int32_t E, int64_t im, int64_t ip,
+                                         Emit&& emit) {
   using Sh = EoShape<P>;
   constexpr int N = Sh::N, H = Sh::H;
-  const fixlimb* T = a.tab + AX * a.TAB;
-  const int64_t im = fix_align_face(gm, E), ip = fix_align_face(gp, E);
   if constexpr (!EO) {
     const fixlimb lm = fix_split(im), lp = fix_split(ip);
     fixlimb f[N];
 #pragma unroll
     for (int l = 0; l < N; l++) f[l] = fix_split(fix_align(F[l], E));
-    const int4* __restrict__ lift = static_cast<const int4*>(a.s.fix_lift) + AX * N * N * N + r;
 #pragma unroll 2
     for (int i = 0; i < N; i++) {
       const int4 c = lift[i * N * N];
@@ -201,7 +203,7 @@ __device__ __forceinline__ void fix_line(const FixStageArgs<P, EO>& a, int r, co
 }
 
 // Exponent of a line formed in FP64: its results are doubles.
-constexpr int kFixDouble = 1 << 20;
+constexpr int kFixDouble = 1 << 14;
 
 // The line of direction AX held in shared memory with stride S, its results
 // over it as integers (or doubles); returns the line's exponent.
@@ -218,7 +220,8 @@ __device__ __forceinline__ int fix_line_shared(const FixStageArgs<P, EO>& a, int
   }
   if (a.ok && fix_in_range(E)) {
     int64_t* out = reinterpret_cast<int64_t*>(line);
-    fix_line<P, EO, AX>(a, r, F, E, gm, gp, [&](int m, int64_t v) { out[m * S] = v; });
+    fix_line<P, EO>(a.tab + AX * a.TAB, a.lift(AX, r), F, E, fix_align_face(gm, E),
+                    fix_align_face(gp, E), [&](int m, int64_t v) { out[m * S] = v; });
     return fix_line_exp(E);
   }
   double out[N];
@@ -235,6 +238,15 @@ static __device__ __noinline__ double fix_node_fp64(int64_t x, int ex, int64_t y
     return e >= kFixDouble / 2 ? __longlong_as_double(v) : v == 0 ? 0.0 : fix_to_double(v, e);
   };
   return (value(x, ex) + value(y, ey)) + value(z, ez);
+}
+
+// A node's tendency from its three line results v with exponents e, as
+// integers (each below 2^61) on the largest of their scales.
+__device__ __forceinline__ double fix_node(int64_t x, int ex, int64_t y, int ey, int64_t z,
+                                           int ez) {
+  const int e = max(ex, max(ey, ez));
+  if (e >= kFixDouble / 2) return fix_node_fp64(x, ex, y, ey, z, ez);
+  return fix_to_double(fix_sar(x, e - ex) + fix_sar(y, e - ey) + fix_sar(z, e - ez), e);
 }
 
 // Neighbour elements of e across the faces -y, +x, +y, -x, -z, +z with
@@ -274,8 +286,9 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
   double* sX = reinterpret_cast<double*>(smem_raw) + le * EW;
   double* sY = sX + epb * EW;
   // exponents of the element's x and y lines
-  int* sEx = reinterpret_cast<int*>(reinterpret_cast<double*>(smem_raw) + 2 * epb * EW) + le * N2;
-  int* sEy = sEx + epb * N2;
+  short* sEx =
+      reinterpret_cast<short*>(reinterpret_cast<double*>(smem_raw) + 2 * epb * EW) + le * N2;
+  short* sEy = sEx + epb * N2;
   const long long ge = (eb + le) * NP;  // the element's first node
   const double* __restrict__ q = a.s.q_in;
   const int zat = i + NS * j;  // the z line's first node in the padded arrays
@@ -347,8 +360,6 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
     const double* __restrict__ q0 = a.s.q0;
     double* __restrict__ qout = a.s.q_out;
     const double c = a.c, ra = a.s.a, rb = a.s.b;
-    // the node's three results on the largest of their scales, added as
-    // integers (each below 2^61)
     const int Bz = a.ok && fix_in_range(E) ? fix_line_exp(E) : kFixDouble;
     const int rx = a.row[Args::row_of(i)], ry = a.row[Args::ROWS + Args::row_of(j)];
     const int64_t* iX = reinterpret_cast<const int64_t*>(sX) + zat;
@@ -357,12 +368,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
       const int64_t x = iX[m * NS * N], y = iY[m * NS * N];
       const int ex = sEx[j + N * m] + rx, ey = sEy[i + N * m] + ry;
       const int ez = Bz + a.row[2 * Args::ROWS + Args::row_of(m)];
-      const int e = max(ex, max(ey, ez));
-      double t;
-      if (e < kFixDouble / 2)
-        t = fix_to_double(fix_sar(x, e - ex) + fix_sar(y, e - ey) + fix_sar(z, e - ez), e);
-      else
-        t = fix_node_fp64(x, ex, y, ey, z, ez);
+      const double t = fix_node(x, ex, y, ey, z, ez);
       const long long n = ge + r + m * N2;
       if constexpr (RK == kRkTend)
         qout[n] = t;
@@ -375,7 +381,8 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
                      : fma(ra, q0[n], rb * fma(c, t, q[n]));
     };
     if (Bz != kFixDouble) {
-      fix_line<P, EO, 2>(a, r, F, E, g[4], g[5], emit);
+      fix_line<P, EO>(a.tab + 2 * a.TAB, a.lift(2, r), F, E, fix_align_face(g[4], E),
+                      fix_align_face(g[5], E), emit);
     } else {
       double in[N], out[N];  // in: F itself stays in registers
 #pragma unroll

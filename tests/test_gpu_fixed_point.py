@@ -106,3 +106,87 @@ def test_steep_fields_and_uneven_axes(opt, p):
     for s in (a, b):
         s.upload(*_fields(c))
     assert rel_l2(a.tendency() * tiny, b.tendency()) <= TOL_TEND
+
+
+def _mesh_arrays(c, scale_of_element=None):
+    m = c.mesh
+    es = m.Escale.copy().reshape(3, m.Ne, m.Np)
+    if scale_of_element is not None:
+        es *= scale_of_element.reshape(3, m.Ne, -1)
+    return es.reshape(-1)
+
+
+@both
+@pytest.mark.parametrize("p,dims", [(1, (9, 8, 7)), (2, (6, 7, 5)), (5, (10, 9, 9)),
+                                    (7, (8, 7, 8)), (8, (7, 7, 6)), (13, (3, 5, 4)),
+                                    (15, (3, 4, 3))])
+@pytest.mark.parametrize("kind", ["affine", "own", "curved", "bad"])
+def test_tendency_and_loop_on_reference_arrays(opt, p, dims, kind):
+    """cal_tend and the time loop with one Escale for the mesh, one an element,
+    one a node in every third element, and a non-finite state, on meshes on
+    both sides of the small-mesh rule, against the oracle on the same arrays."""
+    import copy
+
+    import sdg
+    c = Case(*dims, p)
+    m = copy.copy(c.mesh)
+    r = np.random.RandomState(p)
+    if kind == "own":
+        m.Escale = _mesh_arrays(c, 0.5 + r.rand(3, m.Ne, 1))
+    elif kind == "curved":
+        f = 0.5 + r.rand(3, m.Ne, m.Np)
+        f[:, np.arange(m.Ne) % 3 != 0, :] = 1.0
+        m.Escale = _mesh_arrays(c, f)
+    q = c.q.copy()
+    if kind == "bad":
+        q[m.Np * (m.Ne // 2)] = np.inf
+        m.update_halo(q)
+    want = O.cal_tend(m, q, c.u, c.v, c.w, c.D, c.Dt, c.Lift, O.OPT1)[: c.nown]
+    sdg.dg_optr_kernel_setup(opt[4:])
+    got = np.zeros(m.Np * m.NeA)
+    sdg.advect3d_eq_cal_tend(got, q, c.u, c.v, c.w, c.D, c.Dt, c.Lift, m.VMapM, m.VMapP,
+                             m.normal_fn, m.Escale, m.Fscale, m.Nq, m.Np, m.NfpTot, m.Ne, m.NeA)
+    got = got[: c.nown]
+    fine = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), fine)
+    assert rel_l2(got[fine], want[fine]) <= TOL_TEND
+    if kind == "bad":
+        return
+    args = (m.VMapM, m.VMapP, m.normal_fn, m.Escale, m.Fscale, m.halo_src_map, m.Nq, m.Np,
+            m.NfpTot, m.Ne, m.NeA, m.NhaloNode)
+    a = sdg.advect3d_eq_step(q, c.u, c.v, c.w, c.D, c.Dt, c.Lift, *args, 0.5 * c.dt, 2,
+                             getattr(sdg, opt))
+    qq = q.copy()
+    O.run(m, qq, c.u, c.v, c.w, c.D, c.Dt, c.Lift, 0.5 * c.dt, 2, O.OPT1)
+    assert rel_l2(a[: c.nown], qq[: c.nown]) <= TOL_TEND
+
+
+@both
+@pytest.mark.parametrize("p", [1, 6, 11, 14])
+def test_loop_with_the_least_scratch(opt, p):
+    """Scratch without room for the operator tables (all that was asked for
+    before there were any) still runs, to the same result."""
+    import sdg
+    c = Case(3, 2, 2, p)
+    m = c.mesh
+    A = sdg.DeviceArray
+    need = int(sdg.lib.sdg_advect3d_eq_step_scratch_bytes(m.Nq, m.Ne))
+    N, H, HR = m.Nq, m.Nq // 2, (m.Nq + 1) // 2
+    te = H * H + HR * H + (N & 1) * H + HR + H
+    up = lambda n: (n + 255) // 256 * 256
+    least = (2 * up(8 * m.Np * m.Ne) + up(16 * m.NfpTot * m.Ne) + up(8 * m.NfpTot * m.Ne)
+             + up(24 * te) + up(32 * m.Ne))
+    assert least < need
+    arrs = [A(a) for a in (c.u, c.v, c.w, c.D, c.Dt, c.Lift, m.VMapM, m.VMapP, m.normal_fn,
+                           m.Escale, m.Fscale, m.halo_src_map)]
+    out = []
+    for size, want in ((need, 0), (least, 0), (least - 1, sdg.ERR_INVALID_ARG)):
+        q, scratch, err = A(c.q), A(n=size, dtype=np.uint8), A(np.zeros(1, dtype=np.int32))
+        st = sdg.lib.sdg_advect3d_eq_step_dev(
+            q.ptr, *[a.ptr for a in arrs], m.Nq, m.Np, m.NfpTot, m.Ne, m.NeA, m.NhaloNode, c.dt,
+            2, getattr(sdg, opt), scratch.ptr, size, err.ptr, None)
+        assert st == want
+        if st == 0:
+            assert err.numpy()[0] == 0
+            out.append(q.numpy()[: c.nown])
+    assert rel_l2(out[1], out[0]) <= TOL_TEND
