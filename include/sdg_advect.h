@@ -64,10 +64,9 @@ extern "C" {
                              FP64 arithmetic, which forms the lines that hold
                              infinities, NaN or extreme magnitudes */
 #define SDG_PREC_FP32 1   /* FP32 flux/derivative/lift, FP64 RK state */
-#define SDG_PREC_FP64_EMU 2 /* FP64 state and RK combine; flux/derivative/lift in
-                               double-float (two FP32 numbers, ~48 bits) on the
-                               FP32 pipes; <= 1e-12 relative L2 per tendency
-                               against FP64 */
+#define SDG_PREC_FP64_EMU 2 /* FP64 arithmetic emulated on the integer and FP32 pipes:
+                               since SDG_PREC_FP64 forms its line sums there too,
+                               the same kernels and results as SDG_PREC_FP64 */
 
 const char* sdg_status_string(int status);
 const char* sdg_last_error(void);
@@ -351,8 +350,7 @@ typedef struct sdg_solver sdg_solver;
  * SDG_OPT_EVENODD the even-odd stage (returns SDG_ERR_INVALID_ARG if
  * D1D or Lift_mat lacks the centro-symmetry beyond 1e-13 relative).
  * precision = SDG_PREC_*.  stream may be NULL.
- * With SDG_PREC_FP64, or SDG_OPT_EVENODD and SDG_PREC_FP64_EMU, the solver also
- * holds the face-flux velocity factors of one call (16 bytes per face node,
+ * With SDG_PREC_FP64 or SDG_PREC_FP64_EMU the solver also holds the face-flux velocity factors of one call (16 bytes per face node,
  * 96/Nq bytes per DOF): the first stage of every sdg_solver_step forms them
  * from the current velocity and the others read them.  (With GENERAL and OPT1
  * a solver whose device memory does not hold them forms them in every stage.) */

@@ -77,7 +77,6 @@ __device__ __forceinline__ void batch_item_body(const BatchInst& I, const BatchI
   a.b = c_rk_b[stage];
   a.dt = I.dt;
   a.cdt_hi = I.cdt[stage];  // FP32 increment factor of the FP32 form
-  a.cdt_lo = 0.0f;
   a.b_is_one = (stage == 0);
   a.a_nonzero = (stage != 0);
   a.tend_only = 0;

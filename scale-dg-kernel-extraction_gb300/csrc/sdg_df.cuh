@@ -2,9 +2,10 @@
 // FP32 numbers hi + lo (|lo| <= ulp(hi)/2), computed on the FP32 pipes.
 //
 // GB300 executes FP64 arithmetic at 1/64 of the FP32 rate (measured: 1.2
-// TFLOP/s DFMA against 75 TFLOP/s FFMA), so the emulated FP64 stage kernel does
-// its flux, divergence and lift arithmetic with these error-free
-// transformations and keeps FP64 only for the state and the RK combine.
+// TFLOP/s DFMA against 75 TFLOP/s FFMA).  The kernels use the bit casts and the
+// FP64 <-> FP32 conversions without FP64 operations (df_split, f32_to_f64_bits);
+// sums that need FP64's precision run in fixed point (sdg_fix.cuh), which took
+// the place of the double-float stage kernels built on the rest.
 // Published building blocks:
 //   TwoSum (Knuth, TAOCP vol. 2; Moller 1965): s + e = a + b exactly, 6 ops;
 //   Fast2Sum (Dekker 1971): same when |a| >= |b|, 3 ops;

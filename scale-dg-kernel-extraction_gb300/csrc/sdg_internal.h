@@ -91,17 +91,16 @@ struct StageArgs {
   long long elem_begin;  // first element of this launch
   long long elem_count;  // elements of this launch
   double a, b, dt;      // q_out = a*q0 + b*(q_in + dt*dqdt)
-  float cdt_hi, cdt_lo; // b*dt as a double-float pair (emulated-FP64 kernel)
+  float cdt_hi;         // b*dt in FP32
   int b_is_one;         // b == 1 (stage 1): the kernels branch on integers,
   int a_nonzero;        // since an FP64 comparison also uses the FP64 pipe
   int tend_only;        // write dqdt instead of the RK update
-  // even-odd FP64 stage: per-direction factors of the D part (-c*Es_d) and
-  // of the lift part (-c*Fs_d/4) of the tables, c = b*dt (1 for tend_only);
-  // D then points at the 3-direction table built by the solver
-  double eo_sD[3], eo_sL[3];
-  float eo_sDf[3], eo_sLf[3];  // the same factors for the FP32-compute form
-  // even-odd FP64 stage: the velocity factors of the face flux, (tP, tM) per
-  // face node of each element (2*Nfp*6 doubles an element).  A stage with
+  // even-odd stages: D points at the 3-direction table built by the solver; the
+  // FP32 form's per-direction factors of its D part (-c*Es_d) and of its lift
+  // part (-c*Fs_d/4), c = b*dt (1 for tend_only)
+  float eo_sDf[3], eo_sLf[3];
+  // FP64 stage: the velocity factors of the face flux, two per face node of
+  // each element (2*Nfp*6 doubles an element).  A stage with
   // fc_out forms them from u, v, w and stores them; a stage with fc_in reads
   // them instead (same bits), so the stages of one solver call, which share
   // the velocity (main.f90:58-67 passes the same u, v, w to every

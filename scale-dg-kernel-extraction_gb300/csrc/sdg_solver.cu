@@ -36,10 +36,8 @@ struct sdg_solver {
   void* D = nullptr;
   void* Lift = nullptr;
   double* dqdt = nullptr;
-  // face-flux velocity factors shared by the three stages of a step (even-odd
-  // FP64 and emulated-FP64 stages; null otherwise): 96 / (p + 1) bytes a DOF.
-  // Measured on GB300 against forming them in every stage: 1.04-1.13x for the
-  // FP64 stage (p = 7: 19.3 against 18.5 GDOF-updates/s), 1.01-1.14x emulated.
+  // face-flux velocity factors shared by the stages of a call (not FP32):
+  // 96 / (p + 1) bytes a DOF
   double* fc = nullptr;
   // coefficients of the FP64 stage, and for operators as given (GENERAL, OPT1)
   // its device table of lift limbs
@@ -126,9 +124,7 @@ int one_stage_on(sdg_solver* s, int stage, double dt, const double* qin, const d
   a.a = rk_a[stage];
   a.b = rk_b[stage];
   a.dt = dt;
-  const dfl cdt = df_from_double(a.b * dt);
-  a.cdt_hi = cdt.hi;
-  a.cdt_lo = cdt.lo;
+  a.cdt_hi = (float)(a.b * dt);
   a.b_is_one = (a.b == 1.0) ? 1 : 0;
   a.a_nonzero = (a.a != 0.0) ? 1 : 0;
   a.tend_only = tend_only ? 1 : 0;
@@ -138,10 +134,8 @@ int one_stage_on(sdg_solver* s, int stage, double dt, const double* qin, const d
   a.fix_lift = s->fix_lift;
   const double c = tend_only ? 1.0 : a.b * dt;
   for (int d = 0; d < 3; d++) {
-    a.eo_sD[d] = -c * s->box.Es[d];
-    a.eo_sL[d] = -c * (0.25 * s->box.Fs[d]);
-    a.eo_sDf[d] = (float)a.eo_sD[d];
-    a.eo_sLf[d] = (float)a.eo_sL[d];
+    a.eo_sDf[d] = (float)(-c * s->box.Es[d]);
+    a.eo_sLf[d] = (float)(-c * (0.25 * s->box.Fs[d]));
   }
   return launch_stage(s->p, s->prec, s->opt, a, st);
 }
@@ -160,89 +154,24 @@ int put_velocity(sdg_solver* s, void* dst, const double* src_dev) {
   return SDG_OK;
 }
 
-// Operator tables in the layout and arithmetic each kernel family reads:
-//   FP64: D1D(Nq,Nq) and Lift_mat(Nq,Nq,Nq,6) as given;
-//   FP32: the same rounded to float;
-//   FP64_EMU: double-float (hi, lo) pairs with the geometric factors folded
-//     in: D [3][Nq*Nq] = Es_d*D1D, R [3][Nq] = Es_d * (row sums of D1D, from
-//     the FP64 values), Lift [6*Np] = Lift_mat(n,f)*0.5*Fscale(f).
-void operator_tables(int prec, int Nq, const Box& box, const double* D1D,
-                     const double* Lift_mat, std::vector<unsigned char>& dtab,
-                     std::vector<unsigned char>& ltab) {
-  const size_t nD = (size_t)Nq * Nq, Np = (size_t)Nq * Nq * Nq, nL = 6 * Np;
-  if (prec == SDG_PREC_FP64) {
+// D1D(Nq,Nq) and Lift_mat(Nq,Nq,Nq,6) in the type the form's kernels read: FP64
+// as given, FP32 rounded to float.
+void operator_tables(int prec, int Nq, const double* D1D, const double* Lift_mat,
+                     std::vector<unsigned char>& dtab, std::vector<unsigned char>& ltab) {
+  const size_t nD = (size_t)Nq * Nq, nL = 6 * nD * Nq;
+  if (prec != SDG_PREC_FP32) {
     dtab.resize(8 * nD);
     ltab.resize(8 * nL);
     std::memcpy(dtab.data(), D1D, 8 * nD);
     std::memcpy(ltab.data(), Lift_mat, 8 * nL);
-  } else if (prec == SDG_PREC_FP32) {
-    dtab.resize(4 * nD);
-    ltab.resize(4 * nL);
-    float* d = reinterpret_cast<float*>(dtab.data());
-    float* l = reinterpret_cast<float*>(ltab.data());
-    for (size_t i = 0; i < nD; i++) d[i] = (float)D1D[i];
-    for (size_t i = 0; i < nL; i++) l[i] = (float)Lift_mat[i];
-  } else {
-    // interleaved double-float pairs: D [3][Nq*Nq], R [3][Nq], Lift [6*Np]
-    dtab.resize(8 * (3 * nD + 3 * (size_t)Nq));
-    ltab.resize(8 * nL);
-    float* d = reinterpret_cast<float*>(dtab.data());
-    float* l = reinterpret_cast<float*>(ltab.data());
-    for (int ax = 0; ax < 3; ax++) {
-      for (size_t i = 0; i < nD; i++) {
-        const dfl v = df_from_double(box.Es[ax] * D1D[i]);
-        d[2 * (ax * nD + i)] = v.hi;
-        d[2 * (ax * nD + i) + 1] = v.lo;
-      }
-      // true row sums of the FP64 operator (about 1e-16 |D|), in long double
-      for (int i = 0; i < Nq; i++) {
-        long double rs = 0.0L;
-        for (int c = 0; c < Nq; c++) rs += (long double)D1D[i + (size_t)c * Nq];
-        const dfl v = df_from_double((double)((long double)box.Es[ax] * rs));
-        d[2 * (3 * nD + ax * Nq + i)] = v.hi;
-        d[2 * (3 * nD + ax * Nq + i) + 1] = v.lo;
-      }
-    }
-    const int face_axis[6] = {1, 0, 1, 0, 2, 2};  // -y,+x,+y,-x,-z,+z
-    for (int f = 0; f < 6; f++)
-      for (size_t n = 0; n < Np; n++) {
-        const dfl v = df_from_double(Lift_mat[n + f * Np] * (0.5 * box.Fs[face_axis[f]]));
-        l[2 * (n + f * Np)] = v.hi;
-        l[2 * (n + f * Np) + 1] = v.lo;
-      }
+    return;
   }
-}
-
-// Tables of the emulated even-odd stage (sdg_stage_emu_eo.cuh) as
-// double-float pairs, per axis: the even-odd tables `eo` (unscaled, from
-// eo_tables) with the D parts times -Es_d and the lift parts times
-// -0.5*Fs_d, then the row sums R(i), i < N/2, of the symmetrised operator
-// (long double) times -Es_d.
-void emu_eo_tables(int Nq, const Box& box, const double* D1D, const std::vector<double>& eo,
-                   std::vector<unsigned char>& out) {
-  const int N = Nq, H = N / 2, HR = (N + 1) / 2, ODD = N & 1;
-  const int TE = H * H + HR * H + ODD * H + HR + H, TE2 = TE + H;
-  const int offA = H * H + HR * H + ODD * H;
-  std::vector<float> f(2 * 3 * (size_t)TE2);
-  for (int ax = 0; ax < 3; ax++) {
-    const long double sD = -(long double)box.Es[ax];
-    const long double sL = -0.5L * (long double)box.Fs[ax];
-    auto put = [&](int w, long double v) {
-      const dfl x = df_from_double((double)v);
-      f[2 * ((size_t)ax * TE2 + w)] = x.hi;
-      f[2 * ((size_t)ax * TE2 + w) + 1] = x.lo;
-    };
-    for (int w = 0; w < TE; w++)
-      put(w, (long double)eo[(size_t)ax * TE + w] * (w < offA ? sD : sL));
-    for (int i = 0; i < H; i++) {
-      long double rs = 0.0L;
-      for (int l = 0; l < N; l++)
-        rs += 0.5L * ((long double)D1D[i + l * N] - (long double)D1D[(N - 1 - i) + (N - 1 - l) * N]);
-      put(TE + i, rs * sD);
-    }
-  }
-  out.resize(4 * f.size());
-  std::memcpy(out.data(), f.data(), out.size());
+  dtab.resize(4 * nD);
+  ltab.resize(4 * nL);
+  float* d = reinterpret_cast<float*>(dtab.data());
+  float* l = reinterpret_cast<float*>(ltab.data());
+  for (size_t i = 0; i < nD; i++) d[i] = (float)D1D[i];
+  for (size_t i = 0; i < nL; i++) l[i] = (float)Lift_mat[i];
 }
 
 // A solver on a given box (sizes and scale factors already checked): the
@@ -265,7 +194,7 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
   const size_t nD = (size_t)s->Nq * s->Nq, nL = 6 * (size_t)s->Np;
   // operator tables as the kernels read them (see operator_tables below)
   std::vector<unsigned char> dtab, ltab;
-  operator_tables(precision, s->Nq, s->box, D1D, Lift_mat, dtab, ltab);
+  operator_tables(precision, s->Nq, D1D, Lift_mat, dtab, ltab);
   if (opt == SDG_OPT_EVENODD) {
     std::vector<double> tab;
     const int rc = eo_tables(s->Nq, D1D, Lift_mat, tab);
@@ -273,9 +202,7 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
       delete s;
       return rc;
     }
-    if (precision == SDG_PREC_FP64_EMU) {
-      emu_eo_tables(s->Nq, s->box, D1D, tab, dtab);
-    } else if (precision == SDG_PREC_FP32) {
+    if (precision == SDG_PREC_FP32) {
       // the FP32 form reads FP32 tables
       std::vector<float> f(tab.begin(), tab.end());
       dtab.resize(4 * f.size());
@@ -287,7 +214,7 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
     }
   }
   std::vector<int32_t> fix_lift;
-  if (precision == SDG_PREC_FP64 && opt != SDG_OPT_EVENODD)
+  if (precision != SDG_PREC_FP32 && opt != SDG_OPT_EVENODD)
     fix_tables_general(s->Nq, s->box, D1D, Lift_mat, s->fix, fix_lift);
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < 3 && e == cudaSuccess; i++)
@@ -303,7 +230,7 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
   if (e == cudaSuccess && !fix_lift.empty()) e = cudaMalloc(&s->fix_lift, 4 * fix_lift.size());
   if (e == cudaSuccess && !fix_lift.empty())
     e = cudaMemcpy(s->fix_lift, fix_lift.data(), 4 * fix_lift.size(), cudaMemcpyHostToDevice);
-  // GENERAL and OPT1 in FP64 share the velocity factors too, but a box whose
+  // GENERAL and OPT1 share the velocity factors too, but a box whose
   // other buffers fill the memory runs without them
   if (e == cudaSuccess && !fix_lift.empty() && cudaMalloc(&s->fc, fc_bytes) != cudaSuccess) {
     cudaGetLastError();

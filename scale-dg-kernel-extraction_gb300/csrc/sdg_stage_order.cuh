@@ -3,8 +3,6 @@
 #pragma once
 
 #include "sdg_stage.cuh"
-#include "sdg_stage_emu.cuh"
-#include "sdg_stage_emu_eo.cuh"
 #include "sdg_stage_elem.cuh"
 #include "sdg_stage_eo.cuh"
 #include "sdg_stage_fix.cuh"
@@ -15,13 +13,9 @@ namespace sdg {
 template <int P>
 int launch_stage_order(int prec, int opt, const StageArgs& a, cudaStream_t st) {
   constexpr bool kCanSplit = (P > 7);
-  // EVENODD: the even-odd bodies (FP64, FP32 and emulated FP64)
   const bool split = kCanSplit && (opt != SDG_OPT_GENERAL);
-  if (prec == SDG_PREC_FP64_EMU) {
-    if (opt == SDG_OPT_EVENODD) return launch_stage_emu_eo_impl<P>(a, st);
-    return launch_stage_emu_impl<P>(a, st);
-  }
-  if (prec == SDG_PREC_FP64)
+  // FP64 and emulated FP64 are one arithmetic: the fixed-point stage
+  if (prec != SDG_PREC_FP32)
     return opt == SDG_OPT_EVENODD ? launch_stage_fix_impl<P, true>(a, st)
                                   : launch_stage_fix_impl<P, false>(a, st);
   if (opt == SDG_OPT_EVENODD) {
