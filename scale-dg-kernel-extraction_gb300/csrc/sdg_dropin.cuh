@@ -10,11 +10,14 @@
 //                    per block staged in shared memory: a GENERAL or OPT1
 //                    tendency of so few elements (about Nq) that the flux
 //                    scratch does not hold step_ref_kernel's tables;
-//   divlike_kernel   tensorprod_divlike_dirXYZ (mod_dg_optr_kernel.f90:62-136)
-//                    over a batch of elements;
+//   ops_kernel       tensorprod_divlike_dirXYZ (mod_dg_optr_kernel.f90:62-136),
+//                    gradlike and matvec over a batch of elements
+//                    (sdg_dropin_ops.cuh), and
+//   divlike_kernel, gradlike_kernel  the same in FP64 over few elements;
 //   lift_kernel      tensorprod_Lift_hexahedral (mod_dg_optr_kernel.f90:139-190).
 #pragma once
 
+#include "sdg_dropin_ops.cuh"
 #include "sdg_stage.cuh"
 #include "sdg_stage_eo.cuh"
 
@@ -125,18 +128,6 @@ __global__ void __launch_bounds__(DropCfg<P>::THREADS) dqdt_kernel(const TendArg
     }
   }
 }
-
-struct DivArgs {
-  double* ox;
-  double* oy;
-  double* oz;
-  const double* D;
-  const double* Dt;
-  const double* ix;
-  const double* iy;
-  const double* iz;
-  int nelem;
-};
 
 template <int P>
 constexpr size_t divlike_smem_bytes() {
@@ -323,6 +314,19 @@ struct RefCall {
   size_t bytes;
 };
 
+// Whether a contraction over nelem elements runs in fixed point: from 150k nodes
+// (about one wave of blocks; below it the FP64 kernels' blocks of one node a
+// thread wait less: p = 3 6.6 / 4.6 us at 20k nodes, level at 100k, 16.8 / 25.2 at
+// 1M; p = 7 8.8 / 10.7 at 100k) and always from p = 11 (15 / 23 us at 100k nodes,
+// p = 15 23 / 62).  divlike at p = 1, 48 bytes a node for 6 FP64 instructions,
+// stays in FP64 (115 / 118 us at 10M nodes).
+template <int P>
+constexpr bool ops_always() { return P >= 11; }
+template <int P>
+bool ops_fixed(int nelem) {
+  return ops_always<P>() || (long long)nelem * Ord<P>::NP >= 150000;
+}
+
 // Per-order entry used by the dispatch in sdg_dropin.cu.  what: 0 cal_dqdt,
 // 1 divlike, 2 lift, 3 gradlike, 4 step_ref_kernel, 5 its tables, 6 the bytes
 // of these (into the two size_t args points at: at least, and the whole).
@@ -337,11 +341,22 @@ int dropin_order(int what, int opt, const void* args, cudaStream_t st) {
     }
     case 1: {
       const DivArgs& a = *static_cast<const DivArgs*>(args);
-      return split ? launch_divlike_impl<P, kCanSplit>(a, st)
-                   : launch_divlike_impl<P, false>(a, st);
+      if constexpr (ops_always<P>()) {
+        return launch_ops<P, false>(a, st);
+      } else {
+        if (P > 1 && ops_fixed<P>(a.nelem)) return launch_ops<P, false>(a, st);
+        return split ? launch_divlike_impl<P, kCanSplit>(a, st)
+                     : launch_divlike_impl<P, false>(a, st);
+      }
     }
     case 3:
-      return launch_gradlike_impl<P>(*static_cast<const DivArgs*>(args), st);
+      if constexpr (ops_always<P>()) {
+        return launch_ops<P, true>(*static_cast<const DivArgs*>(args), st);
+      } else {
+        return ops_fixed<P>(static_cast<const DivArgs*>(args)->nelem)
+                   ? launch_ops<P, true>(*static_cast<const DivArgs*>(args), st)
+                   : launch_gradlike_impl<P>(*static_cast<const DivArgs*>(args), st);
+      }
     case 4: {
       const RefCall& c = *static_cast<const RefCall*>(args);
       const bool eo = opt == SDG_OPT_EVENODD;

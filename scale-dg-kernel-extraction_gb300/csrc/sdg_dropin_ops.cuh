@@ -1,0 +1,183 @@
+// The element contractions with their sums in fixed point (sdg_fix.cuh):
+// tensorprod_divlike_dirXYZ (mod_dg_optr_kernel.f90:62-136), gradlike and the
+// single-direction matvecs (opt1 erb:51-129, :166-219).
+//
+// In FP64 these kernels kept the FP64 pipe 93-96 % busy (24 FP64 instructions a
+// node at p = 7 for 48 bytes).  As integer sums they have none; a sum is then
+// the exact one to 2^-61 of its row's bound, rounded once, whatever the order
+// GENERAL or OPT1 asks for.  Lines with infinities, NaN or magnitudes near the
+// ends of the exponent range are summed in FP64.
+//
+// Measured on 10M nodes on GB300, us, against the FP64 kernels: divlike p = 3
+// 126 / 212, p = 7 160 / 406 (3.0 TB/s, 44 % of the measured HBM rate), p = 15
+// 272 / 980; gradlike p = 7 154 / 402; one direction p = 7 60 / 140.  The Lift
+// operator, six products a node with a scale of their own, measured level as
+// integer sums (98-109 / 105-107, and slower below 1M nodes) and stays in FP64.
+#pragma once
+
+#include "sdg_stage_fix.cuh"
+
+namespace sdg {
+
+struct DivArgs {
+  double* ox;
+  double* oy;
+  double* oz;
+  const double* D;
+  const double* Dt;
+  const double* ix;
+  const double* iy;
+  const double* iz;
+  int nelem;
+};
+
+// The exponent of a row whose magnitudes add up to sum (with room for the
+// rounding of the sum and of a coefficient's high limb), kBadRow outside +-200.
+constexpr int kBadRow = 1 << 20;
+__device__ __forceinline__ int fix_row_exp(double sum) {
+  const int e = (int)((unsigned)__double2hiint(sum * (1.0 + 1e-8)) >> 20 & 0x7FFu);
+  if (sum == 0.0) return 0;
+  return e < 1022 - 200 || e > 1022 + 200 ? kBadRow : e - 1022;
+}
+
+// A line's sums in FP64, M(i,l) at M[i * si + l * sl].
+template <int P>
+__device__ __noinline__ void ops_line_fp64(const double* __restrict__ M, int si, int sl,
+                                           const double* F, int fs, double* out, int os) {
+  constexpr int N = P + 1;
+  double r[N];
+#pragma unroll 1
+  for (int i = 0; i < N; i++) {
+    double s = M[i * si] * F[0];
+#pragma unroll 1
+    for (int l = 1; l < N; l++) s = fma(M[i * si + l * sl], F[l * fs], s);
+    r[i] = s;
+  }
+  for (int i = 0; i < N; i++) out[i * os] = r[i];  // out may be F
+}
+
+// One line: out(i) = sum_l M(i,l) F(l), F at in with
+// stride S, out with SO (one array, for lines in shared memory); T and row are the
+// matrix's limbs and row exponents, M, si, sl the matrix itself.
+template <int P, int S, int SO>
+__device__ __forceinline__ void ops_line(const fixlimb* T, const int* row, bool ok,
+                                         const double* __restrict__ M, int si, int sl,
+                                         const double* in, double* out) {
+  constexpr int N = P + 1;
+  double F[N];
+  int32_t E = 0;
+#pragma unroll
+  for (int l = 0; l < N; l++) {
+    F[l] = in[l * S];
+    E = max(E, fix_value_exp(F[l]));
+  }
+  if (!ok || !fix_in_range(E)) {
+    ops_line_fp64<P>(M, si, sl, in, S, out, SO);
+    return;
+  }
+  fixlimb f[N];
+#pragma unroll
+  for (int l = 0; l < N; l++) f[l] = fix_split(fix_align(F[l], E));
+  const int B = fix_line_exp(E) - 61;
+#pragma unroll 2
+  for (int i = 0; i < N; i++) {
+    fixacc o;
+    fix_mul(o, T[i * N], f[0]);
+#pragma unroll
+    for (int l = 1; l < N; l++) fix_fma(o, T[i * N + l], f[l]);
+    const int64_t v = fix_sum(o);
+    const double r = fix_to_double(v, B + row[i]);
+    out[i * SO] = v == 0 ? 0.0 : r;
+  }
+}
+
+template <int P>
+__host__ __device__ constexpr size_t ops_smem() {
+  using Sh = FixShape<P>;
+  return sizeof(double) * Sh::EPB * Sh::EW + sizeof(fixlimb) * 2 * Sh::N2 + sizeof(int) * 2 * Sh::N;
+}
+
+// GRAD: the three derivatives of one field (a.ix; a null output is skipped),
+// else one of each of three.  Blocks walk the elements with a grid stride, so
+// the matrices become limbs once a block; thread r of an element owns line r of
+// each direction.  y and z lines are read and written in place, coalesced along
+// i; x lines go through shared memory.
+template <int P, bool GRAD>
+__global__ void __launch_bounds__(FixShape<P>::THREADS, 1024 / FixShape<P>::THREADS)
+    ops_kernel(const DivArgs a) {
+  using Sh = FixShape<P>;
+  constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NS = Sh::NS, EW = Sh::EW, EPB = Sh::EPB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* sF = reinterpret_cast<double*>(smem_raw);
+  fixlimb* sT = reinterpret_cast<fixlimb*>(sF + EPB * EW);  // D1D, then D1D_tr: (i, l)
+  int* sRow = reinterpret_cast<int*>(sT + 2 * N2);
+  const int le = threadIdx.x / N2, r = threadIdx.x - le * N2;
+  const int i = r % N, j = r / N;
+  auto M = [&](int k) {  // entry k of the two matrices, (i, l) at i N + l
+    const int w = k % N2;
+    return k < N2 ? a.D[w / N + (w % N) * N] : a.Dt[w % N + (w / N) * N];
+  };
+  for (int t = threadIdx.x; t < 2 * N; t += blockDim.x) {
+    double s = 0.0;
+    for (int l = 0; l < N; l++) s += fabs(M(t * N + l));
+    sRow[t] = fix_row_exp(s);
+  }
+  __syncthreads();
+  bool bad = false;
+  for (int t = threadIdx.x; t < 2 * N2; t += blockDim.x) {
+    const int k = sRow[t / N];
+    bad |= k == kBadRow;
+    sT[t] = fix_coef(fix_unit(k == kBadRow ? 0.0 : M(t) * __hiloint2double((1023 - k) << 20, 0)));
+  }
+  const bool ok = !__syncthreads_or(bad);
+  double* sE = sF + le * EW;
+  for (long long eb = (long long)blockIdx.x * EPB; eb < a.nelem;
+       eb += (long long)gridDim.x * EPB) {
+    const bool on = le < EPB && eb + le < a.nelem;
+    const long long g = (eb + le) * NP;
+    const int zat = i + NS * j;
+    if (on && (GRAD || a.ox)) {
+#pragma unroll
+      for (int m = 0; m < N; m++) sE[zat + m * NS * N] = a.ix[g + r + m * N2];
+    }
+    if (!GRAD && on) {
+      ops_line<P, N, N>(sT + N2, sRow + N, ok, a.Dt, N, 1, a.iy + g + i + j * N2,
+                     a.oy + g + i + j * N2);
+      ops_line<P, N2, N2>(sT + N2, sRow + N, ok, a.Dt, N, 1, a.iz + g + r, a.oz + g + r);
+    }
+    __syncthreads();
+    if (GRAD && on) {
+      // from shared memory, the results straight out
+      if (a.oy) ops_line<P, NS, N>(sT + N2, sRow + N, ok, a.Dt, N, 1, sE + i + NS * N * j,
+                                      a.oy + g + i + j * N2);
+      if (a.oz) ops_line<P, NS * N, N2>(sT + N2, sRow + N, ok, a.Dt, N, 1, sE + zat,
+                                           a.oz + g + r);
+    }
+    if (!GRAD || a.ox) {
+      if (GRAD) __syncthreads();
+      if (on) ops_line<P, 1, 1>(sT, sRow, ok, a.D, 1, N, sE + NS * r, sE + NS * r);
+      __syncthreads();
+      if (on) {
+#pragma unroll
+        for (int m = 0; m < N; m++) a.ox[g + r + m * N2] = sE[zat + m * NS * N];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int P, bool GRAD>
+int launch_ops(const DivArgs& a, cudaStream_t st) {
+  using Sh = FixShape<P>;
+  if (a.nelem <= 0) return SDG_OK;
+  constexpr size_t smem = ops_smem<P>();
+  SDG_TRY(set_kernel_smem((const void*)ops_kernel<P, GRAD>, (int)smem, true));
+  // as many blocks as the registers let reside
+  const long long nblk = ((long long)a.nelem + Sh::EPB - 1) / Sh::EPB;
+  const long long most = 152LL * (1024 / Sh::THREADS);
+  ops_kernel<P, GRAD><<<(unsigned)std::min(nblk, most), Sh::THREADS, smem, st>>>(a);
+  SDG_CUDA_TRY(cudaGetLastError());
+  return SDG_OK;
+}
+
+}  // namespace sdg

@@ -33,7 +33,7 @@
 // which gathers 14 values a face node, by them alone (the FP64 pipe 44 %).
 #pragma once
 
-#include "sdg_stage_eo.cuh"
+#include "sdg_dropin_ops.cuh"
 #include "sdg_stage_fix.cuh"
 
 namespace sdg {
@@ -49,7 +49,7 @@ struct RefArgs {
   const double* Dt;
   const double* Lift;
   // tables (ref_tables_kernel): rows of coefficients times 2^-row, the rows'
-  // exponents (kRefBadRow: out of range), the nodes' lift limbs (not EO)
+  // exponents (kBadRow: out of range), the nodes' lift limbs (not EO)
   const double* tab;
   const int* row;
   const int4* lift;
@@ -73,8 +73,6 @@ struct RefArgs {
   int Ne;
   double a, b, dt;      // q_out = a q0 + b (q + dt dqdt)
 };
-
-constexpr int kRefBadRow = 1 << 20;
 
 template <int P, bool EO>
 struct RefShape {
@@ -104,13 +102,6 @@ struct RefShape {
   }
 };
 
-// The exponent of a row whose magnitudes add up to sum (with room for the
-// rounding of the sum and of a coefficient's high limb), kRefBadRow outside +-200.
-__device__ __forceinline__ int ref_row_exp(double sum) {
-  const int e = (int)((unsigned)__double2hiint(sum * (1.0 + 1e-8)) >> 20 & 0x7FFu);
-  if (sum == 0.0) return 0;
-  return e < 1022 - 200 || e > 1022 + 200 ? kRefBadRow : e - 1022;
-}
 __device__ __forceinline__ double ref_pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 
 // Escale of a direction: its exponent x (Es = sig 2^x, sig in [0.5, 1)), and
@@ -193,7 +184,7 @@ __global__ void __launch_bounds__(256) ref_tables_eo_kernel(const double* __rest
     double most = pair(i < H ? Sh::OFF_B + i : Sh::OFF_A + i, Sh::OFF_A + i);
     for (int l = 0; l < H; l++) most += pair(Sh::OFF_E + i * H + l, Sh::OFF_O + i * H + l);
     if (i < H && Sh::ODD) most += fabs(T[Sh::OFF_DM + i]);
-    row[t] = sRow[t] = ref_row_exp(most);
+    row[t] = sRow[t] = fix_row_exp(most);
   }
   unsigned long long mD = 0, mL = 0;
   for (int t = threadIdx.x; t < NQ2; t += blockDim.x)
@@ -205,7 +196,7 @@ __global__ void __launch_bounds__(256) ref_tables_eo_kernel(const double* __rest
   __syncthreads();
   for (int t = threadIdx.x; t < 3 * TE; t += blockDim.x) {
     const int w = t % TE, k = sRow[t / TE * Sh::HR + Rs::row_of_entry(w)];
-    const double c = k == kRefBadRow ? sT[t] : sT[t] * ref_pow2(-k);
+    const double c = k == kBadRow ? sT[t] : sT[t] * ref_pow2(-k);
     tab[t] = c;
     if (shared)
       shared[t] = ref_coef(c, Rs::derivative(w), ref_escale_sig(Es[(t / TE) * NpNe]));
@@ -258,9 +249,9 @@ __global__ void __launch_bounds__(256) ref_tables_kernel(const double* __restric
   auto Dv = [&](int l) { return d == 0 ? D[i + l * N] : Dt[l + i * N]; };
   double sum = __longlong_as_double((long long)smax);
   for (int l = 0; l < N; l++) sum += fabs(Dv(l));
-  const int k = ref_row_exp(sum);
+  const int k = fix_row_exp(sum);
   if (r == 0) row[blockIdx.x] = k;
-  const double scale = k == kRefBadRow ? 1.0 : ref_pow2(-k);
+  const double scale = k == kBadRow ? 1.0 : ref_pow2(-k);
   if (r < N) {
     const double c = Dv(r) * scale;
     tab[blockIdx.x * N + r] = c;
@@ -309,7 +300,7 @@ __device__ __noinline__ void ref_line_fp64(const RefArgs* a, int ax, int r, cons
 #pragma unroll 1
   for (int i = 0; i < Sh::HR; i++) {
     const int k = a->row[ax * Sh::HR + i];
-    const double c = k == kRefBadRow ? -1.0 : -ref_pow2(k);
+    const double c = k == kBadRow ? -1.0 : -ref_pow2(k);
     double o = T[Sh::OFF_O + i * H] * d[0];
 #pragma unroll
     for (int l = 1; l < H; l++) o = fma(T[Sh::OFF_O + i * H + l], d[l], o);
@@ -476,7 +467,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
       mix |= xe[d] < -150 || xe[d] > 150;
       same = same && __double_as_longlong(es[d]) == __double_as_longlong(Es[d * NpNe]);
     }
-    for (int t = r; t < 3 * ROWS; t += N2) mix |= a.row[t] == kRefBadRow;
+    for (int t = r; t < 3 * ROWS; t += N2) mix |= a.row[t] == kBadRow;
     if (mix) sMix[le] = 1;
 #pragma unroll
     for (int m = 0; m < N; m++) {

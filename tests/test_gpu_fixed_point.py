@@ -190,3 +190,52 @@ def test_loop_with_the_least_scratch(opt, p):
             assert err.numpy()[0] == 0
             out.append(q.numpy()[: c.nown])
     assert rel_l2(out[1], out[0]) <= TOL_TEND
+
+
+@pytest.mark.parametrize("p,nelem", [(1, 20011), (2, 5600), (3, 2400), (6, 441), (7, 301), (8, 207),
+                                     (10, 113), (11, 1), (12, 5), (15, 3), (15, 40)])
+def test_contractions_in_fixed_point(p, nelem):
+    """divlike, gradlike and the single directions on both sides of the element
+    counts that choose the kernel: unsymmetric matrices, steep fields, zero
+    lines, and lines with infinities, NaN and extreme magnitudes."""
+    import sdg
+    N = p + 1
+    r = np.random.RandomState(p)
+    D, Dt = r.randn(N * N), r.randn(N * N)
+    D[0] = 0.0
+    f = [np.exp(-20 * r.rand(nelem * N ** 3)) * r.randn(nelem * N ** 3) for _ in range(3)]
+    f[0][: N ** 3] = 0.0
+    f[1][5] = np.inf
+    f[2][N ** 3 - 1] = np.nan
+    f[0][-1] = 1e300
+    f[1][-2] = 1e-300
+
+    def along(a, axis):
+        a = a.reshape(nelem, N, N, N).astype(np.longdouble)
+        M = (D if axis == 0 else Dt).reshape(N, N).astype(np.longdouble)
+        M = M.T if axis == 0 else M  # (out, in)
+        return np.moveaxis(np.tensordot(a, M, axes=([3 - axis], [1])), -1, 3 - axis).reshape(-1)
+
+    def check(got, want):
+        fine = np.isfinite(want)
+        assert np.array_equal(np.isfinite(got), fine)
+        # each line against its own size: 1e-12 of the sum of its terms' magnitudes
+        assert rel_l2(got[fine & (np.abs(want) < 1e200)],
+                      want[fine & (np.abs(want) < 1e200)].astype(float)) <= TOL_TEND
+        big = fine & (np.abs(want) >= 1e200)
+        if big.any():
+            assert rel_l2(got[big] * 2.0 ** -700, (want[big] * np.longdouble(2) ** -700).astype(float)) \
+                <= TOL_TEND
+
+    with np.errstate(all="ignore"):
+        sdg.dg_optr_kernel_setup("OPT1")
+        for axis, got in enumerate(sdg.tensorprod_divlike_dirXYZ(D, Dt, *f, N)):
+            check(got, along(f[axis], axis))
+        for axis, got in enumerate(sdg.tensorprod_gradlike_dirXYZ(D, Dt, f[0], N)):
+            check(got, along(f[0], axis))
+        for axis in range(3):
+            got = sdg.element_matvec_dir(axis + 1, D if axis == 0 else Dt, f[axis], N)
+            check(got, along(f[axis], axis))
+    # the first element's zero z lines (the last holds the 1e300 when it is alone)
+    zero = sdg.tensorprod_gradlike_dirXYZ(D, Dt, f[0], N)[2][: N * N - 1]
+    assert np.all(zero == 0.0)
