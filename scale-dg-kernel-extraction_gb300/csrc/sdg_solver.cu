@@ -4,6 +4,7 @@
 // without update_halo).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -43,6 +44,12 @@ struct sdg_solver {
   // its device table of lift limbs
   FixTables fix;
   void* fix_lift = nullptr;
+  // whole step calls in one launch (sdg_stage_loop.cuh): the most elements it
+  // takes (-1: not asked for yet), its two barrier words, whether it ran since
+  // the second was last looked at
+  long long loop_most = -1;
+  unsigned* bar = nullptr;  // in D's allocation
+  bool loop_ran = false;
   // elements a stage advances: [elem_begin, elem_begin + elem_count) of the
   // box (the whole box by default; a z-slab partition advances its owned
   // layers and keeps a ghost layer on each side)
@@ -91,6 +98,12 @@ void release(sdg_solver* s) {
   cudaFree(s->fix_lift);
 }
 
+// No grid of one-launch steps holds more elements (152 SMs of 1024 threads, 12
+// threads an element at p = 1): spares larger boxes the question.
+constexpr long long kLoopElems = 152 * 1024 / 12;
+// Steps of one launch: some 10-100 ms, past any gain from more.
+constexpr int kLoopSteps = 1024;
+
 // fc: 0 = the stage forms the face-flux velocity factors inline, 1 = it also
 // stores them in s->fc, 2 = it reads them from s->fc (an earlier stage of
 // the same call, same velocity, stored them); 1 and 2 apply only when s->fc
@@ -104,9 +117,9 @@ int one_stage(sdg_solver* s, int stage, double dt, const double* qin,
   return one_stage_on(s, stage, dt, qin, q0, qout, s->u, s->v, s->w, s->stream, tend_only, fc);
 }
 
-int one_stage_on(sdg_solver* s, int stage, double dt, const double* qin, const double* q0,
-                 double* qout, const void* u, const void* v, const void* w, cudaStream_t st,
-                 bool tend_only, int fc) {
+StageArgs stage_args(const sdg_solver* s, int stage, double dt, const double* qin,
+                     const double* q0, double* qout, const void* u, const void* v, const void* w,
+                     bool tend_only, int fc) {
   static const double rk_a[3] = {0.0, 0.75, 1.0 / 3.0};  // mod_common.f90:28-30
   static const double rk_b[3] = {1.0, 0.25, 2.0 / 3.0};
   StageArgs a{};
@@ -137,7 +150,41 @@ int one_stage_on(sdg_solver* s, int stage, double dt, const double* qin, const d
     a.eo_sDf[d] = (float)(-c * s->box.Es[d]);
     a.eo_sLf[d] = (float)(-c * (0.25 * s->box.Fs[d]));
   }
-  return launch_stage(s->p, s->prec, s->opt, a, st);
+  return a;
+}
+
+int one_stage_on(sdg_solver* s, int stage, double dt, const double* qin, const double* q0,
+                 double* qout, const void* u, const void* v, const void* w, cudaStream_t st,
+                 bool tend_only, int fc) {
+  return launch_stage(s->p, s->prec, s->opt,
+                      stage_args(s, stage, dt, qin, q0, qout, u, v, w, tend_only, fc), st);
+}
+
+// Whether a step call of the whole box runs as one launch (a captured call
+// keeps its launch a stage).
+int takes_loop(sdg_solver* s, bool* yes) {
+  *yes = false;
+  if (s->prec == SDG_PREC_FP32 || s->elem_count >= 0 || s->box.Ne > kLoopElems) return SDG_OK;
+  if (s->loop_most < 0)
+    SDG_TRY(launch_loop(s->p, s->opt, StageArgs{}, nullptr, 0.0, 0, nullptr, &s->loop_most,
+                        nullptr));
+  if (s->box.Ne > s->loop_most) return SDG_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s->stream, &cap) != cudaSuccess) cudaGetLastError();
+  *yes = cap == cudaStreamCaptureStatusNone;
+  return SDG_OK;
+}
+
+// After a synchronisation: whether a wait of the one-launch steps ran out.
+int loop_status(sdg_solver* s) {
+  if (!s->loop_ran) return SDG_OK;
+  s->loop_ran = false;
+  unsigned bar[2] = {0, 0};
+  SDG_CUDA_TRY(cudaMemcpyAsync(bar, s->bar, sizeof(bar), cudaMemcpyDeviceToHost, s->stream));
+  SDG_CUDA_TRY(cudaStreamSynchronize(s->stream));
+  if (bar[1] == 0) return SDG_OK;
+  SDG_CUDA_TRY(cudaMemsetAsync(s->bar, 0, sizeof(bar), s->stream));
+  return fail(SDG_ERR_TIMEOUT, "a wait between the stages of a step ran out");
 }
 
 // Uploads one velocity component (device source) in the compute type.
@@ -222,6 +269,9 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
   if (e == cudaSuccess) e = cudaMalloc(&s->u, es * (size_t)s->ndof);
   if (e == cudaSuccess) e = cudaMalloc(&s->v, es * (size_t)s->ndof);
   if (e == cudaSuccess) e = cudaMalloc(&s->w, es * (size_t)s->ndof);
+  // the barrier words of the one-launch steps follow the tables, zero
+  const size_t bar_at = (dtab.size() + 255) & ~size_t(255);
+  dtab.resize(bar_at + 256, 0);
   if (e == cudaSuccess) e = cudaMalloc(&s->D, dtab.size());
   if (e == cudaSuccess) e = cudaMalloc(&s->Lift, ltab.size());
   const size_t fc_bytes = 16 * (size_t)(6 * s->Nq * s->Nq) * (size_t)s->box.Ne;
@@ -237,6 +287,7 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
     s->fc = nullptr;
   }
   if (e == cudaSuccess) e = cudaMemcpy(s->D, dtab.data(), dtab.size(), cudaMemcpyHostToDevice);
+  s->bar = reinterpret_cast<unsigned*>(static_cast<char*>(s->D) + bar_at);
   if (e == cudaSuccess)
     e = cudaMemcpy(s->Lift, ltab.data(), ltab.size(), cudaMemcpyHostToDevice);
   (void)nD;
@@ -376,6 +427,20 @@ int sdg_solver_upload(sdg_solver* s, const double* q, const double* u,
 int sdg_solver_step(sdg_solver* s, double dt, int nstep) {
   if (!s) return fail(SDG_ERR_INVALID_ARG, "NULL solver");
   if (nstep < 0) return fail(SDG_ERR_INVALID_ARG, "nstep < 0");
+  bool loop = false;
+  if (nstep > 0) SDG_TRY(takes_loop(s, &loop));
+  if (loop) {
+    for (int left = nstep; left > 0;) {
+      const int n = std::min(left, kLoopSteps);
+      double* q[3] = {s->q[s->cur], s->q[(s->cur + 1) % 3], s->q[(s->cur + 2) % 3]};
+      const StageArgs a = stage_args(s, 0, dt, q[0], nullptr, q[1], s->u, s->v, s->w, false, 0);
+      SDG_TRY(launch_loop(s->p, s->opt, a, q, dt, n, s->bar, nullptr, s->stream));
+      s->loop_ran = true;
+      s->cur = (s->cur + n) % 3;
+      left -= n;
+    }
+    return SDG_OK;
+  }
   for (int it = 0; it < nstep; it++) {
     const int s0 = s->cur, s1 = (s->cur + 1) % 3, s2 = (s->cur + 2) % 3;
     // the velocity cannot change within one call: the first stage of the
@@ -410,12 +475,13 @@ int sdg_solver_step_timed(sdg_solver* s, double dt, int nstep, double* ms) {
   if (ce != cudaSuccess) return cuda_fail(ce, "solver timing", __FILE__, __LINE__);
   if (st != SDG_OK) return st;
   *ms = f;
-  return SDG_OK;
+  return loop_status(s);
 }
 
 int sdg_solver_minmax(sdg_solver* s, double* qmin, double* qmax) {
   if (!s || !qmin || !qmax) return fail(SDG_ERR_INVALID_ARG, "NULL argument");
-  return sdg_minmax_dev(s->q[s->cur], s->ndof, qmin, qmax, s->stream);
+  SDG_TRY(sdg_minmax_dev(s->q[s->cur], s->ndof, qmin, qmax, s->stream));
+  return loop_status(s);
 }
 
 // The reference's time loop with its diagnostic output (main.f90:51-80): nstep
@@ -450,7 +516,7 @@ int sdg_solver_run(sdg_solver* s, double dt, int nstep, int output_interval, dou
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) return cuda_fail(e, "sdg_solver_run", __FILE__, __LINE__);
   for (size_t i = 0; i < hk.size(); i++) records[i] = minmax_key_to_double(hk[i]);
-  return SDG_OK;
+  return loop_status(s);
 }
 
 int sdg_solver_tendency(sdg_solver* s, double* dqdt) {
@@ -557,7 +623,7 @@ int sdg_solver_download(sdg_solver* s, double* q) {
   SDG_CUDA_TRY(cudaMemcpyAsync(q, s->q[s->cur], 8 * (size_t)s->ndof,
                                cudaMemcpyDeviceToHost, s->stream));
   SDG_CUDA_TRY(cudaStreamSynchronize(s->stream));
-  return SDG_OK;
+  return loop_status(s);
 }
 
 const double* sdg_solver_state_dev(const sdg_solver* s) { return s ? s->q[s->cur] : nullptr; }

@@ -6,6 +6,7 @@
 #include "sdg_stage_elem.cuh"
 #include "sdg_stage_eo.cuh"
 #include "sdg_stage_fix.cuh"
+#include "sdg_stage_loop.cuh"
 #include "sdg_stage_warp.cuh"
 
 namespace sdg {
@@ -29,5 +30,27 @@ int launch_stage_order(int prec, int opt, const StageArgs& a, cudaStream_t st) {
   if (split) return launch_stage_impl<P, float, float, kCanSplit>(a, st);
   return launch_stage_impl<P, float, float, false>(a, st);
 }
+
+// A whole step call of a small box in one launch (sdg_stage_loop.cuh); with q
+// null only *most, the most elements such a launch takes.
+template <int P>
+int launch_loop_order(int opt, const StageArgs& a, double* const* q, double dt, int nstep,
+                      unsigned* bar, long long* most, cudaStream_t st) {
+  const bool eo = opt == SDG_OPT_EVENODD;
+  if (!q) return eo ? fix_loop_most<P, true>(most) : fix_loop_most<P, false>(most);
+  return eo ? launch_stage_fix_loop<P, true>(a, q, dt, nstep, bar, st)
+            : launch_stage_fix_loop<P, false>(a, q, dt, nstep, bar, st);
+}
+
+// The entry points of one order (one translation unit per group of orders, so
+// that the build compiles them in parallel).
+#define SDG_DEFINE_ORDER(p)                                                                 \
+  int launch_stage_p##p(int prec, int opt, const StageArgs& a, cudaStream_t st) {           \
+    return launch_stage_order<p>(prec, opt, a, st);                                         \
+  }                                                                                         \
+  int launch_loop_p##p(int opt, const StageArgs& a, double* const* q, double dt, int nstep, \
+                       unsigned* bar, long long* most, cudaStream_t st) {                   \
+    return launch_loop_order<p>(opt, a, q, dt, nstep, bar, most, st);                       \
+  }
 
 }  // namespace sdg

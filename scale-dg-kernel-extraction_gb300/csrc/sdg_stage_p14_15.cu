@@ -1,12 +1,7 @@
-// Instantiations of the fused stage kernel for orders 14 15 (one translation
-// unit per group so that the build compiles them in parallel).
+// Instantiations of the stage kernels for orders 14, 15.
 #include "sdg_stage_order.cuh"
 
 namespace sdg {
-int launch_stage_p14(int prec, int opt, const StageArgs& a, cudaStream_t st) {
-  return launch_stage_order<14>(prec, opt, a, st);
-}
-int launch_stage_p15(int prec, int opt, const StageArgs& a, cudaStream_t st) {
-  return launch_stage_order<15>(prec, opt, a, st);
-}
+SDG_DEFINE_ORDER(14)
+SDG_DEFINE_ORDER(15)
 }  // namespace sdg

@@ -1,9 +1,6 @@
-// Instantiations of the fused stage kernel for orders 7 (one translation
-// unit per group so that the build compiles them in parallel).
+// Instantiations of the stage kernels for order 7.
 #include "sdg_stage_order.cuh"
 
 namespace sdg {
-int launch_stage_p7(int prec, int opt, const StageArgs& a, cudaStream_t st) {
-  return launch_stage_order<7>(prec, opt, a, st);
-}
+SDG_DEFINE_ORDER(7)
 }  // namespace sdg

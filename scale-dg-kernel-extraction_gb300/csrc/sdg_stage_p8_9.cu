@@ -1,12 +1,7 @@
-// Instantiations of the fused stage kernel for orders 8 9 (one translation
-// unit per group so that the build compiles them in parallel).
+// Instantiations of the stage kernels for orders 8, 9.
 #include "sdg_stage_order.cuh"
 
 namespace sdg {
-int launch_stage_p8(int prec, int opt, const StageArgs& a, cudaStream_t st) {
-  return launch_stage_order<8>(prec, opt, a, st);
-}
-int launch_stage_p9(int prec, int opt, const StageArgs& a, cudaStream_t st) {
-  return launch_stage_order<9>(prec, opt, a, st);
-}
+SDG_DEFINE_ORDER(8)
+SDG_DEFINE_ORDER(9)
 }  // namespace sdg

@@ -239,3 +239,26 @@ def test_contractions_in_fixed_point(p, nelem):
     # the first element's zero z lines (the last holds the 1e300 when it is alone)
     zero = sdg.tensorprod_gradlike_dirXYZ(D, Dt, f[0], N)[2][: N * N - 1]
     assert np.all(zero == 0.0)
+
+
+@both
+@pytest.mark.parametrize("p,dims", [(1, (5, 4, 3)), (1, (20, 19, 17)), (2, (7, 3, 2)),
+                                    (3, (16, 19, 10)), (3, (1, 1, 1)), (5, (4, 5, 3)),
+                                    (7, (8, 5, 19)), (7, (2, 1, 3)), (8, (5, 4, 4)),
+                                    (11, (3, 2, 4)), (12, (3, 3, 2)), (15, (2, 3, 2))])
+@pytest.mark.parametrize("nstep", [1, 5, 1100])
+def test_steps_in_one_launch_equal_a_launch_a_stage(opt, p, dims, nstep):
+    """Whole step calls of small boxes (one resident grid) against the same box as
+    one z-slab, whose stages are launches of their own: the same bits, also over
+    calls that follow one another and with a non-finite state in a corner."""
+    import sdg
+    c = Case(*dims, p)
+    q, u, v, w = _fields(c)
+    q[-1] = np.inf if nstep == 5 else q[-1]
+    a = sdg.Solver(*dims, p, c.D, c.Lift, opt=getattr(sdg, opt))
+    b = sdg.Slabs(*dims, p, c.D, c.Lift, 1, opt=getattr(sdg, opt))
+    for s in (a, b):
+        s.upload(q, u, v, w)
+        s.step(c.dt, nstep)
+        s.step(0.5 * c.dt, 2)
+    assert np.array_equal(a.download(), b.download(), equal_nan=True)
