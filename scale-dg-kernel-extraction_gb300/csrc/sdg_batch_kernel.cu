@@ -390,8 +390,8 @@ static int batch_fused_enqueue(BatchInst* d_inst, int n_inst, const BatchItem* d
     smem = g.smem > smem ? g.smem : smem;
   }
   if (n_items > 0) {
-    SDG_TRY(set_kernel_smem((const void*)batch_stage_kernel<kRkFirst>, (int)smem, false));
-    SDG_TRY(set_kernel_smem((const void*)batch_stage_kernel<kRkGeneral>, (int)smem, false));
+    SDG_TRY(set_kernel_smem((const void*)batch_stage_kernel<kRkFirst>, (int)smem, kCarveDefault));
+    SDG_TRY(set_kernel_smem((const void*)batch_stage_kernel<kRkGeneral>, (int)smem, kCarveDefault));
     int dev = 0, nsm = 0, per_sm = 0;
     SDG_CUDA_TRY(cudaGetDevice(&dev));
     SDG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));

@@ -171,7 +171,7 @@ int launch_ops(const DivArgs& a, cudaStream_t st) {
   using Sh = FixShape<P>;
   if (a.nelem <= 0) return SDG_OK;
   constexpr size_t smem = ops_smem<P>();
-  SDG_TRY(set_kernel_smem((const void*)ops_kernel<P, GRAD>, (int)smem, true));
+  SDG_TRY(set_kernel_smem((const void*)ops_kernel<P, GRAD>, (int)smem, kCarveMax));
   // as many blocks as the registers let reside
   const long long nblk = ((long long)a.nelem + Sh::EPB - 1) / Sh::EPB;
   const long long most = 152LL * (1024 / Sh::THREADS);

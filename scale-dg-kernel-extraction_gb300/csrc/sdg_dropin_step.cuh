@@ -25,12 +25,12 @@
 // node's lift entries (GENERAL, OPT1).
 //
 // Measured on GB300 at about 7M DOF against the FP64 kernels this replaced
-// (GDOF-updates/s): the time loop at p = 7 42.0 from 18.2 (EVENODD) and 35.2
-// from 10.7 (OPT1), p = 3 38.9 / 34.6 from 19.1 / 10.7, p = 15 34.4 / 22.3 from
-// 13.1 / 6.8; the per-stage calls 19.9 from 10.6 at p = 7.  A stage is bound by
+// (GDOF-updates/s): the time loop at p = 7 46.9 from 18.2 (EVENODD) and 39.7
+// from 10.7 (OPT1), p = 3 43.8 / 38.8 from 19.1 / 10.7, p = 15 34.4 / 22.3 from
+// 13.1 / 6.8; the per-stage calls 24.5 from 10.6 at p = 7.  A stage is bound by
 // the latency of its gathers and loads (long-scoreboard stalls 6.5 of 17 cycles
-// an instruction, 32 warps an SM) with the FP64 pipe 44-60 % busy; a tendency,
-// which gathers 14 values a face node, by them alone (the FP64 pipe 44 %).
+// an instruction, 32 warps an SM); a tendency, which gathers 14 values a face
+// node, by them alone.
 #pragma once
 
 #include "sdg_dropin_ops.cuh"
@@ -571,8 +571,12 @@ int launch_ref_mode(const RefArgs& a, cudaStream_t st) {
   const int epb = threads / N2;
   const long long nblk = ((long long)a.Ne + epb - 1) / epb;
   if (nblk == 0) return SDG_OK;
-  SDG_TRY(set_kernel_smem((const void*)step_ref_kernel<P, EO, MODE>,
-                          (int)ref_smem<P, EO>(FixShape<P>::EPB), true));
+  // carveout: the gathers of the faces live on L1 hits, as in launch_stage_fix_kind
+  // (loop, even-odd, 24^3: p = 2 34.5 from 26.3, p = 4 42.1 from 33.2, p = 7 46.9
+  // from 42.0 GDOF-updates/s; level at p = 15, whose blocks need all of it)
+  constexpr size_t smem = ref_smem<P, EO>(FixShape<P>::EPB);
+  SDG_TRY(set_kernel_smem((const void*)step_ref_kernel<P, EO, MODE>, (int)smem,
+                          carve_for(smem, ref_min_blocks<P, EO>())));
   step_ref_kernel<P, EO, MODE><<<(unsigned)nblk, threads, ref_smem<P, EO>(epb), st>>>(a);
   SDG_CUDA_TRY(cudaGetLastError());
   return SDG_OK;

@@ -39,28 +39,27 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
               line);
 }
 
-int set_kernel_smem(const void* func, int smem, bool max_carveout) {
+int set_kernel_smem(const void* func, int smem, int carve) {
   int dev = 0;
   SDG_CUDA_TRY(cudaGetDevice(&dev));
   struct Key {
     const void* func;
-    int dev, smem;
-    bool carve;
+    int dev, smem, carve;
     bool operator==(const Key& o) const {
       return func == o.func && dev == o.dev && smem == o.smem && carve == o.carve;
     }
   };
   static std::mutex mu;
   static std::vector<Key> done;  // a few dozen kernels at most
-  const Key k{func, dev, smem, max_carveout};
+  const Key k{func, dev, smem, carve};
   {
     std::lock_guard<std::mutex> g(mu);
     if (std::find(done.begin(), done.end(), k) != done.end()) return SDG_OK;
   }
   SDG_CUDA_TRY(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  if (max_carveout)
-    SDG_CUDA_TRY(cudaFuncSetAttribute(func, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                      (int)cudaSharedmemCarveoutMaxShared));
+  if (carve != kCarveDefault)
+    SDG_CUDA_TRY(
+        cudaFuncSetAttribute(func, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
   std::lock_guard<std::mutex> g(mu);
   if (std::find(done.begin(), done.end(), k) == done.end()) done.push_back(k);
   return SDG_OK;

@@ -33,12 +33,20 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
-// Raises a kernel's dynamic shared-memory limit to smem bytes (and, when
-// asked, prefers the largest shared-memory carveout) on the current device.
+// Raises a kernel's dynamic shared-memory limit to smem bytes and sets its
+// preferred shared-memory carveout in percent (kCarveDefault: the driver's
+// choice) on the current device.
 // Kernel attributes are per device, so this records (kernel, device, smem)
 // and sets them once per device; it is safe to call from several host
 // threads at once.
-int set_kernel_smem(const void* func, int smem, bool max_carveout);
+int set_kernel_smem(const void* func, int smem, int carve);
+constexpr int kCarveDefault = -1, kCarveMax = 100;
+// The carveout that holds `blocks` blocks of smem bytes on an SM (228 KB, 1 KB
+// of each block's taken by the system): what is left of the 256 KB is L1.
+constexpr int carve_for(size_t smem, int blocks) {
+  const size_t pct = (blocks * (smem + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024);
+  return pct < 100 ? (int)pct : 100;
+}
 
 // Checks the first CUDA device is usable; returns SDG_OK or an error status.
 int require_device();

@@ -343,7 +343,7 @@ template <int P, typename CT, typename VT, bool SPLIT3>
 int launch_stage_impl(const StageArgs& a, cudaStream_t st) {
   using C = StageCfg<P, CT>;
   constexpr size_t smem = stage_smem_bytes<P, CT, VT, SPLIT3>();
-  SDG_TRY(set_kernel_smem((const void*)stage_kernel<P, CT, VT, SPLIT3>, (int)smem, false));
+  SDG_TRY(set_kernel_smem((const void*)stage_kernel<P, CT, VT, SPLIT3>, (int)smem, kCarveDefault));
   const long long nblk = (a.elem_count + C::EPB - 1) / C::EPB;
   if (nblk <= 0) return SDG_OK;
   if (nblk > 0x7fffffffLL) return fail(SDG_ERR_INVALID_ARG, "too many elements");

@@ -5,10 +5,9 @@
 // the FP64 pipe 90 % busy at 19.8 GDOF-updates/s.  Here the even-odd pair
 // sums, the derivative and the lift are integer multiply-adds, and FP64 keeps
 // the products q u_d, the face flux and the RK update (6.8 instructions a
-// DOF): 62 GDOF-updates/s at p = 7 on 32^3 elements (270 us a stage, from
-// 848), 39-62 across p = 1..15 (from 13-22), the FP64 pipe 60-67 % and the
-// issue slots 41-47 % busy, with 32 warps an SM waiting on the loads of its
-// two ends.  Error of a tendency against a long-double one: 0.5-1.1 times the
+// DOF): 68 GDOF-updates/s at p = 7 on 32^3 elements (246 us a stage, from
+// 848), 46-68 across p = 1..15 (from 13-22), with 32 warps an SM waiting on
+// the loads of its two ends.  Error of a tendency against a long-double one: 0.5-1.1 times the
 // FP64 body's at every order, on smooth, narrow and random fields (the
 // coefficients' symmetrisation, common to both, dominates from p = 5).
 //
@@ -407,8 +406,14 @@ int launch_stage_fix_kind(const FixStageArgs<P, EO>& a, cudaStream_t st) {
   const long long nblk = (a.s.elem_count + epb - 1) / epb;
   if (nblk <= 0) return SDG_OK;
   if (nblk > 0x7fffffffLL) return fail(SDG_ERR_INVALID_ARG, "too many elements");
-  SDG_TRY(set_kernel_smem((const void*)stage_fix_kernel<P, EO, RK, FCIN>,
-                          (int)fix_smem<P>(FixShape<P>::EPB), true));
+  // no more shared memory than the resident blocks take: the rest of the SM's
+  // 256 KB is L1, from which a node's value is read again by the RK update and a
+  // face value by the threads that share its sector (all of it as shared memory:
+  // 55.0 against 58.4 GDOF-updates/s at p = 3, 64.0 against 68.2 at p = 7, 46.0
+  // against 53.3 at p = 11)
+  constexpr size_t smem = fix_smem<P>(FixShape<P>::EPB);
+  SDG_TRY(set_kernel_smem((const void*)stage_fix_kernel<P, EO, RK, FCIN>, (int)smem,
+                          carve_for(smem, fix_min_blocks<P>())));
   stage_fix_kernel<P, EO, RK, FCIN><<<(unsigned)nblk, threads, fix_smem<P>(epb), st>>>(a);
   SDG_CUDA_TRY(cudaGetLastError());
   return SDG_OK;

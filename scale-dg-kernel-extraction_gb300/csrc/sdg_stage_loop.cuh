@@ -27,6 +27,7 @@ struct LoopShape {
   static constexpr int EPB = N2 < 32 ? 32 / N2 : 1;           // elements a block
   static constexpr int G = (EPB * N2 + 31) / 32 * 32;         // threads a direction
   static constexpr int THREADS = 3 * G;
+  static constexpr int BLOCKS = THREADS > 512 ? 1 : 1024 / THREADS;   // resident, an SM
   static constexpr int IT = (EPB * N2 * N + THREADS - 1) / THREADS;  // nodes a thread
   static constexpr size_t SMEM =
       sizeof(int64_t) * 3 * EPB * FixShape<P>::EW + sizeof(short) * 3 * EPB * N2;
@@ -114,7 +115,7 @@ __device__ __forceinline__ int fix_loop_line(const FixStageArgs<P, EO>& a, const
 
 template <int P, bool EO>
 __global__ void __launch_bounds__(LoopShape<P>::THREADS,
-                                  LoopShape<P>::THREADS > 512 ? 1 : 1024 / LoopShape<P>::THREADS)
+                                  LoopShape<P>::BLOCKS)
     stage_fix_loop_kernel(const __grid_constant__ FixLoopArgs<P, EO> a) {
   using Ls = LoopShape<P>;
   using Args = FixStageArgs<P, EO>;
@@ -218,7 +219,7 @@ int launch_stage_fix_loop(const StageArgs& s, double* const* q, double dt, int n
   a.nstep = nstep;
   a.bar = bar;
   const void* kernel = (const void*)stage_fix_loop_kernel<P, EO>;
-  SDG_TRY(set_kernel_smem(kernel, (int)Ls::SMEM, true));
+  SDG_TRY(set_kernel_smem(kernel, (int)Ls::SMEM, carve_for(Ls::SMEM, Ls::BLOCKS)));
   const unsigned nblk = (unsigned)((s.elem_count + Ls::EPB - 1) / Ls::EPB);
   void* args[1] = {&a};
   SDG_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(nblk), dim3(Ls::THREADS), args, Ls::SMEM, st));
@@ -237,7 +238,7 @@ template <int P, bool EO>
 int fix_loop_most(long long* elems) {
   using Ls = LoopShape<P>;
   const void* kernel = (const void*)stage_fix_loop_kernel<P, EO>;
-  SDG_TRY(set_kernel_smem(kernel, (int)Ls::SMEM, true));
+  SDG_TRY(set_kernel_smem(kernel, (int)Ls::SMEM, carve_for(Ls::SMEM, Ls::BLOCKS)));
   int dev = 0, sms = 0, per = 0;
   SDG_CUDA_TRY(cudaGetDevice(&dev));
   SDG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -293,7 +293,7 @@ extern "C" int sdg_tensorprod_divlike_dirXYZ_f32_dev(float* out_x, float* out_y,
   switch (Nq) {
 #define SDG_F32_CASE(n)                                                                  \
   case n:                                                                                \
-    SDG_TRY(set_kernel_smem((const void*)divlike_f32_kernel<n>, (int)smem, false));      \
+    SDG_TRY(set_kernel_smem((const void*)divlike_f32_kernel<n>, (int)smem, kCarveDefault));      \
     divlike_f32_kernel<n><<<grid, 256, smem, st>>>(a);                                   \
     break;
     SDG_F32_CASE(2) SDG_F32_CASE(3) SDG_F32_CASE(4) SDG_F32_CASE(5) SDG_F32_CASE(6)
