@@ -107,6 +107,7 @@ struct StageArgs {
   // FP32 form's per-direction factors of its D part (-c*Es_d) and of its lift
   // part (-c*Fs_d/4), c = b*dt (1 for tend_only)
   float eo_sDf[3], eo_sLf[3];
+  const float* eo_host;  // FP32: the table on the host
   // FP64 stage: the velocity factors of the face flux, two per face node of
   // each element (2*Nfp*6 doubles an element).  A stage with
   // fc_out forms them from u, v, w and stores them; a stage with fc_in reads

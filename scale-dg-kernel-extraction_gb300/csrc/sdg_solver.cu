@@ -43,6 +43,7 @@ struct sdg_solver {
   // coefficients of the FP64 stage, and for operators as given (GENERAL, OPT1)
   // its device table of lift limbs
   FixTables fix;
+  std::vector<float> eo32;  // FP32 even-odd table on the host
   void* fix_lift = nullptr;
   // whole step calls in one launch (sdg_stage_loop.cuh): the most elements it
   // takes (-1: not asked for yet), its two barrier words, whether it ran since
@@ -143,6 +144,7 @@ StageArgs stage_args(const sdg_solver* s, int stage, double dt, const double* qi
   a.tend_only = tend_only ? 1 : 0;
   a.fc_out = (s->fc && fc == 1) ? s->fc : nullptr;
   a.fc_in = (s->fc && fc == 2) ? s->fc : nullptr;
+  a.eo_host = s->eo32.data();
   a.fix = &s->fix;
   a.fix_lift = s->fix_lift;
   const double c = tend_only ? 1.0 : a.b * dt;
@@ -251,9 +253,9 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
     }
     if (precision == SDG_PREC_FP32) {
       // the FP32 form reads FP32 tables
-      std::vector<float> f(tab.begin(), tab.end());
-      dtab.resize(4 * f.size());
-      std::memcpy(dtab.data(), f.data(), dtab.size());
+      s->eo32.assign(tab.begin(), tab.end());
+      dtab.resize(4 * tab.size());
+      std::memcpy(dtab.data(), s->eo32.data(), dtab.size());
     } else {
       dtab.resize(8 * tab.size());
       std::memcpy(dtab.data(), tab.data(), dtab.size());

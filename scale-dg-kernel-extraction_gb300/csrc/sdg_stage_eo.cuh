@@ -370,56 +370,4 @@ __device__ __forceinline__ void stage_eo_block(const StageArgs& a, long long eb,
   });
 }
 
-// Resident blocks an SM.  FP32, two threads a line (512 threads, or 256 at
-// p = 7, 9, 10 with twice the blocks): the body issues few instructions per
-// byte and needs warps to hide memory latency, so the registers are capped at
-// 32 for 64 warps (measured 1.0-1.16x the three-block build, 100 against 91.5
-// GDOF-updates/s at p = 7); at p = 15 shared memory admits three blocks and
-// the cap would only spill.  One thread a line (p <= 6 and 11..14): the
-// counts below, each measured on GB300 against its neighbours.
-template <int P, typename CT>
-__host__ __device__ constexpr int eo_min_blocks() {
-  if (P == 4) return 6;  // 40 registers, one thread a line (above)
-  if (P == 5) return 5;  // 48 registers, one thread a line
-  // one thread a line from p = 11 to 14 (eo_parts); p = 11, 12 in blocks
-  // sized to one element's lines (EoCfg: 160 and 192 threads)
-  if (P == 11) return 5;
-  if (P == 12 || P == 13) return 6;
-  if (P == 14) return 4;
-  return (P <= 3 || eo_lines<P, CT>() == 128) ? 8 : P <= 12 ? 4 : 3;
-}
-
-// FP32 single-box kernel: F_y / F_z formed on the fly (FLY) at the orders
-// where that measured faster on GB300 (1.07-1.18x at p = 10, 13 and 15, even
-// at 12 and 14); staging them is faster below (up to 1.15x at p = 6;
-// rechecked with the current shapes at p = 4, 6 and 8: FLY 0.92-0.99x).
-template <int P>
-__host__ __device__ constexpr bool eo_fly_single() {
-  return P == 10 || P >= 12;
-}
-
-template <int P, typename CT>
-__global__ void __launch_bounds__(EoCfg<P, CT>::THREADS, eo_min_blocks<P, CT>())
-    stage_eo_kernel(const StageArgs a) {
-  constexpr int EPB = EoCfg<P, CT>::EPB;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long long eb = a.elem_begin + (long long)blockIdx.x * EPB;
-  const long long eend = a.elem_begin + a.elem_count;
-  const int nloc = (int)((eend - eb) < EPB ? (eend - eb) : EPB);
-  if (nloc <= 0) return;
-  stage_eo_block<P, CT, -1, eo_fly_single<P>(), (P >= 4)>(a, eb, nloc, smem_raw);
-}
-
-template <int P, typename CT>
-int launch_stage_eo_impl(const StageArgs& a, cudaStream_t st) {
-  constexpr size_t smem = eo_block_smem<P, CT, eo_fly_single<P>()>(EoCfg<P, CT>::EPB);
-  SDG_TRY(set_kernel_smem((const void*)stage_eo_kernel<P, CT>, (int)smem, kCarveMax));
-  const long long nblk = (a.elem_count + EoCfg<P, CT>::EPB - 1) / EoCfg<P, CT>::EPB;
-  if (nblk <= 0) return SDG_OK;
-  if (nblk > 0x7fffffffLL) return fail(SDG_ERR_INVALID_ARG, "too many elements");
-  stage_eo_kernel<P, CT><<<(unsigned)nblk, EoCfg<P, CT>::THREADS, smem, st>>>(a);
-  SDG_CUDA_TRY(cudaGetLastError());
-  return SDG_OK;
-}
-
 }  // namespace sdg

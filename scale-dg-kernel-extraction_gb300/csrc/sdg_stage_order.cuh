@@ -3,11 +3,10 @@
 #pragma once
 
 #include "sdg_stage.cuh"
-#include "sdg_stage_elem.cuh"
 #include "sdg_stage_eo.cuh"
 #include "sdg_stage_fix.cuh"
+#include "sdg_stage_line.cuh"
 #include "sdg_stage_loop.cuh"
-#include "sdg_stage_warp.cuh"
 
 namespace sdg {
 
@@ -19,14 +18,7 @@ int launch_stage_order(int prec, int opt, const StageArgs& a, cudaStream_t st) {
   if (prec != SDG_PREC_FP32)
     return opt == SDG_OPT_EVENODD ? launch_stage_fix_impl<P, true>(a, st)
                                   : launch_stage_fix_impl<P, false>(a, st);
-  if (opt == SDG_OPT_EVENODD) {
-    // p = 1: one thread an element (same bits as the block body): 129.7
-    // against 48.2 GDOF-updates/s at 128^3 on GB300
-    if constexpr (P == 1) return launch_stage_elem_impl<P>(a, st);
-    // p = 2, 3: one warp an element (same bits as the block body)
-    if constexpr (P == 2 || P == 3) return launch_stage_warp_impl<P>(a, st);
-    return launch_stage_eo_impl<P, float>(a, st);
-  }
+  if (opt == SDG_OPT_EVENODD) return launch_stage_line_impl<P>(a, st);
   if (split) return launch_stage_impl<P, float, float, kCanSplit>(a, st);
   return launch_stage_impl<P, float, float, false>(a, st);
 }

@@ -262,3 +262,26 @@ def test_steps_in_one_launch_equal_a_launch_a_stage(opt, p, dims, nstep):
         s.step(c.dt, nstep)
         s.step(0.5 * c.dt, 2)
     assert np.array_equal(a.download(), b.download(), equal_nan=True)
+
+
+@pytest.mark.parametrize("p", [1, 2, 4, 7, 8, 10, 15])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 1, 3), (13, 5, 7)])
+def test_fp32_line_stage_within_its_rounding_bound(p, dims):
+    """Tendency of the FP32 form node by node against the oracle's, at one element,
+    at blocks that are not full and at uneven boxes: a line result is a chain of
+    at most N + 4 roundings (coefficient, product, pair, multiply-adds, faces),
+    each at most 2^-24 of the terms' magnitudes; three lines add up."""
+    import sdg
+    c = Case(*dims, p)
+    q, u, v, w = _fields(c)
+    m, N = c.mesh, p + 1
+    _, want = _tendencies(c, q, u, v, w, "OPT_EVENODD")
+    s = sdg.Solver(*dims, p, c.D, c.Lift, opt=sdg.OPT_EVENODD, precision=sdg.PREC_FP32)
+    s.upload(q, u, v, w)
+    rows = np.abs(np.asarray(c.D).reshape(N, N)).sum(axis=0).max()  # of a row, by symmetry
+    rows = max(rows, np.abs(np.asarray(c.D).reshape(N, N)).sum(axis=1).max())
+    lift = np.abs(np.asarray(c.Lift)).max()
+    Es, Fs = np.abs(m.Escale).max(), np.abs(m.Fscale).max()
+    qm, um = np.abs(q).max(), max(np.abs(a).max() for a in (u, v, w))
+    bound = 3 * qm * um * (Es * rows + 2 * Fs * lift * 2) * (N + 4) * 2.0 ** -24
+    assert np.max(np.abs(s.tendency() - want)) <= bound
