@@ -4,13 +4,13 @@
 // Every box is an instance with its own order p, size, dt, rotating state
 // buffers and velocity.  A work item is one block's worth of consecutive
 // elements of one instance.  The item list is sorted by order; each order's
-// items run in one launch of a kernel compiled for that order and body:
-// one block per item for the even-odd body (batch_one_item), or persistent
-// blocks that take items round-robin and prefetch the next item's instance
-// header into shared memory while computing the current one.  A block
-// resolves the instance's buffers for the stage and runs the same fused
-// stage body as the single-box solver (stage_block or stage_eo_block, FP32
-// compute, FP64 state).  Each instance's current
+// items run in one launch of a kernel compiled for that order and body: one
+// block per item for the even-odd body, or persistent blocks that take items
+// round-robin and prefetch the next item's instance header into shared memory
+// while computing the current one for the node body.  A block resolves the
+// instance's buffers for the stage and runs the stage body (stage_block, or
+// line_elements, the single-box solver's; FP32 compute, FP64 state).  Each
+// instance's current
 // buffer index lives on the device and is advanced by a tiny kernel after
 // stage 3, so one captured CUDA graph replays every step.
 #pragma once
@@ -66,12 +66,14 @@ inline void batch_stage_factors(BatchInst& I) {
 
 // The items of one order and stage body, run by one launch of a kernel
 // compiled for that order and body.  The item list is sorted by order
-// (and body), so a group is a contiguous range of it.
+// (and body), so a group is a contiguous range of it.  The even-odd body takes
+// an item's elements a block of lines at a time, with at least one element's
+// lines a block.
 struct BatchGroup {
   int p = 0, eo = 0;       // order, 1 for the even-odd body
   int begin = 0, count = 0;  // item range
   int threads = 256;       // block size
-  size_t smem = 0;         // dynamic shared memory of a block
+  size_t smem = 0;         // bytes that bound an item (batch_smem_bytes)
   int grid = 0;            // blocks: one per item (one-item kernel) or the
                            // resident blocks, at most count (persistent kernel)
 };
@@ -125,8 +127,9 @@ struct BatchForkJoin {
 int batch_step_enqueue(BatchForkJoin& fj, BatchInst* d_inst, int n_inst,
                        const BatchItem* d_items, const std::vector<BatchGroup>& groups,
                        cudaStream_t st);
-// Dynamic shared memory the kernel needs for `epb` elements of order p with
-// the node body (eo = 0) or the even-odd body (eo = 1).
+// Shared memory of `epb` elements of order p staged at once, which bounds an
+// item: what the node body's kernel (eo = 0) takes; the even-odd body's
+// (eo = 1) takes less.
 size_t batch_smem_bytes(int p, int epb, int eo);
 
 // Device-side initial condition: Gaussian tracer exp(-d^2/(2 sigma^2)) around

@@ -1,5 +1,6 @@
-// The persistent batched stage kernel and its helpers (see sdg_batch.cuh).
+// The batched stage kernels and their helpers (see sdg_batch.cuh).
 #include "sdg_batch.cuh"
+#include "sdg_stage_line.cuh"
 
 namespace sdg {
 
@@ -15,42 +16,18 @@ constexpr int kInstWords = (int)(sizeof(BatchInst) / 4);
 static_assert(sizeof(BatchInst) % 4 == 0, "instance header is copied as 32-bit words");
 static_assert(kInstWords < 128, "the smallest block must copy the header in one pass");
 
-// One persistent launch runs the items of one order group (order P, stage
-// body EO: 1 even-odd, 0 node body; RK the stage's update kind).  Compiling
-// one order and one body per kernel keeps each at its own register count
-// (32 or 40, for 4 or 3 blocks of 512 threads an SM), where a switch over
-// the orders would keep the union of their needs.
-//
-// Items are assigned round-robin (block b runs items b, b + G, b + 2G, ...).
-// The next item's instance header is fetched into shared memory while the
-// current item computes, and the item after that into a register, so that a
-// block never waits on the item -> instance -> data chain of dependent loads.
-// Resident blocks of 512 threads an SM the registers are capped for: 4 (32
-// registers) where that measured faster on GB300, else 3 (40 registers).
-// The node body gains 4-16 % from the fourth block at every order; the
-// even-odd body, in its one-item kernel, up to 15 % (p = 2, 3) at every order
-// but p = 10 (0.92x there).
-template <int P, int EO>
-__host__ __device__ constexpr int batch_min_blocks() {
-  return (EO != 0 && P == 10) ? 3 : 4;
-}
-
-// Even-odd body: F_y / F_z formed on the fly rather than staged at the orders
-// where that measured faster in the batch on GB300 (1.05x at p = 6, 1.11x at
-// p = 8; 0.96-0.97x at p = 10 and 11).
+// Bytes of shared memory of a block of `threads` threads of the even-odd body:
+// the instance's scaled coefficients, then the line arrays of the elements a
+// block holds at once.
 template <int P>
-__host__ __device__ constexpr bool batch_eo_fly() {
-  return P == 6 || P == 8;
+__host__ __device__ constexpr size_t batch_line_smem(int threads) {
+  return sizeof(float) * 3 * LineRows<P>::DIR + line_smem<P>(threads / FixShape<P>::N2);
 }
-
-// Even-odd body: threads a line.  One up to p = 4, where a line has at most
-// two output pairs (measured in the batch on GB300: p = 3 81.5 against 75.3,
-// p = 4 82.1 against 71.6 GDOF-updates/s), two above (one at p = 5 with 64
-// registers measured 439 against 450 solves/s on the 256-member ensemble,
-// and at p = 11 level on the serving stream).
+// The block size an item is run with: at least one element's lines.
 template <int P>
-__host__ __device__ constexpr int batch_eo_parts() {
-  return P <= 4 ? 1 : 2;
+__host__ __device__ constexpr int batch_line_threads(int threads) {
+  constexpr int least = (FixShape<P>::N2 + 31) / 32 * 32;
+  return threads < least ? least : threads;
 }
 
 // One work item through one stage: the instance's buffers for the stage from
@@ -58,6 +35,57 @@ __host__ __device__ constexpr int batch_eo_parts() {
 template <int P, int EO, int RK>
 __device__ __forceinline__ void batch_item_body(const BatchInst& I, const BatchItem& w,
                                                 int stage, unsigned char* smem) {
+  if constexpr (EO != 0) {
+    // the even-odd line stage (sdg_stage_line.cuh), the coefficients scaled for
+    // this instance in shared memory; blockDim.x / N^2 elements at a time
+    using Rows = LineRows<P>;
+    constexpr int TE = EoShape<P>::TE, OFF_A = EoShape<P>::OFF_A, NP = FixShape<P>::N * FixShape<P>::N2;
+    float* T = reinterpret_cast<float*>(smem);
+    // read now, stored once the state's loads are on their way; where a
+    // coefficient goes and its factor also now, but for the orders with the
+    // fewest instructions between (p = 3 111.6 from 106.6, p = 7 133.0 from 132.0,
+    // p = 10 123.9 from 116.6 GDOF-updates/s; p = 2 99.3 against 102.3, p = 4 117.0
+    // against 126.8)
+    constexpr int LEAST = (FixShape<P>::N2 + 31) / 32 * 32;  // threads, at least
+    constexpr int PER = (3 * TE + LEAST - 1) / LEAST;
+    constexpr bool EARLY = P == 3 || P >= 5;
+    float c[PER], by[PER];
+    int to[PER];
+    auto place = [&](int k) {
+      const int t = threadIdx.x + k * blockDim.x;
+      const int d = t / TE, n = t - d * TE;
+      to[k] = t < 3 * TE ? d * Rows::DIR + Rows::at(n) : -1;
+      by[k] = t < 3 * TE ? (n < OFF_A ? I.eo_sD[stage][d] : I.eo_sL[stage][d]) : 0.0f;
+    };
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const int t = threadIdx.x + k * blockDim.x;
+      c[k] = t < 3 * TE ? I.eo_tab[t] : 0.0f;
+      if constexpr (EARLY) place(k);
+    }
+    auto store = [&] {
+#pragma unroll
+      for (int k = 0; k < PER; k++) {
+        if constexpr (!EARLY) place(k);
+        if (to[k] >= 0) T[to[k]] = c[k] * by[k];
+      }
+    };
+    const int s0 = I.cur, s1 = s0 == 2 ? 0 : s0 + 1, s2 = s1 == 2 ? 0 : s1 + 1;
+    const double* q = I.q[stage == 0 ? s0 : stage == 1 ? s1 : s2];
+    const int epb = blockDim.x / FixShape<P>::N2;
+    // No barrier between two rounds: a thread reads last, and writes first, its
+    // own z line of the arrays; the first barrier inside orders the coefficients
+    // before their first use.
+    for (int e = 0; e < w.e_count; e += epb)
+      line_elements<P, RK>(
+          q, I.q[s0], I.q[stage == 1 ? s2 : s1], I.u, I.v, I.w, I.box, c_rk_a[stage],
+          c_rk_b[stage], w.e_begin + e, min(epb, w.e_count - e), epb, T + 3 * Rows::DIR,
+          [&](int d) { return Rows{T + d * Rows::DIR}; },
+          [&] {
+            if (e == 0) store();
+          });
+    return;
+  }
   const int s0 = I.cur, s1 = (s0 + 1) % 3, s2 = (s0 + 2) % 3;
   StageArgs a;
   a.q_in = (stage == 0) ? I.q[s0] : (stage == 1) ? I.q[s1] : I.q[s2];
@@ -66,7 +94,7 @@ __device__ __forceinline__ void batch_item_body(const BatchInst& I, const BatchI
   a.u = I.u;
   a.v = I.v;
   a.w = I.w;
-  a.D = EO ? static_cast<const void*>(I.eo_tab) : static_cast<const void*>(I.D);
+  a.D = I.D;
   a.Lift = I.Lift;
   a.box = I.box;
   a.fc_out = nullptr;
@@ -80,49 +108,42 @@ __device__ __forceinline__ void batch_item_body(const BatchInst& I, const BatchI
   a.b_is_one = (stage == 0);
   a.a_nonzero = (stage != 0);
   a.tend_only = 0;
-  if constexpr (EO != 0) {
-    for (int d = 0; d < 3; d++) {
-      a.eo_sDf[d] = I.eo_sD[stage][d];
-      a.eo_sLf[d] = I.eo_sL[stage][d];
-    }
-    stage_eo_block<P, float, RK, batch_eo_fly<P>(), false, batch_eo_parts<P>()>(
-        a, w.e_begin, w.e_count, smem);
-  } else {
-    stage_block<P, float, float, false, RK>(a, w.e_begin, w.e_count, smem);
-  }
+  stage_block<P, float, float, false, RK>(a, w.e_begin, w.e_count, smem);
 }
 
-// One block per work item, no loop: no work-item state stays live across
-// the stage body, so the body keeps the registers the persistent form
-// spends on its prefetch pipeline (the persistent kernel spilled 40-48 bytes
-// at p = 7 under the 32-register cap).  Measured on GB300 for the even-odd
-// body: 1.03-1.15x at every order but p = 8 (p = 7: 103.5 against 89.9
-// GDOF-updates/s), 0.97x at p = 8; the node body is faster persistent.
-template <int P, int EO>
-__host__ __device__ constexpr bool batch_one_item() {
-  return EO != 0 && P != 8;
-}
-
-template <int P, int EO, int RK>
-__global__ void __launch_bounds__(kBatchThreadsMax, batch_min_blocks<P, EO>())
+// Even-odd body: one block per work item; no work-item state stays live across
+// the stage.  64 registers a thread, as in the single-box kernel (40: 0.95x at
+// p = 3, 0.8x at p = 7).  Against a block body with every flux and face staged in
+// shared memory, four boxes of 3.5M DOF, GDOF-updates/s: p = 1 89 from 63, p = 2
+// 104 from 82, p = 3 114 from 96, p = 4 127 from 92, p = 5 122 from 86, p = 7 132
+// from 103, p = 9 116 from 86, p = 11 110 from 89.  A block starts with two
+// dependent reads (item, instance) that the single-box kernel does without:
+// it waits on loads (long-scoreboard stalls 9 of 15 cycles an instruction).
+template <int P, int RK>
+__global__ void __launch_bounds__(kBatchThreadsMax, 2)
     batch_item_kernel(const BatchInst* __restrict__ insts, const BatchItem* __restrict__ items,
                       int n_items, int stage) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(16) BatchInst s_inst;
-  __shared__ BatchItem s_item;
-  const int tid = threadIdx.x;
   if ((int)blockIdx.x >= n_items) return;  // uniform across the block
-  if (tid == 0) s_item = items[blockIdx.x];
+  const BatchItem item = items[blockIdx.x];
+  for (int t = threadIdx.x; t < kInstWords; t += blockDim.x)
+    reinterpret_cast<uint32_t*>(&s_inst)[t] =
+        reinterpret_cast<const uint32_t*>(insts + item.inst)[t];
   __syncthreads();
-  if (tid < kInstWords)
-    reinterpret_cast<uint32_t*>(&s_inst)[tid] =
-        reinterpret_cast<const uint32_t*>(insts + s_item.inst)[tid];
-  __syncthreads();
-  if (s_inst.active) batch_item_body<P, EO, RK>(s_inst, s_item, stage, smem);
+  if (s_inst.active) batch_item_body<P, 1, RK>(s_inst, item, stage, smem);
 }
 
-template <int P, int EO, int RK>
-__global__ void __launch_bounds__(kBatchThreadsMax, batch_min_blocks<P, EO>())
+// Node body: one persistent launch runs the items of one order group.
+// Compiling one order per kernel keeps each at its own register count; four
+// blocks of 512 threads an SM (32 registers) measured 4-16 % above three.
+//
+// Items are assigned round-robin (block b runs items b, b + G, b + 2G, ...).
+// The next item's instance header is fetched into shared memory while the
+// current item computes, and the item after that into a register, so that a
+// block never waits on the item -> instance -> data chain of dependent loads.
+template <int P, int RK>
+__global__ void __launch_bounds__(kBatchThreadsMax, 4)
     batch_order_kernel(const BatchInst* __restrict__ insts, const BatchItem* __restrict__ items,
                        int n_items, int stage) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -155,7 +176,7 @@ __global__ void __launch_bounds__(kBatchThreadsMax, batch_min_blocks<P, EO>())
 
     const BatchItem w = s_items[slot];
     const BatchInst& I = s_inst[slot];
-    if (I.active) batch_item_body<P, EO, RK>(I, w, stage, smem);
+    if (I.active) batch_item_body<P, 0, RK>(I, w, stage, smem);
     // every read of this item's slots happened before the body's barriers
     __syncthreads();
     if (has_next && tid < kInstWords) reinterpret_cast<uint32_t*>(&s_inst[slot ^ 1])[tid] = hw;
@@ -239,10 +260,16 @@ __global__ void init_blob_kernel(double* q, float* u, float* v, float* w, const 
   }
 }
 
+// What bounds an item's elements: the node body stages them all at once; the
+// even-odd body, which takes them a block of lines at a time, keeps the bound of
+// a body that would (q, the fluxes, the sums and the face fluxes of each).
 template <int P>
 size_t smem_for(int epb, int eo) {
-  return eo ? eo_block_smem<P, float, batch_eo_fly<P>(), batch_eo_parts<P>()>(epb)
-            : stage_block_smem<P, float>(epb);
+  if (!eo) return stage_block_smem<P, float>(epb);
+  using O = Ord<P>;
+  constexpr int arrays = P <= 4 ? 4 : (P == 6 || P == 8) ? 3 : 5;
+  return sizeof(float) * (size_t)(3 * EoShape<P>::TE + epb * (arrays * O::NP + O::NFT)) +
+         sizeof(int) * 6 * (size_t)epb;
 }
 
 }  // namespace
@@ -265,49 +292,63 @@ size_t batch_smem_bytes(int p, int epb, int eo) {
 }
 
 namespace {
-// The three functions an order group needs, for one (P, EO) pair.
+// What an order group needs, for one (P, EO) pair: the launch's block size and
+// shared memory for a group's, the blocks an SM holds, the launch.
 template <int P, int EO>
 struct GroupOps {
-  static constexpr bool kOneItem = batch_one_item<P, EO>();
-  static int set_smem(size_t smem) {
-    SDG_CUDA_TRY(cudaFuncSetAttribute(batch_order_kernel<P, EO, kRkFirst>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SDG_CUDA_TRY(cudaFuncSetAttribute(batch_order_kernel<P, EO, kRkGeneral>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if constexpr (kOneItem) {
-      SDG_CUDA_TRY(cudaFuncSetAttribute(batch_item_kernel<P, EO, kRkFirst>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      SDG_CUDA_TRY(cudaFuncSetAttribute(batch_item_kernel<P, EO, kRkGeneral>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
-    return SDG_OK;
+  static int threads(const BatchGroup& g) {
+    return EO ? batch_line_threads<P>(g.threads) : g.threads;
   }
-  static int blocks_per_sm(int threads, size_t smem) {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_order_kernel<P, EO, kRkGeneral>,
-                                                      threads, smem) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
-    return nb;
+  static size_t smem(const BatchGroup& g, int threads) {
+    return EO ? batch_line_smem<P>(threads) : g.smem;
   }
-  static int launch(const BatchInst* d_inst, const BatchItem* d_items, int n, int stage,
-                    int grid, int threads, size_t smem, cudaStream_t st) {
-    if constexpr (kOneItem) {
-      if (stage == 0)
-        batch_item_kernel<P, EO, kRkFirst><<<grid, threads, smem, st>>>(d_inst, d_items, n,
-                                                                        stage);
-      else
-        batch_item_kernel<P, EO, kRkGeneral><<<grid, threads, smem, st>>>(d_inst, d_items, n,
-                                                                          stage);
-      SDG_CUDA_TRY(cudaGetLastError());
+  static int setup(const BatchGroup& g, int* per_sm) {
+    if constexpr (EO != 0) {
+      int dev = 0, most = 0;
+      SDG_CUDA_TRY(cudaGetDevice(&dev));
+      SDG_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+      if (g.smem + 2 * (sizeof(BatchInst) + sizeof(BatchItem)) > (size_t)most)
+        return cuda_fail(cudaErrorInvalidValue, "batch item size", __FILE__, __LINE__);
+      // at most 46 KB at any block size; the carveout holds 1024 threads' worth
+      static_assert(batch_line_smem<P>(kBatchThreadsMax) + sizeof(BatchInst) + sizeof(BatchItem) <=
+                    48 * 1024);
+      constexpr int carve = carve_for(batch_line_smem<P>(128 < FixShape<P>::N2 ? 256 : 128),
+                                      128 < FixShape<P>::N2 ? 4 : 8);
+      constexpr int limit = (int)batch_line_smem<P>(kBatchThreadsMax);
+      SDG_TRY(set_kernel_smem((const void*)batch_item_kernel<P, kRkFirst>, limit, carve));
+      SDG_TRY(set_kernel_smem((const void*)batch_item_kernel<P, kRkGeneral>, limit, carve));
+      *per_sm = 1;
+      return SDG_OK;
+    } else {
+      SDG_CUDA_TRY(cudaFuncSetAttribute(batch_order_kernel<P, kRkFirst>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)g.smem));
+      SDG_CUDA_TRY(cudaFuncSetAttribute(batch_order_kernel<P, kRkGeneral>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)g.smem));
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, batch_order_kernel<P, kRkGeneral>,
+                                                        g.threads, g.smem) != cudaSuccess) {
+        cudaGetLastError();
+        *per_sm = 0;
+      }
       return SDG_OK;
     }
-    if (stage == 0)
-      batch_order_kernel<P, EO, kRkFirst><<<grid, threads, smem, st>>>(d_inst, d_items, n, stage);
-    else
-      batch_order_kernel<P, EO, kRkGeneral><<<grid, threads, smem, st>>>(d_inst, d_items, n,
-                                                                         stage);
+  }
+  static int launch(const BatchInst* d_inst, const BatchItem* d_items, const BatchGroup& g,
+                    int stage, cudaStream_t st) {
+    const int t = threads(g);
+    const size_t sm = smem(g, t);
+    if constexpr (EO != 0) {
+      if (stage == 0)
+        batch_item_kernel<P, kRkFirst><<<g.grid, t, sm, st>>>(d_inst, d_items, g.count, stage);
+      else
+        batch_item_kernel<P, kRkGeneral><<<g.grid, t, sm, st>>>(d_inst, d_items, g.count, stage);
+    } else {
+      if (stage == 0)
+        batch_order_kernel<P, kRkFirst><<<g.grid, t, sm, st>>>(d_inst, d_items, g.count, stage);
+      else
+        batch_order_kernel<P, kRkGeneral><<<g.grid, t, sm, st>>>(d_inst, d_items, g.count, stage);
+    }
     SDG_CUDA_TRY(cudaGetLastError());
     return SDG_OK;
   }
@@ -329,10 +370,13 @@ int with_group(int p, int eo, F&& f) {
 }  // namespace
 
 void batch_default_shape(int p, int* threads, int* epb) {
-  // index = order; measured with sdg_ensemble_tune, block sizes 128/256/512
-  static const int kThreads[kBatchMaxOrder + 1] = {256, 128, 256, 256, 256, 256,
-                                                   256, 512, 256, 256, 256, 512};
-  static const int kEpb[kBatchMaxOrder + 1] = {1, 64, 32, 16, 8, 4, 4, 4, 2, 1, 1, 1};
+  // index = order; block sizes 128/256/512 and one to four rounds of a block's
+  // lines an item, four boxes of 3.5M DOF (p = 3: 111.6 at 128/16, 110.4 at 128/8,
+  // 105.0 at 256/32; p = 6: 117.3 at 256/5, 109.0 at 128/4).  From p = 10 a block
+  // of one element's lines.
+  static const int kThreads[kBatchMaxOrder + 1] = {256, 128, 128, 128, 128, 256,
+                                                   256, 128, 256, 128, 128, 128};
+  static const int kEpb[kBatchMaxOrder + 1] = {1, 128, 56, 16, 10, 14, 5, 2, 3, 3, 2, 2};
   const int i = (p >= 1 && p <= kBatchMaxOrder) ? p : 0;
   *threads = kThreads[i];
   *epb = kEpb[i];
@@ -341,25 +385,18 @@ void batch_default_shape(int p, int* threads, int* epb) {
 int batch_default_eo(int p) { return p >= 1 ? 1 : 0; }
 
 int batch_group_setup(BatchGroup& g) {
-  const int threads = g.threads;
   int dev = 0, nsm = 0;
   SDG_CUDA_TRY(cudaGetDevice(&dev));
   SDG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   int per_sm = 0;
-  bool one_item = false;
-  const int st = with_group<GroupOps>(g.p, g.eo, [&](auto ops) {
-    const int r = decltype(ops)::set_smem(g.smem);
-    if (r != SDG_OK) return r;
-    per_sm = decltype(ops)::blocks_per_sm(threads, g.smem);
-    one_item = decltype(ops)::kOneItem;
-    return SDG_OK;
-  });
+  const int st = with_group<GroupOps>(
+      g.p, g.eo, [&](auto ops) { return decltype(ops)::setup(g, &per_sm); });
   if (st != SDG_OK) return st;
   if (per_sm <= 0)
     return fail(SDG_ERR_INVALID_ARG, "batch kernel of order %d does not fit: %d threads, %zu B",
-                g.p, threads, g.smem);
+                g.p, g.threads, g.smem);
   const long long cap = (long long)nsm * per_sm;
-  g.grid = one_item ? g.count : (int)(g.count < cap ? g.count : cap);
+  g.grid = g.eo ? g.count : (int)(g.count < cap ? g.count : cap);
   return SDG_OK;
 }
 
@@ -367,8 +404,7 @@ int batch_group_launch(const BatchInst* d_inst, const BatchItem* d_items, const 
                        int stage, cudaStream_t st) {
   if (g.count <= 0) return SDG_OK;
   return with_group<GroupOps>(g.p, g.eo, [&](auto ops) {
-    return decltype(ops)::launch(d_inst, d_items + g.begin, g.count, stage, g.grid, g.threads,
-                                 g.smem, st);
+    return decltype(ops)::launch(d_inst, d_items + g.begin, g, stage, st);
   });
 }
 
@@ -386,9 +422,16 @@ static int batch_fused_enqueue(BatchInst* d_inst, int n_inst, const BatchItem* d
   size_t smem = 0;
   for (const BatchGroup& g : groups) {
     n_items = g.begin + g.count > n_items ? g.begin + g.count : n_items;
-    threads = g.threads > threads ? g.threads : threads;
-    smem = g.smem > smem ? g.smem : smem;
+    SDG_TRY(with_group<GroupOps>(g.p, g.eo, [&](auto ops) {
+      threads = std::max(threads, decltype(ops)::threads(g));
+      return SDG_OK;
+    }));
   }
+  for (const BatchGroup& g : groups)
+    SDG_TRY(with_group<GroupOps>(g.p, g.eo, [&](auto ops) {
+      smem = std::max(smem, decltype(ops)::smem(g, threads));
+      return SDG_OK;
+    }));
   if (n_items > 0) {
     SDG_TRY(set_kernel_smem((const void*)batch_stage_kernel<kRkFirst>, (int)smem, kCarveDefault));
     SDG_TRY(set_kernel_smem((const void*)batch_stage_kernel<kRkGeneral>, (int)smem, kCarveDefault));

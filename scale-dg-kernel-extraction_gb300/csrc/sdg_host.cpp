@@ -45,23 +45,24 @@ int set_kernel_smem(const void* func, int smem, int carve) {
   struct Key {
     const void* func;
     int dev, smem, carve;
-    bool operator==(const Key& o) const {
-      return func == o.func && dev == o.dev && smem == o.smem && carve == o.carve;
-    }
   };
   static std::mutex mu;
   static std::vector<Key> done;  // a few dozen kernels at most
-  const Key k{func, dev, smem, carve};
-  {
-    std::lock_guard<std::mutex> g(mu);
-    if (std::find(done.begin(), done.end(), k) != done.end()) return SDG_OK;
-  }
-  SDG_CUDA_TRY(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  // the limit is only ever raised: a caller of fewer bytes must not lower it
+  // under one that was told its own is set
+  std::lock_guard<std::mutex> g(mu);
+  auto k = std::find_if(done.begin(), done.end(),
+                        [&](const Key& o) { return o.func == func && o.dev == dev; });
+  if (k != done.end() && k->smem >= smem && k->carve == carve) return SDG_OK;
+  const int limit = k != done.end() ? std::max(k->smem, smem) : smem;
+  SDG_CUDA_TRY(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
   if (carve != kCarveDefault)
     SDG_CUDA_TRY(
         cudaFuncSetAttribute(func, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-  std::lock_guard<std::mutex> g(mu);
-  if (std::find(done.begin(), done.end(), k) == done.end()) done.push_back(k);
+  if (k != done.end())
+    *k = Key{func, dev, limit, carve};
+  else
+    done.push_back(Key{func, dev, limit, carve});
   return SDG_OK;
 }
 

@@ -4,22 +4,23 @@
 // Thread r of an element's N^2 owns line r of each direction and node r of
 // each face (the layout of stage_fix_kernel): its face fluxes and the z line's
 // pair values never leave its registers, shared memory holds the x and y
-// fluxes and then their line results, and the coefficients, scaled for the
-// stage on the host, are kernel parameters, which a multiply-add takes from
-// the constant bank.  Every value is formed in the order of operations of
-// stage_eo_block (products rounded before the pair sums, x + y + z, widened
-// increment), so both give the same bits.
+// fluxes and then their line results.  The coefficients, scaled for the stage,
+// are kernel parameters, which a multiply-add takes from the constant bank; in
+// the batch, whose instances each have their own, they are in shared memory.
+// Products are rounded before the pair sums, line results add up as x + y + z
+// in FP32 and the increment is widened: the same bits in both kernels.
 //
 // Bound: 28 bytes a node in the first stage and 36 in the others, read and
-// written once, at two thirds of the copy bandwidth; 32 warps an SM wait on
-// the loads at the two ends of a block.  On GB300, 16.8M DOF, against the
-// kernels this replaced (GDOF-updates/s): p = 2 136 from 110, p = 3 140 from
-// 106, p = 4 143 from 82, p = 5 137 from 82, p = 7 151 from 108, p = 9 131 from
-// 87, p = 11 134 from 93, p = 15 130 from 87 (p = 1 level at 130).  Most of it
-// comes from L1: with the largest shared-memory carveout 84 at p = 5.  64
-// registers (1024 threads an SM): 1280 threads 0.85-1.0x, 768 0.9-1.03x.
-// Velocity factors of the faces stored by the call's first stage, as the FP64
-// form does: 0.88-1.03x.
+// written once, at 0.7-0.85 of the copy bandwidth; 32 warps an SM wait on the
+// loads at the two ends of a block.  On GB300, 16.8M DOF, against the kernels
+// this replaced (GDOF-updates/s): p = 2 140 from 110, p = 3 147 from 106, p = 5
+// 145 from 82, p = 7 171 from 108, p = 9 148 from 87, p = 11 146 from 93, p = 15
+// 148 from 87 (p = 1 126-130 from 130).  Half of it comes from L1: with the largest
+// shared-memory carveout 84 at p = 5.  The state is read by __ldg: plain reads of
+// q and q0 wait for the store of the node before (p = 7 151, and 89 against 131 in
+// the batch).  64 registers (1024 threads an SM): 1280 threads 0.85-1.0x, 768
+// 0.9-1.03x.  Velocity factors of the faces stored by the call's first stage, as
+// the FP64 form does: 0.88-1.03x.
 #pragma once
 
 #include "sdg_stage_fix.cuh"
@@ -42,40 +43,109 @@ __host__ __device__ constexpr size_t line_smem(int epb) {
   return sizeof(float) * 2 * epb * FixShape<P>::EW;
 }
 
+// A direction's coefficients as EoShape lays them out (kernel parameters).
+template <int P>
+struct LineTable {
+  using Sh = EoShape<P>;
+  const float* T;
+  // c: E(i, .), D(i, mid) (odd N), B(i), O(i, .), A(i)
+  __device__ __forceinline__ void row(int i, float* c) const {
+    constexpr int H = Sh::H;
+#pragma unroll
+    for (int l = 0; l < H; l++) {
+      c[l] = T[Sh::OFF_E + i * H + l];
+      c[H + Sh::ODD + 1 + l] = T[Sh::OFF_O + i * H + l];
+    }
+    if constexpr (Sh::ODD != 0) c[H] = T[Sh::OFF_DM + i];
+    c[H + Sh::ODD] = T[Sh::OFF_B + i];
+    c[2 * H + Sh::ODD + 1] = T[Sh::OFF_A + i];
+  }
+  // c: O(H, .), A(H): the middle row of an odd N
+  __device__ __forceinline__ void mid(float* c) const {
+#pragma unroll
+    for (int l = 0; l < Sh::H; l++) c[l] = T[Sh::OFF_O + Sh::H * Sh::H + l];
+    c[Sh::H] = T[Sh::OFF_A + Sh::H];
+  }
+};
+
+// The same row by row in shared memory, each row padded to whole 16-byte loads
+// (a quarter of the loads).
+template <int P>
+struct LineRows {
+  using Sh = EoShape<P>;
+  static constexpr int ROW = (2 * Sh::H + 2 + Sh::ODD + 3) / 4 * 4;
+  static constexpr int MID = Sh::ODD ? (Sh::H + 1 + 3) / 4 * 4 : 0;
+  static constexpr int DIR = Sh::H * ROW + MID;  // words of a direction
+  const float* T;                                // 16-byte aligned
+  // where EoShape's entry t of a direction goes
+  static __device__ __forceinline__ int at(int t) {
+    constexpr int H = Sh::H;
+    if (t < Sh::OFF_O) return t / H * ROW + t % H;
+    if (t < Sh::OFF_DM) {
+      const int i = (t - Sh::OFF_O) / H, l = (t - Sh::OFF_O) % H;
+      return i < H ? i * ROW + H + Sh::ODD + 1 + l : H * ROW + l;
+    }
+    if (t < Sh::OFF_A) return (t - Sh::OFF_DM) * ROW + H;
+    if (t < Sh::OFF_B) {
+      const int i = t - Sh::OFF_A;
+      return i < H ? i * ROW + 2 * H + Sh::ODD + 1 : H * ROW + H;
+    }
+    return (t - Sh::OFF_B) * ROW + H + Sh::ODD;
+  }
+  __device__ __forceinline__ void row(int i, float* c) const { load<ROW>(T + i * ROW, c); }
+  __device__ __forceinline__ void mid(float* c) const { load<MID>(T + Sh::H * ROW, c); }
+  template <int W>
+  static __device__ __forceinline__ void load(const float* p, float* c) {
+#pragma unroll
+    for (int k = 0; k < W; k += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(p + k);
+      c[k] = x.x;
+      c[k + 1] = x.y;
+      c[k + 2] = x.z;
+      c[k + 3] = x.w;
+    }
+  }
+};
+
 // One line from its pair values s, d and face fluxes: the N results to
-// emit(m, value), in the order of operations of eo_line_f.
-template <int P, typename Emit>
-__device__ __forceinline__ void line_pairs(const float* s, const float* d, float fm, const float* T,
-                                           float gm, float gp, Emit&& emit) {
+// emit(m, value).
+template <int P, typename Table, typename Emit>
+__device__ __forceinline__ void line_pairs(const float* s, const float* d, float fm,
+                                           const Table& T, float gm, float gp, Emit&& emit) {
   using Sh = EoShape<P>;
   constexpr int N = Sh::N, H = Sh::H;
   const float gs = gm + gp, gd = gm - gp;
 #pragma unroll
   for (int i = 0; i < H; i++) {
-    float e = T[Sh::OFF_E + i * H] * s[0], o = T[Sh::OFF_O + i * H] * d[0];
+    float c[LineRows<P>::ROW];
+    T.row(i, c);
+    const float* co = c + H + Sh::ODD + 1;
+    float e = c[0] * s[0], o = co[0] * d[0];
 #pragma unroll
     for (int l = 1; l < H; l++) {
-      e = fmaf(T[Sh::OFF_E + i * H + l], s[l], e);
-      o = fmaf(T[Sh::OFF_O + i * H + l], d[l], o);
+      e = fmaf(c[l], s[l], e);
+      o = fmaf(co[l], d[l], o);
     }
-    if constexpr (Sh::ODD != 0) e = fmaf(T[Sh::OFF_DM + i], fm, e);
-    e = fmaf(T[Sh::OFF_B + i], gd, e);
-    o = fmaf(T[Sh::OFF_A + i], gs, o);
+    if constexpr (Sh::ODD != 0) e = fmaf(c[H], fm, e);
+    e = fmaf(c[H + Sh::ODD], gd, e);
+    o = fmaf(co[H], gs, o);
     emit(i, e + o);
     emit(N - 1 - i, o - e);
   }
   if constexpr (Sh::ODD != 0) {
-    float o = T[Sh::OFF_O + H * H] * d[0];
+    float c[LineRows<P>::MID];
+    T.mid(c);
+    float o = c[0] * d[0];
 #pragma unroll
-    for (int l = 1; l < H; l++) o = fmaf(T[Sh::OFF_O + H * H + l], d[l], o);
-    o = fmaf(T[Sh::OFF_A + H], gs, o);
+    for (int l = 1; l < H; l++) o = fmaf(c[l], d[l], o);
+    o = fmaf(c[H], gs, o);
     emit(H, o);
   }
 }
 
 // Line at `line` (stride S) in shared memory, results over it.
-template <int P, int S>
-__device__ __forceinline__ void line_shared(float* line, const float* T, float gm, float gp) {
+template <int P, int S, typename Table>
+__device__ __forceinline__ void line_shared(float* line, const Table& T, float gm, float gp) {
   using Sh = EoShape<P>;
   constexpr int N = Sh::N, H = Sh::H;
   float s[H], d[H], fm = 0.0f;
@@ -89,43 +159,42 @@ __device__ __forceinline__ void line_shared(float* line, const float* T, float g
   line_pairs<P>(s, d, fm, T, gm, gp, [&](int m, float v) { line[m * S] = v; });
 }
 
-template <int P, int RK>
-__global__ void __launch_bounds__(FixShape<P>::THREADS, line_min_blocks<P>())
-    stage_line_kernel(const __grid_constant__ LineStageArgs<P> a) {
+// Elements [eb, eb + nloc) through one stage by a block of at least nloc N^2
+// threads; smem: line_smem of epb elements; tab(d): the table of direction d;
+// pre(): runs after the loads and before the block's first barrier.
+template <int P, int RK, typename Tab, typename Pre>
+__device__ __forceinline__ void line_elements(const double* __restrict__ q,
+                                              const double* __restrict__ q0,
+                                              double* __restrict__ qout,
+                                              const float* __restrict__ u,
+                                              const float* __restrict__ v,
+                                              const float* __restrict__ w, const Box& box,
+                                              double ra, double rb, long long eb, int nloc, int epb,
+                                              float* smem, Tab&& tab, Pre&& pre) {
   using Sh = FixShape<P>;
   using Eo = EoShape<P>;
-  constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NS = Sh::NS, EW = Sh::EW,
-                H = Eo::H;
-  const int epb = blockDim.x / N2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const long long eb = a.s.elem_begin + (long long)blockIdx.x * epb;
-  const long long left = a.s.elem_begin + a.s.elem_count - eb;
-  const int nloc = (int)(left < epb ? left : epb);
+  constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NS = Sh::NS, EW = Sh::EW, H = Eo::H;
   const int le = threadIdx.x / N2, r = threadIdx.x - le * N2;
   const bool on = le < nloc;
   const int i = r % N, j = r / N;
-  float* sX = reinterpret_cast<float*>(smem_raw) + le * EW;
+  float* sX = smem + le * EW;
   float* sY = sX + epb * EW;
   const long long ge = (eb + le) * NP;  // the element's first node
-  const double* __restrict__ q = a.s.q_in;
   const int zat = i + NS * j;  // the z line's first node in the padded arrays
 
   // the z line's fluxes, of which it keeps the pair values; the six face fluxes
   float g[6], s[H], d[H], fm = 0.0f;
   if (on) {
     if constexpr (RK == kRkGeneral)
-      for (int t = 16 * r; t < NP; t += 16 * N2) prefetch_l2(a.s.q0 + ge + t);
-    const float* __restrict__ u = static_cast<const float*>(a.s.u);
-    const float* __restrict__ v = static_cast<const float*>(a.s.v);
-    const float* __restrict__ w = static_cast<const float*>(a.s.w);
+      for (int t = 16 * r; t < NP; t += 16 * N2) prefetch_l2(q0 + ge + t);
     float F[N];
 #pragma unroll
     for (int m = 0; m < N; m++) {
       const long long n = ge + r + m * N2;
-      const float qv = to_ct<float>(q[n]);
-      sX[zat + m * NS * N] = qv * u[n];
-      sY[zat + m * NS * N] = qv * v[n];
-      F[m] = __fmul_rn(qv, w[n]);
+      const float qv = to_ct<float>(__ldg(q + n));
+      sX[zat + m * NS * N] = qv * __ldg(u + n);
+      sY[zat + m * NS * N] = qv * __ldg(v + n);
+      F[m] = __fmul_rn(qv, __ldg(w + n));
     }
 #pragma unroll
     for (int l = 0; l < H; l++) {
@@ -134,42 +203,54 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, line_min_blocks<P>())
     }
     if constexpr (Eo::ODD != 0) fm = F[H];
     unsigned nb[6];
-    fix_neighbors(a.s.box, (unsigned)(eb + le), nb);
+    fix_neighbors(box, (unsigned)(eb + le), nb);
     const int x0 = i * N + j * N2, y0 = i + j * N2;
     const int nM[6] = {y0, x0 + (N - 1), y0 + (N - 1) * N, x0, r, r + (N - 1) * N2};
     const int nP[6] = {y0 + (N - 1) * N, x0, y0, x0 + (N - 1), r + (N - 1) * N2, r};
 #pragma unroll
     for (int f = 0; f < 6; f++) {
       const long long gP = (long long)nb[f] * NP + nP[f];
-      const float qP = to_ct<float>(q[gP]), qM = to_ct<float>(q[ge + nM[f]]);
+      const float qP = to_ct<float>(__ldg(q + gP)), qM = to_ct<float>(__ldg(q + ge + nM[f]));
       const float* vel = (f == 1 || f == 3) ? u : (f == 0 || f == 2) ? v : w;
-      const float uM = vel[ge + nM[f]], uP = vel[gP];
+      const float uM = __ldg(vel + ge + nM[f]), uP = __ldg(vel + gP);
       const float a2 = fabsf(uP + uM);
       const float tw = (f == 1 || f == 2 || f == 5) ? 2.0f : -2.0f;
       g[f] = fmaf(qP, fmaf(tw, uP, -a2), -(qM * fmaf(tw, uM, -a2)));
     }
   }
+  pre();
   __syncthreads();
   if (on) {
     // lines along i (r = j + N k) and along j (r = i + N k)
-    line_shared<P, 1>(sX + NS * r, a.tab, g[3], g[1]);
-    line_shared<P, NS>(sY + i + NS * N * j, a.tab + Eo::TE, g[0], g[2]);
+    line_shared<P, 1>(sX + NS * r, tab(0), g[3], g[1]);
+    line_shared<P, NS>(sY + i + NS * N * j, tab(1), g[0], g[2]);
   }
   __syncthreads();
   if (on) {
-    const double* __restrict__ q0 = a.s.q0;
-    double* __restrict__ qout = a.s.q_out;
-    const double ra = a.s.a, rb = a.s.b;
-    line_pairs<P>(s, d, fm, a.tab + 2 * Eo::TE, g[4], g[5], [&](int m, float z) {
+    line_pairs<P>(s, d, fm, tab(2), g[4], g[5], [&](int m, float z) {
       const int at = zat + m * NS * N;
       const double inc = f32_to_f64_bits((sX[at] + sY[at]) + z);
       const long long n = ge + r + m * N2;
       if constexpr (RK == kRkTend)
         qout[n] = inc;
       else
-        qout[n] = rk_combine<RK>(inc, q[n], RK == kRkGeneral ? q0[n] : 0.0, ra, rb);
+        qout[n] = rk_combine<RK>(inc, __ldg(q + n), RK == kRkGeneral ? __ldg(q0 + n) : 0.0, ra, rb);
     });
   }
+}
+
+template <int P, int RK>
+__global__ void __launch_bounds__(FixShape<P>::THREADS, line_min_blocks<P>())
+    stage_line_kernel(const __grid_constant__ LineStageArgs<P> a) {
+  const int epb = blockDim.x / FixShape<P>::N2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const long long eb = a.s.elem_begin + (long long)blockIdx.x * epb;
+  const long long left = a.s.elem_begin + a.s.elem_count - eb;
+  line_elements<P, RK>(a.s.q_in, a.s.q0, a.s.q_out, static_cast<const float*>(a.s.u),
+                       static_cast<const float*>(a.s.v), static_cast<const float*>(a.s.w), a.s.box,
+                       a.s.a, a.s.b, eb, (int)(left < epb ? left : epb), epb,
+                       reinterpret_cast<float*>(smem_raw),
+                       [&](int d) { return LineTable<P>{a.tab + d * EoShape<P>::TE}; }, [] {});
 }
 
 template <int P, int RK>

@@ -285,3 +285,34 @@ def test_fp32_line_stage_within_its_rounding_bound(p, dims):
     qm, um = np.abs(q).max(), max(np.abs(a).max() for a in (u, v, w))
     bound = 3 * qm * um * (Es * rows + 2 * Fs * lift * 2) * (N + 4) * 2.0 ** -24
     assert np.max(np.abs(s.tendency() - want)) <= bound
+
+
+@pytest.mark.parametrize("threads,epb", [(32, 1), (96, 5), (128, 2), (512, 8)])
+def test_batched_line_stage_equals_the_single_box_bit_for_bit(threads, epb):
+    """Every order of the batch at block sizes below and above one element's
+    lines, items of part of a block's lines and of several rounds: the members'
+    bits are the single-box solver's."""
+    import sdg
+    import workloads as W
+    orders = list(range(1, 12))
+    tab = {p: W.reference_operators(p) for p in orders}
+    dims = [(3 + p % 3, 2 + p % 2, 3) for p in orders]
+    dt = [1e-3 / (2 * p + 1) for p in orders]
+    ens = sdg.Ensemble(dims, orders, dt, tab)
+    for p in orders:
+        ens.set_epb(p, 1)
+        ens.set_threads(threads, p=p)
+        ens.set_epb(p, min(epb, 8 if p < 9 else 4))
+    states = []
+    for i, p in enumerate(orders):
+        c = Case(*dims[i], p)
+        f = _fields(c)
+        states.append((c, f))
+        ens.upload(i, *f)
+    ens.step(3)
+    for i, (c, f) in enumerate(states):
+        s = sdg.Solver(*dims[i], orders[i], *tab[orders[i]][1::2], opt=sdg.OPT_EVENODD,
+                       precision=sdg.PREC_FP32)
+        s.upload(*f)
+        s.step(dt[i], 3)
+        assert np.array_equal(ens.download(i), s.download()), orders[i]
