@@ -386,7 +386,8 @@ def bench_ensemble(sdg, args):
                        [m["dt"] for m in members], ops)
     if args.batch_opt != "auto":
         ens.set_opt(OPTS[args.batch_opt])
-    ens.set_parallel_groups(args.parallel_groups)
+    if args.parallel_groups:
+        ens.set_parallel_groups(True)
     for i, m in enumerate(members):
         ens.init_blob(i, m["centre"], m["sigma"], m["vel"])
     sdg.synchronize()
@@ -1148,8 +1149,8 @@ def main() -> int:
     ap.add_argument("--serve-rate", type=float, default=20.0)
     ap.add_argument("--serve-rate-saturated", type=float, default=200.0)
     ap.add_argument("--parallel-groups", action="store_true",
-                    help="run the batched forms' order groups on parallel streams instead of "
-                         "one after the other")
+                    help="run the batched forms' order groups on parallel streams (the default "
+                         "of the library)")
     ap.add_argument("--serve-sweep", default="10,50,100,500,2000",
                     help="offered rates (req/s) of the serving sweep, comma separated")
     ap.add_argument("--serve-max-ne", type=int, default=32)

@@ -483,9 +483,9 @@ int sdg_ensemble_set_order_threads(sdg_ensemble* e, int p, int threads);
 /* threads_by_order receives 12 entries (index = order). */
 int sdg_ensemble_get_threads(const sdg_ensemble* e, int* threads_by_order);
 /* on = 1: the order groups of a step run on parallel graph branches (one
- * stream each, joined before the index advance); on = 0 (the default): one
- * after the other on the ensemble's stream.  Results are the same either
- * way. */
+ * stream each, joined before the index advance), as they do by default;
+ * on = 0: one after the other on the ensemble's stream.  Results are the same
+ * either way. */
 int sdg_ensemble_set_parallel_groups(sdg_ensemble* e, int on);
 /* on = 1: every RK stage is ONE persistent launch over the work items of all
  * orders (blocks take items round-robin and switch on the item's order and
@@ -536,8 +536,9 @@ typedef struct {
                                (running sums) */
   int threads_by_order[16]; /* block size by order (0: `threads`, else the
                                default of the order) */
-  int parallel_groups;      /* 0: the order groups of a step run one after the
-                               other on one stream; 1: on parallel streams */
+  int parallel_groups;      /* 1: the order groups of a step run on parallel
+                               streams; 0: the library's choice, which is the
+                               same (same results either way) */
 } sdg_server_config;
 typedef struct {
   int NeX, NeY, NeZ, p, nstep;

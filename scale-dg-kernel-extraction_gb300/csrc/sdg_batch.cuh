@@ -103,16 +103,17 @@ int batch_advance_launch(BatchInst* d_inst, int n_inst, cudaStream_t st);
 // One side stream per order group, when `parallel` is set.  Groups touch
 // disjoint instances, so a step can fork from the caller's stream into the
 // groups' streams (each runs its group's three stages in order) and join
-// them before the index advance, letting a small group's blocks fill the
-// tail of a large group's launch.  Measured on GB300 it is slower (333
-// against 369 solves/s on a 256-member ensemble of orders 3, 5 and 7; 27.4
-// against 28.8 on the saturated serving stream), so the default runs the
-// groups one after the other on the caller's stream.
+// them before the index advance, which lets one group's blocks fill the tail
+// of another's launch.  Measured on GB300, us a step, one after the other /
+// in parallel: 12 members of 4^3..24^3 at p = 3, 5, 7 200 / 167, 5 small ones 59 /
+// 29, 64 members 1181 / 1130, 256 of 8^3..24^3 6443 / 6391, 24 members of ten
+// orders 541 / 384; a burst of 16 served requests of ten orders 68 / 49 ms.
+// Never slower, so it is the default.
 struct BatchForkJoin {
   std::vector<cudaStream_t> streams;
   std::vector<cudaEvent_t> done;
   cudaEvent_t fork = nullptr;
-  bool parallel = false;  // false: every group on the caller's stream
+  bool parallel = true;  // false: every group on the caller's stream
   // true: each stage is ONE persistent launch over the items of every order
   // (batch_stage_kernel), instead of one launch per order group
   bool fused = false;
