@@ -328,6 +328,7 @@ int sdg_advect3d_eq_cal_tend(double* dqdt, const double* q, const double* u,
              ar.at<double>(oS), ar.at<double>(oX), ar.at<int>(oR), Ne,
              (long long)Np * NeA};
   SDG_TRY(tend_dev(a, Nq - 1, NfpTot, opt, st));
+  touch_pages(dqdt, 8 * nO);
   int err = 0;
   SDG_CUDA_TRY(cudaMemcpyAsync(&err, ar.at<void>(oR), sizeof(int), cudaMemcpyDeviceToHost, st));
   SDG_CUDA_TRY(cudaMemcpyAsync(dqdt, ar.at<void>(od), 8 * nO, cudaMemcpyDeviceToHost, st));
@@ -379,6 +380,7 @@ int sdg_tensorprod_divlike_dirXYZ(double* ox, double* oy, double* oz,
             ar.at<double>(o[3]), ar.at<double>(o[4]), ar.at<double>(o[5]),
             ar.at<double>(o[6]), ar.at<double>(o[7]), nelem};
   SDG_TRY(dropin(Nq - 1, 1, opt, &a, nullptr));
+  for (double* o : {ox, oy, oz}) touch_pages(o, 8 * n);
   SDG_CUDA_TRY(cudaMemcpy(ox, a.ox, 8 * n, cudaMemcpyDeviceToHost));
   SDG_CUDA_TRY(cudaMemcpy(oy, a.oy, 8 * n, cudaMemcpyDeviceToHost));
   SDG_CUDA_TRY(cudaMemcpy(oz, a.oz, 8 * n, cudaMemcpyDeviceToHost));
@@ -439,6 +441,7 @@ int host_contract(int what, double* ox, double* oy, double* oz, const double* Ma
             nin > 1 ? ar.at<double>(o[6]) : nullptr, nin > 2 ? ar.at<double>(o[7]) : nullptr,
             nblocks};
   SDG_TRY(dropin(Nq - 1, what, opt, &a, nullptr));
+  for (double* o : {ox, oy, oz}) touch_pages(o, 8 * n);
   SDG_CUDA_TRY(cudaMemcpy(ox, a.ox, 8 * n, cudaMemcpyDeviceToHost));
   SDG_CUDA_TRY(cudaMemcpy(oy, a.oy, 8 * n, cudaMemcpyDeviceToHost));
   SDG_CUDA_TRY(cudaMemcpy(oz, a.oz, 8 * n, cudaMemcpyDeviceToHost));
@@ -501,6 +504,7 @@ int sdg_element_matvec_dir(int dir, double* vec_out, const double* Mat, const do
   SDG_CUDA_TRY(cudaMemcpy(ar.at<void>(oi), vec_in, 8 * n, cudaMemcpyHostToDevice));
   SDG_TRY(sdg_element_matvec_dir_dev(dir, ar.at<double>(oo), ar.at<double>(oM),
                                      ar.at<double>(oi), Nq, nelem, nullptr));
+  touch_pages(vec_out, 8 * n);
   SDG_CUDA_TRY(cudaMemcpy(vec_out, ar.at<void>(oo), 8 * n, cudaMemcpyDeviceToHost));
   return SDG_OK;
 }
@@ -533,6 +537,7 @@ int sdg_tensorprod_Lift_hexahedral(double* out, const double* Lift,
   DivArgs a{ar.at<double>(oo), nullptr, nullptr, ar.at<double>(oL), nullptr,
             ar.at<double>(oi), nullptr, nullptr, nelem};
   SDG_TRY(dropin(Nq - 1, 2, SDG_OPT_GENERAL, &a, nullptr));
+  touch_pages(out, 8 * n);
   SDG_CUDA_TRY(cudaMemcpy(out, a.ox, 8 * n, cudaMemcpyDeviceToHost));
   return SDG_OK;
 }

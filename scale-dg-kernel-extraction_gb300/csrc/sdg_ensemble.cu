@@ -459,6 +459,7 @@ int sdg_ensemble_download(sdg_ensemble* e, int i, double* q) {
   if (!e || i < 0 || i >= e->n || !q) return fail(SDG_ERR_INVALID_ARG, "bad ensemble download");
   const BatchInst& I = e->inst[i];
   const long long nd = (long long)(I.p + 1) * (I.p + 1) * (I.p + 1) * I.box.Ne;
+  touch_pages(q, 8 * nd);  // while the steps run
   SDG_CUDA_TRY(cudaStreamSynchronize(e->stream));
   SDG_CUDA_TRY(cudaMemcpy(q, I.q[e->cur_host[i]], 8 * nd, cudaMemcpyDeviceToHost));
   return SDG_OK;

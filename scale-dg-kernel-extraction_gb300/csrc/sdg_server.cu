@@ -432,6 +432,7 @@ int sdg_server_submit(sdg_server* s, const sdg_request* r, double* out_state, ui
   q->r = *r;
   q->out = out_state;
   q->t_submit = Clock::now();
+  touch_pages(out_state, 8 * (size_t)request_dofs(*r));  // not by the worker's copy
   {
     std::lock_guard<std::mutex> lk(s->mu);
     if (s->stop) {

@@ -525,6 +525,7 @@ int sdg_solver_tendency(sdg_solver* s, double* dqdt) {
   if (!s || !dqdt) return fail(SDG_ERR_INVALID_ARG, "NULL argument");
   if (!s->dqdt) SDG_CUDA_TRY(cudaMalloc(&s->dqdt, 8 * (size_t)s->ndof));
   SDG_TRY(one_stage(s, 0, 0.0, s->q[s->cur], nullptr, s->dqdt, true));
+  touch_pages(dqdt, 8 * (size_t)s->ndof);
   SDG_CUDA_TRY(cudaMemcpyAsync(dqdt, s->dqdt, 8 * (size_t)s->ndof, cudaMemcpyDeviceToHost,
                                s->stream));
   SDG_CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -622,6 +623,7 @@ int sdg_solver_solve_host_pipelined(sdg_solver* s, int count, const double* cons
 
 int sdg_solver_download(sdg_solver* s, double* q) {
   if (!s || !q) return fail(SDG_ERR_INVALID_ARG, "NULL argument");
+  touch_pages(q, 8 * (size_t)s->ndof);  // while the steps run
   SDG_CUDA_TRY(cudaMemcpyAsync(q, s->q[s->cur], 8 * (size_t)s->ndof,
                                cudaMemcpyDeviceToHost, s->stream));
   SDG_CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -865,6 +867,7 @@ int sdg_slabs_step(sdg_slabs* s, double dt, int nstep) {
 int sdg_slabs_download(sdg_slabs* s, double* q) {
   if (!s || !q) return fail(SDG_ERR_INVALID_ARG, "NULL argument");
   const long long lay = (long long)s->NeX * s->NeY * s->Np;
+  touch_pages(q, 8 * (size_t)(lay * s->NeZ));
   for (int k = 0; k < s->nparts; k++) {
     const sdg_solver* ps = s->part[k];
     SDG_CUDA_TRY(cudaMemcpyAsync(q + s->z_begin[k] * lay, ps->q[ps->cur] + lay,

@@ -316,3 +316,20 @@ def test_batched_line_stage_equals_the_single_box_bit_for_bit(threads, epb):
         s.upload(*f)
         s.step(dt[i], 3)
         assert np.array_equal(ens.download(i), s.download()), orders[i]
+
+
+@pytest.mark.parametrize("offset", [0, 1, 4099])
+def test_download_into_fresh_and_offset_memory(offset):
+    """A download that maps its destination first: fresh memory, any alignment,
+    nothing outside the destination."""
+    import sdg
+    c = Case(9, 8, 7, 3)
+    f = _fields(c)
+    s = sdg.Solver(9, 8, 7, 3, c.D, c.Lift)
+    s.upload(*f)
+    whole = np.empty(c.nown + offset + 8192)
+    whole[:offset] = 7.0
+    whole[offset + c.nown:] = 7.0
+    s.download(out=whole[offset: offset + c.nown])
+    assert np.array_equal(whole[offset: offset + c.nown], f[0])
+    assert np.all(whole[:offset] == 7.0) and np.all(whole[offset + c.nown:] == 7.0)
