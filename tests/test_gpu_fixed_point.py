@@ -333,3 +333,23 @@ def test_download_into_fresh_and_offset_memory(offset):
     s.download(out=whole[offset: offset + c.nown])
     assert np.array_equal(whole[offset: offset + c.nown], f[0])
     assert np.all(whole[:offset] == 7.0) and np.all(whole[offset + c.nown:] == 7.0)
+
+
+@pytest.mark.parametrize("stage", [1, 2, 3])
+@pytest.mark.parametrize("n,offset", [(1, 0), (2, 0), (1001, 0), (1000, 1), (4097, 1)])
+def test_rk_stage_at_odd_sizes_and_alignments(stage, n, offset):
+    """The 8- and 16-byte forms against numpy: five roundings there and three here,
+    each of at most the terms' size, weigh no more than 7 units of it."""
+    import sdg
+    r = np.random.RandomState(n + stage)
+    q, q0, t = [r.randn(n + offset + 1) for _ in range(3)]
+    dq, d0, dt = [sdg.DeviceArray(x) for x in (q, q0, t)]
+    assert sdg.lib.sdg_rk_stage_dev(dq.ptr + 8 * offset, d0.ptr + 8 * offset,
+                                    dt.ptr + 8 * offset, n, 1, stage, 0.37, None) == 0
+    got = dq.numpy()
+    a, b = [(0.0, 1.0), (0.75, 0.25), (1.0 / 3.0, 2.0 / 3.0)][stage - 1]
+    m = slice(offset, offset + n)
+    want = a * q0[m] + b * (q[m] + 0.37 * t[m])
+    size = np.abs(q0[m]) + np.abs(q[m]) + np.abs(t[m])
+    assert np.all(np.abs(got[m] - want) <= 7 * 2.0 ** -53 * size)
+    assert np.array_equal(got[:offset], q[:offset]) and got[offset + n] == q[offset + n]
