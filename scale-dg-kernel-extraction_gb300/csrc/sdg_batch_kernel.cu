@@ -77,7 +77,7 @@ __device__ __forceinline__ void batch_item_body(const BatchInst& I, const BatchI
     // own z line of the arrays; the first barrier inside orders the coefficients
     // before their first use.
     for (int e = 0; e < w.e_count; e += epb)
-      line_elements<P, RK>(
+      line_elements<P, RK, true>(
           q, I.q[s0], I.q[stage == 1 ? s2 : s1], I.u, I.v, I.w, I.box, c_rk_a[stage],
           c_rk_b[stage], w.e_begin + e, min(epb, w.e_count - e), epb, T + 3 * Rows::DIR,
           [&](int d) { return Rows{T + d * Rows::DIR}; },

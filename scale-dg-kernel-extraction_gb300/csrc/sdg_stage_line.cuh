@@ -15,7 +15,7 @@
 // loads at the two ends of a block.  On GB300, 16.8M DOF, against the kernels
 // this replaced (GDOF-updates/s): p = 2 140 from 110, p = 3 147 from 106, p = 5
 // 145 from 82, p = 7 171 from 108, p = 9 148 from 87, p = 11 146 from 93, p = 15
-// 148 from 87 (p = 1 126-130 from 130).  Half of it comes from L1: with the largest
+// 148 from 87 (p = 1 level at 130).  Half of it comes from L1: with the largest
 // shared-memory carveout 84 at p = 5.  The state is read by __ldg: plain reads of
 // q and q0 wait for the store of the node before (p = 7 151, and 89 against 131 in
 // the batch).  64 registers (1024 threads an SM): 1280 threads 0.85-1.0x, 768
@@ -159,10 +159,19 @@ __device__ __forceinline__ void line_shared(float* line, const Table& T, float g
   line_pairs<P>(s, d, fm, T, gm, gp, [&](int m, float v) { line[m * S] = v; });
 }
 
+// A read of what this launch does not write (RO: as a read-only load).
+template <bool RO, typename T>
+__device__ __forceinline__ T line_read(const T* p) {
+  if constexpr (RO)
+    return __ldg(p);
+  else
+    return *p;
+}
+
 // Elements [eb, eb + nloc) through one stage by a block of at least nloc N^2
 // threads; smem: line_smem of epb elements; tab(d): the table of direction d;
 // pre(): runs after the loads and before the block's first barrier.
-template <int P, int RK, typename Tab, typename Pre>
+template <int P, int RK, bool RO, typename Tab, typename Pre>
 __device__ __forceinline__ void line_elements(const double* __restrict__ q,
                                               const double* __restrict__ q0,
                                               double* __restrict__ qout,
@@ -191,10 +200,10 @@ __device__ __forceinline__ void line_elements(const double* __restrict__ q,
 #pragma unroll
     for (int m = 0; m < N; m++) {
       const long long n = ge + r + m * N2;
-      const float qv = to_ct<float>(__ldg(q + n));
-      sX[zat + m * NS * N] = qv * __ldg(u + n);
-      sY[zat + m * NS * N] = qv * __ldg(v + n);
-      F[m] = __fmul_rn(qv, __ldg(w + n));
+      const float qv = to_ct<float>(line_read<RO>(q + n));
+      sX[zat + m * NS * N] = qv * line_read<RO>(u + n);
+      sY[zat + m * NS * N] = qv * line_read<RO>(v + n);
+      F[m] = __fmul_rn(qv, line_read<RO>(w + n));
     }
 #pragma unroll
     for (int l = 0; l < H; l++) {
@@ -210,9 +219,9 @@ __device__ __forceinline__ void line_elements(const double* __restrict__ q,
 #pragma unroll
     for (int f = 0; f < 6; f++) {
       const long long gP = (long long)nb[f] * NP + nP[f];
-      const float qP = to_ct<float>(__ldg(q + gP)), qM = to_ct<float>(__ldg(q + ge + nM[f]));
+      const float qP = to_ct<float>(line_read<RO>(q + gP)), qM = to_ct<float>(line_read<RO>(q + ge + nM[f]));
       const float* vel = (f == 1 || f == 3) ? u : (f == 0 || f == 2) ? v : w;
-      const float uM = __ldg(vel + ge + nM[f]), uP = __ldg(vel + gP);
+      const float uM = line_read<RO>(vel + ge + nM[f]), uP = line_read<RO>(vel + gP);
       const float a2 = fabsf(uP + uM);
       const float tw = (f == 1 || f == 2 || f == 5) ? 2.0f : -2.0f;
       g[f] = fmaf(qP, fmaf(tw, uP, -a2), -(qM * fmaf(tw, uM, -a2)));
@@ -234,7 +243,7 @@ __device__ __forceinline__ void line_elements(const double* __restrict__ q,
       if constexpr (RK == kRkTend)
         qout[n] = inc;
       else
-        qout[n] = rk_combine<RK>(inc, __ldg(q + n), RK == kRkGeneral ? __ldg(q0 + n) : 0.0, ra, rb);
+        qout[n] = rk_combine<RK>(inc, line_read<RO>(q + n), RK == kRkGeneral ? line_read<RO>(q0 + n) : 0.0, ra, rb);
     });
   }
 }
@@ -246,7 +255,8 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, line_min_blocks<P>())
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const long long eb = a.s.elem_begin + (long long)blockIdx.x * epb;
   const long long left = a.s.elem_begin + a.s.elem_count - eb;
-  line_elements<P, RK>(a.s.q_in, a.s.q0, a.s.q_out, static_cast<const float*>(a.s.u),
+  // p = 1: its two nodes a line wait little; plain reads 130 against 126
+  line_elements<P, RK, (P > 1)>(a.s.q_in, a.s.q0, a.s.q_out, static_cast<const float*>(a.s.u),
                        static_cast<const float*>(a.s.v), static_cast<const float*>(a.s.w), a.s.box,
                        a.s.a, a.s.b, eb, (int)(left < epb ? left : epb), epb,
                        reinterpret_cast<float*>(smem_raw),
