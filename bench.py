@@ -235,7 +235,7 @@ def run_reference(args, ws, rank):
     return 0
 
 
-PREC_LABEL = {"fp64": "FP64", "fp64emu": "FP64 state, double-float arithmetic",
+PREC_LABEL = {"fp64": "FP64", "fp64emu": "FP64 state, fixed-point sums",
               "fp32": "FP32-compute/FP64-state"}
 
 
@@ -292,8 +292,9 @@ def roofline(precision, p, ne, ndof, t, steps, peaks, opt="opt1"):
     (`implementation_bytes_per_dof_update`) and not counted.  `traffic` is
     the ncu DRAM bytes per launch of the same kernel.
 
-    Compute: the FP64 pipe binds the FP64 forms (1.2 TFLOP/s DFMA against
-    88.75 flops a DOF-update at p = 7).  `compute.frac` is that pipe's busy
+    Compute: the FP64 forms' line sums are integer multiply-adds; FP64 keeps
+    the products, the face fluxes and the RK update, and its pipe is the busiest
+    unit.  `compute.frac` is that pipe's busy
     share from the kernel's ncu capture (sm__pipe_fp64_cycles_active);
     `achieved_tflops` counts the reference's formulas (25 + 6 Nq + 126 / Nq
     flops a DOF-update) against the DFMA peak measured live.  The FP32 and
@@ -308,18 +309,12 @@ def roofline(precision, p, ne, ndof, t, steps, peaks, opt="opt1"):
     per_gpu = ndof * 3 * steps / t / 1e9
     fl = flops_per_dof_update(p)
     pipe = "dfma_tflops" if precision == "fp64" else "ffma_tflops"
-    kernel = {"fp64": f"stage_kernel<{p},double>", "fp32": f"stage_kernel<{p},float>",
-              "fp64emu": f"stage_emu_kernel<{p}>"}[precision]
-    tkey = f"stage_{precision}_p{p}_ne{ne}"
-    if precision == "fp64" and opt == "evenodd":
-        kernel, tkey = f"stage_eo_kernel<{p},double>", f"stage_fp64eo_p{p}_ne{ne}"
-    elif precision == "fp64emu" and opt == "evenodd":
-        kernel, tkey = f"stage_emu_eo_kernel<{p}>", f"stage_fp64emueo_p{p}_ne{ne}"
-    elif precision == "fp32" and opt == "evenodd":
-        # the single box's own kernels at the lowest orders (same arithmetic)
-        k32 = {1: "stage_p1_kernel", 2: "stage_col_kernel<2>", 3: "stage_p3_kernel"}
-        kernel = k32.get(p, f"stage_eo_kernel<{p},float>")
-        tkey = f"stage_fp32eo_p{p}_ne{ne}"
+    eo = opt == "evenodd"
+    if precision == "fp32":
+        kernel = f"stage_line_kernel<{p}>" if eo else f"stage_kernel<{p},float>"
+    else:  # FP64 and emulated FP64 are one arithmetic
+        kernel = f"stage_fix_kernel<{p},{str(eo).lower()}>"
+    tkey = f"stage_{precision}{'eo' if eo else ''}_p{p}_ne{ne}"
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak,
             "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
@@ -667,7 +662,7 @@ def bench_dropin_step(sdg, args, wl, fused_rate, opt=None):
     (sdg_advect3d_eq_step_dev): mesh arrays built on the device, then K
     SSP-RK3 steps; EVENODD runs one fused launch a stage (face flux from
     VMapM/VMapP, normal_fn and Fscale, per-node Escale, lift, RK update),
-    OPT1 the reference's per-stage sequence.  Timed on the host around the
+    OPT1 the same with the operators as given.  Timed on the host around the
     call with a synchronize on both sides."""
     opt = sdg.OPT_EVENODD if opt is None else opt
     p, ne = args.p, args.ne
@@ -712,12 +707,12 @@ def bench_dropin_step(sdg, args, wl, fused_rate, opt=None):
     t = time.perf_counter() - t0
     assert err.numpy()[0] == 0
     rate = np_ * ne3 * 3 * k / t / 1e9
-    oname = {sdg.OPT_OPT1: "OPT1 order, the reference's per-stage sequence",
+    oname = {sdg.OPT_OPT1: "OPT1, one fused launch a stage",
              sdg.OPT_EVENODD: "one fused even-odd launch a stage"}[opt]
     return {"workload": f"same {ne}^3 p={p} box, sdg_advect3d_eq_step_dev on the reference's "
                         f"arrays (VMapM/VMapP, halo_src_map, normal_fn, Escale, Fscale), {oname}",
             "gdof_updates_per_s": rate, "ms_per_step": 1e3 * t / k, "steps": k,
-            "launches_per_step": 3 if opt == sdg.OPT_EVENODD else 13,
+            "launches_per_step": 3,
             "ratio_to_fused_structured_stage": rate / fused_rate,
             "scratch_bytes": nbytes}
 
@@ -934,7 +929,7 @@ def headline_line(args, ws, value, t, roof, cpu, e2e, clk, parity, sections) -> 
         "metric": metric_name(args), "value": value, "unit": "GDOF-updates/s", "n_gpus": ws,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * t / args.steps,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": {"fp64": "f64", "fp64emu": "f64-state/double-float",
+        "dtype": {"fp64": "f64", "fp64emu": "f64-state/fixed-point",
                   "fp32": "f32-compute/f64-state"}[args.precision],
         "data": "synthetic (seeded Gaussian tracer, seeded smooth velocity)",
         "config": config(args),
@@ -1029,8 +1024,8 @@ def run_ours(args, ws, rank, local):
                                  args.warmup, local, barrier, False, OPTS[args.opt])
         te_ = tmax(te_)
         other = {"precision": "fp64emu",
-                 "description": "FP64 state and RK combine; flux, divergence and lift in "
-                                "double-float (two FP32 numbers) on the FP32 pipes",
+                 "description": "FP64 state, face flux and RK combine; divergence and lift "
+                                "in 60-bit fixed point (the FP64 form's stage)",
                  "value": ws * ndof * 3 * args.steps / te_ / 1e9, "unit": "GDOF-updates/s",
                  "ms_per_step": 1e3 * te_ / args.steps,
                  "roofline": roofline("fp64emu", p, ne, ndof, te_, args.steps, peaks, args.opt)}

@@ -406,7 +406,8 @@ int sdg_solver_run(sdg_solver* s, double dt, int nstep, int output_interval,
 /* Evaluates the tendency of the current state into dqdt (owned part,
  * host memory), the fused-kernel analogue of advect3d_eq_cal_tend. */
 int sdg_solver_tendency(sdg_solver* s, double* dqdt);
-/* Kernel launches one step issues (for launch accounting). */
+/* Kernel launches one step issues (for launch accounting) where its stages are
+ * launches of their own; a small box takes one launch a step call. */
 int sdg_solver_launches_per_step(const sdg_solver* s);
 /* The solver's stream as void*. */
 void* sdg_solver_stream(const sdg_solver* s);
