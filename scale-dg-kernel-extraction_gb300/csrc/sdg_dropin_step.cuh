@@ -113,6 +113,12 @@ __device__ __forceinline__ int64_t ref_escale_sig(double es) {
   return fix_unit(
       __hiloint2double(__double2hiint(es) - (ref_escale_exp(es) << 20), __double2loint(es)));
 }
+// The exponent field of a line's two faces, less that of its Escale; past the
+// fields of a double (an Escale below a half, faces infinite, NaN or huge) the
+// largest, which no line takes in fixed point.
+__device__ __forceinline__ int32_t ref_face_exp(double gm, double gp, int xe) {
+  return min((max(fix_value_exp(gm), fix_value_exp(gp)) >> 20) - xe, 2047) << 20;
+}
 // The limbs of a table entry (its minus sign is dqdt's), a derivative entry
 // with the significand of Escale.
 __device__ __forceinline__ fixlimb ref_coef(double entry, bool derivative, int64_t sig) {
@@ -372,7 +378,7 @@ __device__ __forceinline__ int ref_line_shared(const RefArgs& a, const fixlimb* 
                                                const double* Es) {
   constexpr int N = P + 1;
   double F[N];
-  int32_t E = max(0, max(fix_value_exp(gm), fix_value_exp(gp)) - (xe << 20));
+  int32_t E = max(0, ref_face_exp(gm, gp, xe));
 #pragma unroll
   for (int l = 0; l < N; l++) {
     F[l] = line[l * S];
@@ -513,7 +519,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
   double F[N];
   int32_t E = 0;
   if (on) {
-    E = max(0, max(fix_value_exp(g[4]), fix_value_exp(g[5])) - (xe[2] << 20));
+    E = max(0, ref_face_exp(g[4], g[5], xe[2]));
 #pragma unroll
     for (int m = 0; m < N; m++) {
       F[m] = q[ge + r + m * N2] * a.w[ge + r + m * N2];

@@ -1,0 +1,90 @@
+"""Calls at the edges of the fixed-point forms' ranges: face fluxes and scale
+factors whose exponents lie far apart, on the reference's arrays.  The expected
+values are the oracle's; the tolerance is the FP64 form's 1e-12 relative L2 per
+tendency."""
+import copy
+
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import Case, TOL_TEND, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+both = pytest.mark.parametrize("opt", ["OPT_EVENODD", "OPT_OPT1"])
+
+
+def _cal_tend(c, m, q, opt, D=None, Lift=None):
+    """(GPU tendency, oracle tendency) of state q on mesh m."""
+    import sdg
+    D = c.D if D is None else D
+    Dt = np.ascontiguousarray(D.reshape(m.Nq, m.Nq).T).reshape(-1)
+    Lift = c.Lift if Lift is None else Lift
+    want = O.cal_tend(m, q, c.u, c.v, c.w, D, Dt, Lift, O.OPT1)[: c.nown]
+    sdg.dg_optr_kernel_setup(opt[4:])
+    got = np.zeros(m.Np * m.NeA)
+    sdg.advect3d_eq_cal_tend(got, q, c.u, c.v, c.w, D, Dt, Lift, m.VMapM, m.VMapP, m.normal_fn,
+                             m.Escale, m.Fscale, m.Nq, m.Np, m.NfpTot, m.Ne, m.NeA)
+    return got[: c.nown], want
+
+
+def _loop(c, m, q, dt, nstep, opt):
+    """(GPU state, oracle state) after nstep steps of the loop on mesh m."""
+    import sdg
+    got = sdg.advect3d_eq_step(q, c.u, c.v, c.w, c.D, c.Dt, c.Lift, m.VMapM, m.VMapP, m.normal_fn,
+                               m.Escale, m.Fscale, m.halo_src_map, m.Nq, m.Np, m.NfpTot, m.Ne,
+                               m.NeA, m.NhaloNode, dt, nstep, getattr(sdg, opt))[: c.nown]
+    want = q.copy()
+    O.run(m, want, c.u, c.v, c.w, c.D, c.Dt, c.Lift, dt, nstep, O.OPT1)
+    return got, want[: c.nown]
+
+
+def _agree(got, want):
+    fine = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), fine)
+    assert rel_l2(got[fine], want[fine]) <= TOL_TEND
+
+
+# element counts on the fixed-point side of the small-mesh rule
+MESHES = pytest.mark.parametrize("p,dims", [(3, (15, 14, 13)), (7, (8, 7, 8)), (8, (7, 7, 6)),
+                                            (13, (3, 5, 4))])
+
+
+@both
+@MESHES
+@pytest.mark.parametrize("length", [1.0, 30.0, 1e4])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_non_finite_neighbours_reach_elements_of_any_size(opt, p, dims, length, bad):
+    """A face value that is not finite reaches the element beyond the face
+    whatever the elements' size: with Escale = 2 / h far above one, near and far
+    below a half."""
+    c = Case(*dims, p)
+    m = O.Mesh(*dims, p, c.x1D, L=(length,) * 3)
+    q = c.q.copy()
+    q[m.Np * (m.Ne // 2)] = bad  # a corner: on the -x, -y and -z face
+    m.update_halo(q)
+    with np.errstate(all="ignore"):
+        got, want = _cal_tend(c, m, q, opt)
+        beyond = [i for i in range(m.Ne) if i != m.Ne // 2
+                  and not np.isfinite(want[i * m.Np:(i + 1) * m.Np]).all()]
+        assert len(beyond) == 3
+        _agree(got, want)
+        _agree(*_loop(c, m, q, 0.5 * c.dt * length, 1, opt))
+
+
+@both
+@MESHES
+def test_huge_face_fluxes_over_small_scale_factors(opt, p, dims):
+    """Face fluxes of 2^1011 beside Escale of 2^-16: their ratio passes the
+    largest double, every result is finite."""
+    c = Case(*dims, p)
+    m = copy.copy(c.mesh)
+    m.Escale = m.Escale * 2.0 ** -20
+    q = c.q.copy()
+    q[m.Np * (m.Ne // 2 + 1) - 1] = 2.0 ** 1008  # flows out through three faces
+    m.update_halo(q)
+    got, want = _cal_tend(c, m, q, opt)
+    assert np.isfinite(want).all() and np.abs(want).max() > 2.0 ** 1005
+    k = 2.0 ** -900
+    _agree(got * k, want * k)
