@@ -88,3 +88,20 @@ def test_huge_face_fluxes_over_small_scale_factors(opt, p, dims):
     assert np.isfinite(want).all() and np.abs(want).max() > 2.0 ** 1005
     k = 2.0 ** -900
     _agree(got * k, want * k)
+
+
+@both
+@MESHES
+def test_scales_that_lie_apart_only_together(opt, p, dims):
+    """State, Escale and operators whose exponents each lie within the fixed-point
+    range and add up past a double's: the largest results near 2^-1005, those of
+    the tracer's tail subnormal."""
+    c = Case(*dims, p)
+    m = copy.copy(c.mesh)
+    m.Escale, m.Fscale = m.Escale * 2.0 ** -148, m.Fscale * 2.0 ** -148
+    q = c.q * 2.0 ** -685
+    D, Lift = c.D * 2.0 ** -180, c.Lift * 2.0 ** -180
+    got, want = _cal_tend(c, m, q, opt, D, Lift)
+    assert 0.0 < np.abs(want).max() < 2.0 ** -995
+    assert np.count_nonzero(np.abs(want) < 2.0 ** -1022) > 0
+    _agree(np.ldexp(got, 1000), np.ldexp(want, 1000))
