@@ -370,8 +370,18 @@ int sdg_solver_upload(sdg_solver* s, const double* q, const double* u,
 /* The same from device memory (asynchronous on the solver's stream). */
 int sdg_solver_upload_dev(sdg_solver* s, const double* q, const double* u,
                           const double* v, const double* w);
-/* Advances nstep SSP-RK3 steps of size dt (asynchronous). */
+/* Advances nstep SSP-RK3 steps of size dt (asynchronous).  A small FP64 box
+ * takes a step call as one launch, whose blocks wait for one another between
+ * the stages.  Should such a wait run out, the state is undefined: the next of
+ * step_timed, minmax, run, tendency, download and solve_host_pipelined returns
+ * SDG_ERR_TIMEOUT, and step calls before it do nothing on the device.  (A caller
+ * who only reads sdg_solver_state_dev learns of it from any of them, as
+ * sdg_solver_step_timed with nstep 0.)  After that an upload and further steps
+ * work again. */
 int sdg_solver_step(sdg_solver* s, double dt, int nstep);
+/* How often such a wait looks before it gives up: negative for the default
+ * (some seconds), 0 to give up at once (to test a caller's handling). */
+int sdg_solver_set_wait_limit(sdg_solver* s, int polls);
 /* sdg_solver_step bracketed by CUDA events on the solver's stream; waits
  * for the end event and returns the elapsed device time in *ms. */
 int sdg_solver_step_timed(sdg_solver* s, double dt, int nstep, double* ms);

@@ -139,10 +139,11 @@ int eo_tables(int Nq, const double* D1D, const double* Lift_mat, std::vector<dou
 // Fused stage launchers (sdg_stage_*.cu).  prec = SDG_PREC_*.
 int launch_stage(int p, int prec, int opt, const StageArgs& a, cudaStream_t st);
 // nstep whole steps of a small box in one launch (FP64 form): q the rotating
-// state buffers, the current one first; bar two device words, the first zero;
+// state buffers, the current one first; bar two device words, zero (the second
+// set by a wait between the stages that gave up after `polls` reads);
 // the result is in q[nstep % 3].  With q null: *most = the most elements.
 int launch_loop(int p, int opt, const StageArgs& a, double* const* q, double dt, int nstep,
-                unsigned* bar, long long* most, cudaStream_t st);
+                unsigned* bar, int polls, long long* most, cudaStream_t st);
 
 // min / max of q[0..n) as order keys (see sdg_minmax.cu); resets both keys first.
 int minmax_launch(const double* q, long long n, unsigned long long* kmin, unsigned long long* kmax,

@@ -24,6 +24,10 @@ struct IoSlot {
   cudaEvent_t uploaded = nullptr, computed = nullptr, downloaded = nullptr;
 };
 
+// Reads of the arrivals a wait of the one-launch steps takes before it gives up:
+// some seconds.
+constexpr int kLoopPolls = 1 << 22;
+
 struct sdg_solver {
   int p = 0, Nq = 0, Np = 0, opt = 0, prec = 0;
   Box box{};
@@ -51,6 +55,7 @@ struct sdg_solver {
   long long loop_most = -1;
   unsigned* bar = nullptr;  // in D's allocation
   bool loop_ran = false;
+  int loop_polls = kLoopPolls;
   // elements a stage advances: [elem_begin, elem_begin + elem_count) of the
   // box (the whole box by default; a z-slab partition advances its owned
   // layers and keeps a ghost layer on each side)
@@ -168,7 +173,7 @@ int takes_loop(sdg_solver* s, bool* yes) {
   *yes = false;
   if (s->prec == SDG_PREC_FP32 || s->elem_count >= 0 || s->box.Ne > kLoopElems) return SDG_OK;
   if (s->loop_most < 0)
-    SDG_TRY(launch_loop(s->p, s->opt, StageArgs{}, nullptr, 0.0, 0, nullptr, &s->loop_most,
+    SDG_TRY(launch_loop(s->p, s->opt, StageArgs{}, nullptr, 0.0, 0, nullptr, 0, &s->loop_most,
                         nullptr));
   if (s->box.Ne > s->loop_most) return SDG_OK;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -436,7 +441,7 @@ int sdg_solver_step(sdg_solver* s, double dt, int nstep) {
       const int n = std::min(left, kLoopSteps);
       double* q[3] = {s->q[s->cur], s->q[(s->cur + 1) % 3], s->q[(s->cur + 2) % 3]};
       const StageArgs a = stage_args(s, 0, dt, q[0], nullptr, q[1], s->u, s->v, s->w, false, 0);
-      SDG_TRY(launch_loop(s->p, s->opt, a, q, dt, n, s->bar, nullptr, s->stream));
+      SDG_TRY(launch_loop(s->p, s->opt, a, q, dt, n, s->bar, s->loop_polls, nullptr, s->stream));
       s->loop_ran = true;
       s->cur = (s->cur + n) % 3;
       left -= n;
@@ -453,6 +458,12 @@ int sdg_solver_step(sdg_solver* s, double dt, int nstep) {
     SDG_TRY(one_stage(s, 2, dt, s->q[s2], s->q[s0], s->q[s1], false, 2));
     s->cur = s1;
   }
+  return SDG_OK;
+}
+
+int sdg_solver_set_wait_limit(sdg_solver* s, int polls) {
+  if (!s) return fail(SDG_ERR_INVALID_ARG, "NULL solver");
+  s->loop_polls = polls >= 0 ? polls : kLoopPolls;
   return SDG_OK;
 }
 
@@ -529,7 +540,7 @@ int sdg_solver_tendency(sdg_solver* s, double* dqdt) {
   SDG_CUDA_TRY(cudaMemcpyAsync(dqdt, s->dqdt, 8 * (size_t)s->ndof, cudaMemcpyDeviceToHost,
                                s->stream));
   SDG_CUDA_TRY(cudaStreamSynchronize(s->stream));
-  return SDG_OK;
+  return loop_status(s);
 }
 
 // Pipelined host-to-host solves: two device buffer sets, an upload stream, a
@@ -618,7 +629,7 @@ int sdg_solver_solve_host_pipelined(sdg_solver* s, int count, const double* cons
   SDG_CUDA_TRY(cudaStreamSynchronize(s->h2d));
   SDG_CUDA_TRY(cudaStreamSynchronize(s->comp));
   SDG_CUDA_TRY(cudaStreamSynchronize(s->d2h));
-  return SDG_OK;
+  return loop_status(s);
 }
 
 int sdg_solver_download(sdg_solver* s, double* q) {

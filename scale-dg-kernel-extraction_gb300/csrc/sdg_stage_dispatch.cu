@@ -8,7 +8,7 @@ namespace sdg {
 #define SDG_DECL_ORDER(p)                                                                   \
   int launch_stage_p##p(int prec, int opt, const StageArgs& a, cudaStream_t st);            \
   int launch_loop_p##p(int opt, const StageArgs& a, double* const* q, double dt, int nstep, \
-                       unsigned* bar, long long* most, cudaStream_t st);
+                       unsigned* bar, int polls, long long* most, cudaStream_t st);
 SDG_DECL_ORDER(1) SDG_DECL_ORDER(2) SDG_DECL_ORDER(3) SDG_DECL_ORDER(4)
 SDG_DECL_ORDER(5) SDG_DECL_ORDER(6) SDG_DECL_ORDER(7) SDG_DECL_ORDER(8)
 SDG_DECL_ORDER(9) SDG_DECL_ORDER(10) SDG_DECL_ORDER(11) SDG_DECL_ORDER(12)
@@ -42,9 +42,9 @@ int launch_stage(int p, int prec, int opt, const StageArgs& a, cudaStream_t st) 
 }
 
 int launch_loop(int p, int opt, const StageArgs& a, double* const* q, double dt, int nstep,
-                unsigned* bar, long long* most, cudaStream_t st) {
-  using Fn = int (*)(int, const StageArgs&, double* const*, double, int, unsigned*, long long*,
-                     cudaStream_t);
+                unsigned* bar, int polls, long long* most, cudaStream_t st) {
+  using Fn = int (*)(int, const StageArgs&, double* const*, double, int, unsigned*, int,
+                     long long*, cudaStream_t);
   static const Fn fn[kMaxOrder] = {launch_loop_p1,  launch_loop_p2,  launch_loop_p3,
                                    launch_loop_p4,  launch_loop_p5,  launch_loop_p6,
                                    launch_loop_p7,  launch_loop_p8,  launch_loop_p9,
@@ -52,7 +52,7 @@ int launch_loop(int p, int opt, const StageArgs& a, double* const* q, double dt,
                                    launch_loop_p13, launch_loop_p14, launch_loop_p15};
   if (p < 1 || p > kMaxOrder)
     return fail(SDG_ERR_UNSUPPORTED_ORDER, "PolyOrder %d outside 1..15", p);
-  return fn[p - 1](opt, a, q, dt, nstep, bar, most, st);
+  return fn[p - 1](opt, a, q, dt, nstep, bar, polls, most, st);
 }
 
 }  // namespace sdg

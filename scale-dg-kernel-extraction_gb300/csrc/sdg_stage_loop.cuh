@@ -13,8 +13,10 @@
 // Measured on GB300, us a stage (100 steps), against one stage_fix_kernel launch
 // a stage: see fix_loop_most.
 //
-// The wait at the grid barrier is bounded: a block that gives up sets a flag,
-// which the solver's next call that waits for its stream reports, and leaves.
+// The wait at the grid barrier is bounded: a block that gives up sets a flag and
+// leaves.  Launches that find the flag set leave at once (the arrivals of the
+// one that gave up would let their stages run unordered); the solver's next
+// call that waits for its stream reports it and clears both words.
 #pragma once
 
 #include "sdg_stage_fix.cuh"
@@ -40,11 +42,12 @@ struct FixLoopArgs {
   double dt;
   int nstep;
   unsigned* bar;          // [0] arrivals (zero between launches), [1] a wait ran out
+  int polls;              // reads of the arrivals before a wait gives up
 };
 
 // Waits until every block has arrived `round` times; false when the wait ran
 // out (here or in another block).
-__device__ __forceinline__ bool fix_grid_barrier(unsigned* bar, unsigned round) {
+__device__ __forceinline__ bool fix_grid_barrier(unsigned* bar, unsigned round, int polls) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -52,7 +55,7 @@ __device__ __forceinline__ bool fix_grid_barrier(unsigned* bar, unsigned round) 
     atomicAdd(&bar[0], 1u);
     const unsigned want = round * gridDim.x;
     int good = 0;
-    for (int t = 0; t < (1 << 22); t++) {
+    for (int t = 0; t < polls; t++) {
       unsigned v;
       asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
       if ((int)(v - want) >= 0) {  // both may pass 2^32
@@ -124,6 +127,8 @@ __global__ void __launch_bounds__(LoopShape<P>::THREADS,
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int64_t* s0 = reinterpret_cast<int64_t*>(smem_raw);           // [3][EPB][EW]
   short* sE = reinterpret_cast<short*>(s0 + 3 * EPB * EW);      // [3][EPB][N2]
+  // one thread's answer for the block: another block may give up meanwhile
+  if (__syncthreads_or(threadIdx.x == 0 && __ldcg(a.bar + 1) != 0)) return;
   const long long eb = (long long)blockIdx.x * EPB;
   const int nloc = (int)min((long long)EPB, a.f.s.elem_count - eb);
   // one direction a group of whole warps
@@ -199,7 +204,7 @@ __global__ void __launch_bounds__(LoopShape<P>::THREADS,
                        : fma(ra, q0[it], rb * fma(c, v, qv[it]));
       }
       if (step + 1 < a.nstep || stage < 2)
-        if (!fix_grid_barrier(a.bar, ++round)) return;
+        if (!fix_grid_barrier(a.bar, ++round, a.polls)) return;
     }
     c0 = c0 == 2 ? 0 : c0 + 1;
   }
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(LoopShape<P>::THREADS,
 
 template <int P, bool EO>
 int launch_stage_fix_loop(const StageArgs& s, double* const* q, double dt, int nstep, unsigned* bar,
-                          cudaStream_t st) {
+                          int polls, cudaStream_t st) {
   using Ls = LoopShape<P>;
   FixLoopArgs<P, EO> a;
   fix_fill<P, EO>(a.f, s);
@@ -218,6 +223,7 @@ int launch_stage_fix_loop(const StageArgs& s, double* const* q, double dt, int n
   a.dt = dt;
   a.nstep = nstep;
   a.bar = bar;
+  a.polls = polls;
   const void* kernel = (const void*)stage_fix_loop_kernel<P, EO>;
   SDG_TRY(set_kernel_smem(kernel, (int)Ls::SMEM, carve_for(Ls::SMEM, Ls::BLOCKS)));
   const unsigned nblk = (unsigned)((s.elem_count + Ls::EPB - 1) / Ls::EPB);

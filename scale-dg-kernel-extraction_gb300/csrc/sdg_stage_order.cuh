@@ -27,11 +27,11 @@ int launch_stage_order(int prec, int opt, const StageArgs& a, cudaStream_t st) {
 // null only *most, the most elements such a launch takes.
 template <int P>
 int launch_loop_order(int opt, const StageArgs& a, double* const* q, double dt, int nstep,
-                      unsigned* bar, long long* most, cudaStream_t st) {
+                      unsigned* bar, int polls, long long* most, cudaStream_t st) {
   const bool eo = opt == SDG_OPT_EVENODD;
   if (!q) return eo ? fix_loop_most<P, true>(most) : fix_loop_most<P, false>(most);
-  return eo ? launch_stage_fix_loop<P, true>(a, q, dt, nstep, bar, st)
-            : launch_stage_fix_loop<P, false>(a, q, dt, nstep, bar, st);
+  return eo ? launch_stage_fix_loop<P, true>(a, q, dt, nstep, bar, polls, st)
+            : launch_stage_fix_loop<P, false>(a, q, dt, nstep, bar, polls, st);
 }
 
 // The entry points of one order (one translation unit per group of orders, so
@@ -41,8 +41,8 @@ int launch_loop_order(int opt, const StageArgs& a, double* const* q, double dt, 
     return launch_stage_order<p>(prec, opt, a, st);                                         \
   }                                                                                         \
   int launch_loop_p##p(int opt, const StageArgs& a, double* const* q, double dt, int nstep, \
-                       unsigned* bar, long long* most, cudaStream_t st) {                   \
-    return launch_loop_order<p>(opt, a, q, dt, nstep, bar, most, st);                       \
+                       unsigned* bar, int polls, long long* most, cudaStream_t st) {        \
+    return launch_loop_order<p>(opt, a, q, dt, nstep, bar, polls, most, st);                \
   }
 
 }  // namespace sdg

@@ -134,6 +134,7 @@ def _load() -> C.CDLL:
         "sdg_solver_upload_dev": ([_vp, _vp, _vp, _vp, _vp], _i),
         "sdg_solver_step": ([_vp, _d, _i], _i),
         "sdg_solver_step_timed": ([_vp, _d, _i, C.POINTER(_d)], _i),
+        "sdg_solver_set_wait_limit": ([_vp, _i], _i),
         "sdg_solver_download": ([_vp, _vp], _i),
         "sdg_solver_solve_host_pipelined": ([_vp, _i, C.POINTER(_vp), C.POINTER(_vp),
                                              C.POINTER(_vp), C.POINTER(_vp), C.POINTER(_vp), _d,
@@ -531,6 +532,11 @@ class Solver:
 
     def step(self, dt: float, nstep: int) -> None:
         _check(lib.sdg_solver_step(self._h, float(dt), int(nstep)), "sdg_solver_step")
+
+    def set_wait_limit(self, polls: int) -> None:
+        """How often a wait between the stages of a one-launch step looks before it
+        gives up (negative: the default)."""
+        _check(lib.sdg_solver_set_wait_limit(self._h, int(polls)), "sdg_solver_set_wait_limit")
 
     def step_timed(self, dt: float, nstep: int) -> float:
         """Steps and returns the device time in milliseconds (CUDA events)."""
