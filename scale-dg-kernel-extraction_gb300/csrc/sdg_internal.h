@@ -142,6 +142,9 @@ int launch_stage(int p, int prec, int opt, const StageArgs& a, cudaStream_t st);
 // state buffers, the current one first; bar two device words, zero (the second
 // set by a wait between the stages that gave up after `polls` reads);
 // the result is in q[nstep % 3].  With q null: *most = the most elements.
+// kLoopTooLarge, with nothing launched, where the stream has fewer SMs than the
+// device (a green context's) and they do not hold the grid.
+constexpr int kLoopTooLarge = 1;
 int launch_loop(int p, int opt, const StageArgs& a, double* const* q, double dt, int nstep,
                 unsigned* bar, int polls, long long* most, cudaStream_t st);
 

@@ -436,19 +436,22 @@ int sdg_solver_step(sdg_solver* s, double dt, int nstep) {
   if (nstep < 0) return fail(SDG_ERR_INVALID_ARG, "nstep < 0");
   bool loop = false;
   if (nstep > 0) SDG_TRY(takes_loop(s, &loop));
-  if (loop) {
-    for (int left = nstep; left > 0;) {
-      const int n = std::min(left, kLoopSteps);
-      double* q[3] = {s->q[s->cur], s->q[(s->cur + 1) % 3], s->q[(s->cur + 2) % 3]};
-      const StageArgs a = stage_args(s, 0, dt, q[0], nullptr, q[1], s->u, s->v, s->w, false, 0);
-      SDG_TRY(launch_loop(s->p, s->opt, a, q, dt, n, s->bar, s->loop_polls, nullptr, s->stream));
-      s->loop_ran = true;
-      s->cur = (s->cur + n) % 3;
-      left -= n;
+  int left = nstep;
+  while (loop && left > 0) {
+    const int n = std::min(left, kLoopSteps);
+    double* q[3] = {s->q[s->cur], s->q[(s->cur + 1) % 3], s->q[(s->cur + 2) % 3]};
+    const StageArgs a = stage_args(s, 0, dt, q[0], nullptr, q[1], s->u, s->v, s->w, false, 0);
+    const int rc = launch_loop(s->p, s->opt, a, q, dt, n, s->bar, s->loop_polls, nullptr, s->stream);
+    if (rc == kLoopTooLarge) {  // from now on a launch a stage
+      s->loop_most = 0;
+      break;
     }
-    return SDG_OK;
+    SDG_TRY(rc);
+    s->loop_ran = true;
+    s->cur = (s->cur + n) % 3;
+    left -= n;
   }
-  for (int it = 0; it < nstep; it++) {
+  for (int it = 0; it < left; it++) {
     const int s0 = s->cur, s1 = (s->cur + 1) % 3, s2 = (s->cur + 2) % 3;
     // the velocity cannot change within one call: the first stage of the
     // call forms the face-flux velocity factors and every later stage of the

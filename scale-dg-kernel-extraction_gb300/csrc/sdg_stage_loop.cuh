@@ -228,7 +228,13 @@ int launch_stage_fix_loop(const StageArgs& s, double* const* q, double dt, int n
   SDG_TRY(set_kernel_smem(kernel, (int)Ls::SMEM, carve_for(Ls::SMEM, Ls::BLOCKS)));
   const unsigned nblk = (unsigned)((s.elem_count + Ls::EPB - 1) / Ls::EPB);
   void* args[1] = {&a};
-  SDG_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(nblk), dim3(Ls::THREADS), args, Ls::SMEM, st));
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel(kernel, dim3(nblk), dim3(Ls::THREADS), args, Ls::SMEM, st);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return kLoopTooLarge;
+  }
+  SDG_CUDA_TRY(e);
   return SDG_OK;
 }
 

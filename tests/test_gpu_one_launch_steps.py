@@ -102,3 +102,51 @@ def test_two_boxes_on_two_streams_at_once(opt):
             s.step(c.dt, 3)
     for s, want in zip(both_, alone):
         assert np.array_equal(s.download(), want)
+
+
+class _GreenStream:
+    """A stream confined to some of the device's SMs (a green context)."""
+
+    def __init__(self, sms):
+        import ctypes as C
+
+        import sdg
+        sdg.DeviceArray(n=1)  # the primary context
+        self.cu = C.CDLL("libcuda.so.1")
+        dev, n = C.c_int(), C.c_uint(1)
+        resource = lambda: C.create_string_buffer(256)
+        whole, part, rest = resource(), resource(), resource()
+        desc, self.ctx, self.stream = C.c_void_p(), C.c_void_p(), C.c_void_p()
+        self._ok(self.cu.cuDeviceGet(C.byref(dev), 0))
+        self._ok(self.cu.cuDeviceGetDevResource(dev, whole, 1))
+        self._ok(self.cu.cuDevSmResourceSplitByCount(part, C.byref(n), whole, rest, 0, sms))
+        self._ok(self.cu.cuDevResourceGenerateDesc(C.byref(desc), part, 1))
+        self._ok(self.cu.cuGreenCtxCreate(C.byref(self.ctx), desc, dev, 1))
+        self._ok(self.cu.cuGreenCtxStreamCreate(C.byref(self.stream), self.ctx, 1, 0))
+
+    @staticmethod
+    def _ok(status):
+        if status != 0:
+            pytest.skip("no green context here: CUresult %d" % status)
+
+    def close(self):
+        self.cu.cuStreamSynchronize(self.stream)
+        self.cu.cuStreamDestroy_v2(self.stream)
+        self.cu.cuGreenCtxDestroy(self.ctx)
+
+
+@both
+def test_a_stream_of_few_sms_takes_a_launch_a_stage(opt):
+    """A box whose one-launch grid the device holds and the stream's SMs do not:
+    the step call succeeds with the same bits."""
+    c = Case(13, 12, 13, 3)
+    s = _solver(c, opt)
+    green = _GreenStream(16)
+    g = _solver(c, opt, stream=green.stream.value)
+    for x in (s, g):
+        x.upload(*_fields(c))
+        x.step(c.dt, 3)
+        x.step(c.dt, 2)
+    assert np.array_equal(s.download(), g.download())
+    g.close()
+    green.close()
