@@ -201,7 +201,8 @@ int sdg_mesh_setup_dev(int NeX, int NeY, int NeZ, int p, double Lx, double Ly,
 /* tensorprod_divlike_dirXYZ (mod_dg_optr_kernel.f90:62-136) over nelem
  * consecutive elements (nelem = 1 is the reference call made per element from
  * mod_advect3d_eq.f90:185-188).  Each array holds nelem blocks of Nq^3
- * values.  Host pointers; uses the type set by sdg_dg_optr_kernel_setup. */
+ * values.  An output of the device form may be any of its inputs, at the same
+ * offset.  Host pointers; uses the type set by sdg_dg_optr_kernel_setup. */
 int sdg_tensorprod_divlike_dirXYZ(double* vec_out_x, double* vec_out_y,
                                   double* vec_out_z, const double* Mat,
                                   const double* Mat_tr, const double* vec_in_x,

@@ -66,6 +66,24 @@ static int check_tend_shape(int Nq, int Np, int NfpTot, int Ne, int NeA) {
   return SDG_OK;
 }
 
+// Whether n doubles at a and m at b share memory.
+static bool overlap(const double* a, long long n, const double* b, long long m) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + 8 * (uintptr_t)m && y < x + 8 * (uintptr_t)n;
+}
+
+// divlike on the caller's device arrays; notes an output that shares memory
+// with an input other than its own direction's.
+static int divlike(DivArgs a, int p, int opt, cudaStream_t st) {
+  const long long n = (long long)(p + 1) * (p + 1) * (p + 1) * a.nelem;
+  const double* out[3] = {a.ox, a.oy, a.oz};
+  const double* in[3] = {a.ix, a.iy, a.iz};
+  for (int o = 0; o < 3; o++)
+    for (int i = 0; i < 3; i++)
+      if (overlap(out[o], n, in[i], n) && !(o == i && out[o] == in[i])) a.staged = true;
+  return dropin(p, 1, opt, &a, st);
+}
+
 // One device allocation carved into aligned pieces; freed on scope exit.
 class Arena {
  public:
@@ -395,8 +413,8 @@ int sdg_tensorprod_divlike_dirXYZ_dev(double* ox, double* oy, double* oz,
   if (nelem == 0) return SDG_OK;
   if (!ox || !oy || !oz || !Mat || !Mat_tr || !ix || !iy || !iz)
     return fail(SDG_ERR_INVALID_ARG, "NULL device pointer");
-  DivArgs a{ox, oy, oz, Mat, Mat_tr, ix, iy, iz, nelem};
-  return dropin(Nq - 1, 1, opt, &a, as_stream(stream));
+  return divlike(DivArgs{ox, oy, oz, Mat, Mat_tr, ix, iy, iz, nelem}, Nq - 1, opt,
+                 as_stream(stream));
 }
 
 int sdg_tensorprod_divlike_dirXYZ(double* ox, double* oy, double* oz,
@@ -457,8 +475,8 @@ int sdg_tensorprod_divlike_dirXYZ_var5_dev(double* ox, double* oy, double* oz,
   if (nelem == 0) return SDG_OK;
   if (!ox || !oy || !oz || !Mat || !Mat_tr || !ix || !iy || !iz)
     return fail(SDG_ERR_INVALID_ARG, "NULL device pointer");
-  DivArgs a{ox, oy, oz, Mat, Mat_tr, ix, iy, iz, 5 * nelem};
-  return dropin(Nq - 1, 1, SDG_OPT_OPT1, &a, as_stream(stream));
+  return divlike(DivArgs{ox, oy, oz, Mat, Mat_tr, ix, iy, iz, 5 * nelem}, Nq - 1, SDG_OPT_OPT1,
+                 as_stream(stream));
 }
 
 namespace {

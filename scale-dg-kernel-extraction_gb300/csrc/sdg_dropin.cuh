@@ -340,14 +340,12 @@ int dropin_order(int what, int opt, const void* args, cudaStream_t st) {
       return split ? launch_dqdt_impl<P, kCanSplit>(a, st) : launch_dqdt_impl<P, false>(a, st);
     }
     case 1: {
+      // ops_kernel writes y and z lines while other lines of the element's inputs
+      // are still read; divlike_kernel reads all three inputs of an element first
       const DivArgs& a = *static_cast<const DivArgs*>(args);
-      if constexpr (ops_always<P>()) {
-        return launch_ops<P, false>(a, st);
-      } else {
-        if (P > 1 && ops_fixed<P>(a.nelem)) return launch_ops<P, false>(a, st);
-        return split ? launch_divlike_impl<P, kCanSplit>(a, st)
-                     : launch_divlike_impl<P, false>(a, st);
-      }
+      if (P > 1 && ops_fixed<P>(a.nelem) && !a.staged) return launch_ops<P, false>(a, st);
+      return split ? launch_divlike_impl<P, kCanSplit>(a, st)
+                   : launch_divlike_impl<P, false>(a, st);
     }
     case 3:
       if constexpr (ops_always<P>()) {

@@ -29,6 +29,7 @@ struct DivArgs {
   const double* iy;
   const double* iz;
   int nelem;
+  bool staged = false;  // divlike: an output is another direction's input
 };
 
 // The exponent of a row whose magnitudes add up to sum (with room for the
@@ -101,7 +102,8 @@ __host__ __device__ constexpr size_t ops_smem() {
 // else one of each of three.  Blocks walk the elements with a grid stride, so
 // the matrices become limbs once a block; thread r of an element owns line r of
 // each direction.  y and z lines are read and written in place, coalesced along
-// i; x lines go through shared memory.
+// i; x lines go through shared memory.  An output may be its own direction's
+// input, and any of gradlike's, which stages its field, may be the field.
 template <int P, bool GRAD>
 __global__ void __launch_bounds__(FixShape<P>::THREADS, 1024 / FixShape<P>::THREADS)
     ops_kernel(const DivArgs a) {
