@@ -133,7 +133,8 @@ int sdg_advect3d_eq_cal_tend(double* dqdt, const double* q, const double* u,
                              int Nq, int Np, int NfpTot, int Ne, int NeA);
 
 /* The same on device pointers, asynchronous on `stream`, with the
- * optimisation type explicit.  `flux_scratch` is caller-owned device memory
+ * optimisation type explicit.  dqdt may be one of the fields, in place.
+ * `flux_scratch` is caller-owned device memory
  * of NfpTot*Ne doubles for the element-boundary flux (the reference's
  * automatic array ebnd_flux, mod_advect3d_eq.f90:66); `err_flag` is a
  * caller-owned device int that the kernels set to 1 when a VMap index is out

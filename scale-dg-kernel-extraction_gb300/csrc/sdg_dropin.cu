@@ -148,7 +148,13 @@ int tend_dev(const TendArgs& a, int p, int NfpTot, int opt, cudaStream_t st) {
   SDG_TRY(dropin(p, 6, opt, need, st));
   const uintptr_t at = (reinterpret_cast<uintptr_t>(a.flux) + 15) & ~uintptr_t(15);
   const uintptr_t end = reinterpret_cast<uintptr_t>(a.flux + NT);
-  const long long dof = (long long)(p + 1) * (p + 1) * (p + 1) * a.Ne;
+  const long long np = (long long)(p + 1) * (p + 1) * (p + 1), dof = np * a.Ne;
+  // dqdt over an array that the kernel still reads elsewhere: the flux kernel
+  // gathers first, and cal_dqdt reads an element's fields before it writes any
+  const bool over = overlap(a.dqdt, dof, a.q, a.NpNeA) || overlap(a.dqdt, dof, a.u, a.NpNeA) ||
+                    overlap(a.dqdt, dof, a.v, a.NpNeA) || overlap(a.dqdt, dof, a.w, a.NpNeA) ||
+                    overlap(a.dqdt, dof, a.Escale, 3 * dof) ||
+                    overlap(a.dqdt, dof, a.normal_fn, 3 * NT) || overlap(a.dqdt, dof, a.Fscale, NT);
   if (at + need[0] <= end && (opt == SDG_OPT_EVENODD || dof >= 160000 || p >= 12)) {
     RefArgs r{};
     r.q_in = a.q;
@@ -168,8 +174,9 @@ int tend_dev(const TendArgs& a, int p, int NfpTot, int opt, cudaStream_t st) {
     r.Escale = a.Escale;
     r.Ne = a.Ne;
     RefCall c{&r, kRkTend, reinterpret_cast<void*>(at), (size_t)(end - at)};
-    SDG_TRY(dropin(p, 5, opt, &c, st));
-    return dropin(p, 4, opt, &c, st);
+    // (of an EVENODD call the tables' symmetry check counts either way)
+    if (!over || opt == SDG_OPT_EVENODD) SDG_TRY(dropin(p, 5, opt, &c, st));
+    if (!over) return dropin(p, 4, opt, &c, st);
   }
   long long nb = (NT + 255) / 256;
   if (nb > 152LL * 64) nb = 152LL * 64;

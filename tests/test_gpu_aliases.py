@@ -61,3 +61,36 @@ def test_gradlike_and_a_direction_over_the_field(p, nelem, over):
     M = m if over == 0 else mt
     assert sdg.lib.sdg_element_matvec_dir_dev(over + 1, x.ptr, M.ptr, x.ptr, N, nelem, None) == 0
     assert rel_l2(x.numpy(), want[over]) <= TOL_TEND
+
+
+@pytest.mark.parametrize("opt", ["OPT_EVENODD", "OPT_OPT1"])
+@pytest.mark.parametrize("p,dims", [(3, (4, 5, 3)), (3, (15, 14, 13)), (7, (8, 7, 8)),
+                                    (13, (3, 5, 4))])
+@pytest.mark.parametrize("over", ["q", "u", "v", "w", "Escale"])
+def test_tendency_over_one_of_its_fields(opt, p, dims, over):
+    """dqdt in place of a field (or of Escale's x part), on both sides of the
+    small-mesh rule; an EVENODD call still reports operators without the
+    symmetries."""
+    import sdg
+    c = Case(*dims, p)
+    m = c.mesh
+    want = c.oracle_tend(O.OPT1)
+    A = sdg.DeviceArray
+    f = {"q": A(c.q), "u": A(c.u), "v": A(c.v), "w": A(c.w), "Escale": A(m.Escale)}
+    D, Dt, L, M, P, n, S = [A(a) for a in (c.D, c.Dt, c.Lift, m.VMapM, m.VMapP, m.normal_fn,
+                                           m.Fscale)]
+    flux, err = A(n=m.NfpTot * m.Ne), A(np.zeros(1, dtype=np.int32))
+
+    def call(D):
+        return sdg.lib.sdg_advect3d_eq_cal_tend_dev(
+            f[over].ptr, f["q"].ptr, f["u"].ptr, f["v"].ptr, f["w"].ptr, D.ptr, Dt.ptr, L.ptr,
+            M.ptr, P.ptr, n.ptr, f["Escale"].ptr, S.ptr, m.Nq, m.Np, m.NfpTot, m.Ne, m.NeA,
+            getattr(sdg, opt), flux.ptr, err.ptr, None)
+
+    assert call(D) == 0
+    assert rel_l2(f[over].numpy()[: c.nown], want) <= TOL_TEND
+    assert err.numpy()[0] == 0
+    bad = c.D.copy()
+    bad[1] *= 1.5
+    assert call(A(bad)) == 0
+    assert err.numpy()[0] == (2 if opt == "OPT_EVENODD" else 0)
