@@ -319,7 +319,10 @@ int sdg_rk_stage_dev(double* q, const double* q0, const double* dqdt, int Np,
  * operator tables, the last 48 Nq^3 bytes and some, is taken too: OPT1 / GENERAL
  * then run the per-stage sequence, 10 launches a step and more.)  Errors found on the device set *err_flag
  * (not cleared here): 1 for a VMapM / VMapP / halo_src_map entry outside the
- * DOFs it may name, 2 for operators without the even-odd symmetries.  On
+ * DOFs it may name, 2 for operators without the even-odd symmetries.  (Slots
+ * beyond the NhaloNode that halo_src_map fills are the caller's: OPT1 and
+ * GENERAL read their values, a boundary condition say, through the whole call;
+ * EVENODD sets 1.)  On
  * return the halo slots of q hold the final state's halo values.  Runs
  * asynchronously on `stream`. */
 size_t sdg_advect3d_eq_step_scratch_bytes(int Nq, int Ne);

@@ -237,7 +237,8 @@ __global__ void __launch_bounds__(256)
 
 // Once per call, one thread per face node m: the owned nodes its qM and qP
 // come from (VMapM(m), VMapP(m), a halo slot b followed through
-// halo_src_map(b)) and the velocity factors of its flux qP tP - qM tM from the
+// halo_src_map(b), or as given where the operators are and the map leaves the
+// slot to the caller) and the velocity factors of its flux qP tP - qM tM from the
 // caller's velocity at VMapM / VMapP, normal_fn and Fscale: (tP, tM), or with
 // `jump` (tP - tM, tM).  An entry out of
 // range sets *err = 1 and gives the face node a zero flux.
@@ -257,8 +258,13 @@ __global__ void step_face_kernel(const int* __restrict__ VMapM, const int* __res
     for (int side = 0; side < 2; side++)
       if (r[side] >= NpNe && r[side] < NpNeA && r[side] - NpNe < NhaloNode)
         r[side] = (long long)halo_src_map[r[side] - NpNe] - 1;
-    const bool ok = vM >= 0 && vM < NpNeA && vP >= 0 && vP < NpNeA && r[0] >= 0 &&
-                    r[0] < NpNe && r[1] >= 0 && r[1] < NpNe;
+    // beyond the map's slots: a value the caller keeps (a boundary condition),
+    // which the reference's loop reads as it is; the even-odd type refuses it
+    auto named = [&](long long v, long long n) {
+      return v >= 0 && v < NpNeA && n >= 0 &&
+             (n < NpNe || (jump && n == v && v >= NpNe + NhaloNode));
+    };
+    const bool ok = named(vM, r[0]) && named(vP, r[1]);
     if (!ok) {
       atomicExch(err, 1);
       res[m] = make_int2(-1, -1);
@@ -748,6 +754,7 @@ int sdg_advect3d_eq_step_dev(double* q, const double* u, const double* v, const 
   a.Lift = Lift_mat;
   a.err = err_flag;
   a.res = res;
+  a.q_halo = q;
   a.fc = fc;
   a.Escale = Escale;
   a.Ne = Ne;

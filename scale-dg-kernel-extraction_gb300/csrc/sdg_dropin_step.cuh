@@ -60,9 +60,12 @@ struct RefArgs {
   const double* Fscale;
   int* err;             // set to 1 on an out-of-range VMap entry
   long long NpNeA;      // valid 1-based indices are 1..NpNeA
-  // faces of the time loop: the 0-based owned nodes qM and qP come from (-1: a
-  // map entry was out of range), and the velocity factors
+  // faces of the time loop: the 0-based nodes qM and qP come from (-1: a map
+  // entry was out of range), and the velocity factors.  Operators as given may
+  // name halo slots beyond halo_src_map's, whose values q_halo (the caller's q)
+  // holds through the call
   const int2* res;
+  const double* q_halo;
   const double2* fc;
   const double* Escale;
   // coefficients for the Escale of the mesh's first node (null: not built), and
@@ -504,7 +507,8 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
         const double2 fc = a.fc[m];
         g[f] = 0.0;
         if (at[f].x >= 0) {
-          const double qP = q[at[f].y], qM = q[at[f].x];
+          auto from = [&](int n) { return EO || n < (int)NpNe ? q : a.q_halo; };
+          const double qP = from(at[f].y)[at[f].y], qM = from(at[f].x)[at[f].x];
           g[f] = EO ? fma(qP, fc.x, -(qM * fc.y)) : fma(qP, fc.x, (qP - qM) * fc.y);
         }
       }
