@@ -355,10 +355,12 @@ typedef struct sdg_solver sdg_solver;
  * SDG_OPT_EVENODD the even-odd stage (returns SDG_ERR_INVALID_ARG if
  * D1D or Lift_mat lacks the centro-symmetry beyond 1e-13 relative).
  * precision = SDG_PREC_*.  stream may be NULL.
- * With SDG_PREC_FP64 or SDG_PREC_FP64_EMU the solver also holds the face-flux velocity factors of one call (16 bytes per face node,
- * 96/Nq bytes per DOF): the first stage of every sdg_solver_step forms them
- * from the current velocity and the others read them.  (With GENERAL and OPT1
- * a solver whose device memory does not hold them forms them in every stage.) */
+ * With SDG_PREC_FP64 or SDG_PREC_FP64_EMU the solver also holds the face-flux
+ * velocity factors of one call (16 bytes per face node, 96/Nq bytes per DOF):
+ * the first stage of every sdg_solver_step forms them from the current velocity
+ * and the others read them.  (With GENERAL and OPT1 only where they are at most
+ * an eighth of the device memory that is left; else every stage forms them, to
+ * the same bits.) */
 int sdg_solver_create(sdg_solver** out, int NeX, int NeY, int NeZ, int p,
                       double Lx, double Ly, double Lz, const double* D1D,
                       const double* Lift_mat, int opt, int precision,

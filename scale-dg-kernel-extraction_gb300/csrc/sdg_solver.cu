@@ -287,9 +287,13 @@ int solver_create_box(sdg_solver** out, const Box& box, int p, const double* D1D
   if (e == cudaSuccess && !fix_lift.empty()) e = cudaMalloc(&s->fix_lift, 4 * fix_lift.size());
   if (e == cudaSuccess && !fix_lift.empty())
     e = cudaMemcpy(s->fix_lift, fix_lift.data(), 4 * fix_lift.size(), cudaMemcpyHostToDevice);
-  // GENERAL and OPT1 share the velocity factors too, but a box whose
-  // other buffers fill the memory runs without them
-  if (e == cudaSuccess && !fix_lift.empty() && cudaMalloc(&s->fc, fc_bytes) != cudaSuccess) {
+  // GENERAL and OPT1 share the velocity factors too, where they are an eighth of
+  // what is left at most: the caller's next allocations (and this solver's
+  // tendency, of 4/3 their size at most) have to find room as they would without
+  size_t room = 0, whole = 0;
+  if (e == cudaSuccess && !fix_lift.empty() &&
+      (cudaMemGetInfo(&room, &whole) != cudaSuccess || fc_bytes > room / 8 ||
+       cudaMalloc(&s->fc, fc_bytes) != cudaSuccess)) {
     cudaGetLastError();
     s->fc = nullptr;
   }
