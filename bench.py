@@ -381,8 +381,8 @@ def bench_ensemble(sdg, args):
                        [m["dt"] for m in members], ops)
     if args.batch_opt != "auto":
         ens.set_opt(OPTS[args.batch_opt])
-    if args.parallel_groups:
-        ens.set_parallel_groups(True)
+    if args.serial_groups:
+        ens.set_parallel_groups(False)
     for i, m in enumerate(members):
         ens.init_blob(i, m["centre"], m["sigma"], m["vel"])
     sdg.synchronize()
@@ -816,7 +816,7 @@ def bench_serving(sdg, args, rate=None, plain_cache=None):
         arrivals.append(t)
     srv = sdg.Server(ops, hbm_budget_bytes=int(args.serve_budget_gb * (1 << 30)),
                      opt=0 if args.batch_opt == "auto" else OPTS[args.batch_opt],
-                     parallel_groups=args.parallel_groups)
+                     parallel_groups=False if args.serial_groups else None)
     # warm the batched kernel and the pool
     srv.wait(srv.submit(**reqs[0]))
     srv.reset_stats()
@@ -1143,9 +1143,11 @@ def main() -> int:
     ap.add_argument("--serve-n", type=int, default=60)
     ap.add_argument("--serve-rate", type=float, default=20.0)
     ap.add_argument("--serve-rate-saturated", type=float, default=200.0)
-    ap.add_argument("--parallel-groups", action="store_true",
-                    help="run the batched forms' order groups on parallel streams (the default "
-                         "of the library)")
+    ap.add_argument("--serial-groups", action="store_true",
+                    help="run the batched forms' order groups one after the other instead of on "
+                         "parallel streams (the library's default)")
+    ap.add_argument("--parallel-groups", dest="serial_groups", action="store_false",
+                    help="run them on parallel streams")
     ap.add_argument("--serve-sweep", default="10,50,100,500,2000",
                     help="offered rates (req/s) of the serving sweep, comma separated")
     ap.add_argument("--serve-max-ne", type=int, default=32)

@@ -555,8 +555,9 @@ typedef struct {
   int threads_by_order[16]; /* block size by order (0: `threads`, else the
                                default of the order) */
   int parallel_groups;      /* 1: the order groups of a step run on parallel
-                               streams; 0: the library's choice, which is the
-                               same (same results either way) */
+                               streams; -1: one after the other on one; 0: the
+                               library's choice (parallel, which measured
+                               faster).  Same results either way */
 } sdg_server_config;
 typedef struct {
   int NeX, NeY, NeZ, p, nstep;

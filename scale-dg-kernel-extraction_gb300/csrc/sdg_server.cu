@@ -353,6 +353,7 @@ int sdg_server_create(sdg_server** out, const sdg_server_config* cfg,
   sdg_server* s = new (std::nothrow) sdg_server();
   if (!s) return fail(SDG_ERR_OUT_OF_MEMORY, "host allocation failed");
   s->cfg = *cfg;
+  s->fj.parallel = cfg->parallel_groups >= 0;  // parallel is the library's choice
   for (int p = 0; p <= kBatchMaxOrder; p++) {
     batch_default_shape(p, &s->threads[p], &s->epb[p]);
     if (cfg->threads > 0) s->threads[p] = cfg->threads;

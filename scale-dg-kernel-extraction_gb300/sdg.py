@@ -738,9 +738,11 @@ class Server:
 
     def __init__(self, ops_by_order, hbm_budget_bytes=64 << 30, max_active=512,
                  max_window_steps=8, threads=0, device=0, opt=0, threads_by_order=None,
-                 epb_by_order=None, parallel_groups=False):
+                 epb_by_order=None, parallel_groups=None):
         """threads_by_order / epb_by_order: {p: value} overrides of the
-        batched kernels' launch shape (results do not depend on it)."""
+        batched kernels' launch shape; parallel_groups: order groups on parallel
+        streams (True), on one (False), or the library's choice (None).  Results
+        do not depend on either."""
         self._arrs, D, L, X = _order_table(ops_by_order)
         cfg = ServerConfig()
         cfg.device = device
@@ -749,7 +751,7 @@ class Server:
         cfg.max_active = max_active
         cfg.max_window_steps = max_window_steps
         cfg.threads = threads
-        cfg.parallel_groups = 1 if parallel_groups else 0
+        cfg.parallel_groups = 0 if parallel_groups is None else 1 if parallel_groups else -1
         for p, t in (threads_by_order or {}).items():
             cfg.threads_by_order[p] = t
         for p, e in (epb_by_order or {}).items():
