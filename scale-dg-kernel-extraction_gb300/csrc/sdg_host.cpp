@@ -4,8 +4,6 @@
 
 #include <atomic>
 #include <cctype>
-#include <unistd.h>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -17,6 +15,7 @@
 
 #include "sdg_fix.cuh"
 #include "sdg_internal.h"
+#include "sdg_pages.h"
 
 namespace sdg {
 
@@ -76,10 +75,7 @@ void touch_pages(void* p, size_t bytes) {
     return;
   }
   if (a.type != cudaMemoryTypeUnregistered) return;
-  static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-  volatile char* b = static_cast<volatile char*>(p);
-  for (size_t at = 0; at < bytes; at += page) b[at] = b[at];
-  b[bytes - 1] = b[bytes - 1];
+  map_pages(p, bytes);
 }
 
 int require_device() {
