@@ -390,8 +390,8 @@ __device__ __forceinline__ int ref_line_shared(const RefArgs& a, const fixlimb* 
   if (ok && fix_in_range(E)) {
     int64_t* out = reinterpret_cast<int64_t*>(line);
     const int32_t Ef = E + (xe << 20);
-    fix_line<P, EO>(T, EO ? nullptr : a.lift + AX * N * N * N + r, F, E, fix_align(gm, Ef),
-                    fix_align(gp, Ef), [&](int m, int64_t v) { out[m * S] = v; });
+    fix_line<P, EO>(T, EO ? nullptr : a.lift + AX * N * N * N + r, F, E, fix_align_signed(gm, Ef),
+                    fix_align_signed(gp, Ef), [&](int m, int64_t v) { out[m * S] = v; });
     return fix_line_exp(E) + xe;
   }
   double out[N];
@@ -486,8 +486,8 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
 #pragma unroll
     for (int m = 0; m < N; m++) {
       const double qv = q[ge + r + m * N2];
-      sX[zat + m * NS * N] = qv * a.u[ge + r + m * N2];
-      sY[zat + m * NS * N] = qv * a.v[ge + r + m * N2];
+      sX[zat + m * NS * N] = fix_product(qv, a.u[ge + r + m * N2]);
+      sY[zat + m * NS * N] = fix_product(qv, a.v[ge + r + m * N2]);
     }
     if (same) {
       for (int t = r; t < 3 * TAB; t += N2) sT[t] = a.shared[t];
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
     E = max(0, ref_face_exp(g[4], g[5], xe[2]));
 #pragma unroll
     for (int m = 0; m < N; m++) {
-      F[m] = q[ge + r + m * N2] * a.w[ge + r + m * N2];
+      F[m] = fix_product(q[ge + r + m * N2], a.w[ge + r + m * N2]);
       E = max(E, fix_value_exp(F[m]));
     }
   }
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
     if (zok) {
       const int32_t Ef = E + (xe[2] << 20);
       fix_line<P, EO>(sT + 2 * TAB, EO ? nullptr : a.lift + 2 * NP + r, F, E,
-                      fix_align(g[4], Ef), fix_align(g[5], Ef), emit);
+                      fix_align_signed(g[4], Ef), fix_align_signed(g[5], Ef), emit);
     } else {
       double in[N], out[N];  // in: F itself stays in registers
 #pragma unroll

@@ -151,7 +151,17 @@ SDG_HD bool fix_in_range(int32_t E) {
 SDG_HD int fix_line_exp(int32_t E) { return (E >> 20) - 1022; }
 
 // A value F 2^(59 - B), off by at most one unit (the magnitude truncated, a
-// negative one then complemented); a face g / 4 2^(59 - B).
+// negative one then complemented, which is two instructions less than its
+// negative: 2 % of a stage).  +0 gives zero, -0 minus one: products are formed by
+// fix_product.  A face g / 4 2^(59 - B), its magnitude truncated: either zero gives
+// zero.
+SDG_HD double fix_product(double q, double u) {
+#if defined(__CUDA_ARCH__)
+  return __fma_rn(q, u, 0.0);  // -0 + 0 = +0
+#else
+  return q * u + 0.0;
+#endif
+}
 SDG_HD int64_t fix_align(double x, int32_t E) {
   uint32_t hi, lo;
   d2words(x, hi, lo);
@@ -159,14 +169,17 @@ SDG_HD int64_t fix_align(double x, int32_t E) {
   const uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32 | lo) << 6;
   return (int64_t)fix_shr(m, s) ^ (int64_t)((int32_t)hi >> 31);
 }
+SDG_HD int64_t fix_align_signed(double x, int32_t E) {
+  return fix_align(x, E) - ((int32_t)fix_high(x) >> 31);
+}
 SDG_HD int64_t fix_align_face(double g, int32_t E) {
-  return fix_align(g, E + (2 << 20));
+  return fix_align_signed(g, E + (2 << 20));
 }
 
 // x 2^E, |x| < 2^63, to one unit of x and half an ulp of the result, for
-// results in the normal range; no FP64 operation and no conversion
-// instruction, which run on the FP64 pipe, and no branch.  A negative x is
-// complemented (a unit less); zero becomes half a unit.
+// results in the normal range, and zero for zero; no FP64 operation and no
+// conversion instruction, which run on the FP64 pipe, and no branch.  A negative
+// x is complemented (a unit less).
 SDG_HD double fix_to_double(int64_t x, int E) {
   const uint32_t xh = (uint32_t)(x >> 32), neg = (uint32_t)((int32_t)xh >> 31);
   uint32_t ah = xh ^ neg, al = (uint32_t)x ^ neg;
@@ -187,7 +200,7 @@ SDG_HD double fix_to_double(int64_t x, int E) {
   // the exponent field
   const uint64_t m = ((uint64_t)mh << 32 | (al << sh)) + 0x200u;
   const uint32_t hi = (uint32_t)(m >> 42) + ((uint32_t)(1023 + 61 + E - sh) << 20);
-  return words2d(hi | (xh & 0x80000000u), (uint32_t)(m >> 10));
+  return words2d(x == 0 ? 0u : hi | (xh & 0x80000000u), (uint32_t)(m >> 10));
 }
 
 }  // namespace sdg

@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
 #pragma unroll
     for (int m = 0; m < N; m++) {
       const double qv = q[ge + r + m * N2];
-      sX[zat + m * NS * N] = qv * u[ge + r + m * N2];
-      sY[zat + m * NS * N] = qv * v[ge + r + m * N2];
+      sX[zat + m * NS * N] = fix_product(qv, u[ge + r + m * N2]);
+      sY[zat + m * NS * N] = fix_product(qv, v[ge + r + m * N2]);
     }
     unsigned nb[6];
     fix_neighbors(a.s.box, (unsigned)(eb + le), nb);
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
     E = max(0, max(fix_face_exp(g[4]), fix_face_exp(g[5])));
 #pragma unroll
     for (int m = 0; m < N; m++) {
-      F[m] = q[ge + r + m * N2] * w[ge + r + m * N2];
+      F[m] = fix_product(q[ge + r + m * N2], w[ge + r + m * N2]);
       E = max(E, fix_value_exp(F[m]));
     }
   }

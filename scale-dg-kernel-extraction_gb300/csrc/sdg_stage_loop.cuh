@@ -95,7 +95,7 @@ __device__ __forceinline__ int fix_loop_line(const FixStageArgs<P, EO>& a, const
     const double v = __ldcg(q + at + l * S);
     if (l == 0) qm = v;
     if (l == N - 1) qp = v;
-    F[l] = v * u[at + l * S];
+    F[l] = fix_product(v, u[at + l * S]);
     E = max(E, fix_value_exp(F[l]));
   }
   auto flux = [](double qP, double qM, double2 c) {
