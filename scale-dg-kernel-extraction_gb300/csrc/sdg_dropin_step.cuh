@@ -474,13 +474,13 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
     for (int d = 0; d < 3; d++) {
       xe[d] = ref_escale_exp(es[d]);
       mix |= xe[d] < -150 || xe[d] > 150;
-      // a row's exponent with Escale's: with a line's, whose results have to lie
-      // in the normal range, at most the 900 of the box solver
-      if (r < ROWS) {
-        const int x = a.row[d * ROWS + r] + xe[d];
-        mix |= x < -200 || x > 200;
-      }
       same = same && __double_as_longlong(es[d]) == __double_as_longlong(Es[d * NpNe]);
+    }
+    // a row's exponent with Escale's: with a line's, whose results have to lie in
+    // the normal range, at most the 900 of the box solver
+    for (int t = r; t < 3 * ROWS; t += N2) {
+      const int x = a.row[t] + (t < ROWS ? xe[0] : t < 2 * ROWS ? xe[1] : xe[2]);
+      mix |= x < -200 || x > 200;
     }
     if (mix) sMix[le] = 1;
 #pragma unroll
