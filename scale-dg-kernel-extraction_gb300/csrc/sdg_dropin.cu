@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(256)
 // Once per call, one thread per face node m: the owned nodes its qM and qP
 // come from (VMapM(m), VMapP(m), a halo slot b followed through
 // halo_src_map(b), or as given where the operators are and the map leaves the
-// slot to the caller) and the velocity factors of its flux qP tP - qM tM from the
+// slot to the caller, which *slots notes) and the velocity factors of its flux qP tP - qM tM from the
 // caller's velocity at VMapM / VMapP, normal_fn and Fscale: (tP, tM), or with
 // `jump` (tP - tM, tM).  An entry out of
 // range sets *err = 1 and gives the face node a zero flux.
@@ -249,7 +249,7 @@ __global__ void step_face_kernel(const int* __restrict__ VMapM, const int* __res
                                  const double* __restrict__ normal_fn,
                                  const double* __restrict__ Fscale, int2* res, double2* fc,
                                  long long NT, long long NpNe, long long NpNeA,
-                                 long long NhaloNode, int jump, int* err) {
+                                 long long NhaloNode, int jump, int* slots, int* err) {
   for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < NT;
        m += (long long)gridDim.x * blockDim.x) {
     const long long vM = (long long)VMapM[m] - 1, vP = (long long)VMapP[m] - 1;
@@ -271,6 +271,7 @@ __global__ void step_face_kernel(const int* __restrict__ VMapM, const int* __res
       fc[m] = make_double2(0.0, 0.0);
       continue;
     }
+    if (r[0] >= NpNe || r[1] >= NpNe) *slots = 1;
     res[m] = make_int2((int)r[0], (int)r[1]);
     const double n1 = normal_fn[m], n2 = normal_fn[m + NT], n3 = normal_fn[m + 2 * NT];
     const double velM = u[vM] * n1 + v[vM] * n2 + w[vM] * n3;
@@ -284,8 +285,9 @@ __global__ void step_face_kernel(const int* __restrict__ VMapM, const int* __res
 // Once per call, one warp per element: whether the element's Escale is one
 // value per direction over all its nodes (compared bit for bit), stored as
 // (Es_x, Es_y, Es_z, 1), else (.., 0).
-__global__ void step_escale_kernel(const double* __restrict__ Es, double4* esu, long long Ne,
-                                   int Np) {
+__global__ void step_escale_kernel(const double* __restrict__ Es, double4* esu, int* slots,
+                                   long long Ne, int Np) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *slots = 0;  // step_face_kernel's
   const long long NpNe = (long long)Np * Ne;
   const int lane = threadIdx.x & 31;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -762,15 +764,19 @@ int sdg_advect3d_eq_step_dev(double* q, const double* u, const double* v, const 
   const bool whole = scratch_bytes >= need;
   RefCall call{&a, 0, base + off[whole ? 5 : 4], whole ? need - off[5] : off[5] - off[4]};
   SDG_TRY(dropin(p, 5, opt, &call, st));
+  int* slots = nullptr;  // behind the elements' Escale, in the room of the tables
   if (whole) {
     double4* esu = reinterpret_cast<double4*>(base + off[4]);
-    step_escale_kernel<<<grid_for(32LL * Ne), 256, 0, st>>>(Escale, esu, Ne, Np);
+    slots = reinterpret_cast<int*>(esu + Ne);
+    a.slots = slots;
+    step_escale_kernel<<<grid_for(32LL * Ne), 256, 0, st>>>(Escale, esu, slots, Ne, Np);
     SDG_CUDA_TRY(cudaGetLastError());
     a.esu = esu;
   }
   step_face_kernel<<<grid_for(nft), 256, 0, st>>>(VMapM, VMapP, halo_src_map, u, v, w,
                                                   normal_fn, Fscale, res, fc, nft, npne,
-                                                  np * NeA, NhaloNode, eo ? 0 : 1, err_flag);
+                                                  np * NeA, NhaloNode, eo ? 0 : 1, slots,
+                                                  err_flag);
   SDG_CUDA_TRY(cudaGetLastError());
   for (int s = 0; s < nstep; s++) {
     // stage 1: q -> B; 2: B, q0 = q -> C; 3: C, q0 = q -> q
