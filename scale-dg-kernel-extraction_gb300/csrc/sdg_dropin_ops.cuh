@@ -72,6 +72,7 @@ __device__ __forceinline__ void ops_line(const fixlimb* T, const int* row, bool 
     F[l] = in[l * S];
     E = max(E, fix_value_exp(F[l]));
   }
+  E = fix_line_scale<N>(F, E, 0.0, 0.0);
   if (!ok || !fix_in_range(E)) {
     ops_line_fp64<P>(M, si, sl, in, S, out, SO);
     return;
@@ -86,9 +87,7 @@ __device__ __forceinline__ void ops_line(const fixlimb* T, const int* row, bool 
     fix_mul(o, T[i * N], f[0]);
 #pragma unroll
     for (int l = 1; l < N; l++) fix_fma(o, T[i * N + l], f[l]);
-    const int64_t v = fix_sum(o);
-    const double r = fix_to_double(v, B + row[i]);
-    out[i * SO] = v == 0 ? 0.0 : r;
+    out[i * SO] = fix_to_double(fix_sum(o), B + row[i]);
   }
 }
 

@@ -396,6 +396,7 @@ __device__ __forceinline__ int ref_line_shared(const RefArgs& a, const fixlimb* 
                     fix_align_signed(gp, Ef), [&](int m, int64_t v) { out[m * S] = v; });
     return fix_line_exp(E) + xe;
   }
+  if (ok && fix_line_scale<N>(F, E, gm, gp) == kFixZeros) return fix_line_exp(kFixZeros);
   double out[N];
   ref_line_fp64<P, EO>(&a, AX, r, line, S, gm, gp, Es, ES, out);
   for (int m = 0; m < N; m++) line[m * S] = out[m];
@@ -547,6 +548,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
       F[m] = fix_product(q[ge + r + m * N2], a.w[ge + r + m * N2]);
       E = max(E, fix_value_exp(F[m]));
     }
+    E = fix_line_scale<N>(F, E, g[4], g[5]);
   }
   __syncthreads();
   if (on) {

@@ -148,7 +148,11 @@ SDG_HD int32_t fix_face_exp(double g) { return (int32_t)(fix_high(g) & kFixExp) 
 SDG_HD bool fix_in_range(int32_t E) {
   return (uint32_t)E - (322u << 20) < (1400u << 20);
 }
-SDG_HD int fix_line_exp(int32_t E) { return (E >> 20) - 1022; }
+// The scale of a line of zeros: the least of the range, marked in a bit that no
+// other has, so that the line's exponent lies below all others and a node's sum
+// is formed on the scale of its other lines.
+constexpr int32_t kFixZeros = 322 << 20 | 1;
+SDG_HD int fix_line_exp(int32_t E) { return (E >> 20) - 1022 - ((E & 1) << 11); }
 
 // A value F 2^(59 - B), off by at most one unit (the magnitude truncated, a
 // negative one then complemented, which is two instructions less than its

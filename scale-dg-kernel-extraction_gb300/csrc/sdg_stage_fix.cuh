@@ -88,22 +88,15 @@ __host__ __device__ constexpr size_t fix_smem(int epb) {
   return sizeof(double) * 2 * epb * FixShape<P>::EW + sizeof(short) * 2 * epb * FixShape<P>::N2;
 }
 
-// A line in FP64, for values the fixed-point path does not take (E: their
-// largest exponent, 0 when there is nothing but zeros and subnormals): F
-// holds the line's fluxes with stride fs, results to out[0..N).  A call of
-// its own, so that its registers do not count against the kernel's.
+// A line in FP64, for values the fixed-point path does not take: F holds the
+// line's fluxes with stride fs, results to out[0..N).  A call of its own, so that
+// its registers do not count against the kernel's.
 template <int P, bool EO>
 __device__ __noinline__ void fix_line_fp64(const StageArgs* a, int ax, int r, const double* F,
                                            int fs, double gm, double gp, double* out) {
   using Sh = EoShape<P>;
   constexpr int N = Sh::N, H = Sh::H, N2 = N * N, NP = N * N2;
   const double sD = -a->box.Es[ax], sL = -(0.25 * a->box.Fs[ax]);
-  bool some = gm != 0.0 || gp != 0.0;
-  for (int l = 0; l < N; l++) {
-    out[l] = 0.0;
-    some = some || F[l * fs] != 0.0;
-  }
-  if (!some) return;
   const double* __restrict__ T = static_cast<const double*>(a->D);
   if constexpr (!EO) {
     const int fm = ax == 0 ? 3 : ax == 1 ? 0 : 4, fp = ax == 0 ? 1 : ax == 1 ? 2 : 5;
@@ -203,6 +196,21 @@ __device__ __forceinline__ void fix_line(const fixlimb* T, const int4* __restric
   }
 }
 
+// The scale of a line whose largest exponent field is E: a line of zeros (a
+// tracer that fills part of the box, a velocity without a component) stays in
+// fixed point; in FP64 its nodes' sums cost more than all others (p = 7 113 us a
+// stage against 72).
+template <int N>
+__device__ __forceinline__ int32_t fix_line_scale(const double* F, int32_t E, double gm,
+                                                  double gp) {
+  if (E > 0) return E;
+  auto bits = [](double x) { return __double2hiint(x) << 1 | __double2loint(x); };
+  int any = bits(gm) | bits(gp);
+#pragma unroll
+  for (int l = 0; l < N; l++) any |= bits(F[l]);
+  return any == 0 ? kFixZeros : 0;
+}
+
 // Exponent of a line formed in FP64: its results are doubles.
 constexpr int kFixDouble = 1 << 14;
 
@@ -225,6 +233,8 @@ __device__ __forceinline__ int fix_line_shared(const FixStageArgs<P, EO>& a, int
                     fix_align_face(gp, E), [&](int m, int64_t v) { out[m * S] = v; });
     return fix_line_exp(E);
   }
+  // zeros (fix_product's are +0) are their own results
+  if (a.ok && fix_line_scale<N>(F, E, gm, gp) == kFixZeros) return fix_line_exp(kFixZeros);
   double out[N];
   fix_line_fp64<P, EO>(&a.s, AX, r, line, S, gm, gp, out);
   for (int m = 0; m < N; m++) line[m * S] = out[m];
@@ -355,6 +365,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
       F[m] = fix_product(q[ge + r + m * N2], w[ge + r + m * N2]);
       E = max(E, fix_value_exp(F[m]));
     }
+    E = fix_line_scale<N>(F, E, g[4], g[5]);
   }
   __syncthreads();
   if (on) {

@@ -103,6 +103,7 @@ __device__ __forceinline__ int fix_loop_line(const FixStageArgs<P, EO>& a, const
   };
   const double gm = flux(qPm, qm, fc[0]), gp = flux(qPp, qp, fc[1]);
   E = max(E, max(fix_face_exp(gm), fix_face_exp(gp)));
+  E = fix_line_scale<N>(F, E, gm, gp);
   if (a.ok && fix_in_range(E)) {
     fix_line<P, EO>(a.tab + AX * a.TAB, a.lift(AX, r), F, E, fix_align_face(gm, E),
                     fix_align_face(gp, E), [&](int m, int64_t v) { out[m * SO] = v; });

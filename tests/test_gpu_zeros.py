@@ -57,3 +57,35 @@ def test_rows_whose_terms_are_zero_give_zero(opt, p, dims):
     assert rel_l2(got, want) <= TOL_TEND
     assert np.count_nonzero(want[e != 0]) > 0
     assert np.all(got[want == 0.0] == 0.0)
+
+
+@both
+@ORDERS
+@pytest.mark.parametrize("exp", [0, -690])
+def test_lines_of_zeros_beside_others(opt, p, dims, exp):
+    """A velocity without one of its components, and a tracer of one element, in a
+    box whose axes' scale factors lie 2^40 apart, with the tracer also near the
+    least magnitude the fixed-point lines take."""
+    import sdg
+    c = Case(*dims, p)
+    L = (1.0, 2.0 ** -40, 1.0)
+    m = O.Mesh(*dims, p, c.x1D, L=L)
+    e = np.arange(c.nown) // m.Np
+    q, u, v, w = [a[: c.nown].copy() for a in (c.q, c.u, c.v, c.w)]
+    q = np.ldexp(q + 0.25, exp)
+    for f in ([q, u, 0.0 * v, w], [q, u, 0.0 * v, 0.0 * w], [q * (e == 1), u, v * 2.0 ** -40, w]):
+        full = []
+        for a in f:
+            x = np.zeros(m.Np * m.NeA)
+            x[: c.nown] = a
+            m.update_halo(x)
+            full.append(x)
+        want = O.cal_tend(m, *full, c.D, c.Dt, c.Lift, O.OPT1)[: c.nown]
+        s = sdg.Solver(*dims, p, c.D, c.Lift, opt=getattr(sdg, opt), L=L)
+        s.upload(*f)
+        assert rel_l2(np.ldexp(s.tendency(), -exp), np.ldexp(want, -exp)) <= TOL_TEND
+        sdg.dg_optr_kernel_setup(opt[4:])
+        got = np.zeros(m.Np * m.NeA)
+        sdg.advect3d_eq_cal_tend(got, *full, c.D, c.Dt, c.Lift, m.VMapM, m.VMapP, m.normal_fn,
+                                 m.Escale, m.Fscale, m.Nq, m.Np, m.NfpTot, m.Ne, m.NeA)
+        assert rel_l2(np.ldexp(got[: c.nown], -exp), np.ldexp(want, -exp)) <= TOL_TEND
