@@ -17,8 +17,9 @@
 //     direction over all its nodes (mesh_setup's affine elements,
 //     mod_mesh.f90:147-149), its significand is folded into the element's copy
 //     of the derivative coefficients and its exponent into the line's (the
-//     faces aligned against it); the lines of other elements are formed in FP64, Escale applied per node
-//     before the lift is added (mod_advect3d_eq.f90:185-198).
+//     faces aligned against it); in other elements a line's derivative and lift
+//     sums become doubles and Escale is applied per node in between
+//     (mod_advect3d_eq.f90:185-198).
 //
 // EO: coefficients of the even-odd pairs, for operators with the symmetries
 // (type EVENODD); else rows of D1D (x) and D1D_tr (y, z) as given and every
@@ -330,6 +331,99 @@ __device__ __noinline__ void ref_line_fp64(const RefArgs* a, int ax, int r, cons
   }
 }
 
+// A line's derivative and lift sums apart, each in fixed point on a scale of its
+// own: im / ip the faces' fluxes as integers, the rest as fix_line; emit(m, d, l).
+template <int P, bool EO, typename Emit>
+__device__ __forceinline__ void ref_line_parts(const fixlimb* T, const int4* __restrict__ lift,
+                                               const double* F, int32_t E, int64_t im, int64_t ip,
+                                               Emit&& emit) {
+  using Sh = EoShape<P>;
+  constexpr int N = Sh::N, H = Sh::H;
+  fixacc l;
+  if constexpr (!EO) {
+    const fixlimb lm = fix_split(im), lp = fix_split(ip);
+    fixlimb f[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) f[k] = fix_split(fix_align(F[k], E));
+#pragma unroll 1
+    for (int i = 0; i < N; i++) {
+      const int4 c = lift[i * N * N];
+      fix_mul(l, fixlimb{c.x, c.y}, lm);
+      fix_fma(l, fixlimb{c.z, c.w}, lp);
+      fixacc d;
+      fix_mul(d, T[i * N], f[0]);
+#pragma unroll
+      for (int k = 1; k < N; k++) fix_fma(d, T[i * N + k], f[k]);
+      emit(i, fix_sum(d), fix_sum(l));
+    }
+    return;
+  }
+  fixlimb s[H], d[H], fm{0, 0};
+#pragma unroll
+  for (int k = 0; k < H; k++) {
+    const int64_t f1 = fix_align(F[k], E), f2 = fix_align(F[N - 1 - k], E);
+    s[k] = fix_split(f1 + f2);
+    d[k] = fix_split(f1 - f2);
+  }
+  if constexpr (Sh::ODD != 0) fm = fix_split(fix_align(F[H], E));
+  const fixlimb gs = fix_split(im + ip), gd = fix_split(im - ip);
+#pragma unroll 1
+  for (int i = 0; i < Sh::HR; i++) {
+    fix_mul(l, T[Sh::OFF_A + i], gs);
+    const int64_t ol = fix_sum(l);
+    fixacc o, e;
+    fix_mul(o, T[Sh::OFF_O + i * H], d[0]);
+#pragma unroll
+    for (int k = 1; k < H; k++) fix_fma(o, T[Sh::OFF_O + i * H + k], d[k]);
+    const int64_t od = fix_sum(o);
+    if (i == H) {
+      emit(i, od, ol);
+      continue;
+    }
+    fix_mul(e, T[Sh::OFF_E + i * H], s[0]);
+#pragma unroll
+    for (int k = 1; k < H; k++) fix_fma(e, T[Sh::OFF_E + i * H + k], s[k]);
+    if constexpr (Sh::ODD != 0) fix_fma(e, T[Sh::OFF_DM + i], fm);
+    const int64_t ed = fix_sum(e);
+    fix_mul(l, T[Sh::OFF_B + i], gd);
+    const int64_t el = fix_sum(l);
+    emit(i, od + ed, ol + el);
+    emit(N - 1 - i, od - ed, ol - el);
+  }
+}
+
+// A line the folded coefficients do not take: F its fluxes (stride fs), Es its
+// nodes' Escale (stride es), out[m] = -(Es(m) (D F)(m) + lift(m)).  With T (an
+// element whose Escale varies: its coefficients without Escale) the sums are
+// formed in fixed point where F and the faces allow.
+template <int P, bool EO>
+__device__ __noinline__ void ref_line_nodes(const RefArgs* a, const fixlimb* T, int ax, int r,
+                                            const double* F, int fs, double gm, double gp,
+                                            const double* __restrict__ Es, int es, double* out) {
+  constexpr int N = P + 1;
+  using Rs = RefShape<P, EO>;
+  double f[N];
+  int32_t E = 0, Eg = max(fix_value_exp(gm), fix_value_exp(gp));
+#pragma unroll
+  for (int l = 0; l < N; l++) {
+    f[l] = F[l * fs];
+    E = max(E, fix_value_exp(f[l]));
+  }
+  E = fix_line_scale<N>(f, E, 0.0, 0.0);
+  if (gm == 0.0 && gp == 0.0) Eg = kFixZeros;
+  if (T == nullptr || !fix_in_range(E) || !fix_in_range(Eg)) {
+    ref_line_fp64<P, EO>(a, ax, r, F, fs, gm, gp, Es, es, out);
+    return;
+  }
+  const int B = fix_line_exp(E) - 61, Bg = fix_line_exp(Eg) - 61;
+  ref_line_parts<P, EO>(T, EO ? nullptr : a->lift + ax * N * N * N + r, f, E,
+                        fix_align_signed(gm, Eg), fix_align_signed(gp, Eg),
+                        [&](int m, int64_t d, int64_t l) {
+                          const int k = a->row[ax * Rs::ROWS + Rs::row_of(m)];
+                          out[m] = fma(Es[m * es], fix_to_double(d, B + k), fix_to_double(l, Bg + k));
+                        });
+}
+
 // u . n with the components whose normal entry is a zero left out: the same
 // value, as long as those components are finite, for two of three FP64
 // operations a side on the axis-aligned normals of mesh_setup.
@@ -376,10 +470,11 @@ __host__ __device__ constexpr size_t ref_smem(int epb) {
 
 // The line of direction AX held in shared memory with stride S, its results
 // over it; returns its exponent.  T: the element's coefficients of the
-// direction, xe: the exponent of its Escale, ok: they are usable.
+// direction, with Escale folded in but for its exponent xe (ok), without it
+// (curved) or not usable (neither).
 template <int P, bool EO, int AX, int S, int ES>
 __device__ __forceinline__ int ref_line_shared(const RefArgs& a, const fixlimb* T, int xe, bool ok,
-                                               int r, double* line, double gm, double gp,
+                                               bool curved, int r, double* line, double gm, double gp,
                                                const double* Es) {
   constexpr int N = P + 1;
   double F[N];
@@ -396,9 +491,11 @@ __device__ __forceinline__ int ref_line_shared(const RefArgs& a, const fixlimb* 
                     fix_align_signed(gp, Ef), [&](int m, int64_t v) { out[m * S] = v; });
     return fix_line_exp(E) + xe;
   }
-  if (ok && fix_line_scale<N>(F, E, gm, gp) == kFixZeros) return fix_line_exp(kFixZeros);
+  // zeros (fix_product's are +0, as doubles too) are their own results
+  if ((ok || curved) && fix_line_scale<N>(F, E, gm, gp) == kFixZeros)
+    return fix_line_exp(kFixZeros);
   double out[N];
-  ref_line_fp64<P, EO>(&a, AX, r, line, S, gm, gp, Es, ES, out);
+  ref_line_nodes<P, EO>(&a, curved ? T : nullptr, AX, r, line, S, gm, gp, Es, ES, out);
   for (int m = 0; m < N; m++) line[m * S] = out[m];
   return kFixDouble;
 }
@@ -418,7 +515,8 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
   constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NFT = 6 * N2, NS = Sh::NS, EW = Sh::EW,
                 TAB = Rs::TAB, ROWS = Rs::ROWS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int sMix[FixShape<P>::EPB];  // elements whose lines go in FP64
+  // elements whose Escale the coefficients do not take (1), rows out of range (2)
+  __shared__ int sMix[FixShape<P>::EPB];
   const int epb = blockDim.x / N2;
   const long long eb = (long long)blockIdx.x * epb;
   const long long left = (long long)a.Ne - eb;
@@ -442,6 +540,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
   // 0: the z line's x and y fluxes, the element's coefficients, the face fluxes
   double g[6];
   int xe[3] = {0, 0, 0};
+  bool mix = false;
   if (on) {
     // the gathers wait for these: first
     const bool slots = !EO && MODE != kRkTend && *a.slots != 0;
@@ -456,7 +555,6 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
       prefetch_l2(a.w + ge + t);
       if constexpr (MODE == kRkGeneral) prefetch_l2(a.q0 + ge + t);
     }
-    bool mix = false;
     double es[3];
     if (MODE == kRkTend || a.esu == nullptr) {
 #pragma unroll
@@ -482,11 +580,13 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
     }
     // a row's exponent with Escale's: with a line's, whose results have to lie in
     // the normal range, at most the 900 of the box solver
+    bool bad = false;
     for (int t = r; t < 3 * ROWS; t += N2) {
-      const int x = a.row[t] + (t < ROWS ? xe[0] : t < 2 * ROWS ? xe[1] : xe[2]);
+      const int k = a.row[t], x = k + (t < ROWS ? xe[0] : t < 2 * ROWS ? xe[1] : xe[2]);
       mix |= x < -200 || x > 200;
+      bad |= k == kBadRow;
     }
-    if (mix) sMix[le] = 1;
+    if (mix) atomicOr(&sMix[le], bad ? 3 : 1);
 #pragma unroll
     for (int m = 0; m < N; m++) {
       const double qv = q[ge + r + m * N2];
@@ -528,15 +628,20 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
       }
     }
   }
-  __syncthreads();
-  const bool ok = on && sMix[le] == 0;
+  if (__syncthreads_or(mix)) {
+    if (on && sMix[le] == 1)
+      for (int t = r; t < 3 * TAB; t += N2) sT[t] = fix_coef(-fix_unit(a.tab[t]));
+    __syncthreads();
+  }
+  const int cls = on ? sMix[le] : 0;
+  const bool ok = cls == 0, curved = cls == 1;
   if (on) {
     // lines along i (r = j + N k), faces -x (3) and +x (1); along j (r = i + N k),
     // faces -y (0) and +y (2)
-    sEx[r] = ref_line_shared<P, EO, 0, 1, 1>(a, sT, xe[0], ok, r, sX + NS * r, g[3], g[1],
+    sEx[r] = ref_line_shared<P, EO, 0, 1, 1>(a, sT, xe[0], ok, curved, r, sX + NS * r, g[3], g[1],
                                              Es + ge + N * r);
-    sEy[r] = ref_line_shared<P, EO, 1, NS, N>(a, sT + TAB, xe[1], ok, r, sY + i + NS * N * j, g[0],
-                                              g[2], Es + NpNe + ge + i + j * N2);
+    sEy[r] = ref_line_shared<P, EO, 1, NS, N>(a, sT + TAB, xe[1], ok, curved, r, sY + i + NS * N * j,
+                                              g[0], g[2], Es + NpNe + ge + i + j * N2);
   }
   // lines along k (r = i + N j), faces -z (4) and +z (5); the node's result
   double F[N];
@@ -560,10 +665,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
     const int64_t* iY = reinterpret_cast<const int64_t*>(sY) + zat;
     // a line in FP64 has doubles whatever its row (a bad row's exponent is large)
     auto add = [](int line, int row) { return line == kFixDouble ? kFixDouble : line + row; };
-    auto emit = [&](int m, int64_t z) {
-      const double t = fix_node(iX[m * NS * N], add(sEx[j + N * m], rx), iY[m * NS * N],
-                                add(sEy[i + N * m], ry), z,
-                                add(Bz, a.row[2 * ROWS + Rs::row_of(m)] - 61));
+    auto finish = [&](int m, double t) {
       const long long n = ge + r + m * N2;
       if constexpr (MODE == kRkTend)
         a.out[n] = t;
@@ -577,6 +679,11 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
         a.out[n] = EO ? fma(ra, a.q0[n], fma(rb, q[n], (rb * dt) * t))
                       : fma(ra, a.q0[n], rb * fma(dt, t, q[n]));
     };
+    auto emit = [&](int m, int64_t z) {
+      finish(m, fix_node(iX[m * NS * N], add(sEx[j + N * m], rx), iY[m * NS * N],
+                         add(sEy[i + N * m], ry), z,
+                         add(Bz, a.row[2 * ROWS + Rs::row_of(m)] - 61)));
+    };
     if (zok) {
       const int32_t Ef = E + (xe[2] << 20);
       fix_line<P, EO>(sT + 2 * TAB, EO ? nullptr : a.lift + 2 * NP + r, F, E,
@@ -585,9 +692,16 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
       double in[N], out[N];  // in: F itself stays in registers
 #pragma unroll
       for (int m = 0; m < N; m++) in[m] = F[m];
-      ref_line_fp64<P, EO>(&a, 2, r, in, 1, g[4], g[5], Es + 2 * NpNe + ge + r, N2, out);
+      ref_line_nodes<P, EO>(&a, curved ? sT + 2 * TAB : nullptr, 2, r, in, 1, g[4], g[5],
+                            Es + 2 * NpNe + ge + r, N2, out);
+      if (curved) {  // all lines are doubles
 #pragma unroll 1
-      for (int m = 0; m < N; m++) emit(m, __double_as_longlong(out[m]));
+        for (int m = 0; m < N; m++)
+          finish(m, (sX[zat + m * NS * N] + sY[zat + m * NS * N]) + out[m]);
+      } else {
+#pragma unroll 1
+        for (int m = 0; m < N; m++) emit(m, __double_as_longlong(out[m]));
+      }
     }
   }
 }

@@ -105,3 +105,44 @@ def test_scales_that_lie_apart_only_together(opt, p, dims):
     assert 0.0 < np.abs(want).max() < 2.0 ** -995
     assert np.count_nonzero(np.abs(want) < 2.0 ** -1022) > 0
     _agree(np.ldexp(got, 1000), np.ldexp(want, 1000))
+
+
+@both
+@pytest.mark.parametrize("p,dims", [(1, (9, 8, 7)), (2, (6, 7, 5)), (3, (15, 14, 13)),
+                                    (7, (8, 7, 8)), (8, (7, 7, 6)), (13, (3, 5, 4)),
+                                    (15, (3, 4, 3))])
+@pytest.mark.parametrize("kind", ["mild", "wide", "edges", "nonfinite"])
+def test_escale_per_node(opt, p, dims, kind):
+    """Escale that varies over an element's nodes: mildly, over 60 powers of two,
+    with zeros, negative values and exponents past the folded ones, and with an
+    infinity and a NaN; beside elements of one Escale and elements of zeros.  A
+    result's error is held against its own terms where they differ in size: the
+    sums' bound on the element times its Escale, 1e-12 of it."""
+    c = Case(*dims, p)
+    m = copy.copy(c.mesh)
+    r = np.random.RandomState(p)
+    es = m.Escale.reshape(3, m.Ne, m.Np).copy()
+    curved = np.arange(m.Ne) % 3 == 1
+    f = 0.5 + r.rand(3, m.Ne, m.Np)
+    if kind == "wide":
+        f = np.ldexp(f, r.randint(-30, 31, f.shape))
+    if kind == "edges":
+        f[:, :, 0], f[:, :, 1], f[:, :, 2], f[:, :, 3] = 0.0, -1.0, 2.0 ** 160, 2.0 ** -160
+    if kind == "nonfinite":
+        f[1, 1, 0], f[2, 4, 5] = np.inf, np.nan
+    es[:, curved] *= f[:, curved]
+    m.Escale = es.reshape(-1)
+    q = c.q.copy()
+    q[: c.nown].reshape(m.Ne, m.Np)[np.arange(m.Ne) % 5 == 0] = 0.0
+    m.update_halo(q)
+    with np.errstate(all="ignore"):
+        got, want = _cal_tend(c, m, q, opt)
+        fine = np.isfinite(want)
+        assert np.array_equal(np.isfinite(got), fine)
+        N = p + 1
+        rows = np.abs(c.D.reshape(N, N)).sum(axis=0).max() + 2 * np.abs(c.Lift).max()
+        vel = max(np.abs(a).max() for a in (c.u, c.v, c.w))
+        size = rows * vel * np.abs(c.q).max() * (np.abs(es).sum(axis=0) + 3 * m.Fscale.max())
+    assert np.all(np.abs(got - want)[fine] <= 1e-12 * size.reshape(-1)[fine])
+    if kind in ("mild", "wide"):
+        _agree(*_loop(c, m, q, 0.25 * c.dt / f.max(), 1, opt))
