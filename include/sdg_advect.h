@@ -203,7 +203,17 @@ int sdg_mesh_setup_dev(int NeX, int NeY, int NeZ, int p, double Lx, double Ly,
  * consecutive elements (nelem = 1 is the reference call made per element from
  * mod_advect3d_eq.f90:185-188).  Each array holds nelem blocks of Nq^3
  * values.  An output of the device form may be any of its inputs, at the same
- * offset.  Host pointers; uses the type set by sdg_dg_optr_kernel_setup. */
+ * offset.  Host pointers; uses the type set by sdg_dg_optr_kernel_setup.
+ *
+ * How the contractions (divlike, gradlike, matvec, var5) sum: calls of fewer than
+ * 150,000 nodes at p <= 10, and any whose matrix has an entry off its diagonal
+ * below 2^-10 of its row's magnitudes (filters, identities, triangular matrices),
+ * and divlike at p = 1 in FP64 in the order of the type.  Others (the derivative matrices of every
+ * order) in 60-bit fixed point, which has no order: a result is off by at most
+ * (1.5 Nq + 4) 2^-59 times its row's magnitudes times its line's largest value,
+ * and half a unit of itself; the row of a value eight times all others of its
+ * line, where the diagonal holds zeros, by what FP64 gives.  -f then gives the
+ * negative to that bound, not to the bit. */
 int sdg_tensorprod_divlike_dirXYZ(double* vec_out_x, double* vec_out_y,
                                   double* vec_out_z, const double* Mat,
                                   const double* Mat_tr, const double* vec_in_x,
@@ -219,7 +229,8 @@ int sdg_tensorprod_divlike_dirXYZ_dev(double* vec_out_x, double* vec_out_y,
 
 /* element_operation_kernel_matvec_gradlike_dirXYZ_P* (opt1 erb:166-219) over
  * nelem elements: the x, y and z derivatives of ONE field, vec_out_x =
- * Mat along i, vec_out_y / vec_out_z = Mat_tr along j / k, running sums.
+ * Mat along i, vec_out_y / vec_out_z = Mat_tr along j / k, summed as divlike's
+ * GENERAL type says.
  * The template's z direction starts with vec_in(i,1,k)*Mat_tr(1,j)
  * (erb:209), a typo; this computes the consistent sum_l vec_in(i,j,l) *
  * Mat_tr(l,k). */
@@ -236,7 +247,8 @@ int sdg_tensorprod_gradlike_dirXYZ_dev(double* vec_out_x, double* vec_out_y,
 /* element_operation_kernel_matvec_dirX_P* / dirY_P* / dirZ_P* (opt1
  * erb:51-129) over nelem elements, dir = 1, 2, 3: one running-sum
  * contraction along i with Mat_x, or along j / k with the transposed
- * Mat_y_tr / Mat_z_tr, exactly as the templates take them. */
+ * Mat_y_tr / Mat_z_tr, exactly as the templates take them;
+ * summed as divlike's GENERAL type says. */
 int sdg_element_matvec_dir(int dir, double* vec_out, const double* Mat,
                            const double* vec_in, int Nq, int nelem);
 int sdg_element_matvec_dir_dev(int dir, double* vec_out, const double* Mat,
@@ -245,7 +257,7 @@ int sdg_element_matvec_dir_dev(int dir, double* vec_out, const double* Mat,
 
 /* element_operation_kernel_matvec_divlike_dirXYZ_var5_P* (opt1
  * erb:347-465): the divlike contraction of 5 variables per element, in the
- * OPT1 summation order (three partial sums for p > 7).  Each array holds
+ * OPT1 order (three partial sums for p > 7) where divlike sums in FP64.  Each array holds
  * nelem blocks of (Nq,Nq,Nq,5) values, outputs in the same layout.  The
  * template's y output index, j + (kv-1)*5*Nq (erb:400), runs past
  * vec_out_y for kv > 1; this writes vec_out_y(i,j,k,v) like x and z. */

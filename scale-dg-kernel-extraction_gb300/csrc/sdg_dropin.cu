@@ -81,6 +81,7 @@ static int divlike(DivArgs a, int p, int opt, cudaStream_t st) {
   for (int o = 0; o < 3; o++)
     for (int i = 0; i < 3; i++)
       if (overlap(out[o], n, in[i], n) && !(o == i && out[o] == in[i])) a.staged = true;
+  a.split = p > 7 && opt == SDG_OPT_OPT1;
   return dropin(p, 1, opt, &a, st);
 }
 
@@ -456,7 +457,7 @@ int sdg_tensorprod_divlike_dirXYZ(double* ox, double* oy, double* oz,
   DivArgs a{ar.at<double>(o[0]), ar.at<double>(o[1]), ar.at<double>(o[2]),
             ar.at<double>(o[3]), ar.at<double>(o[4]), ar.at<double>(o[5]),
             ar.at<double>(o[6]), ar.at<double>(o[7]), nelem};
-  SDG_TRY(dropin(Nq - 1, 1, opt, &a, nullptr));
+  SDG_TRY(divlike(a, Nq - 1, opt, nullptr));
   for (double* o : {ox, oy, oz}) touch_pages(o, 8 * n);
   SDG_CUDA_TRY(cudaMemcpy(ox, a.ox, 8 * n, cudaMemcpyDeviceToHost));
   SDG_CUDA_TRY(cudaMemcpy(oy, a.oy, 8 * n, cudaMemcpyDeviceToHost));
@@ -517,7 +518,7 @@ int host_contract(int what, double* ox, double* oy, double* oz, const double* Ma
             ar.at<double>(o[3]), ar.at<double>(o[4]), ar.at<double>(o[5]),
             nin > 1 ? ar.at<double>(o[6]) : nullptr, nin > 2 ? ar.at<double>(o[7]) : nullptr,
             nblocks};
-  SDG_TRY(dropin(Nq - 1, what, opt, &a, nullptr));
+  SDG_TRY(what == 1 ? divlike(a, Nq - 1, opt, nullptr) : dropin(Nq - 1, what, opt, &a, nullptr));
   for (double* o : {ox, oy, oz}) touch_pages(o, 8 * n);
   SDG_CUDA_TRY(cudaMemcpy(ox, a.ox, 8 * n, cudaMemcpyDeviceToHost));
   SDG_CUDA_TRY(cudaMemcpy(oy, a.oy, 8 * n, cudaMemcpyDeviceToHost));
