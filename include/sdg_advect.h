@@ -59,10 +59,22 @@ extern "C" {
 
 /* Arithmetic of a solver (the reference is FP64 throughout). */
 #define SDG_PREC_FP64 0   /* FP64 state, fluxes and RK update; the line sums of
-                             the fused stage as exact integer sums of 60-bit
-                             fixed-point products, as near to the exact sum as
-                             FP64 arithmetic, which forms the lines that hold
-                             infinities, NaN or extreme magnitudes */
+                             the fused stage in 60-bit fixed point on a scale
+                             of the line.  A sum is off by at most (1.5 Nq + 4)
+                             2^-59 times its row's magnitudes times the line's
+                             largest value: measured over a tendency no more
+                             than FP64 sums are, but relative to the line, not
+                             to each node's own terms.  FP64 forms the lines
+                             with infinities, NaN, extreme magnitudes or a
+                             value more than 128 times all others that the
+                             derivative does not see; any operators with
+                             entries below 2^-10 of their row (zeros on D's
+                             diagonal and in the lift excepted).  Sums of zeros
+                             are zero; -q gives the negative tendency to the
+                             bound, not to the bit.  The same holds for
+                             cal_tend (GENERAL and OPT1 from 160,000 DOF or
+                             p = 12; below that FP64 sums in their order) and
+                             the loop on the reference's arrays. */
 #define SDG_PREC_FP32 1   /* FP32 flux/derivative/lift, FP64 RK state */
 #define SDG_PREC_FP64_EMU 2 /* FP64 arithmetic emulated on the integer and FP32 pipes:
                                since SDG_PREC_FP64 forms its line sums there too,
@@ -211,7 +223,7 @@ int sdg_mesh_setup_dev(int NeX, int NeY, int NeZ, int p, double Lx, double Ly,
  * and divlike at p = 1 in FP64 in the order of the type.  Others (the derivative matrices of every
  * order) in 60-bit fixed point, which has no order: a result is off by at most
  * (1.5 Nq + 4) 2^-59 times its row's magnitudes times its line's largest value,
- * and half a unit of itself; the row of a value eight times all others of its
+ * and half a unit of itself; the row of a value 128 times all others of its
  * line, where the diagonal holds zeros, by what FP64 gives.  -f then gives the
  * negative to that bound, not to the bit. */
 int sdg_tensorprod_divlike_dirXYZ(double* vec_out_x, double* vec_out_y,

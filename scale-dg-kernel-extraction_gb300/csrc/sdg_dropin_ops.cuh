@@ -13,8 +13,8 @@
 //     filter, an identity, a triangular matrix: the derivative's smallest is 2^-9 at
 //     p = 15) keeps FP64 sums, in the order asked for;
 //   * where the diagonal has such entries (a derivative's interior rows), the row of
-//     a line's largest value is summed in FP64 when all other values are less than
-//     an eighth of it;
+//     a line's largest value is summed in FP64 when no other value is within 2^6
+//     of it (kFixAlone);
 //   * lines with infinities, NaN or magnitudes near the ends of the exponent range
 //     are summed in FP64.
 //
@@ -71,7 +71,6 @@ __device__ __noinline__ void ops_line_fp64(const double* __restrict__ M, int si,
 // How a matrix's rows are summed: kOpsFixed in fixed point, kOpsDiag the same with
 // small entries on the diagonal, kOpsDouble in FP64.
 constexpr int kOpsFixed = 0, kOpsDiag = 1, kOpsDouble = 2;
-constexpr int kOpsSpike = 3 << 20;  // a largest value eight times all others
 
 // The kind row i of a matrix allows: v(l) its entries, sum their magnitudes.
 template <int N, typename V>
@@ -117,7 +116,7 @@ __device__ __forceinline__ void ops_line(const fixlimb* T, const int* row, int k
     E2 = max(E2, min(E, x));
     E = max(E, x);
   }
-  const bool spike = kind == kOpsDiag && E - E2 > kOpsSpike;
+  const bool spike = kind == kOpsDiag && E - E2 > kFixAlone;
   E = fix_line_scale<N>(F, E, 0.0, 0.0);
   if (!fix_in_range(E)) {
     ops_line_fp64<P>(M, si, sl, in, S, out, SO);

@@ -50,7 +50,8 @@ struct RefArgs {
   const double* Dt;
   const double* Lift;
   // tables (ref_tables_kernel): rows of coefficients times 2^-row, the rows'
-  // exponents (kBadRow: out of range), the nodes' lift limbs (not EO)
+  // exponents (kBadRow: out of range) and, behind them, which rows' lift has zeros
+  // and the nodes' lift limbs (both not EO)
   const double* tab;
   const int* row;
   const int4* lift;
@@ -87,7 +88,8 @@ struct RefShape {
   static constexpr int ROWS = EO ? EoShape<P>::HR : N;
   // bytes of the tables: lift limbs, coefficients, rows (16-byte aligned base)
   static constexpr size_t LIFT = EO ? 0 : sizeof(int4) * 3 * N * N * N;
-  static constexpr size_t LEAST = LIFT + sizeof(double) * 3 * TAB + sizeof(int) * 3 * ROWS;
+  static constexpr size_t LEAST =
+      LIFT + sizeof(double) * 3 * TAB + sizeof(int) * (EO ? 3 : 6) * ROWS;
   // with the coefficients for the first node's Escale
   static constexpr size_t SHARED = (LEAST + 7) / 8 * 8;
   static constexpr size_t BYTES = SHARED + sizeof(fixlimb) * 3 * TAB;
@@ -234,7 +236,8 @@ __global__ void __launch_bounds__(256) ref_tables_eo_kernel(const double* __rest
 }
 
 // Operators as given: block (d, i) forms row i of direction d -- its scale over
-// the derivative entries and all its nodes' lift entries, the scaled
+// the derivative entries and all its nodes' lift entries (kBadRow where an entry is
+// below 2^-10 of those: the reference's smallest is 2^-9.6 at p = 15), the scaled
 // derivative entries (D1D for x, D1D_tr for y and z), the nodes' lift limbs
 // (-, + face) and the coefficients for the Escale of the mesh's first node.
 template <int P>
@@ -261,8 +264,16 @@ __global__ void __launch_bounds__(256) ref_tables_kernel(const double* __restric
   auto Dv = [&](int l) { return d == 0 ? D[i + l * N] : Dt[l + i * N]; };
   double sum = __longlong_as_double((long long)smax);
   for (int l = 0; l < N; l++) sum += fabs(Dv(l));
-  const int k = fix_row_exp(sum);
-  if (r == 0) row[blockIdx.x] = k;
+  // entries too small for the row's scale: in FP64 (lift entries may be zero)
+  const double least = sum * (1.0 / 1024.0);
+  bool small = r < N && r != i && fabs(Dv(r)) < least;
+  small |= r < N2 && ((m != 0.0 && fabs(m) < least) || (p != 0.0 && fabs(p) < least));
+  const int k = __syncthreads_or(small) ? kBadRow : fix_row_exp(sum);
+  const int thin = __syncthreads_or(r < N2 && (m == 0.0 || p == 0.0));
+  if (r == 0) {
+    row[blockIdx.x] = k;
+    row[3 * N + blockIdx.x] = thin;
+  }
   const double scale = k == kBadRow ? 1.0 : ref_pow2(-k);
   if (r < N) {
     const double c = Dv(r) * scale;
@@ -403,13 +414,15 @@ __device__ __noinline__ void ref_line_nodes(const RefArgs* a, const fixlimb* T, 
   constexpr int N = P + 1;
   using Rs = RefShape<P, EO>;
   double f[N];
-  int32_t E = 0, Eg = max(fix_value_exp(gm), fix_value_exp(gp));
+  FixScan<P, EO> scan;
 #pragma unroll
   for (int l = 0; l < N; l++) {
     f[l] = F[l * fs];
-    E = max(E, fix_value_exp(f[l]));
+    scan.add(l, fix_value_exp(f[l]));
   }
-  E = fix_line_scale<N>(f, E, 0.0, 0.0);
+  // (the faces have a scale of their own)
+  const int32_t E = fix_line_scale<N>(f, scan.scale(0, false), 0.0, 0.0);
+  int32_t Eg = max(fix_value_exp(gm), fix_value_exp(gp));
   if (gm == 0.0 && gp == 0.0) Eg = kFixZeros;
   if (T == nullptr || !fix_in_range(E) || !fix_in_range(Eg)) {
     ref_line_fp64<P, EO>(a, ax, r, F, fs, gm, gp, Es, es, out);
@@ -474,16 +487,17 @@ __host__ __device__ constexpr size_t ref_smem(int epb) {
 // (curved) or not usable (neither).
 template <int P, bool EO, int AX, int S, int ES>
 __device__ __forceinline__ int ref_line_shared(const RefArgs& a, const fixlimb* T, int xe, bool ok,
-                                               bool curved, int r, double* line, double gm, double gp,
+                                               bool curved, bool thin, int r, double* line, double gm, double gp,
                                                const double* Es) {
   constexpr int N = P + 1;
   double F[N];
-  int32_t E = max(0, ref_face_exp(gm, gp, xe));
+  FixScan<P, EO> scan;
 #pragma unroll
   for (int l = 0; l < N; l++) {
     F[l] = line[l * S];
-    E = max(E, fix_value_exp(F[l]));
+    scan.add(l, fix_value_exp(F[l]));
   }
+  const int32_t E = scan.scale(ref_face_exp(gm, gp, xe), thin);
   if (ok && fix_in_range(E)) {
     int64_t* out = reinterpret_cast<int64_t*>(line);
     const int32_t Ef = E + (xe << 20);
@@ -515,7 +529,8 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
   constexpr int N = Sh::N, N2 = Sh::N2, NP = N * N2, NFT = 6 * N2, NS = Sh::NS, EW = Sh::EW,
                 TAB = Rs::TAB, ROWS = Rs::ROWS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  // elements whose Escale the coefficients do not take (1), rows out of range (2)
+  // elements whose Escale the coefficients do not take (1), rows out of range (2),
+  // a lift with zeros (4)
   __shared__ int sMix[FixShape<P>::EPB];
   const int epb = blockDim.x / N2;
   const long long eb = (long long)blockIdx.x * epb;
@@ -585,6 +600,7 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
       const int k = a.row[t], x = k + (t < ROWS ? xe[0] : t < 2 * ROWS ? xe[1] : xe[2]);
       mix |= x < -200 || x > 200;
       bad |= k == kBadRow;
+      if (!EO && a.row[3 * ROWS + t] != 0) atomicOr(&sMix[le], 4);
     }
     if (mix) atomicOr(&sMix[le], bad ? 3 : 1);
 #pragma unroll
@@ -629,31 +645,31 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, ref_min_blocks<P, EO>())
     }
   }
   if (__syncthreads_or(mix)) {
-    if (on && sMix[le] == 1)
+    if (on && (sMix[le] & 3) == 1)
       for (int t = r; t < 3 * TAB; t += N2) sT[t] = fix_coef(-fix_unit(a.tab[t]));
     __syncthreads();
   }
   const int cls = on ? sMix[le] : 0;
-  const bool ok = cls == 0, curved = cls == 1;
+  const bool ok = (cls & 3) == 0, curved = (cls & 3) == 1, thin = !EO && cls >= 4;
   if (on) {
     // lines along i (r = j + N k), faces -x (3) and +x (1); along j (r = i + N k),
     // faces -y (0) and +y (2)
-    sEx[r] = ref_line_shared<P, EO, 0, 1, 1>(a, sT, xe[0], ok, curved, r, sX + NS * r, g[3], g[1],
+    sEx[r] = ref_line_shared<P, EO, 0, 1, 1>(a, sT, xe[0], ok, curved, thin, r, sX + NS * r, g[3], g[1],
                                              Es + ge + N * r);
-    sEy[r] = ref_line_shared<P, EO, 1, NS, N>(a, sT + TAB, xe[1], ok, curved, r, sY + i + NS * N * j,
+    sEy[r] = ref_line_shared<P, EO, 1, NS, N>(a, sT + TAB, xe[1], ok, curved, thin, r, sY + i + NS * N * j,
                                               g[0], g[2], Es + NpNe + ge + i + j * N2);
   }
   // lines along k (r = i + N j), faces -z (4) and +z (5); the node's result
   double F[N];
   int32_t E = 0;
   if (on) {
-    E = max(0, ref_face_exp(g[4], g[5], xe[2]));
+    FixScan<P, EO> scan;
 #pragma unroll
     for (int m = 0; m < N; m++) {
       F[m] = fix_product(q[ge + r + m * N2], a.w[ge + r + m * N2]);
-      E = max(E, fix_value_exp(F[m]));
+      scan.add(m, fix_value_exp(F[m]));
     }
-    E = fix_line_scale<N>(F, E, g[4], g[5]);
+    E = fix_line_scale<N>(F, scan.scale(ref_face_exp(g[4], g[5], xe[2]), thin), g[4], g[5]);
   }
   __syncthreads();
   if (on) {

@@ -148,6 +148,12 @@ SDG_HD int32_t fix_face_exp(double g) { return (int32_t)(fix_high(g) & kFixExp) 
 SDG_HD bool fix_in_range(int32_t E) {
   return (uint32_t)E - (322u << 20) < (1400u << 20);
 }
+// A line's values within 2^6 of its largest are held exactly (59 bits of that for
+// 53).  Where none but the largest lies within, a sum that does not see it (a zero
+// on the diagonal) has fewer bits of the others than FP64.
+constexpr int32_t kFixAlone = 6 << 20;
+// The scale of a line that is to be formed in FP64: above the range.
+constexpr int32_t kFixRefused = 2047 << 20;
 // The scale of a line of zeros: the least of the range, marked in a bit that no
 // other has, so that the line's exponent lies below all others and a node's sum
 // is formed on the scale of its other lines.

@@ -339,7 +339,7 @@ void fix_tables_general(int Nq, const Box& box, const double* D1D, const double*
                         FixTables& t, std::vector<int32_t>& lift) {
   const int N = Nq, N2 = N * N, NP = N * N2;
   const int fminus[3] = {3, 0, 4}, fplus[3] = {1, 2, 5};
-  t.ok = 0;
+  t.ok = t.thin = 0;
   t.coef.assign(2 * 3 * (size_t)N2, 0);
   t.row.assign(3 * (size_t)N, 0);
   lift.assign(4 * 3 * (size_t)NP, 0);
@@ -360,6 +360,18 @@ void fix_tables_general(int Nq, const Box& box, const double* D1D, const double*
       for (int l = 0; l < N; l++) sum += std::fabs(D1D[i + l * N] * Es);
       int k = 0;
       if (!fix_row_exp(sum + most * Fs, &k)) return;
+      // entries too small for the row's scale (the reference's smallest is 2^-9.6 of
+      // it at p = 15; a zero on the diagonal and zeros of the lift are no matter)
+      const double least = (sum + most * Fs) / 1024.0;
+      auto small = [&](double x) { return std::fabs(x) < least; };
+      for (int l = 0; l < N; l++)
+        if (l != i && small(D1D[i + l * N] * Es)) return;
+      for (int r = 0; r < N2; r++)
+        for (double x : {Lm[node(r)], Lp[node(r)]})
+          if (x == 0.0)
+            t.thin = 1;
+          else if (small(x * Fs))
+            return;
       t.row[(size_t)d * N + i] = k - 61;
       for (int l = 0; l < N; l++)
         fix_put(&t.coef[2 * ((size_t)d * N2 + i * N + l)], D1D[i + l * N], Es, k);

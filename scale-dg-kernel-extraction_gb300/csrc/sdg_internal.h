@@ -84,6 +84,7 @@ struct FixTables {
   std::vector<int32_t> coef;
   std::vector<int> row;
   int ok = 0;
+  int thin = 0;  // operators as given: the lift has zeros
 };
 // Fills t from the unscaled tables of eo_tables.
 void fix_tables(int Nq, const Box& box, const std::vector<double>& eo, FixTables& t);

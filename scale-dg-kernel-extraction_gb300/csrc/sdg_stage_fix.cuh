@@ -75,6 +75,7 @@ struct FixStageArgs {
   fixlimb tab[3 * TAB];  // per direction: EoShape's table, or D(i,l) at i N + l
   int row[3 * ROWS];     // exponent of a row's scale, less 61
   int ok;                // 0: coefficients out of range, every line in FP64
+  int thin;              // the lift has zeros
   static __host__ __device__ constexpr int row_of(int m) {
     return EO ? (m < P - m ? m : P - m) : m;
   }
@@ -196,6 +197,35 @@ __device__ __forceinline__ void fix_line(const fixlimb* T, const int4* __restric
   }
 }
 
+// The largest exponent field of a line's values, and whether a node of the line
+// would lose what FP64 has: one whose own value is alone (kFixAlone), where
+// the derivative has a zero on its diagonal (every row between the ends, of
+// operators as given; the middle one of the even-odd pairs, whose other rows form
+// sums and differences of the two values in either arithmetic), or, where the lift
+// has zeros (thin), one that does not see a face flux that is.  Such a line's scale
+// lies out of range: it is formed in FP64.  (A face flux counted so for every lift
+// takes a tracer's fronts to FP64: OPT1, p = 7 147 us a stage against 95; a value
+// eight times all others for alone 110.)
+template <int P, bool EO>
+struct FixScan {
+  static constexpr int N = P + 1, MID = EO && (N & 1) ? N / 2 : -1;
+  static constexpr bool SECOND = !EO && P > 1;
+  int32_t e = 0, next = 0;  // next: the second largest (SECOND), all but MID's
+  __device__ __forceinline__ void add(int l, int32_t x) {
+    if constexpr (SECOND) next = max(next, min(e, x));
+    if constexpr (MID >= 0) {
+      if (l != MID) next = max(next, x);
+    }
+    e = max(e, x);
+  }
+  // face: the larger exponent field of the line's faces (negative: none)
+  __device__ __forceinline__ int32_t scale(int32_t face, bool thin) const {
+    const int32_t E = max(e, face);
+    const int32_t rest = thin ? next : max(next, face);
+    return (SECOND || MID >= 0) && E - rest > kFixAlone ? kFixRefused : E;
+  }
+};
+
 // The scale of a line whose largest exponent field is E: a line of zeros (a
 // tracer that fills part of the box, a velocity without a component) stays in
 // fixed point; in FP64 its nodes' sums cost more than all others (p = 7 113 us a
@@ -221,12 +251,13 @@ __device__ __forceinline__ int fix_line_shared(const FixStageArgs<P, EO>& a, int
                                                double gm, double gp) {
   constexpr int N = P + 1;
   double F[N];
-  int32_t E = max(0, max(fix_face_exp(gm), fix_face_exp(gp)));
+  FixScan<P, EO> scan;
 #pragma unroll
   for (int l = 0; l < N; l++) {
     F[l] = line[l * S];
-    E = max(E, fix_value_exp(F[l]));
+    scan.add(l, fix_value_exp(F[l]));
   }
+  const int32_t E = scan.scale(max(fix_face_exp(gm), fix_face_exp(gp)), !EO && a.thin);
   if (a.ok && fix_in_range(E)) {
     int64_t* out = reinterpret_cast<int64_t*>(line);
     fix_line<P, EO>(a.tab + AX * a.TAB, a.lift(AX, r), F, E, fix_align_face(gm, E),
@@ -359,12 +390,13 @@ __global__ void __launch_bounds__(FixShape<P>::THREADS, fix_min_blocks<P>())
   int32_t E = 0;
   if (on) {
     const double* __restrict__ w = static_cast<const double*>(a.s.w);
-    E = max(0, max(fix_face_exp(g[4]), fix_face_exp(g[5])));
+    FixScan<P, EO> scan;
 #pragma unroll
     for (int m = 0; m < N; m++) {
       F[m] = fix_product(q[ge + r + m * N2], w[ge + r + m * N2]);
-      E = max(E, fix_value_exp(F[m]));
+      scan.add(m, fix_value_exp(F[m]));
     }
+    E = scan.scale(max(fix_face_exp(g[4]), fix_face_exp(g[5])), !EO && a.thin);
     E = fix_line_scale<N>(F, E, g[4], g[5]);
   }
   __syncthreads();
@@ -438,6 +470,7 @@ void fix_fill(FixStageArgs<P, EO>& a, const StageArgs& s) {
     a.tab[t] = fixlimb{s.fix->coef[2 * t], s.fix->coef[2 * t + 1]};
   for (int t = 0; t < 3 * a.ROWS; t++) a.row[t] = s.fix->row[t];
   a.ok = s.fix->ok;
+  a.thin = s.fix->thin;
 }
 
 template <int P, bool EO>

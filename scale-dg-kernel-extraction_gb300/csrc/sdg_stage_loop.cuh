@@ -89,21 +89,21 @@ __device__ __forceinline__ int fix_loop_line(const FixStageArgs<P, EO>& a, const
   // the state was written by other blocks during this launch: not through L1
   const double qPm = __ldcg(q + nbr[0]), qPp = __ldcg(q + nbr[1]);
   double F[N], qm = 0.0, qp = 0.0;
-  int32_t E = 0;
+  FixScan<P, EO> scan;
 #pragma unroll
   for (int l = 0; l < N; l++) {
     const double v = __ldcg(q + at + l * S);
     if (l == 0) qm = v;
     if (l == N - 1) qp = v;
     F[l] = fix_product(v, u[at + l * S]);
-    E = max(E, fix_value_exp(F[l]));
+    scan.add(l, fix_value_exp(F[l]));
   }
   auto flux = [](double qP, double qM, double2 c) {
     return EO ? fma(qP, c.x, -(qM * c.y)) : fma(qP, c.x, (qP - qM) * c.y);
   };
   const double gm = flux(qPm, qm, fc[0]), gp = flux(qPp, qp, fc[1]);
-  E = max(E, max(fix_face_exp(gm), fix_face_exp(gp)));
-  E = fix_line_scale<N>(F, E, gm, gp);
+  const int32_t E = fix_line_scale<N>(
+      F, scan.scale(max(fix_face_exp(gm), fix_face_exp(gp)), !EO && a.thin), gm, gp);
   if (a.ok && fix_in_range(E)) {
     fix_line<P, EO>(a.tab + AX * a.TAB, a.lift(AX, r), F, E, fix_align_face(gm, E),
                     fix_align_face(gp, E), [&](int m, int64_t v) { out[m * SO] = v; });
