@@ -204,7 +204,8 @@ def load_traffic(key: str, field: str = "bytes_per_launch"):
     with open(path) as f:
         d = json.load(f)
     v = d.get(key)
-    return float(v[field]) if isinstance(v, dict) and field in v else None
+    x = v.get(field) if isinstance(v, dict) else None
+    return x if x is None or isinstance(x, str) else float(x)
 
 
 def run_reference(args, ws, rank):
@@ -281,6 +282,11 @@ def time_solver(sdg, wl, p, ne, prec, steps, warmup, local, barrier, sample_cloc
     return s, ms / 1e3, clk
 
 
+def stage_form(precision):
+    """The form whose stage kernel a precision runs."""
+    return "fp64" if precision == "fp64emu" else precision
+
+
 def roofline(precision, p, ne, ndof, t, steps, peaks, opt="opt1"):
     """The stage kernel against its roofs.
 
@@ -295,11 +301,12 @@ def roofline(precision, p, ne, ndof, t, steps, peaks, opt="opt1"):
     Compute: the FP64 forms' line sums are integer multiply-adds; FP64 keeps
     the products, the face fluxes and the RK update, and its pipe is the busiest
     unit.  `compute.frac` is that pipe's busy
-    share from the kernel's ncu capture (sm__pipe_fp64_cycles_active);
+    share from the kernel's ncu capture (the record names the metric);
     `achieved_tflops` counts the reference's formulas (25 + 6 Nq + 126 / Nq
-    flops a DOF-update) against the DFMA peak measured live.  The FP32 and
-    emulated forms report those flops against the live FFMA peak, and the
-    emulated form its FP64 pipe's busy share apart (`fp64_pipe_busy`)."""
+    flops a DOF-update) against the DFMA peak measured live.  The FP32 form
+    reports those flops against the live FFMA peak.  The emulated form runs the
+    FP64 form's kernel and is reported as that (stage_form); called with
+    "fp64emu" this gives the record of the double-float kernel it used to run."""
     launches = 3 * steps
     avg_launch = t / launches
     bpd = BYTES_PER_DOF_UPDATE[precision]
@@ -330,16 +337,17 @@ def roofline(precision, p, ne, ndof, t, steps, peaks, opt="opt1"):
         busy = load_traffic(tkey, "fp64_pipe_active")
         if busy is not None and precision == "fp64":
             comp["frac"] = busy
-            comp["frac_source"] = "sm__pipe_fp64_cycles_active, ncu capture of this kernel"
+            metric = load_traffic(tkey, "fp64_pipe_metric")
+            comp["frac_source"] = f"{metric}, ncu capture of this kernel"
         else:
             comp["frac"] = fl * per_gpu / 1e3 / peaks[pipe]
             comp["frac_source"] = "reference-formula flops / live peak"
             if busy is not None:
-                # the emulated form's FP64 work (face flux, RK combine) on
-                # the 1/64-rate pipe, beside its FP32 contraction
+                # that kernel's FP64 work (face flux, RK combine) on the 1/64-rate
+                # pipe, beside its FP32 contraction
                 comp["fp64_pipe_busy"] = busy
                 comp["fp64_pipe_busy_source"] = ("sm__pipe_fp64_cycles_active, ncu capture "
-                                                 "of this kernel")
+                                                 "of the double-float kernel")
         roof["compute"] = comp
         if precision == "fp64":
             # the FP64 pipe binds when it is busier than HBM
@@ -984,7 +992,7 @@ def run_ours(args, ws, rank, local):
     t = tmax(t)
     value = whole_job_rate(ws, ndof, args.steps, t)
     peaks = None if args.no_microbench else sdg.microbench_peaks()
-    roof = roofline(args.precision, p, ne, ndof, t, args.steps, peaks, args.opt)
+    roof = roofline(stage_form(args.precision), p, ne, ndof, t, args.steps, peaks, args.opt)
 
     # ---- end to end through the C ABI with pinned host buffers ----
     # every step uploads q, u, v, w from page-locked host memory and downloads
@@ -1028,7 +1036,8 @@ def run_ours(args, ws, rank, local):
                                 "in 60-bit fixed point (the FP64 form's stage)",
                  "value": ws * ndof * 3 * args.steps / te_ / 1e9, "unit": "GDOF-updates/s",
                  "ms_per_step": 1e3 * te_ / args.steps,
-                 "roofline": roofline("fp64emu", p, ne, ndof, te_, args.steps, peaks, args.opt)}
+                 "roofline": roofline(stage_form("fp64emu"), p, ne, ndof, te_, args.steps, peaks,
+                                      args.opt)}
         if rank == 0 and not args.no_cpu_baseline:
             se.upload(wl["q"], wl["u"], wl["v"], wl["w"])
             tend_emu = se.tendency()

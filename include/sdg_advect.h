@@ -147,8 +147,9 @@ int sdg_advect3d_eq_cal_tend(double* dqdt, const double* q, const double* u,
 /* The same on device pointers, asynchronous on `stream`, with the
  * optimisation type explicit.  dqdt may be one of the fields, in place.
  * `flux_scratch` is caller-owned device memory
- * of NfpTot*Ne doubles for the element-boundary flux (the reference's
- * automatic array ebnd_flux, mod_advect3d_eq.f90:66); `err_flag` is a
+ * of NfpTot*Ne doubles, as many as the element-boundary flux has (the
+ * reference's automatic array ebnd_flux, mod_advect3d_eq.f90:66); it holds the
+ * fluxes or the operators' tables, and its contents on return are unspecified; `err_flag` is a
  * caller-owned device int that the kernels set to 1 when a VMap index is out
  * of range, and with opt = SDG_OPT_EVENODD to 2 when D1D is not
  * centro-antisymmetric, D1D_tr not its transpose or Lift_mat not separable

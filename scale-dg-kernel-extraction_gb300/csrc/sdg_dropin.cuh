@@ -3,17 +3,21 @@
 // Fscale), so any connectivity the caller builds is honoured.
 //
 //   step_ref_kernel  the whole tendency, and the stages of the time loop
-//                    (sdg_dropin_step.cuh);
+//                    (sdg_dropin_step.cuh); EVENODD always, GENERAL and OPT1
+//                    tendencies from 160,000 DOF or p = 12;
 //   flux_kernel      cal_elembnd_flux (mod_advect3d_eq.f90:89-142), one
 //                    thread per face node, VMap indices range-checked, and
 //   dqdt_kernel      cal_dqdt (mod_advect3d_eq.f90:146-201), EPB elements
-//                    per block staged in shared memory: a GENERAL or OPT1
-//                    tendency of so few elements (about Nq) that the flux
-//                    scratch does not hold step_ref_kernel's tables;
+//                    per block staged in shared memory: the GENERAL and OPT1
+//                    tendencies of smaller meshes (tend_dev has the
+//                    measurements) and of so few elements (about Nq) that the
+//                    flux scratch does not hold step_ref_kernel's tables, and
+//                    a tendency written over one of its fields;
 //   ops_kernel       tensorprod_divlike_dirXYZ (mod_dg_optr_kernel.f90:62-136),
 //                    gradlike and matvec over a batch of elements
 //                    (sdg_dropin_ops.cuh), and
-//   divlike_kernel, gradlike_kernel  the same in FP64 over few elements;
+//   divlike_kernel, gradlike_kernel  the same in FP64 over few elements, and
+//                    divlike with outputs over other directions' inputs;
 //   lift_kernel      tensorprod_Lift_hexahedral (mod_dg_optr_kernel.f90:139-190).
 #pragma once
 
