@@ -31,9 +31,9 @@
 // and its two face fluxes, and a row of coefficients has a power of two of its
 // own, so every line result keeps about 2^-61 of its own bound.  The three
 // results of a node are added as integers on the largest of their scales and
-// become one double.  A line with infinities, NaN, or magnitudes near the ends
-// of the exponent range is formed in FP64 by its thread, and its nodes add up
-// in FP64.
+// become one double.  A line with infinities, NaN, magnitudes near the ends of
+// the exponent range or a value alone in it (FixScan) is formed in FP64 by its
+// thread, and its nodes add up in FP64.
 //
 // Thread layout: thread r of an element's N^2 owns line r of each direction
 // and node r of each face, so a line's face fluxes never leave their thread.
